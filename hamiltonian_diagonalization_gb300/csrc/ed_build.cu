@@ -20,6 +20,7 @@
 #include <vector>
 
 #include "ed_hop.cuh"
+#include "ed_split.h"
 
 namespace edgb {
 
@@ -882,6 +883,7 @@ void ham_build_crs(const ed_basis& b, const ed_terms& t, int upper, ed_crs& a, c
     ED_REQUIRE(n < (int64_t)0x7fffffff, ED_ERR_RANGE, "sector dimension exceeds int32 column indices");
     a.n = n;
     a.upper = upper ? 1 : 0;
+    a.source = std::make_shared<const SplitSource>(split_source(b, t));
     a.rowptr.alloc(n + 1);
     if (n == 0) {
         ED_CUDA(cudaMemsetAsync(a.rowptr.p, 0, sizeof(int64_t), st));
@@ -1010,6 +1012,8 @@ void ham2_build_crs(const ed_basis& b, const ed_terms& t0, const ed_terms& t1, c
     ED_REQUIRE(n < (int64_t)0x7fffffff, ED_ERR_RANGE, "sector dimension exceeds int32 column indices");
     a.n = n;
     a.upper = upper ? 1 : 0;
+    a.source = std::make_shared<const SplitSource>(
+        SplitSource{2, b.N, b.norb0, b.norb1, b.sector_sum, t0.hop, t1.hop});
     a.rowptr.alloc(n + 1);
     if (n == 0) {
         ED_CUDA(cudaMemsetAsync(a.rowptr.p, 0, sizeof(int64_t), st));

@@ -8,6 +8,7 @@
 #include <vector>
 
 #include "ed_lanczos.h"
+#include "ed_split.h"
 
 namespace edgb {
 
@@ -431,9 +432,13 @@ ed_status ed_hv_matfree(const ed_basis* b, const ed_terms* t, const double* x_de
         ED_REQUIRE(x_dev != y_dev, ED_ERR_ARG, "x and y must be distinct");
         cudaStream_t st = (cudaStream_t)stream;
         basis_compact_tables(*b, st);
-        DevBuf<double> diag(b->dim);
-        ham_diagonal(*b, *t, diag.p, st);
-        hv_matfree(*b, *t, diag.p, x_dev, y_dev, st);
+        const std::shared_ptr<SplitPlan> plan = matfree_plan(*b, *t, nullptr, st);
+        DevBuf<double> diag;
+        if (!plan) {
+            diag.alloc(b->dim);
+            ham_diagonal(*b, *t, diag.p, st);
+        }
+        hv_matfree(*b, *t, plan.get(), diag.p, x_dev, y_dev, st);
         ED_CUDA(cudaStreamSynchronize(st));
     });
 }

@@ -18,6 +18,9 @@
 
 namespace edgb {
 
+struct SplitSource;   // ed_split.h
+struct SplitPlan;
+
 // Largest orbital count of the device path: the two-table rank splits a word
 // into a low and a high half of at most 20 bits each, and the per-hop tables
 // must fit in shared memory.
@@ -204,6 +207,10 @@ struct ed_terms {
     edgb::DevBuf<int> hop_off_dev;    // hop.hop_off
     edgb::DevBuf<double> diag_a_dev;  // hop.diag_a
     edgb::DevBuf<double> diag_b_dev;  // hop.diag_b
+    // plans of the matrix-free product by sector (N, twice Lz), the latest
+    // few; null where the row kernel runs instead
+    mutable std::mutex plans_mu;
+    mutable std::vector<std::pair<std::pair<int, int>, std::shared_ptr<edgb::SplitPlan>>> plans;
 };
 
 // Sliced-ELL copy of a full-storage CRS (SELL-C-sigma with C = 32): within
@@ -265,6 +272,11 @@ struct ed_crs {
     // 96 and more elements on average), same states
     mutable std::unique_ptr<ed_fixq> fixq;
     mutable int fix_state = 0;
+    // the Hamiltonian it was built from (null: read from a file), and the
+    // split product's plan made on the first product; same states
+    std::shared_ptr<const edgb::SplitSource> source;
+    mutable std::shared_ptr<edgb::SplitPlan> split;
+    mutable int split_state = 0;
     int product_kernel = 0;   // 0: chosen by shape; else an ed_spmv_kernel id for every product
 };
 
@@ -333,6 +345,8 @@ void spmv(const ed_crs& a, const double* x, double* y, cudaStream_t st);
 // made, declined, or the stream is capturing); solvers call it before they
 // capture their cycles.
 void spmv_prepare(const ed_crs& a, cudaStream_t st);
+// Gives back what products on st keep for that stream, before it is destroyed.
+void spmv_release(const ed_crs& a, cudaStream_t st);
 // kernel 0: as spmv; 1: row lanes k_spmv_full<8,4>; 2, 3: shared reduction k_spmv_rows<8,4,2>,
 // <8,2,2>; 4, 5: sliced ELL k_spmv_sell<16>, <8>; 6: fixed-point integer rows k_spmv_fix<8,8>;
 // 7: the same with the rows staged in shared memory by bulk copies, k_spmv_fix_staged; 8: fixed-point
@@ -345,7 +359,14 @@ void spmv_check(const ed_crs& a, cudaStream_t st);
 // cycles: returns the number of waits that ran out (reset afterwards).
 int spmv_staged_wait_test(const ed_crs& a, const double* x, double* y, long long cycles, cudaStream_t st);
 double measure_dfma_rate(int iters, int blocks_per_sm);
-void hv_matfree(const ed_basis& b, const ed_terms& t, const double* diag, const double* x, double* y,
+// The plan of the matrix-free product for this sector, made when missing
+// (diag: the Hamiltonian's diagonal, computed here when null); null where the
+// row kernel runs instead, or in a capture before the plan is there.
+std::shared_ptr<SplitPlan> matfree_plan(const ed_basis& b, const ed_terms& t, const double* diag, cudaStream_t st);
+// y = H x without a stored matrix.  plan: from matfree_plan, or null; the row
+// kernel runs without one (with diag) and, with one, for an x that is not
+// finite.
+void hv_matfree(const ed_basis& b, const ed_terms& t, SplitPlan* plan, const double* diag, const double* x, double* y,
                 cudaStream_t st);
 void exclusive_scan_i64(const int64_t* in, int64_t* out, int64_t n, cudaStream_t st);
 int64_t reduce_max_i64_host(const int64_t* in, int64_t n, cudaStream_t st);

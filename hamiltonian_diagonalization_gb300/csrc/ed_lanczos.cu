@@ -34,6 +34,7 @@
 #include <vector>
 
 #include "ed_lanczos.h"
+#include "ed_split.h"
 
 namespace edgb {
 
@@ -398,6 +399,17 @@ void op_prepare(const ed_op& op, cudaStream_t st)
 {
     if (op.kind == ed_op::CRS) spmv_prepare(*op.crs, st);
     else if (op.kind == ed_op::DEFLATED && op.inner) op_prepare(*op.inner, st);
+    else if (op.kind == ed_op::MATFREE) {
+        op.plan = matfree_plan(*op.basis, *op.terms, op.diag.p, st);
+        if (op.plan) split_ready(*op.plan, st);
+    }
+}
+
+void op_release(const ed_op& op, cudaStream_t st)
+{
+    if (op.kind == ed_op::CRS) spmv_release(*op.crs, st);
+    else if (op.kind == ed_op::DEFLATED && op.inner) op_release(*op.inner, st);
+    else if (op.plan) split_release(*op.plan, st);
 }
 
 // Throws when one of the operator's products ran out of a bounded wait.
@@ -414,7 +426,8 @@ void op_apply(const ed_op& op, const double* x, double* y, cudaStream_t st)
         spmv(*op.crs, x, y, st);
         break;
     case ed_op::MATFREE:
-        hv_matfree(*op.basis, *op.terms, op.diag.p, x, y, st);
+        if (!op.plan) op.plan = matfree_plan(*op.basis, *op.terms, op.diag.p, st);
+        hv_matfree(*op.basis, *op.terms, op.plan.get(), op.diag.p, x, y, st);
         break;
     case ed_op::HOST: {
         std::vector<double>& hx = const_cast<std::vector<double>&>(op.hx);
@@ -579,6 +592,11 @@ void lanczos_once(const ed_op& op, const ed_lanczos_params& p, const double* v0_
     cudaStream_t st = ss.s;
     const int nsm = sm_count();
     op_prepare(op, st);
+    struct Release {     // before the stream goes
+        const ed_op& op;
+        cudaStream_t st;
+        ~Release() { op_release(op, st); }
+    } release{op, st};
 
     if (v0_dev) {
         // a start vector must be finite and nonzero on every path

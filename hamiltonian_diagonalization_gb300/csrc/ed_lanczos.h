@@ -13,6 +13,7 @@ struct ed_op {
     const ed_basis* basis = nullptr;
     const ed_terms* terms = nullptr;
     edgb::DevBuf<double> diag;          // matrix-free: stored diagonal
+    mutable std::shared_ptr<edgb::SplitPlan> plan;   // matrix-free: the split product's plan, made on first use
     ed_host_matvec fn = nullptr;
     void* user = nullptr;
     mutable std::vector<double> hx, hy; // host staging for HOST operators
@@ -88,6 +89,8 @@ void rotate_basis(const double* V, int64_t n, int m, const double* Y_host, int l
 void op_apply(const ed_op& op, const double* x, double* y, cudaStream_t st);
 // once-per-operator work of the product, before a solver captures its cycles
 void op_prepare(const ed_op& op, cudaStream_t st);
+// gives back what the operator's products keep for st, before it is destroyed
+void op_release(const ed_op& op, cudaStream_t st);
 // throws when one of the operator's products ran out of a bounded wait
 void op_check(const ed_op& op, cudaStream_t st);
 // Lowest p.nev eigenpairs; v0_dev may be null; evecs_dev (n*nev) may be null.

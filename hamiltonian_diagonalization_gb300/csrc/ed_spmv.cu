@@ -29,6 +29,7 @@
 
 #include "ed_fixed.cuh"
 #include "ed_hop.cuh"
+#include "ed_split.h"
 
 namespace edgb {
 
@@ -758,8 +759,10 @@ __global__ void __launch_bounds__(256) k_hv_matfree(const uint64_t* __restrict__
                                                     int nw, const double* __restrict__ da,
                                                     const double* __restrict__ db, const int* __restrict__ off, int K,
                                                     const uint64_t* __restrict__ hi, const uint64_t* __restrict__ lo_tab,
-                                                    int L, const double* __restrict__ x, double* __restrict__ y)
+                                                    int L, const double* __restrict__ x, double* __restrict__ y,
+                                                    const int* __restrict__ xexp)
 {
+    if (xexp && *xexp < 2047) return;   // x is finite: y is there already
     extern __shared__ __align__(16) unsigned char smem[];
     const HopView hv = load_hop_smem(smem, w, nw, da, db, off, K);
     for (int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; r < n; r += (int64_t)gridDim.x * blockDim.x) {
@@ -795,8 +798,10 @@ __global__ void __launch_bounds__(1024) k_hv_matfree_c(const uint64_t* __restric
                                                      const double* __restrict__ diag, const double* __restrict__ w,
                                                      int nw, const int* __restrict__ off, int K,
                                                      const uint64_t* __restrict__ mhi, const uint32_t* __restrict__ mlo,
-                                                     int L, const double* __restrict__ x, double* __restrict__ y)
+                                                     int L, const double* __restrict__ x, double* __restrict__ y,
+                                                     const int* __restrict__ xexp)
 {
+    if (xexp && *xexp < 2047) return;   // x is finite: y is there already
     extern __shared__ __align__(16) unsigned char smem[];
     double* sw = reinterpret_cast<double*>(smem);
     int* soff = reinterpret_cast<int*>(sw + nw);
@@ -1107,10 +1112,37 @@ void fix_launch_sell(const ed_crs& a, const double* x, double* y, cudaStream_t s
 
 }  // namespace
 
+// Stored matrices of at least this many rows take the split product.  Below,
+// the matrix streams from HBM and L2 faster than the short segments of small
+// sectors can be summed.  Measured on GB300, split against the stored kernel:
+// one level 0.92M rows (N=11, 2S=29) 487 / 474 us, 1.37M (N=11, 2S=30) 709 /
+// 772, 1.44M (N=12, 2S=29) 725 / 812, 3.45M (N=12, 2S=31) 1768 / 2274; two
+// levels 0.90M (N=8, 2S=16) 126 / 108, 1.36M 173 / 177, 2.03M 254 / 281,
+// 5.90M (N=8, 2S=21) 760 / 993.
+constexpr int64_t kSplitMinRows = 1 << 20;
+
+// The split product's plan and this stream's scratch, made when missing and
+// not capturing; false when the stored product runs instead.
+static bool split_prepare(const ed_crs& a, cudaStream_t st)
+{
+    if (a.n < kSplitMinRows) return false;
+    if (a.split_state == 0 && !stream_capturing(st)) {
+        a.split = split_build_crs(a, st);
+        a.split_state = a.split ? 1 : -1;
+    }
+    return a.split_state == 1 && split_ready(*a.split, st);
+}
+
+void spmv_release(const ed_crs& a, cudaStream_t st)
+{
+    if (a.split) split_release(*a.split, st);
+}
+
 void spmv_prepare(const ed_crs& a, cudaStream_t st)
 {
     if (a.n == 0 || stream_capturing(st)) return;
     const int k = a.product_kernel;
+    if (k == 0 && split_prepare(a, st)) return;
     if (k == 6 || k == 7 || (k == 0 && fix_shape(a))) fix_ready(a, st);
     if ((k == 4 || k == 5 || k == 8) && a.sell_state == 0) sell_build(a, st);
     if (k == 0 && a.sell_state == 0) {
@@ -1199,6 +1231,10 @@ void spmv(const ed_crs& a, const double* x, double* y, cudaStream_t st)
         spmv_kernel(a, a.product_kernel, x, y, st);
         return;
     }
+    if (split_prepare(a, st)) {
+        split_product(*a.split, x, y, st);
+        return;
+    }
     if (a.sell_state == 0) spmv_prepare(a, st);   // waits for a solver's explicit call while capturing
     if (a.sell_state == 1) {
         if (fix_ready(a, st, true)) {
@@ -1244,10 +1280,40 @@ void spmv(const ed_crs& a, const double* x, double* y, cudaStream_t st)
     ED_CUDA(cudaGetLastError());
 }
 
-void hv_matfree(const ed_basis& b, const ed_terms& t, const double* diag, const double* x, double* y, cudaStream_t st)
+std::shared_ptr<SplitPlan> matfree_plan(const ed_basis& b, const ed_terms& t, const double* diag, cudaStream_t st)
+{
+    constexpr size_t kMaxPlans = 4;
+    if (b.levels != 1 || b.dimX != 0 || b.dim == 0 || t.norb != b.norb) return nullptr;
+    const std::pair<int, int> key(b.N, b.two_lz);
+    std::lock_guard<std::mutex> lk(t.plans_mu);
+    for (auto& e : t.plans)
+        if (e.first == key) return e.second;
+    if (stream_capturing(st)) return nullptr;
+    DevBuf<double> own;
+    if (!diag) {
+        own.alloc((size_t)b.dim);
+        ham_diagonal(b, t, own.p, st);
+    }
+    std::shared_ptr<SplitPlan> p = split_build(split_source(b, t), diag ? diag : own.p, (int64_t)b.dim, 0, st);
+    if (p) {
+        // the row kernel's diagonal, for an x that is not finite
+        p->values.alloc((size_t)b.dim);
+        ED_CUDA(cudaMemcpyAsync(p->values.p, diag ? diag : own.p, (size_t)b.dim * 8, cudaMemcpyDeviceToDevice, st));
+        ED_CUDA(cudaStreamSynchronize(st));
+    }
+    if (t.plans.size() == kMaxPlans) t.plans.erase(t.plans.begin());
+    t.plans.push_back({key, p});
+    return p;
+}
+
+void hv_matfree(const ed_basis& b, const ed_terms& t, SplitPlan* plan, const double* diag, const double* x, double* y,
+                cudaStream_t st)
 {
     ED_REQUIRE(b.levels == 1 && b.dimX == 0, ED_ERR_ARG, "the matrix-free product takes a one-level Lz basis");
     if (b.dim == 0) return;
+    const int* xexp = nullptr;
+    if (plan && split_ready(*plan, st)) xexp = split_product(*plan, x, y, st);
+    if (plan) diag = plan->values.p;
     const int K = t.norb;
     const int nw = (int)t.hop.w.size();
     if (b.mf_lo.p) {
@@ -1268,7 +1334,7 @@ void hv_matfree(const ed_basis& b, const ed_terms& t, const double* diag, const 
                 it = occ.emplace(std::make_pair(dev, smem), std::max(1, ob)).first;
             }
             k_hv_matfree_c<<<sms() * it->second, 1024, smem, st>>>(b.words.p, (int64_t)b.dim, diag, t.w_dev.p, nw,
-                                                                   t.hop_off_dev.p, K, b.mf_hi.p, b.mf_lo.p, L, x, y);
+                                                                   t.hop_off_dev.p, K, b.mf_hi.p, b.mf_lo.p, L, x, y, xexp);
             count_launch();
             ED_CUDA(cudaGetLastError());
             return;
@@ -1277,7 +1343,8 @@ void hv_matfree(const ed_basis& b, const ed_terms& t, const double* diag, const 
     const size_t smem = hop_smem_bytes(K, nw);
     ED_CUDA(cudaFuncSetAttribute(k_hv_matfree, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     k_hv_matfree<<<sms() * 4, 256, smem, st>>>(b.words.p, (int64_t)b.dim, diag, t.w_dev.p, nw, t.diag_a_dev.p,
-                                                t.diag_b_dev.p, t.hop_off_dev.p, K, b.hi.p, b.lo.p, b.low_bits, x, y);
+                                                t.diag_b_dev.p, t.hop_off_dev.p, K, b.hi.p, b.lo.p, b.low_bits, x, y,
+                                                xexp);
     count_launch();
     ED_CUDA(cudaGetLastError());
 }
