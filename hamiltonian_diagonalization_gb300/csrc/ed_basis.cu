@@ -206,7 +206,17 @@ int grid_for(int64_t work, int threads)
 
 }  // namespace
 
-void exclusive_scan_i64(const int64_t* in, int64_t* out, int64_t n, cudaStream_t st)
+int64_t scan_workspace_i64(int64_t n)
+{
+    int64_t total = 0;
+    for (int64_t t = n; t > 1;) {
+        t = (t + kScanTile - 1) / kScanTile;
+        total += 2 * (t + 1);
+    }
+    return total + 2;
+}
+
+void exclusive_scan_i64(const int64_t* in, int64_t* out, int64_t n, int64_t* ws, cudaStream_t st)
 {
     // out has n+1 entries; out[n] = total
     if (n <= 0) {
@@ -214,18 +224,24 @@ void exclusive_scan_i64(const int64_t* in, int64_t* out, int64_t n, cudaStream_t
         return;
     }
     const int64_t tiles = (n + kScanTile - 1) / kScanTile;
-    DevBuf<int64_t> sums(tiles + 1);
-    k_scan_tiles<<<(unsigned)tiles, kScanThreads, 0, st>>>(in, out, n, sums.p); ::edgb::count_launch();
+    int64_t* sums = ws;
+    k_scan_tiles<<<(unsigned)tiles, kScanThreads, 0, st>>>(in, out, n, sums); ::edgb::count_launch();
     ED_CUDA(cudaGetLastError());
     if (tiles == 1) {
-        ED_CUDA(cudaMemcpyAsync(out + n, sums.p, sizeof(int64_t), cudaMemcpyDeviceToDevice, st));
+        ED_CUDA(cudaMemcpyAsync(out + n, sums, sizeof(int64_t), cudaMemcpyDeviceToDevice, st));
     } else {
-        DevBuf<int64_t> offs(tiles + 1);
-        exclusive_scan_i64(sums.p, offs.p, tiles, st);
-        k_scan_add<<<(unsigned)tiles, 256, 0, st>>>(out, n, offs.p); ::edgb::count_launch();
+        int64_t* offs = sums + tiles + 1;
+        exclusive_scan_i64(sums, offs, tiles, offs + tiles + 1, st);
+        k_scan_add<<<(unsigned)tiles, 256, 0, st>>>(out, n, offs); ::edgb::count_launch();
         ED_CUDA(cudaGetLastError());
-        ED_CUDA(cudaMemcpyAsync(out + n, offs.p + tiles, sizeof(int64_t), cudaMemcpyDeviceToDevice, st));
+        ED_CUDA(cudaMemcpyAsync(out + n, offs + tiles, sizeof(int64_t), cudaMemcpyDeviceToDevice, st));
     }
+}
+
+void exclusive_scan_i64(const int64_t* in, int64_t* out, int64_t n, cudaStream_t st)
+{
+    DevBuf<int64_t> ws((size_t)scan_workspace_i64(n));
+    exclusive_scan_i64(in, out, n, ws.p, st);
     // the temporaries are freed when they go out of scope; make sure the
     // kernels that read them are done first
     ED_CUDA(cudaStreamSynchronize(st));

@@ -14,6 +14,8 @@
 namespace edgb {
 namespace {
 
+constexpr int kFixMaxRow = 2048;     // row elements: |S| < 2048 * 2^116 = 2^127
+
 // Biased exponent field, 1 for zeros and subnormals (their scale).
 __device__ __forceinline__ int fix_exp(double v)
 {
@@ -155,6 +157,26 @@ __device__ __forceinline__ void fix_mac(int2 a, int2 b, long long& p2, long long
 __device__ __forceinline__ __int128 fix_combine(long long p2, long long p1, long long p0)
 {
     return ((__int128)p2 << 60) + ((__int128)p1 << 30) + (__int128)p0;
+}
+
+// An exact sum hi 2^60 + lo, 0 <= lo < 2^60, kept over many products: the
+// next ones go on from (p2, p1, p0) = (hi, 0, lo), at most kFixFlush of them
+// (p1 < 12 2^59, p0 < 13 2^60) until the next carry.  The sum of |p2| over all
+// products must stay below 2^63.
+struct FixSum {
+    long long hi;
+    unsigned long long lo;
+};
+
+constexpr unsigned long long kFixLow60 = (1ull << 60) - 1ull;
+constexpr int kFixFlush = 12;
+
+// The limb sums p2 2^60 + p1 2^30 + p0 as a FixSum (p0 taken unsigned).
+__device__ __forceinline__ FixSum fix_carry(long long p2, long long p1, long long p0)
+{
+    unsigned long long t;
+    asm("mad.wide.u32 %0, %1, %2, %3;" : "=l"(t) : "r"((unsigned)p1 & 0x3FFFFFFFu), "r"(1u << 30), "l"((unsigned long long)p0));
+    return FixSum{p2 + (p1 >> 30) + (long long)(t >> 60), t & kFixLow60};
 }
 
 // The sum of an int128 over the 32 lanes of a warp (exact).

@@ -369,5 +369,8 @@ std::shared_ptr<SplitPlan> matfree_plan(const ed_basis& b, const ed_terms& t, co
 void hv_matfree(const ed_basis& b, const ed_terms& t, SplitPlan* plan, const double* diag, const double* x, double* y,
                 cudaStream_t st);
 void exclusive_scan_i64(const int64_t* in, int64_t* out, int64_t n, cudaStream_t st);
+// The same in a given workspace of scan_workspace_i64(n) words, without waiting.
+int64_t scan_workspace_i64(int64_t n);
+void exclusive_scan_i64(const int64_t* in, int64_t* out, int64_t n, int64_t* ws, cudaStream_t st);
 int64_t reduce_max_i64_host(const int64_t* in, int64_t n, cudaStream_t st);
 }  // namespace edgb

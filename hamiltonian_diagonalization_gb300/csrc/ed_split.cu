@@ -58,6 +58,7 @@ constexpr int kMaxMovable = 12;      // of kMaxSideBits orbitals, by one distanc
 static_assert(kSegRows == 1 << kRowBits, "row field");
 
 enum GammaType { kKeep = 0, kEmpty = 1, kFill = 2 };   // and the moves, in lists of their own
+constexpr int kKeepParts = 8;        // kKeep's alpha entries are listed in so many parts, one after another
 constexpr int kMaxSideBits = 24;     // tables over one part's words
 
 int sms()
@@ -102,10 +103,12 @@ __device__ __forceinline__ void for_alpha(const GenArgs& g, uint32_t P, int gm, 
         const int odd = (1 + __popcll(rest & (bits_between(a, b) ^ bits_between(c, d)))) & 1;
         f((uint32_t)(out >> plo), odd ? -w : w);
     };
-    if (type == kKeep) {
+    if (type == kKeep) {               // part o: every kKeepParts-th pair
+        int pair = kKeepParts - o;
         for (uint64_t ta = W; ta; ta &= ta - 1) {
             const int a = __ffsll((long long)ta) - 1;
             for (uint64_t tb = ta & (ta - 1); tb; tb &= tb - 1) {
+                if (pair++ % kKeepParts) continue;
                 const int b = __ffsll((long long)tb) - 1;
                 const uint64_t rest = W ^ (1ull << a) ^ (1ull << b);
                 for (uint32_t m = (uint32_t)hop_targets(P, a - plo, b - plo, g.pbits, false); m; m &= m - 1) {
@@ -219,42 +222,43 @@ __global__ void __launch_bounds__(128) k_split_alpha(GenArgs g, const uint32_t* 
 __host__ __device__ __forceinline__ int move_distance(int i) { return (i & 1) ? -(i / 2 + 1) : i / 2 + 1; }
 
 // Moves of one secondary particle by a distance d, one thread per (primary
-// word, d): each way the primary word makes up for it (x -> x - d) gets its
-// segment base and two rows of weights over the orbital o that the secondary
-// particle leaves (o -> o + d), sbits of each sign.
+// word, d), or, filling, per (primary word, d, orbital o): each way the primary
+// word makes up for the move (x -> x - d) gets its segment base and two rows of
+// weights over the orbital o that the secondary particle leaves (o -> o + d),
+// sbits of each sign.
+template <bool FILL>
 __global__ void __launch_bounds__(128) k_split_moves(GenArgs g, const uint32_t* __restrict__ pword, int np,
                                                      const int* __restrict__ by_word, int64_t* __restrict__ cnt,
                                                      const int64_t* __restrict__ start, int ea, int* __restrict__ base,
                                                      int64_t* __restrict__ weight)
 {
     const int nm = 2 * (g.sbits - 1);
-    const int64_t total = (int64_t)np * nm;
-    for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t total = (int64_t)np * nm * (FILL ? g.sbits : 1);
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t t = FILL ? i / g.sbits : i;
+        const int o = FILL ? (int)(i % g.sbits) : 0;
         const uint32_t P = pword[t / nm];
-        const int d = move_distance((int)(t % nm));
-        int64_t k = base ? start[t] : 0;
+        const int d = move_distance((int)(t % nm)), q = o + d;
+        int64_t k = FILL ? start[t] : 0;
         for (uint32_t tx = P; tx; tx &= tx - 1) {
             const int x = __ffs((int)tx) - 1, z = x - d;
             if (z < 0 || z >= g.pbits || ((P >> z) & 1)) continue;
             const int b = by_word[P ^ (1u << x) ^ (1u << z)];
             if (b < 0) continue;
-            if (base) {
-                base[k] = b;
+            if (FILL) {
+                if (o == 0) base[k] = b;
                 const int odd = (1 + __popc(P & ((1u << max(x, z)) - 1u) & ~((2u << min(x, z)) - 1u))) & 1;
-                for (int o = 0; o < g.sbits; ++o) {
-                    const int q = o + d;
-                    double w = 0.0;
-                    if (q >= 0 && q < g.sbits) {
-                        const int so = g.slo + o, sq = g.slo + q, gx = g.plo + x, gz = g.plo + z;
-                        w = hop_weight(g, min(so, gx), max(so, gx), min(sq, gz));
-                    }
-                    weight[2 * k * g.sbits + o] = fix_pair(odd ? -w : w, ea);
-                    weight[(2 * k + 1) * g.sbits + o] = fix_pair(odd ? w : -w, ea);
+                double w = 0.0;
+                if (q >= 0 && q < g.sbits) {
+                    const int so = g.slo + o, sq = g.slo + q, gx = g.plo + x, gz = g.plo + z;
+                    w = hop_weight(g, min(so, gx), max(so, gx), min(sq, gz));
                 }
+                weight[2 * k * g.sbits + o] = fix_pair(odd ? -w : w, ea);
+                weight[(2 * k + 1) * g.sbits + o] = fix_pair(odd ? w : -w, ea);
             }
             ++k;
         }
-        if (!base) cnt[t] = k;
+        if (!FILL) cnt[t] = k;
     }
 }
 
@@ -410,22 +414,7 @@ __global__ void __launch_bounds__(256) k_split_conv(const double* __restrict__ v
     }
 }
 
-// An exact sum hi 2^60 + lo, 0 <= lo < 2^60.
-struct Sum {
-    long long hi;
-    unsigned long long lo;
-};
-
-constexpr unsigned long long kLow60 = (1ull << 60) - 1ull;
-constexpr int kFlush = 12;           // products between two carries: p1 < 12 2^59, p0 < 13 2^60
-
-// The limb sums p2 2^60 + p1 2^30 + p0 as a Sum (p0 taken unsigned).
-__device__ __forceinline__ Sum carry(long long p2, long long p1, long long p0)
-{
-    unsigned long long t;
-    asm("mad.wide.u32 %0, %1, %2, %3;" : "=l"(t) : "r"((unsigned)p1 & 0x3FFFFFFFu), "r"(1u << 30), "l"((unsigned long long)p0));
-    return Sum{p2 + (p1 >> 30) + (long long)(t >> 60), t & kLow60};
-}
+using Sum = FixSum;
 
 __device__ __forceinline__ Sum negated(Sum s) { return Sum{~s.hi, (1ull << 60) - s.lo}; }
 
@@ -433,7 +422,7 @@ __device__ __forceinline__ void add_to(Sum& a, Sum b)   // b.lo <= 2^60
 {
     const unsigned long long t = a.lo + b.lo;
     a.hi += b.hi + (long long)(t >> 60);
-    a.lo = t & kLow60;
+    a.lo = t & kFixLow60;
 }
 
 // s[u] += sum over the n entries w of weight * x(entry, u).
@@ -441,7 +430,7 @@ template <int NU, class F>
 __device__ __forceinline__ void keep_sum(const int4* w, int n, F&& x, Sum (&s)[NU])
 {
     for (int i = 0; i < n;) {
-        const int e = min(i + kFlush, n);
+        const int e = min(i + kFixFlush, n);
         long long p2[NU], p1[NU], p0[NU];
 #pragma unroll
         for (int u = 0; u < NU; ++u) {
@@ -456,7 +445,7 @@ __device__ __forceinline__ void keep_sum(const int4* w, int n, F&& x, Sum (&s)[N
             for (int u = 0; u < NU; ++u) fix_mac(make_int2(v.y, v.z), x(v, u), p2[u], p1[u], p0[u]);
         }
 #pragma unroll
-        for (int u = 0; u < NU; ++u) s[u] = carry(p2[u], p1[u], p0[u]);
+        for (int u = 0; u < NU; ++u) s[u] = fix_carry(p2[u], p1[u], p0[u]);
     }
 }
 
@@ -498,7 +487,7 @@ __device__ __forceinline__ void keep_rows(const SplitArgs& g, int a0, int a1, in
 }
 
 // One list of a gamma that changes one orbital: U blocks of 32 entries at a
-// time, up to kFlush alpha entries (the same for all lanes) each.
+// time, up to kFixFlush alpha entries (the same for all lanes) each.
 template <int U>
 __device__ __forceinline__ void change_block(const SplitArgs& g, int a0, int a1, int e, int e1, Sum* acc)
 {
@@ -520,7 +509,7 @@ __device__ __forceinline__ void change_block(const SplitArgs& g, int a0, int a1,
     }
 #pragma unroll
     for (int u = 0; u < U; ++u) {
-        Sum s = carry(p2[u], p1[u], p0[u]);
+        Sum s = fix_carry(p2[u], p1[u], p0[u]);
         if ((int)ent[u] < 0) s = negated(s);
         if (e + 32 * u < e1) add_to(acc[ent[u] & (kSegRows - 1)], s);
     }
@@ -528,8 +517,8 @@ __device__ __forceinline__ void change_block(const SplitArgs& g, int a0, int a1,
 
 __device__ __forceinline__ void change_list(const SplitArgs& g, int a0, int a1, int e0, int e1, Sum* acc)
 {
-    for (; a0 < a1; a0 += kFlush) {
-        const int a = min(a1, a0 + kFlush);
+    for (; a0 < a1; a0 += kFixFlush) {
+        const int a = min(a1, a0 + kFixFlush);
         int eb = e0, e = e0 + (threadIdx.x & 31);
         for (; eb + 32 < e1; eb += 64, e += 64) change_block<2>(g, a0, a, e, e1, acc);
         if (eb < e1) change_block<1>(g, a0, a, e, e1, acc);
@@ -543,7 +532,7 @@ __device__ __forceinline__ void change_list(const SplitArgs& g, int a0, int a1, 
 template <int CA>
 __device__ __forceinline__ void move_list(const SplitArgs& g, int a0, int e0, int e1, Sum* acc)
 {
-    constexpr int kSteps = kFlush / CA;
+    constexpr int kSteps = kFixFlush / CA;
     int b[CA];
 #pragma unroll
     for (int a = 0; a < CA; ++a) b[a] = __ldg(g.mbase + a0 + a);
@@ -570,14 +559,14 @@ __device__ __forceinline__ void move_list(const SplitArgs& g, int a0, int e0, in
             for (int a = 0; a < CA; ++a) fix_mac(w[a], x[a], p2, p1, p0);
             if (--left == 0) break;
             if (--step == 0) {
-                const Sum s = carry(p2, p1, p0);
+                const Sum s = fix_carry(p2, p1, p0);
                 p2 = s.hi;
                 p1 = 0;
                 p0 = (long long)s.lo;
                 step = kSteps;
             }
         }
-        const Sum s = carry(p2, p1, p0);
+        const Sum s = fix_carry(p2, p1, p0);
         if (!(head & kNullEntry)) add_to(acc[(head >> kRowShift) & (kSegRows - 1)], s);
     }
     __syncwarp();
@@ -616,14 +605,14 @@ __global__ void __launch_bounds__(kThreads, 18) k_split_product(SplitArgs g)
     const int* __restrict__ ms = g.mstart + (int64_t)p * g.moves;
     if (threadIdx.x == 0) queue = count = 0;
     __syncthreads();
-    for (int i = threadIdx.x; i < g.moves + g.gammas - 1; i += kThreads) {
+    for (int i = threadIdx.x; i < g.moves + g.gammas - kKeepParts; i += kThreads) {
         // the moves first, the short distances before the long ones: the largest lists
         int4 v;
         if (i < g.moves) {
             const int* l = g.mlstart + ((int64_t)c * g.moves + i) * g.nseg + seg;
             v = make_int4(ms[i], ms[i + 1], l[0], ~l[1]);
         } else {
-            const int gm = i - g.moves + 1;
+            const int gm = i - g.moves + kKeepParts;
             const int* l = g.lstart + ((int64_t)c * g.gammas + gm) * g.nseg + seg;
             v = make_int4(as[gm], as[gm + 1], l[0], l[1]);
         }
@@ -633,7 +622,7 @@ __global__ void __launch_bounds__(kThreads, 18) k_split_product(SplitArgs g)
 #pragma unroll
         for (int w = 1; w < kWarps; ++w) acc[w * g.rows + r] = Sum{0, 0};
     {
-        const int a0 = as[0], a1 = as[1], r0 = seg * kSegRows;
+        const int a0 = as[0], a1 = as[kKeepParts], r0 = seg * kSegRows;
         int r = 0;
         for (; r + kThreads < rows; r += 2 * kThreads) keep_rows<2>(g, a0, a1, r0, r, rows, acc);
         if (r < rows) keep_rows<1>(g, a0, a1, r0, r, rows, acc);
@@ -688,7 +677,7 @@ __device__ __forceinline__ void keep_task(const SplitArgs& g, int p, int size, i
         at[u] = min(r0 + width * u, size - 1);
         s[u] = Sum{0, 0};
     }
-    const int a0 = g.astart[p], a1 = g.astart[p + 1];
+    const int a0 = g.astart[(int64_t)p * kKeepParts], a1 = g.astart[(int64_t)(p + 1) * kKeepParts];
     auto x = [&](const int4& v, int u) { return __ldg(g.x + (v.x + at[u])); };
     if (width == 32) staged_sum<NU>(g.alpha, a0, a1, x, s, stage);
     else keep_sum<NU>(g.alpha + a0, a1 - a0, x, s);
@@ -721,7 +710,6 @@ __global__ void __launch_bounds__(kThreads, 20) k_split_keep(SplitArgs g, int nt
 
 // ------------------------------------------------------------------ the plan
 
-constexpr int kMaxRow = 2048;        // exact row sums stay below 2^127 (ed_spmv.cu)
 // The words of one part with at most N bits set, grouped by class.
 struct PartWords {
     std::vector<uint32_t> word;      // by class, ascending
@@ -729,8 +717,19 @@ struct PartWords {
     std::vector<int> start, size;    // per class
 };
 
-// (popcount, weight sum) -> words, ascending within each key
-void enumerate_part(const std::vector<int>& w, int N, int min_pop, std::vector<std::pair<int, uint32_t>>& out, int span)
+// words of each key = popcount * span + weight sum, up to N bits set
+void count_part(const std::vector<int>& w, int N, int span, std::vector<int>& count)
+{
+    count[0] = 1;
+    for (int wk : w)
+        for (int pop = N; pop >= 1; --pop)
+            for (int sum = span - 1; sum >= wk; --sum) count[pop * span + sum] += count[(pop - 1) * span + sum - wk];
+}
+
+// f(key, word) for every word of min_pop .. N bits set, ascending within each
+// key = popcount * span + weight sum
+template <class F>
+void for_part(const std::vector<int>& w, int N, int min_pop, int span, F&& f)
 {
     const int B = (int)w.size(), lo_bits = std::min(B, 12);
     std::vector<int> lo(1u << lo_bits), hi(1u << (B - lo_bits));
@@ -739,10 +738,10 @@ void enumerate_part(const std::vector<int>& w, int N, int min_pop, std::vector<s
     for (int pop = std::max(0, min_pop); pop <= std::min(N, B); ++pop) {
         uint64_t v = (1ull << pop) - 1, end = 1ull << B;
         while (v < end) {
-            out.push_back({pop * span + lo[v & ((1u << lo_bits) - 1)] + hi[v >> lo_bits], (uint32_t)v});
+            f(pop * span + lo[v & ((1u << lo_bits) - 1)] + hi[v >> lo_bits], (uint32_t)v);
             if (v == 0) break;
-            const uint64_t t = v & (0 - v), r = v + t;   // next word of the same popcount
-            v = r | (((v ^ r) >> 2) / t);
+            const uint64_t r = v + (v & (0 - v));   // next word of the same popcount
+            v = r | ((v ^ r) >> (2 + __builtin_ctzll(v)));
         }
     }
 }
@@ -767,161 +766,193 @@ int grid_of(int64_t work, int threads)
     return (int)std::max<int64_t>(1, std::min<int64_t>((work + threads - 1) / threads, (int64_t)sms() * 16));
 }
 
-// One pass: primary words P (by class), secondary words S of the same classes.
-// given_base: the segments' bases (transposed pass), else the scan over the
-// primary words in ascending order (native).  False when it does not fit.
-bool build_side(SplitSide& out, const PartWords& P, const PartWords& S, GenArgs g, const std::vector<int>& gamma, bool moves, int ea,
-                const std::vector<int>* given_base, size_t& room, cudaStream_t st)
-{
-    const int np = (int)P.word.size(), nc = (int)P.start.size();
-    const int G = (int)gamma.size();
-    out.gammas = G;
-    int longest = 0;
-    for (int c = 0; c < nc; ++c) longest = std::max(longest, S.size[c]);
-    if (G > 1 && longest > (int)kRankMask) return false;
-    out.nseg = (longest + kSegRows - 1) / kSegRows;
-    out.rows = G == 1 ? 0 : (std::min(longest, kSegRows) + 31) / 32 * 32;
-    DevBuf<uint32_t> pword;
-    DevBuf<int> dgamma;
-    upload(pword, P.word, st);
-    upload(dgamma, gamma, st);
-    upload(out.pcls, P.cls, st);
-    upload(out.ssize, S.size, st);
-    g.gamma = dgamma.p;
-    g.gammas = G;
-    // segment bases, also by word
-    const int64_t nw = 1ll << g.pbits;
-    DevBuf<int> by_word((size_t)nw);
-    ED_CUDA(cudaMemsetAsync(by_word.p, 0xFF, (size_t)nw * 4, st));
-    DevBuf<int64_t> scan;
-    if (given_base) {
-        upload(out.pbase, *given_base, st);
-    } else {
-        DevBuf<int64_t> len((size_t)nw);
-        scan.alloc((size_t)nw + 1);
-        out.pbase.alloc(np);
-        ED_CUDA(cudaMemsetAsync(len.p, 0, (size_t)nw * 8, st));
-        k_split_lengths<<<grid_of(np, 256), 256, 0, st>>>(pword.p, out.pcls.p, out.ssize.p, np, len.p);
-        count_launch();
-        exclusive_scan_i64(len.p, scan.p, nw, st);
-    }
-    k_split_bases<<<grid_of(np, 256), 256, 0, st>>>(pword.p, np, scan.p, out.pbase.p, by_word.p);
-    count_launch();
-    // alpha lists
-    const int64_t na = (int64_t)np * G;
-    int64_t total = 0;
+int exp_parts() { return sms() * 2; }
+
+// Device memory for the build's temporaries: few allocations, freed together.
+struct Arena {
+    std::vector<DevBuf<char>> blocks;
+    size_t used = 0;
+    template <class T>
+    T* take(size_t count)
     {
-        DevBuf<int64_t> cnt((size_t)na), start((size_t)na + 1);
-        k_split_alpha<<<grid_of(na, 128), 128, 0, st>>>(g, pword.p, np, by_word.p, cnt.p, nullptr, ea, nullptr);
-        count_launch();
-        exclusive_scan_i64(cnt.p, start.p, na, st);
-        ED_CUDA(cudaMemcpyAsync(&total, start.p + na, 8, cudaMemcpyDeviceToHost, st));
-        ED_CUDA(cudaStreamSynchronize(st));
-        if (total >= (1ll << 31) || (size_t)total * 16 > room) return false;
-        room -= (size_t)total * 16;
-        out.alpha.alloc((size_t)total + 1);
-        out.astart.alloc((size_t)na + 1);
-        k_split_alpha<<<grid_of(na, 128), 128, 0, st>>>(g, pword.p, np, by_word.p, nullptr, start.p, ea, out.alpha.p);
-        count_launch();
-        k_split_narrow<<<grid_of(na + 1, 256), 256, 0, st>>>(start.p, na + 1, out.astart.p);
-        count_launch();
-        ED_CUDA(cudaGetLastError());
-        ED_CUDA(cudaStreamSynchronize(st));
-    }
-    if (moves) {
-        const int nm = out.moves = 2 * (g.sbits - 1);
-        out.sbits = g.sbits;
-        const int64_t nt = (int64_t)np * nm;
-        DevBuf<int64_t> cnt((size_t)nt), start((size_t)nt + 1);
-        k_split_moves<<<grid_of(nt, 128), 128, 0, st>>>(g, pword.p, np, by_word.p, cnt.p, nullptr, ea, nullptr, nullptr);
-        count_launch();
-        exclusive_scan_i64(cnt.p, start.p, nt, st);
-        ED_CUDA(cudaMemcpyAsync(&total, start.p + nt, 8, cudaMemcpyDeviceToHost, st));
-        ED_CUDA(cudaStreamSynchronize(st));
-        const size_t bytes = (size_t)total * (4 + 16 * (size_t)g.sbits);
-        if (total >= (1ll << 31) || bytes > room) return false;
-        room -= bytes;
-        out.mbase.alloc((size_t)total + 1);
-        out.mweight.alloc((size_t)total * 2 * g.sbits + 1);
-        out.mstart.alloc((size_t)nt + 1);
-        k_split_moves<<<grid_of(nt, 128), 128, 0, st>>>(g, pword.p, np, by_word.p, nullptr, start.p, ea, out.mbase.p,
-                                                        out.mweight.p);
-        count_launch();
-        k_split_narrow<<<grid_of(nt + 1, 256), 256, 0, st>>>(start.p, nt + 1, out.mstart.p);
-        count_launch();
-        ED_CUDA(cudaGetLastError());
-        ED_CUDA(cudaStreamSynchronize(st));
-    }
-    std::vector<int2> task;
-    std::vector<int> order(nc);
-    for (int c = 0; c < nc; ++c) order[c] = c;
-    std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return S.size[a] > S.size[b]; });   // longest first
-    if (G == 1) {
-        for (int c : order) {
-            const int m = S.size[c], words = P.size[c];
-            int width = 32;                       // lanes a word: the fewest that hold its segment
-            while (width > 2 && m <= width / 2) width /= 2;
-            const int per = 32 / width, rows = width == 32 ? 32 * kIdRows : width;
-            for (int i = 0; i < words; i += per)
-                for (int seg = 0; seg * rows < m; ++seg)
-                    task.push_back(make_int2(P.start[c] + i, width | std::min(per, words - i) << 6 | seg << 12));
+        const size_t bytes = (count * sizeof(T) + 255) / 256 * 256;
+        if (blocks.empty() || used + bytes > blocks.back().n) {
+            blocks.emplace_back(std::max<size_t>(bytes, (size_t)32 << 20));
+            used = 0;
         }
-    } else {
-        // secondary lists
-        DevBuf<uint32_t> sword;
-        DevBuf<int> scls, sstart, rank((size_t)1 << g.sbits);
-        upload(sword, S.word, st);
-        upload(scls, S.cls, st);
-        upload(sstart, S.start, st);
-        k_split_ranks<<<grid_of((int64_t)S.word.size(), 256), 256, 0, st>>>(sword.p, scls.p, sstart.p, (int)S.word.size(), rank.p);
+        used += bytes;
+        return reinterpret_cast<T*>(blocks.back().p + used - bytes);
+    }
+    template <class T>
+    T* put(const std::vector<T>& h, cudaStream_t st)
+    {
+        T* p = take<T>(std::max<size_t>(1, h.size()));
+        if (!h.empty()) ED_CUDA(cudaMemcpyAsync(p, h.data(), h.size() * sizeof(T), cudaMemcpyHostToDevice, st));
+        return p;
+    }
+};
+
+// One pass: primary words P (by class), secondary words S of the same classes.
+// count() enqueues the list lengths' counts and scans, fill(), after the
+// stream has been waited for, allocates and enqueues the lists.
+struct SideBuild {
+    SplitSide& out;
+    const PartWords &P, &S;
+    GenArgs g;
+    const std::vector<int>& gamma;
+    bool moves;
+    Arena& tmp;
+    cudaStream_t st;
+    int np = 0, nc = 0, G = 0;
+    uint32_t *pword = nullptr, *sword = nullptr;
+    int *by_word = nullptr, *sstart = nullptr, *rank = nullptr;
+    struct Lists {                 // of one kind
+        int64_t n = 0, total = 0;
+        int64_t* start = nullptr;
+    } alpha, move, list, mlist;
+
+    template <class F>
+    void counted(Lists& l, int64_t n, F&& count)
+    {
+        l.n = n;
+        int64_t* cnt = tmp.take<int64_t>((size_t)n);
+        l.start = tmp.take<int64_t>((size_t)n + 1);
+        count(cnt);
         count_launch();
-        const int64_t nl = (int64_t)nc * G * out.nseg;
-        DevBuf<int64_t> cnt((size_t)nl), start((size_t)nl + 1);
-        k_split_lists<<<sms() * 8, 256, 0, st>>>(g, sword.p, sstart.p, out.ssize.p, rank.p, nc, out.nseg, cnt.p, nullptr, nullptr);
+        exclusive_scan_i64(cnt, l.start, n, tmp.take<int64_t>((size_t)scan_workspace_i64(n)), st);
+        ED_CUDA(cudaMemcpyAsync(&l.total, l.start + n, 8, cudaMemcpyDeviceToHost, st));
+    }
+    // the starts as 32-bit indices
+    void starts(const Lists& l, DevBuf<int>& d)
+    {
+        d.alloc((size_t)l.n + 1);
+        k_split_narrow<<<grid_of(l.n + 1, 256), 256, 0, st>>>(l.start, l.n + 1, d.p);
         count_launch();
-        exclusive_scan_i64(cnt.p, start.p, nl, st);
-        ED_CUDA(cudaMemcpyAsync(&total, start.p + nl, 8, cudaMemcpyDeviceToHost, st));
-        ED_CUDA(cudaStreamSynchronize(st));
-        if (total >= (1ll << 31) || (size_t)total * 4 > room) return false;
-        room -= (size_t)total * 4;
-        out.list.alloc((size_t)total + 1);
-        out.lstart.alloc((size_t)nl + 1);
-        k_split_lists<<<sms() * 8, 256, 0, st>>>(g, sword.p, sstart.p, out.ssize.p, rank.p, nc, out.nseg, nullptr, start.p, out.list.p);
+    }
+
+    // given_base: the segments' bases (transposed pass), else the scan over
+    // the primary words in ascending order (native)
+    bool count(const std::vector<int>* given_base)
+    {
+        np = (int)P.word.size();
+        nc = (int)P.start.size();
+        out.gammas = g.gammas = G = (int)gamma.size();
+        int longest = 0;
+        for (int c = 0; c < nc; ++c) longest = std::max(longest, S.size[c]);
+        const bool lists = G > kKeepParts;
+        if (lists && longest > (int)kRankMask) return false;
+        out.nseg = (longest + kSegRows - 1) / kSegRows;
+        out.rows = (std::min(longest, kSegRows) + 31) / 32 * 32;
+        pword = tmp.put(P.word, st);
+        g.gamma = tmp.put(gamma, st);
+        upload(out.pcls, P.cls, st);
+        upload(out.ssize, S.size, st);
+        const int64_t nw = 1ll << g.pbits;
+        by_word = tmp.take<int>((size_t)nw);
+        ED_CUDA(cudaMemsetAsync(by_word, 0xFF, (size_t)nw * 4, st));
+        int64_t* scan = nullptr;
+        if (given_base) {
+            upload(out.pbase, *given_base, st);
+        } else {
+            int64_t* len = tmp.take<int64_t>((size_t)nw);
+            scan = tmp.take<int64_t>((size_t)nw + 1);
+            out.pbase.alloc(np);
+            ED_CUDA(cudaMemsetAsync(len, 0, (size_t)nw * 8, st));
+            k_split_lengths<<<grid_of(np, 256), 256, 0, st>>>(pword, out.pcls.p, out.ssize.p, np, len);
+            count_launch();
+            exclusive_scan_i64(len, scan, nw, tmp.take<int64_t>((size_t)scan_workspace_i64(nw)), st);
+        }
+        k_split_bases<<<grid_of(np, 256), 256, 0, st>>>(pword, np, scan, out.pbase.p, by_word);
         count_launch();
-        k_split_narrow<<<grid_of(nl + 1, 256), 256, 0, st>>>(start.p, nl + 1, out.lstart.p);
-        count_launch();
-        ED_CUDA(cudaGetLastError());
-        ED_CUDA(cudaStreamSynchronize(st));
+        const int64_t na = (int64_t)np * G;
+        counted(alpha, na, [&](int64_t* cnt) {
+            k_split_alpha<<<grid_of(na, 128), 128, 0, st>>>(g, pword, np, by_word, cnt, nullptr, 0, nullptr);
+        });
+        if (lists) {
+            sword = tmp.put(S.word, st);
+            sstart = tmp.put(S.start, st);
+            rank = tmp.take<int>((size_t)1 << g.sbits);
+            k_split_ranks<<<grid_of((int64_t)S.word.size(), 256), 256, 0, st>>>(sword, tmp.put(S.cls, st), sstart, (int)S.word.size(),
+                                                                               rank);
+            count_launch();
+            counted(list, (int64_t)nc * G * out.nseg, [&](int64_t* cnt) {
+                k_split_lists<<<sms() * 8, 256, 0, st>>>(g, sword, sstart, out.ssize.p, rank, nc, out.nseg, cnt, nullptr, nullptr);
+            });
+        }
         if (moves) {
-            const int64_t nm = (int64_t)nc * out.moves * out.nseg;
-            DevBuf<int64_t> mcnt((size_t)nm), mstart((size_t)nm + 1);
-            k_split_move_lists<<<sms() * 16, 128, 0, st>>>(g, sword.p, sstart.p, out.ssize.p, rank.p, nc, out.nseg,
-                                                                 mcnt.p, nullptr, nullptr);
-            count_launch();
-            exclusive_scan_i64(mcnt.p, mstart.p, nm, st);
-            ED_CUDA(cudaMemcpyAsync(&total, mstart.p + nm, 8, cudaMemcpyDeviceToHost, st));
-            ED_CUDA(cudaStreamSynchronize(st));
-            if (total >= (1ll << 31) || (size_t)total * 4 > room) return false;
-            room -= (size_t)total * 4;
-            out.mlist.alloc((size_t)total + 32);
-            out.mlstart.alloc((size_t)nm + 1);
-            k_split_move_lists<<<sms() * 16, 128, 0, st>>>(g, sword.p, sstart.p, out.ssize.p, rank.p, nc, out.nseg,
-                                                                 nullptr, mstart.p, out.mlist.p);
-            count_launch();
-            k_split_narrow<<<grid_of(nm + 1, 256), 256, 0, st>>>(mstart.p, nm + 1, out.mlstart.p);
-            count_launch();
-            ED_CUDA(cudaGetLastError());
-            ED_CUDA(cudaStreamSynchronize(st));
+            out.moves = 2 * (g.sbits - 1);
+            out.sbits = g.sbits;
+            const int64_t nt = (int64_t)np * out.moves;
+            counted(move, nt, [&](int64_t* cnt) {
+                k_split_moves<false><<<grid_of(nt, 128), 128, 0, st>>>(g, pword, np, by_word, cnt, nullptr, 0, nullptr, nullptr);
+            });
+            counted(mlist, (int64_t)nc * out.moves * out.nseg, [&](int64_t* cnt) {
+                k_split_move_lists<<<sms() * 16, 128, 0, st>>>(g, sword, sstart, out.ssize.p, rank, nc, out.nseg, cnt, nullptr, nullptr);
+            });
         }
-        for (int c : order)
-            for (int i = 0; i < P.size[c]; ++i)
-                for (int seg = 0; seg * kSegRows < S.size[c]; ++seg) task.push_back(make_int2(P.start[c] + i, seg));
+        ED_CUDA(cudaGetLastError());
+        return true;
     }
-    out.ntasks = (int)task.size();
-    upload(out.task, task, st);
-    ED_CUDA(cudaStreamSynchronize(st));   // the host vectors go out of scope
-    return true;
-}
+
+    size_t bytes() const
+    {
+        return (size_t)alpha.total * 16 + (size_t)move.total * (4 + 16 * (size_t)g.sbits) + (size_t)(list.total + mlist.total) * 4 +
+               (size_t)(alpha.n + move.n + list.n + mlist.n) * 4;
+    }
+    bool fits() const
+    {
+        return std::max(std::max(alpha.total, move.total), std::max(list.total, mlist.total)) < (1ll << 31);
+    }
+
+    void fill(int ea)
+    {
+        const int64_t na = alpha.n;
+        out.alpha.alloc((size_t)alpha.total + 1);
+        k_split_alpha<<<grid_of(na, 128), 128, 0, st>>>(g, pword, np, by_word, nullptr, alpha.start, ea, out.alpha.p);
+        count_launch();
+        starts(alpha, out.astart);
+        std::vector<int2> task;
+        std::vector<int> order(nc);
+        for (int c = 0; c < nc; ++c) order[c] = c;
+        std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return S.size[a] > S.size[b]; });   // longest first
+        if (G == kKeepParts) {
+            for (int c : order) {
+                const int m = S.size[c], words = P.size[c];
+                int width = 32;                       // lanes a word: the fewest that hold its segment
+                while (width > 2 && m <= width / 2) width /= 2;
+                const int per = 32 / width, rows = width == 32 ? 32 * kIdRows : width;
+                for (int i = 0; i < words; i += per)
+                    for (int seg = 0; seg * rows < m; ++seg)
+                        task.push_back(make_int2(P.start[c] + i, width | std::min(per, words - i) << 6 | seg << 12));
+            }
+        } else {
+            out.list.alloc((size_t)list.total + 1);
+            k_split_lists<<<sms() * 8, 256, 0, st>>>(g, sword, sstart, out.ssize.p, rank, nc, out.nseg, nullptr, list.start, out.list.p);
+            count_launch();
+            starts(list, out.lstart);
+            for (int c : order)
+                for (int i = 0; i < P.size[c]; ++i)
+                    for (int seg = 0; seg * kSegRows < S.size[c]; ++seg) task.push_back(make_int2(P.start[c] + i, seg));
+        }
+        if (moves) {
+            out.mbase.alloc((size_t)move.total + 1);
+            out.mweight.alloc((size_t)move.total * 2 * g.sbits + 1);
+            k_split_moves<true><<<grid_of(move.n * g.sbits, 128), 128, 0, st>>>(g, pword, np, by_word, nullptr, move.start, ea,
+                                                                               out.mbase.p, out.mweight.p);
+            count_launch();
+            starts(move, out.mstart);
+            out.mlist.alloc((size_t)mlist.total + 32);    // the product reads one block past a list
+            ED_CUDA(cudaMemsetAsync(out.mlist.p + mlist.total, 0, 32 * 4, st));
+            k_split_move_lists<<<sms() * 16, 128, 0, st>>>(g, sword, sstart, out.ssize.p, rank, nc, out.nseg, nullptr, mlist.start,
+                                                          out.mlist.p);
+            count_launch();
+            starts(mlist, out.mlstart);
+        }
+        ED_CUDA(cudaGetLastError());
+        out.ntasks = (int)task.size();
+        upload(out.task, task, st);     // pageable: read before the call returns
+    }
+};
 
 SplitArgs args_of(const SplitPlan& p, const SplitSide& s, const int64_t* x, const SplitPlan::Scratch& sc, double* y, int parts)
 {
@@ -954,16 +985,14 @@ SplitArgs args_of(const SplitPlan& p, const SplitSide& s, const int64_t* x, cons
     return g;
 }
 
-int exp_parts() { return sms() * 2; }
-
 template <bool NATIVE>
 void launch_pass(const SplitSide& s, const SplitArgs& g, cudaStream_t st)
 {
     if (s.ntasks == 0) return;
-    if (s.gammas == 1)
+    if (s.gammas == kKeepParts)
         k_split_keep<NATIVE><<<(s.ntasks + kWarps - 1) / kWarps, kThreads, 0, st>>>(g, s.ntasks);
     else
-        k_split_product<NATIVE><<<s.ntasks, kThreads, (size_t)kWarps * sizeof(Sum) * s.rows + sizeof(int4) * (s.moves + s.gammas - 1), st>>>(g);
+        k_split_product<NATIVE><<<s.ntasks, kThreads, (size_t)kWarps * sizeof(Sum) * s.rows + sizeof(int4) * (s.moves + s.gammas - kKeepParts), st>>>(g);
     count_launch();
 }
 
@@ -984,7 +1013,7 @@ std::unique_ptr<SplitPlan> split_build(const SplitSource& s, const double* diag,
     const int B0 = (int)wl.size(), B1 = (int)wh.size();
     if (B0 < 2 || B1 < 2 || B0 > kMaxSideBits || B1 > kMaxSideBits || n < 1 || n >= (1ll << 31)) return nullptr;
     if (max_row <= 0) max_row = s.N * (s.N - 1) / 2 * ((s.norb0 + s.norb1 + 1) / 2) + 1;
-    if (max_row > kMaxRow) return nullptr;
+    if (max_row > kFixMaxRow) return nullptr;
     int ea = 1;
     double wmax = 0.0;
     for (const HopTables* h : {&s.hop0, &s.hop1})
@@ -996,13 +1025,10 @@ std::unique_ptr<SplitPlan> split_build(const SplitSource& s, const double* diag,
     int span = 1;
     for (int w : wl) span += w;
     for (int w : wh) span += w;
-    std::vector<std::pair<int, uint32_t>> lw, hw;
-    enumerate_part(wl, s.N, s.N - B1, lw, span);
-    enumerate_part(wh, s.N, s.N - B0, hw, span);
     const int nkeys = (s.N + 1) * span;
     std::vector<int> lcount(nkeys, 0), hcount(nkeys, 0), lclass(nkeys, -1), hclass(nkeys, -1);
-    for (auto& e : lw) ++lcount[e.first];
-    for (auto& e : hw) ++hcount[e.first];
+    count_part(wl, s.N, span, lcount);
+    count_part(wh, s.N, span, hcount);
     PartWords L, H;
     int64_t rows = 0;
     for (int k = 0; k < nkeys; ++k) {
@@ -1022,15 +1048,15 @@ std::unique_ptr<SplitPlan> split_build(const SplitSource& s, const double* diag,
     }
     if (rows != n) return nullptr;
     for (auto* part : {&L, &H}) {
-        auto& src = part == &L ? lw : hw;
         auto& cls = part == &L ? lclass : hclass;
         std::vector<int> at = part->start;
         part->cls.resize(part->word.size());
-        for (auto& e : src)
-            if (cls[e.first] >= 0) {
-                part->cls[at[cls[e.first]]] = cls[e.first];
-                part->word[at[cls[e.first]]++] = e.second;
-            }
+        for_part(part == &L ? wl : wh, s.N, s.N - (part == &L ? B1 : B0), span, [&](int key, uint32_t word) {
+            const int c = cls[key];
+            if (c < 0) return;
+            part->cls[at[c]] = c;
+            part->word[at[c]++] = word;
+        });
     }
     const int nc = (int)L.start.size();
     std::vector<int> cbase(nc), tbase(L.word.size());
@@ -1044,70 +1070,57 @@ std::unique_ptr<SplitPlan> split_build(const SplitSource& s, const double* diag,
     auto p = std::make_unique<SplitPlan>();
     p->n = n;
     p->lists = s.levels == 1;
+    Arena tmp;
+    GenArgs gn{}, gt{};
+    std::vector<int> gamman, gammat;
+    for (int i = 0; i < kKeepParts; ++i) {
+        gamman.push_back(kKeep | i << 4);
+        gammat.push_back(kKeep | i << 4);
+    }
+    const double *w0 = tmp.put(s.hop0.w, st), *w1 = tmp.put(s.hop1.w, st);
+    const int *off0 = tmp.put(s.hop0.hop_off, st), *off1 = tmp.put(s.hop1.hop_off, st);
+    if (s.levels == 1) {
+        gn = GenArgs{B0, B1, 0, B0, 0, nullptr, s.norb0, w0, off0};
+        gt = GenArgs{0, B0, B0, B1, 0, nullptr, s.norb0, w0, off0};
+        for (int o = 0; o < B0 + B1; ++o)
+            for (int type : {kEmpty, kFill}) (o < B0 ? gamman : gammat).push_back(type | o << 4);
+    } else {
+        gn = GenArgs{0, B1, 0, B0, 0, nullptr, s.norb0, w0, off0};
+        gt = GenArgs{0, B0, 0, B1, 0, nullptr, s.norb1, w1, off1};
+    }
+    SideBuild bn{p->native, H, L, gn, gamman, s.levels == 1, tmp, st};
+    SideBuild bt{p->trans, L, H, gt, gammat, false, tmp, st};
+    if (!bn.count(nullptr) || !bt.count(&tbase)) return nullptr;
+    // the diagonal's exponent joins the weights'
+    const int parts = exp_parts();
+    int* part = tmp.take<int>((size_t)parts + 1);
+    k_fix_exp<<<parts, 256, 0, st>>>(diag, n, part);
+    count_launch();
+    std::vector<int> h(parts);
+    ED_CUDA(cudaMemcpyAsync(h.data(), part, (size_t)parts * 4, cudaMemcpyDeviceToHost, st));
+    ED_CUDA(cudaStreamSynchronize(st));
+    for (int e : h) ea = std::max(ea, e);
+    if (ea >= 2047) return nullptr;
+    // a row's high limb products fit 63 bits: |w| < ah 2^30 in units of the
+    // fixed point, |xh| <= 2^28 (always so where the diagonal, a sum over all
+    // pairs, is well above the single weights)
+    if ((double)max_row * (std::ldexp(wmax, 1050 - ea) + 1.0) >= std::ldexp(1.0, 34)) return nullptr;
+    p->ea = ea;
     size_t free_b = 0, total_b = 0;
     ED_CUDA(cudaMemGetInfo(&free_b, &total_b));
-    size_t room = free_b / 2;
-    if ((size_t)n * 56 > room) return nullptr;
-    room -= (size_t)n * 56;
-    // the diagonal's exponent joins the weights'
-    {
-        const int P = exp_parts();
-        DevBuf<int> part((size_t)P + 1);
-        k_fix_exp<<<P, 256, 0, st>>>(diag, n, part.p);
-        count_launch();
-        std::vector<int> h(P);
-        ED_CUDA(cudaMemcpyAsync(h.data(), part.p, (size_t)P * 4, cudaMemcpyDeviceToHost, st));
-        ED_CUDA(cudaStreamSynchronize(st));
-        for (int e : h) ea = std::max(ea, e);
-        if (ea >= 2047) return nullptr;
-        // a row's high limb products fit 63 bits: |w| < ah 2^30 in units of
-        // the fixed point, |xh| <= 2^28 (always so where the diagonal, a sum
-        // over all pairs, is well above the single weights)
-        if ((double)max_row * (std::ldexp(wmax, 1050 - ea) + 1.0) >= std::ldexp(1.0, 34)) return nullptr;
-        p->ea = ea;
-        p->diag.alloc((size_t)n);
-        ED_CUDA(cudaMemcpyAsync(part.p, &ea, sizeof(int), cudaMemcpyHostToDevice, st));
-        k_fix_conv<<<sms() * 4, 256, 0, st>>>(diag, n, part.p, 1, p->diag.p);
-        count_launch();
-        ED_CUDA(cudaStreamSynchronize(st));
-    }
-    DevBuf<double> w0, w1;
-    DevBuf<int> off0, off1;
-    upload(w0, s.hop0.w, st);
-    upload(off0, s.hop0.hop_off, st);
-    upload(w1, s.hop1.w, st);
-    upload(off1, s.hop1.hop_off, st);
-    GenArgs gn{}, gt{};
-    std::vector<int> gamman{kKeep}, gammat{kKeep};
-    if (s.levels == 1) {
-        gn = GenArgs{B0, B1, 0, B0, 0, nullptr, s.norb0, w0.p, off0.p};
-        gt = GenArgs{0, B0, B0, B1, 0, nullptr, s.norb0, w0.p, off0.p};
-        for (int o = 0; o < B0; ++o) {
-            gamman.push_back(kEmpty | o << 4);
-            gamman.push_back(kFill | o << 4);
-        }
-        for (int o = B0; o < B0 + B1; ++o) {
-            gammat.push_back(kEmpty | o << 4);
-            gammat.push_back(kFill | o << 4);
-        }
-    } else {
-        gn = GenArgs{0, B1, 0, B0, 0, nullptr, s.norb0, w0.p, off0.p};
-        gt = GenArgs{0, B0, 0, B1, 0, nullptr, s.norb1, w1.p, off1.p};
-    }
-    if (!build_side(p->native, H, L, gn, gamman, s.levels == 1, ea, nullptr, room, st)) return nullptr;
-    if (!build_side(p->trans, L, H, gt, gammat, false, ea, &tbase, room, st)) return nullptr;
-    {
-        DevBuf<int> pstart, psize, cb;
-        upload(pstart, H.start, st);
-        upload(psize, H.size, st);
-        upload(cb, cbase, st);
-        p->perm.alloc((size_t)n);
-        k_split_perm<<<sms() * 8, 256, 0, st>>>(p->native.pbase.p, p->native.pcls.p, pstart.p, psize.p, p->native.ssize.p,
-                                                cb.p, (int)H.word.size(), p->perm.p);
-        count_launch();
-        ED_CUDA(cudaGetLastError());
-        ED_CUDA(cudaStreamSynchronize(st));
-    }
+    if (!bn.fits() || !bt.fits() || (size_t)n * 56 + bn.bytes() + bt.bytes() > free_b / 2) return nullptr;
+    p->diag.alloc((size_t)n);
+    ED_CUDA(cudaMemcpyAsync(part, &ea, sizeof(int), cudaMemcpyHostToDevice, st));
+    k_fix_conv<<<sms() * 4, 256, 0, st>>>(diag, n, part, 1, p->diag.p);
+    count_launch();
+    bn.fill(ea);
+    bt.fill(ea);
+    p->perm.alloc((size_t)n);
+    k_split_perm<<<sms() * 8, 256, 0, st>>>(p->native.pbase.p, p->native.pcls.p, tmp.put(H.start, st), tmp.put(H.size, st),
+                                            p->native.ssize.p, tmp.put(cbase, st), (int)H.word.size(), p->perm.p);
+    count_launch();
+    ED_CUDA(cudaGetLastError());
+    ED_CUDA(cudaStreamSynchronize(st));   // the temporaries and the host vectors go
     return p;
 }
 

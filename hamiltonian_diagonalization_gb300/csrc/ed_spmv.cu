@@ -201,7 +201,6 @@ __global__ void __launch_bounds__(256) k_spmv_rows(const int64_t* __restrict__ r
 // elements keep the FP64 kernels.
 
 constexpr int kFixPartPerSm = 2;     // blocks of the exponent pass per SM
-constexpr int kFixMaxRow = 2048;     // |S| < 2048 * 2^116 = 2^127
 
 // The one-level row kernel on the fixed-point values: G lanes per row, each
 // lane one element in G, U elements' loads issued ahead of their
