@@ -7,6 +7,18 @@
 
 #include "ed_internal.h"
 
+namespace edgb {
+// A block product's operands in the integer product's fixed point: weights
+// [2 nhop][B] (each hop and its negative), diagonals [n][B], the exponent bound
+// of each Hamiltonian; and the scratch for X [n][B] with its bounds (the last
+// entry the largest of all).
+struct BlockFixed {
+    bool ready = false;
+    DevBuf<int64_t> w, diag, x;
+    DevBuf<int> ea, ex;
+};
+}  // namespace edgb
+
 struct ed_batch {
     int B = 0;                    // Hamiltonians
     int K = 0, N = 0;
@@ -27,6 +39,10 @@ struct ed_batch {
     // per CTA, hop values through L1 (1) or staged in shared memory (0)
     int tb = 32, unroll = 4, nt = 256, l1 = 1;
     int tuned = 0;                // 1 after batch_autotune: subsets get their own tuned tiles
+    int max_row = 0;              // most off-diagonal entries of a row
+    // the fixed-point operands of ed_batch_spmm, per (device, stream)
+    mutable std::mutex fix_mu;
+    mutable std::map<std::pair<int, cudaStream_t>, std::unique_ptr<edgb::BlockFixed>> fixed;
 };
 
 namespace edgb {

@@ -28,6 +28,7 @@
 #include <mutex>
 #include <vector>
 
+#include "ed_fixed.cuh"
 #include "ed_hop.cuh"
 #include "ed_lanczos.h"
 #include "ed_batch.h"
@@ -36,7 +37,7 @@ namespace edgb {
 
 namespace {
 
-constexpr uint16_t kCodeSign = 0x8000;
+// an element's code: hop << 1 | sign
 
 int sms_b() { return batch_sms(); }
 
@@ -56,7 +57,7 @@ __device__ __forceinline__ uint16_t hop_code(const HopView& hv, uint64_t in, uin
         par = hop_parity(out, c, d, a, b);
     }
     keep = hv.w[h] != 0.0;
-    return (uint16_t)((par ? kCodeSign : 0) | h);
+    return (uint16_t)(h << 1 | par);
 }
 
 // off-diagonal entries per row of the union pattern
@@ -211,11 +212,11 @@ __global__ void k_bdiag(const uint64_t* __restrict__ words, int64_t n, const dou
     }
 }
 
-// W with the element's fermionic sign applied: bit 15 of the code moved to the
+// W with the element's fermionic sign applied: bit 0 of the code moved to the
 // sign bit of the high word, an integer XOR that leaves the FP64 pipe to the FMAs.
 __device__ __forceinline__ double signed_w(double w, uint16_t code)
 {
-    return __hiloint2double(__double2hiint(w) ^ (int)((unsigned)(code & kCodeSign) << 16), __double2loint(w));
+    return __hiloint2double(__double2hiint(w) ^ (int)((unsigned)code << 31), __double2loint(w));
 }
 
 // Y[r][b] = diag[r][b] X[r][b] + sum_k sign_k W_b[h_k] X[col_k][b] for b in
@@ -225,8 +226,9 @@ template <int TB, int U, int NT>
 __global__ void __launch_bounds__(NT) k_bspmm(const int64_t* __restrict__ rowptr, const int32_t* __restrict__ col,
                                               const uint16_t* __restrict__ code, const double* __restrict__ w,
                                               int nhop, const double* __restrict__ diag, const double* __restrict__ X,
-                                              double* __restrict__ Y, int64_t n, int B)
+                                              double* __restrict__ Y, int64_t n, int B, const int* __restrict__ gate)
 {
+    if (gate && *gate < 2047) return;   // X is finite: Y is there already
     extern __shared__ double sw[];   // [nhop][TB]
     const int b0 = blockIdx.y * TB;
     for (int i = threadIdx.x; i < nhop * TB; i += NT) {
@@ -256,7 +258,7 @@ __global__ void __launch_bounds__(NT) k_bspmm(const int64_t* __restrict__ rowptr
 #pragma unroll
             for (int u = 0; u < U; ++u) {
                 if (k + u < e) {
-                    const double wv = signed_w(sw[(cd[u] & 0x7FFF) * TB + bl], cd[u]);
+                    const double wv = signed_w(sw[(cd[u] >> 1) * TB + bl], cd[u]);
                     if (u & 1) acc1 = fma(wv, xv[u], acc1);
                     else acc0 = fma(wv, xv[u], acc0);
                 }
@@ -276,8 +278,10 @@ template <int U, int TB>
 __global__ void __launch_bounds__(256) k_bspmm_warp(const int64_t* __restrict__ rowptr, const int32_t* __restrict__ col,
                                                     const uint16_t* __restrict__ code, const double* __restrict__ w,
                                                     const double* __restrict__ diag, const double* __restrict__ X,
-                                                    double* __restrict__ Y, int64_t n, int B)
+                                                    double* __restrict__ Y, int64_t n, int B,
+                                                    const int* __restrict__ gate)
 {
+    if (gate && *gate < 2047) return;   // X is finite: Y is there already
     constexpr int RPW = 32 / TB;
     const int lane = threadIdx.x & 31;
     const int b = blockIdx.y * TB + (lane % TB);
@@ -298,7 +302,7 @@ __global__ void __launch_bounds__(256) k_bspmm_warp(const int64_t* __restrict__ 
 #pragma unroll
             for (int u = 0; u < U; ++u) {
                 xv[u] = bv ? __ldg(X + (int64_t)c[u] * B + b) : 0.0;
-                wv[u] = bv ? __ldg(w + (int64_t)(cd[u] & 0x7FFF) * B + b) : 0.0;
+                wv[u] = bv ? __ldg(w + (int64_t)(cd[u] >> 1) * B + b) : 0.0;
             }
 #pragma unroll
             for (int u = 0; u < U; ++u) {
@@ -309,6 +313,124 @@ __global__ void __launch_bounds__(256) k_bspmm_warp(const int64_t* __restrict__ 
             }
         }
         if (bv) Y[r * B + b] = acc0 + acc1;
+    }
+}
+
+// ------------------------------------------------------ integer block product
+//
+// The block product in the stored products' exact fixed point (ed_fixed.cuh;
+// the bits of the single products), off the FP64 pipe: one FMA an element and Hamiltonian at 0.53e12 FMA/s is
+// what bound k_bspmm* (87 % of that pipe).  Each Hamiltonian has its own
+// exponent bounds, for its weights and diagonal (2046 at most) and for its
+// column of X.
+
+// Column maxima of the exponents of v [total / B][B] into exps[B], and over
+// all columns into exps[B] (zeroed by the caller).  blockDim.x is a multiple of B.
+__global__ void __launch_bounds__(256) k_bfix_exp(const double* __restrict__ v, int64_t total, int B, int* __restrict__ exps)
+{
+    extern __shared__ int se[];
+    for (int t = threadIdx.x; t < B; t += blockDim.x) se[t] = 1;
+    __syncthreads();
+    int m = 1;
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x)
+        m = max(m, fix_exp(v[i]));
+    atomicMax(&se[threadIdx.x % B], m);
+    __syncthreads();
+    for (int t = threadIdx.x; t < B; t += blockDim.x) {
+        atomicMax(exps + t, se[t]);
+        atomicMax(exps + B, se[t]);
+    }
+}
+
+// q = v in fixed point by column; with both, rows 2h and 2h + 1 of q are row h
+// of v and its negative.
+__global__ void __launch_bounds__(256) k_bfix_conv(const double* __restrict__ v, int64_t total, int B,
+                                                   const int* __restrict__ exps, int both, int64_t* __restrict__ q)
+{
+    const int E = exps[threadIdx.x % B];
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
+        if (both) {
+            const int64_t h = i / B, b = i - h * B;
+            q[2 * h * B + b] = fix_pair(v[i], E);
+            q[(2 * h + 1) * B + b] = fix_pair(-v[i], E);
+        } else {
+            q[i] = fix_pair(v[i], E);
+        }
+    }
+}
+
+// The eight elements at k (a multiple of 8) of a row whose elements are
+// [s, e), the ones outside dropped with MASK.
+template <bool MASK>
+__device__ __forceinline__ void bspmm_fix_block(const int32_t* __restrict__ col, const uint16_t* __restrict__ code,
+                                                const int2* __restrict__ w, const int2* __restrict__ X, unsigned B, unsigned b,
+                                                int64_t k, int64_t s, int64_t e, long long& p2, long long& p1, long long& p0)
+{
+    const int4 c0 = __ldg(reinterpret_cast<const int4*>(col + k)), c1 = __ldg(reinterpret_cast<const int4*>(col + k + 4));
+    const uint4 h = __ldg(reinterpret_cast<const uint4*>(code + k));
+    const unsigned c[8] = {(unsigned)c0.x, (unsigned)c0.y, (unsigned)c0.z, (unsigned)c0.w,
+                           (unsigned)c1.x, (unsigned)c1.y, (unsigned)c1.z, (unsigned)c1.w};
+    const unsigned hh[4] = {h.x, h.y, h.z, h.w};
+    const int lo = (int)(s - k), hi = (int)min(e - k, (int64_t)8);
+    int2 x[8], a[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+        const unsigned cd = (u & 1) ? hh[u / 2] >> 16 : hh[u / 2] & 0xFFFFu;
+        x[u] = __ldg(X + (c[u] * B + b));      // 32-bit indices: fewer address instructions
+        a[u] = __ldg(w + (cd * B + b));
+    }
+    if (MASK) {
+#pragma unroll
+        for (int u = 0; u < 8; ++u)
+            if (u < lo || u >= hi) a[u] = make_int2(0, 0);
+    }
+#pragma unroll
+    for (int u = 0; u < 8; ++u) fix_mac(a[u], x[u], p2, p1, p0);
+    const FixSum t = fix_carry(p2, p1, p0);
+    p2 = t.hi;
+    p1 = 0;
+    p0 = (long long)t.lo;
+}
+
+// TB lanes a row, lane = Hamiltonian: eight elements' columns and codes come
+// in three aligned broadcast loads, then each element takes one word of the
+// signed weight table [2 nhop][B] and one of X.  p2 / p0 carry the exact sum
+// p2 2^60 + p0 from block to block.  Measured on GB300, the passes over X
+// included, against the tuned FP64 tile: N=10, 2S=27 (4.6e7 entries), 32
+// Hamiltonians 1.57 ms / 2.67, 16 0.82 / 1.67, 5 0.45 / 0.67, 2 0.26 / 0.40;
+// N=9, 2S=24, 32 Hamiltonians 0.23 / 0.38, 2 0.058 / 0.066.  Bound by L2: 17
+// GB of X and weight rows a product at 10.9 TB/s (an L1 hit rate of 35 %;
+// blocks of 512 or 1024 threads, whose rows share more, run 1.54 and 1.58
+// ms, five blocks per SM 1.59).
+template <int TB>
+__global__ void __launch_bounds__(256, 4) k_bspmm_fix(const int64_t* __restrict__ rowptr, const int32_t* __restrict__ col,
+                                                      const uint16_t* __restrict__ code, const int2* __restrict__ w,
+                                                      const int2* __restrict__ diag, const int* __restrict__ ea,
+                                                      const int2* __restrict__ X, const int* __restrict__ ex,
+                                                      double* __restrict__ Y, int64_t n, int B)
+{
+    constexpr int RPW = 32 / TB;
+    const int lane = threadIdx.x & 31;
+    const int b = blockIdx.y * TB + (lane % TB);
+    const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
+    const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
+    if (b >= B) return;
+    const int e_x = ex[b];
+    for (int64_t r = warp * RPW + lane / TB; r < n; r += nwarps * RPW) {
+        const int64_t s = rowptr[r], e = rowptr[r + 1];
+        long long p2 = 0, p1 = 0, p0 = 0;
+        int64_t k = s & ~7ll;
+        if (k < s && k < e) {
+            bspmm_fix_block<true>(col, code, w, X, (unsigned)B, (unsigned)b, k, s, e, p2, p1, p0);
+            k += 8;
+        }
+        for (; k + 8 <= e; k += 8) bspmm_fix_block<false>(col, code, w, X, (unsigned)B, (unsigned)b, k, s, e, p2, p1, p0);
+        if (k < e) bspmm_fix_block<true>(col, code, w, X, (unsigned)B, (unsigned)b, k, s, e, p2, p1, p0);
+        const int2 d = __ldg(diag + r * B + b), x = __ldg(X + r * B + b);
+        long long q2 = 0, q1 = 0, q0 = 0;
+        fix_mac(d, x, q2, q1, q0);
+        const __int128 S = ((__int128)p2 << 60) + (__int128)(unsigned long long)p0 + fix_combine(q2, q1, q0);
+        Y[r * B + b] = e_x < 2047 ? round_i128(S, ea[b] + e_x - 2160) : __longlong_as_double(0x7FF8000000000000ll);
     }
 }
 
@@ -681,6 +803,7 @@ void batch_create(ed_batch& bt, const ed_basis& basis, int K, int B, const uint1
     ED_CUDA(cudaMemcpyAsync(&bt.nnz, bt.rowptr.p + n, 8, cudaMemcpyDeviceToHost, st));
     const int64_t maxrow = reduce_max_i64_host(rowlen.p, n, st);
     ED_CUDA(cudaStreamSynchronize(st));
+    bt.max_row = (int)maxrow;
     bt.col.alloc((size_t)bt.nnz + kCrsPad);
     bt.code.alloc((size_t)bt.nnz + kCrsPad);
     ED_CUDA(cudaMemsetAsync(bt.col.p + bt.nnz, 0, kCrsPad * 4, st));
@@ -712,7 +835,7 @@ constexpr size_t kSmemOptIn = 227 * 1024;   // dynamic shared memory per CTA on 
 
 template <int TB, int U, int NT>
 void launch_bspmm(const ed_batch& bt, const BlockOperands& o, const double* X, double* Y, int64_t rows,
-                  cudaStream_t st)
+                  const int* gate, cudaStream_t st)
 {
     const size_t smem = (size_t)bt.nhop * TB * 8;
     static_assert(U <= kCrsPad, "batch overruns the padding");
@@ -723,18 +846,18 @@ void launch_bspmm(const ed_batch& bt, const BlockOperands& o, const double* X, d
     ED_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_bspmm<TB, U, NT>, NT, smem));
     dim3 grid((unsigned)(sms_b() * std::max(1, per_sm)), (unsigned)((o.B + TB - 1) / TB));
     k_bspmm<TB, U, NT><<<grid, NT, smem, st>>>(bt.rowptr.p, bt.col.p, bt.code.p, o.w, bt.nhop, o.diag, X, Y, rows,
-                                                 o.B);
+                                                 o.B, gate);
     count_launch();
     ED_CUDA(cudaGetLastError());
 }
 
 template <int U, int TB>
 void launch_bspmm_warp(const ed_batch& bt, const BlockOperands& o, const double* X, double* Y, int64_t rows,
-                       cudaStream_t st)
+                       const int* gate, cudaStream_t st)
 {
     static_assert(U <= kCrsPad, "batch overruns the padding");
     dim3 grid((unsigned)(sms_b() * 8), (unsigned)((o.B + TB - 1) / TB));
-    k_bspmm_warp<U, TB><<<grid, 256, 0, st>>>(bt.rowptr.p, bt.col.p, bt.code.p, o.w, o.diag, X, Y, rows, o.B);
+    k_bspmm_warp<U, TB><<<grid, 256, 0, st>>>(bt.rowptr.p, bt.col.p, bt.code.p, o.w, o.diag, X, Y, rows, o.B, gate);
     count_launch();
     ED_CUDA(cudaGetLastError());
 }
@@ -743,18 +866,18 @@ void launch_bspmm_warp(const ed_batch& bt, const BlockOperands& o, const double*
 // through L1 (TB 16 or 32 lanes per row); l1 = 0 stages the tile's hop table
 // in shared memory (TB 4, 8 or 16 Hamiltonians, 256 or 1024 threads).
 void bspmm_variant(const ed_batch& bt, const BlockOperands& o, int tb, int u, int nt, int l1, const double* X,
-                   double* Y, int64_t rows, cudaStream_t st)
+                   double* Y, int64_t rows, const int* gate, cudaStream_t st)
 {
     if (l1) {
         if (tb == 32)
-            u == 4 ? launch_bspmm_warp<4, 32>(bt, o, X, Y, rows, st) : launch_bspmm_warp<8, 32>(bt, o, X, Y, rows, st);
+            u == 4 ? launch_bspmm_warp<4, 32>(bt, o, X, Y, rows, gate, st) : launch_bspmm_warp<8, 32>(bt, o, X, Y, rows, gate, st);
         else
-            u == 4 ? launch_bspmm_warp<4, 16>(bt, o, X, Y, rows, st) : launch_bspmm_warp<8, 16>(bt, o, X, Y, rows, st);
+            u == 4 ? launch_bspmm_warp<4, 16>(bt, o, X, Y, rows, gate, st) : launch_bspmm_warp<8, 16>(bt, o, X, Y, rows, gate, st);
         return;
     }
 #define ED_BSPMM_CASE(TB_, U_, NT_)                                                   \
     if (tb == TB_ && u == U_ && nt == NT_) {                                          \
-        launch_bspmm<TB_, U_, NT_>(bt, o, X, Y, rows, st);                            \
+        launch_bspmm<TB_, U_, NT_>(bt, o, X, Y, rows, gate, st);                            \
         return;                                                                       \
     }
     ED_BSPMM_CASE(4, 4, 256) ED_BSPMM_CASE(4, 8, 256) ED_BSPMM_CASE(8, 4, 256) ED_BSPMM_CASE(8, 8, 256)
@@ -797,10 +920,115 @@ BlockOperands gather_operands(const ed_batch& bt, const int* sel_host, int nsel,
     return {w.p, diag.p, nsel};
 }
 
+namespace {
+
+// threads of a block whose stride keeps each thread in one column
+int column_threads(int B) { return 256 / B * B; }
+int column_grid(int64_t total, int B)
+{
+    return (int)std::max<int64_t>(1, std::min<int64_t>(batch_sms() * 8, (total + column_threads(B) - 1) / column_threads(B)));
+}
+
+template <int TB>
+void launch_bspmm_fix(const ed_batch& bt, const BlockFixed& f, int B, double* Y, cudaStream_t st)
+{
+    const int64_t rows_per_block = 256 / TB;
+    dim3 grid((unsigned)std::max<int64_t>(1, std::min<int64_t>(sms_b() * 16, (bt.n + rows_per_block - 1) / rows_per_block)),
+              (unsigned)((B + TB - 1) / TB));
+    k_bspmm_fix<TB><<<grid, 256, 0, st>>>(bt.rowptr.p, bt.col.p, bt.code.p, reinterpret_cast<const int2*>(f.w.p),
+                                          reinterpret_cast<const int2*>(f.diag.p), f.ea.p,
+                                          reinterpret_cast<const int2*>(f.x.p), f.ex.p, Y, bt.n, B);
+    count_launch();
+}
+
+}  // namespace
+
+// The operands' fixed-point form; false where the exact sums do not apply
+// (a weight or diagonal entry that is not finite, a row of more than 2048
+// elements, weights so near the diagonal's size that a row's high limb
+// products could pass 2^62).  Waits for the stream.
+bool fix_operands(const ed_batch& bt, const BlockOperands& o, BlockFixed& f, cudaStream_t st)
+{
+    f.ready = false;
+    const int B = o.B;
+    if (bt.max_row > kFixMaxRow || bt.n * B >= (1ll << 32)) return false;
+    const int64_t nw = (int64_t)bt.nhop * B, nd = bt.n * B;
+    f.ea.alloc_at_least(B + 1);
+    f.ex.alloc_at_least(B + 1);
+    f.w.alloc_at_least((size_t)(2 * nw));
+    f.diag.alloc_at_least((size_t)nd);
+    f.x.alloc_at_least((size_t)nd);
+    DevBuf<int> ew(B + 1);
+    ED_CUDA(cudaMemsetAsync(f.ea.p, 0, (size_t)(B + 1) * 4, st));
+    ED_CUDA(cudaMemsetAsync(ew.p, 0, (size_t)(B + 1) * 4, st));
+    const int T = column_threads(B);
+    k_bfix_exp<<<column_grid(nw, B), T, B * 4, st>>>(o.w, nw, B, f.ea.p); count_launch();
+    ED_CUDA(cudaMemcpyAsync(ew.p, f.ea.p, (size_t)(B + 1) * 4, cudaMemcpyDeviceToDevice, st));
+    k_bfix_exp<<<column_grid(nd, B), T, B * 4, st>>>(o.diag, nd, B, f.ea.p); count_launch();
+    std::vector<int> ea(B + 1), eh(B + 1);
+    ED_CUDA(cudaMemcpyAsync(ea.data(), f.ea.p, (size_t)(B + 1) * 4, cudaMemcpyDeviceToHost, st));
+    ED_CUDA(cudaMemcpyAsync(eh.data(), ew.p, (size_t)(B + 1) * 4, cudaMemcpyDeviceToHost, st));
+    ED_CUDA(cudaStreamSynchronize(st));
+    for (int b = 0; b < B; ++b) {
+        // |w| < 2^(eh - 1022), so its high limb is below 2^(28 + eh - ea) (and 1), x's below 2^28
+        const double high = std::ldexp(1.0, 28 + eh[b] - ea[b]) + 1.0;
+        if (ea[b] >= 2047 || (double)bt.max_row * high >= std::ldexp(1.0, 34)) return false;
+    }
+    k_bfix_conv<<<column_grid(nw, B), T, 0, st>>>(o.w, nw, B, f.ea.p, 1, f.w.p); count_launch();
+    k_bfix_conv<<<column_grid(nd, B), T, 0, st>>>(o.diag, nd, B, f.ea.p, 0, f.diag.p); count_launch();
+    ED_CUDA(cudaGetLastError());
+    ED_CUDA(cudaStreamSynchronize(st));   // ew goes
+    f.ready = true;
+    return true;
+}
+
+// Y = H X through the fixed-point operands f of o; where X is not finite the
+// FP64 kernel of tile t follows and its answer stands.
+void fixed_block_product(const ed_batch& bt, const BlockOperands& o, const BlockFixed& f, const std::array<int, 4>& t,
+                         const double* X, double* Y, cudaStream_t st)
+{
+    const int B = o.B, T = column_threads(B);
+    const int64_t total = bt.n * B;
+    ED_CUDA(cudaMemsetAsync(f.ex.p, 0, (size_t)(B + 1) * 4, st));
+    k_bfix_exp<<<column_grid(total, B), T, B * 4, st>>>(X, total, B, f.ex.p); count_launch();
+    k_bfix_conv<<<column_grid(total, B), T, 0, st>>>(X, total, B, f.ex.p, 0, f.x.p); count_launch();
+    if (B > 16) launch_bspmm_fix<32>(bt, f, B, Y, st);
+    else if (B > 8) launch_bspmm_fix<16>(bt, f, B, Y, st);
+    else if (B > 4) launch_bspmm_fix<8>(bt, f, B, Y, st);
+    else launch_bspmm_fix<4>(bt, f, B, Y, st);
+    ED_CUDA(cudaGetLastError());
+    bspmm_variant(bt, o, t[0], t[1], t[2], t[3], X, Y, bt.n, f.ex.p + B, st);
+}
+
+namespace {
+
+// The whole batch's fixed-point operands with this stream's scratch for X,
+// made when missing and not capturing; null for a part of the batch or where
+// they do not apply.
+BlockFixed* batch_fixed(const ed_batch& bt, const BlockOperands& o, cudaStream_t st)
+{
+    if (o.w != bt.w.p) return nullptr;
+    int dev = 0;
+    ED_CUDA(cudaGetDevice(&dev));
+    const std::pair<int, cudaStream_t> key(dev, st);
+    std::lock_guard<std::mutex> lk(bt.fix_mu);
+    auto it = bt.fixed.find(key);
+    if (it != bt.fixed.end()) return it->second->ready ? it->second.get() : nullptr;
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    ED_CUDA(cudaStreamIsCapturing(st, &cs));
+    if (cs != cudaStreamCaptureStatusNone) return nullptr;
+    auto f = std::make_unique<BlockFixed>();
+    fix_operands(bt, o, *f, st);
+    return (bt.fixed[key] = std::move(f))->ready ? bt.fixed[key].get() : nullptr;
+}
+
+}  // namespace
+
 void batch_block_product(const ed_batch& bt, const BlockOperands& o, const double* X, double* Y, cudaStream_t st)
 {
     const std::array<int, 4> t = batch_tile(bt, o, st);
-    bspmm_variant(bt, o, t[0], t[1], t[2], t[3], X, Y, bt.n, st);
+    if (BlockFixed* f = batch_fixed(bt, o, st)) fixed_block_product(bt, o, *f, t, X, Y, st);
+    else bspmm_variant(bt, o, t[0], t[1], t[2], t[3], X, Y, bt.n, nullptr, st);
 }
 
 void batch_spmm(const ed_batch& bt, const double* X, double* Y, cudaStream_t st)
@@ -890,9 +1118,9 @@ std::array<int, 4> tune_tile(const ed_batch& bt, const BlockOperands& o, cudaStr
         for (int u : {4, 8}) cands.push_back({tb, u, 256, 1});
     }
     for (const auto& c : cands) {
-        bspmm_variant(bt, o, c[0], c[1], c[2], c[3], X.p, Y.p, rows, st);
+        bspmm_variant(bt, o, c[0], c[1], c[2], c[3], X.p, Y.p, rows, nullptr, st);
         ED_CUDA(cudaEventRecord(a, st));
-        for (int r = 0; r < 3; ++r) bspmm_variant(bt, o, c[0], c[1], c[2], c[3], X.p, Y.p, rows, st);
+        for (int r = 0; r < 3; ++r) bspmm_variant(bt, o, c[0], c[1], c[2], c[3], X.p, Y.p, rows, nullptr, st);
         ED_CUDA(cudaEventRecord(b, st));
         ED_CUDA(cudaEventSynchronize(b));
         float ms = 0.f;
@@ -990,6 +1218,8 @@ void batch_solve(const ed_batch& bt, const int* sel, int nsel, const ed_lanczos_
     const BlockOperands ops0 = sel ? gather_operands(bt, sel, nsel, wsel, dsel, st) : full_operands(bt);
     BlockOperands ops = ops0;
     std::array<int, 4> tile = batch_tile(bt, ops, st);
+    BlockFixed fixed;
+    fix_operands(bt, ops, fixed, st);
     int64_t vs = vs0;
 
     auto grid_for = [&](int64_t work) { return (int)std::max<int64_t>(1, std::min<int64_t>(sms_b() * 8, (work + 255) / 256)); };
@@ -1064,7 +1294,8 @@ void batch_solve(const ed_batch& bt, const int* sel, int nsel, const ed_lanczos_
             const bool first = (j == k);
             if (capturing) ED_CUDA(cudaEventRecordWithFlags(ev[2 * j], st, cudaEventRecordExternal));
             else ED_CUDA(cudaEventRecord(ev[2 * j], st));
-            bspmm_variant(bt, ops, tile[0], tile[1], tile[2], tile[3], vj, w, n, st);
+            if (fixed.ready) fixed_block_product(bt, ops, fixed, tile, vj, w, st);
+            else bspmm_variant(bt, ops, tile[0], tile[1], tile[2], tile[3], vj, w, n, nullptr, st);
             if (capturing) ED_CUDA(cudaEventRecordWithFlags(ev[2 * j + 1], st, cudaEventRecordExternal));
             else ED_CUDA(cudaEventRecord(ev[2 * j + 1], st));
             if (!first) {
@@ -1240,6 +1471,7 @@ void batch_solve(const ed_batch& bt, const int* sel, int nsel, const ed_lanczos_
             ED_CUDA(cudaGetLastError());
             ops = {wc[nxt].p, dc[nxt].p, Bn};
             tile = batch_tile(bt, ops, st);
+            fix_operands(bt, ops, fixed, st);
             std::vector<int> no(Bn);
             for (int q = 0; q < Bn; ++q) no[q] = orig[live[q]];
             orig = no;

@@ -128,7 +128,7 @@ __global__ void k_sub_store(const double* __restrict__ u, int64_t n, double s, d
 
 __device__ __forceinline__ double signed_hop(double w, uint16_t code)
 {
-    return __longlong_as_double(__double_as_longlong(w) ^ ((long long)(code & 0x8000u) << 48));
+    return __longlong_as_double(__double_as_longlong(w) ^ ((long long)code << 63));
 }
 
 // Y[r][j] = H_b X[r][j] for j < ncols (X, Y row-major with leading dimensions
@@ -156,7 +156,7 @@ __global__ void __launch_bounds__(256) k_sub_apply(const int64_t* __restrict__ r
             for (int t = 0; t < U; ++t) {
                 c[t] = __ldg(col + k + t);
                 const uint16_t cd = __ldg(code + k + t);
-                wv[t] = signed_hop(__ldg(w + (int64_t)(cd & 0x7FFF) * B + b), cd);
+                wv[t] = signed_hop(__ldg(w + (int64_t)(cd >> 1) * B + b), cd);
             }
 #pragma unroll
             for (int t = 0; t < U; ++t) xv[t] = jv ? __ldg(X + (int64_t)c[t] * ldx + j) : 0.0;
