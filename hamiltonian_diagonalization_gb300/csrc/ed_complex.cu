@@ -281,8 +281,10 @@ __global__ void __launch_bounds__(kCThreads) k_clocal(const double2* __restrict_
                                                       int64_t n, double* __restrict__ part,
                                                       unsigned int* __restrict__ counter, double* __restrict__ coefcol,
                                                       int j, const double* __restrict__ beta_prev,
-                                                      double* __restrict__ hv2, const int* __restrict__ stop)
+                                                      double* __restrict__ hv2, const int* __restrict__ stop,
+                                                      unsigned long long* __restrict__ ended)
 {
+    if (blockIdx.x == 0) stamp(ended);
     if (*stop) return;
     __shared__ double red[kCThreads / 32];
     int64_t r0, r1;
@@ -326,8 +328,10 @@ __global__ void __launch_bounds__(kCThreads) k_cmdot(const double2* __restrict__
                                                      const double* __restrict__ beta_prev, double* __restrict__ part,
                                                      unsigned int* __restrict__ counter, double2* __restrict__ c,
                                                      double* __restrict__ coefcol, double* __restrict__ before,
-                                                     const int* __restrict__ run, const int* __restrict__ stop)
+                                                     const int* __restrict__ run, const int* __restrict__ stop,
+                                                     unsigned long long* __restrict__ ended)
 {
+    if (blockIdx.x == 0) stamp(ended);
     if ((run && !*run) || (stop && *stop)) return;
     extern __shared__ double2 csw[];
     const int64_t r0 = (int64_t)blockIdx.x * R;
@@ -489,16 +493,19 @@ __global__ void __launch_bounds__(kCThreads) k_cupd(const double2* __restrict__ 
 
 // w /= *beta unless the cycle stopped.
 __global__ void __launch_bounds__(kCThreads) k_cscale_dev(double2* __restrict__ w, int64_t n,
-                                                          const double* __restrict__ beta, const int* __restrict__ stop)
+                                                          const double* __restrict__ beta, const int* __restrict__ stop,
+                                                          unsigned long long* __restrict__ started)
 {
-    if (*stop) return;
-    const double inv = 1.0 / *beta;
-    for (int64_t r = blockIdx.x * (int64_t)kCThreads + threadIdx.x; r < n; r += (int64_t)gridDim.x * kCThreads) {
-        double2 a = w[r];
-        a.x *= inv;
-        a.y *= inv;
-        w[r] = a;
+    if (!*stop) {
+        const double inv = 1.0 / *beta;
+        for (int64_t r = blockIdx.x * (int64_t)kCThreads + threadIdx.x; r < n; r += (int64_t)gridDim.x * kCThreads) {
+            double2 a = w[r];
+            a.x *= inv;
+            a.y *= inv;
+            w[r] = a;
+        }
     }
+    stamp(started);
 }
 
 __global__ void __launch_bounds__(kCThreads) k_cnorm2(const double2* __restrict__ w, int64_t n, double* __restrict__ part)
@@ -579,20 +586,19 @@ struct CWork {
     DevBuf<unsigned int> counters;
 
     void mdot(const double2* V, int J, double2* w, int local, const double* alpha, const double* beta_prev,
-              double* coefcol, double* before, const int* run, const int* stop, cudaStream_t st)
+              double* coefcol, double* before, const int* run, const int* stop, cudaStream_t st,
+              unsigned long long* ended = nullptr)
     {
-        k_cmdot<<<nbm, kCThreads, (size_t)R * 16, st>>>(V, n, R, J, w, local, alpha, beta_prev, part.p,
+        launch(k_cmdot, nbm, kCThreads, (size_t)R * 16, st, V, n, R, J, w, local, alpha, beta_prev, part.p,
                                                         counters.p + 1, reinterpret_cast<double2*>(c.p), coefcol,
-                                                        before, run, stop);
-        count_launch();
+                                                        before, run, stop, ended);
     }
     void update(const double2* V, int J, double2* w, int mode, int force2, const double* before, int* need2,
                 double* b, const double* ref2, int j, const int* run, int* stop, cudaStream_t st)
     {
-        k_cupd<<<nb, kCThreads, (size_t)J * 16, st>>>(V, n, J, reinterpret_cast<const double2*>(c.p), w, npart.p,
+        launch(k_cupd, nb, kCThreads, (size_t)J * 16, st, V, n, J, reinterpret_cast<const double2*>(c.p), w, npart.p,
                                                       counters.p + 2, mode, force2, before, need2, b, ref2, j, run,
                                                       stop);
-        count_launch();
     }
 };
 
@@ -842,10 +848,8 @@ void cfix_build(const ed_ccrs& a, cudaStream_t st)
     DevBuf<int> part((size_t)P + 1);
     fq->val.alloc(2 * (size_t)(a.nnz + kCrsPad));
     ED_CUDA(cudaMemsetAsync(fq->val.p + 2 * a.nnz, 0, (size_t)kCrsPad * 16, st));
-    k_fix_exp<<<P, 256, 0, st>>>(a.val.p, 2 * a.nnz, part.p);
-    count_launch();
-    k_fix_conv<<<csms() * 8, 256, 0, st>>>(a.val.p, 2 * a.nnz, part.p, P, fq->val.p);
-    count_launch();
+    launch(k_fix_exp, P, 256, 0, st, a.val.p, 2 * a.nnz, part.p);
+    launch(k_fix_conv, csms() * 8, 256, 0, st, a.val.p, 2 * a.nnz, part.p, P, fq->val.p);
     ED_CUDA(cudaGetLastError());
     int ea = 1;
     ED_CUDA(cudaMemcpyAsync(&ea, part.p + P, sizeof(int), cudaMemcpyDeviceToHost, st));
@@ -887,10 +891,7 @@ void cfix_launch(const ed_ccrs& a, const double* x, double* y, cudaStream_t st)
     const ed_fixq& f = *a.fixq;
     ed_fixq::Scratch& sc = *cfix_scratch(a, st);
     const int P = cfix_parts();
-    k_fix_exp<<<P, 256, 0, st>>>(x, 2 * a.n, sc.part.p);
-    count_launch();
-    k_fix_conv<<<csms() * 4, 256, 0, st>>>(x, 2 * a.n, sc.part.p, P, sc.xq.p);
-    count_launch();
+    fix_convert(x, 2 * a.n, sc.part.p, P, csms() * 4, sc.xq.p, st);
     const double avg = (double)a.nnz / (double)a.n;
     const int4* A = reinterpret_cast<const int4*>(f.val.p);
     const int4* X = reinterpret_cast<const int4*>(sc.xq.p);
@@ -899,9 +900,8 @@ void cfix_launch(const ed_ccrs& a, const double* x, double* y, cudaStream_t st)
     // (GB300, N=10 on 5x6: 1.363 ms; 92 registers and two CTAs 1.77, 2
     // ahead 2.69, 16 lanes 2.72, 48 registers with spills 1.62; the FP64
     // kernel 2.31)
-    if (avg >= 48) k_cspmv_fix<8, 4, 4><<<csms() * 8, kCThreads, 0, st>>>(a.rowptr.p, a.col.p, A, X, sc.part.p + P, f.ea, yy, a.n);
-    else k_cspmv_fix<4, 4, 4><<<csms() * 8, kCThreads, 0, st>>>(a.rowptr.p, a.col.p, A, X, sc.part.p + P, f.ea, yy, a.n);
-    count_launch();
+    if (avg >= 48) launch(k_cspmv_fix<8, 4, 4>, csms() * 8, kCThreads, 0, st, a.rowptr.p, a.col.p, A, X, sc.part.p + P, f.ea, yy, a.n);
+    else launch(k_cspmv_fix<4, 4, 4>, csms() * 8, kCThreads, 0, st, a.rowptr.p, a.col.p, A, X, sc.part.p + P, f.ea, yy, a.n);
     ED_CUDA(cudaGetLastError());
 }
 
@@ -1000,13 +1000,15 @@ void clanczos_solve(const ed_ccrs& a, const ed_lanczos_params& p, const double* 
     CWork cw;
     cw.n = n;
     cw.m = m;
-    cw.nb = (int)std::max<int64_t>(1, std::min<int64_t>(nsm * 4, n / 1024));
-    // multi-dot slices: three blocks per SM, 512 to 6144 rows (96 KB of
+    // as the real solver's
+    const bool small = n < 16384;
+    cw.nb = (int)std::max<int64_t>(1, std::min<int64_t>(nsm * 4, n / (small ? 128 : 256)));
+    // multi-dot slices: three blocks per SM, 256 (128 in a small sector) to 6144 rows (96 KB of
     // shared memory) a block, a multiple of 128
     {
         int64_t nbt = (int64_t)nsm * 3, R = 0;
         for (;;) {
-            R = std::max<int64_t>(512, ((n + nbt - 1) / nbt + 127) / 128 * 128);
+            R = std::max<int64_t>(small ? 128 : 256, ((n + nbt - 1) / nbt + 127) / 128 * 128);
             if (R <= 6144) break;
             nbt += nsm;
         }
@@ -1036,12 +1038,10 @@ void clanczos_solve(const ed_ccrs& a, const ed_lanczos_params& p, const double* 
     }
     corthonormalise(cw, col(Vb, 0), 0, st);
 
-    std::vector<cudaEvent_t> ev(2 * (m + 1), nullptr);
-    for (auto& e : ev) ED_CUDA(cudaEventCreate(&e));
-    struct EvGuard {
-        std::vector<cudaEvent_t>& v;
-        ~EvGuard() { for (auto e : v) if (e) cudaEventDestroy(e); }
-    } evguard{ev};
+    // start and end of each step's product
+    DevBuf<unsigned long long> clock(2 * (size_t)(m + 1));
+    ED_CUDA(cudaMemsetAsync(clock.p, 0, clock.bytes(), st));
+    std::vector<unsigned long long> clock_h(2 * (size_t)(m + 1));
 
     // One restart cycle, steps k..m-1, all on the device (the real solver's
     // scheme): the step scalars stay in device memory, the second
@@ -1049,45 +1049,45 @@ void clanczos_solve(const ed_ccrs& a, const ed_lanczos_params& p, const double* 
     // the cycle is replayed as one CUDA graph.
     int* need2 = cw.flags.p;
     int* stop = cw.flags.p + 1;
-    auto enqueue_cycle = [&](double2* V, int k, bool capturing) {
-        ED_CUDA(cudaMemsetAsync(cw.flags.p, 0, 2 * sizeof(int), st));
-        ED_CUDA(cudaMemsetAsync(cw.coef.p + (size_t)k * (m + 1), 0, (size_t)(m - k) * (m + 1) * 8, st));
+    auto enqueue_cycle = [&](double2* V, int k) {
+        const int64_t coefs = (int64_t)(m - k) * (m + 1);
+        launch(k_cycle_begin, (unsigned)std::min<int64_t>(64, (coefs + 255) / 256), 256, 0, st, cw.coef.p + (size_t)k * (m + 1), coefs,
+                   cw.flags.p, 2, clock.p + 2 * k);
         for (int j = k; j < m; ++j) {
             double2* vj = V + (int64_t)j * n;
             double2* w = V + (int64_t)(j + 1) * n;
             double* coefcol = cw.coef.p + (size_t)j * (m + 1);
             const bool first = (j == k);
-            if (capturing) ED_CUDA(cudaEventRecordWithFlags(ev[2 * j], st, cudaEventRecordExternal));
-            else ED_CUDA(cudaEventRecord(ev[2 * j], st));
             cspmv(a, reinterpret_cast<const double*>(vj), reinterpret_cast<double*>(w), st);
-            if (capturing) ED_CUDA(cudaEventRecordWithFlags(ev[2 * j + 1], st, cudaEventRecordExternal));
-            else ED_CUDA(cudaEventRecord(ev[2 * j + 1], st));
+            unsigned long long* ended = clock.p + 2 * j + 1;
             if (!first) {
-                k_clocal<<<cw.nb, kCThreads, 0, st>>>(vj, w, n, cw.part.p, cw.counters.p, coefcol, j,
-                                                      cw.beta.p + (j - 1), cw.scal.p + 1, stop);
-                count_launch();
+                launch(k_clocal, cw.nb, kCThreads, 0, st, vj, w, n, cw.part.p, cw.counters.p, coefcol, j,
+                                                      cw.beta.p + (j - 1), cw.scal.p + 1, stop, ended);
             }
             const int J = j + 1;
             const double* ref2 = first ? cw.scal.p : cw.scal.p + 1;
             cw.mdot(V, J, w, first ? 0 : 1, first ? nullptr : coefcol + j, first ? nullptr : cw.beta.p + (j - 1),
-                    coefcol, cw.scal.p, nullptr, stop, st);
+                    coefcol, cw.scal.p, nullptr, stop, st, first ? ended : nullptr);
             cw.update(V, J, w, 1, first ? 1 : 0, cw.scal.p, need2, cw.beta.p + j, ref2, j, nullptr, stop, st);
             cw.mdot(V, J, w, 0, nullptr, nullptr, coefcol, cw.scal.p + 2, need2, stop, st);
             cw.update(V, J, w, 2, 0, nullptr, nullptr, cw.beta.p + j, ref2, j, need2, stop, st);
-            k_cscale_dev<<<cw.nb, kCThreads, 0, st>>>(w, n, cw.beta.p + j, stop);
-            count_launch();
+            launch(k_cscale_dev, cw.nb, kCThreads, 0, st, w, n, cw.beta.p + j, stop, clock.p + 2 * (j + 1));
             ED_CUDA(cudaGetLastError());
         }
     };
     CycleGraphs cache;
     auto run_cycle = [&](int k) {
         double2* V = col(Vb, 0);
+        if (k == 0) {    // the first cycle runs once: a graph of it would cost more than its launches
+            enqueue_cycle(V, k);
+            return;
+        }
         CycleGraphs::Entry* g = cache.find(k, Vb.p);
         if (!g) {
             const uint64_t c0 = launch_count();
             ED_CUDA(cudaStreamBeginCapture(st, cudaStreamCaptureModeRelaxed));
             try {
-                enqueue_cycle(V, k, true);
+                enqueue_cycle(V, k);
             } catch (...) {
                 cudaGraph_t broken = nullptr;
                 cudaStreamEndCapture(st, &broken);
@@ -1113,7 +1113,7 @@ void clanczos_solve(const ed_ccrs& a, const ed_lanczos_params& p, const double* 
     std::vector<double> theta, Y, prev_theta;
     int k = 0, m_eff = m;
     bool converged = false;
-    double spmv_ms = 0.0;
+    double spmv_ns = 0.0;
     for (;;) {
         run_cycle(k);
         inf.matvecs += m - k;
@@ -1121,12 +1121,9 @@ void clanczos_solve(const ed_ccrs& a, const ed_lanczos_params& p, const double* 
         ED_CUDA(cudaMemcpyAsync(&hstop, stop, sizeof(int), cudaMemcpyDeviceToHost, st));
         ED_CUDA(cudaMemcpyAsync(coef_h.data(), cw.coef.p, coef_h.size() * 8, cudaMemcpyDeviceToHost, st));
         ED_CUDA(cudaMemcpyAsync(beta_h.data(), cw.beta.p, (size_t)(m + 1) * 8, cudaMemcpyDeviceToHost, st));
+        ED_CUDA(cudaMemcpyAsync(clock_h.data(), clock.p, clock.bytes(), cudaMemcpyDeviceToHost, st));
         ED_CUDA(cudaStreamSynchronize(st));
-        for (int j = k; j < m; ++j) {
-            float ms = 0.f;
-            if (cudaEventElapsedTime(&ms, ev[2 * j], ev[2 * j + 1]) == cudaSuccess) spmv_ms += ms;
-        }
-        (void)cudaGetLastError();
+        spmv_ns += stamped_ns(clock_h, k, hstop ? hstop : m);
         m_eff = hstop ? hstop : m;
         if (hstop) {
             ++inf.breakdowns;
@@ -1182,7 +1179,12 @@ void clanczos_solve(const ed_ccrs& a, const ed_lanczos_params& p, const double* 
             ED_CUDA(cudaGetLastError());
             corthonormalise(cw, col(V2b, 0), kk, st);
         }
-        std::swap(Vb.p, V2b.p);
+        // a small sector's basis goes back to where the later cycles' one
+        // graph expects it (as the real solver's); a large one's buffers swap
+        if (n < kCopyBackRows)
+            ED_CUDA(cudaMemcpyAsync(Vb.p, V2b.p, 2 * (size_t)n * (kk + 1) * 8, cudaMemcpyDeviceToDevice, st));
+        else
+            std::swap(Vb.p, V2b.p);
         std::fill(T.begin(), T.end(), 0.0);
         for (int i = 0; i < kk; ++i) {
             T[(size_t)i * m + i] = theta[i];
@@ -1232,7 +1234,7 @@ void clanczos_solve(const ed_ccrs& a, const ed_lanczos_params& p, const double* 
         inf.converged = nc;
     }
     ED_CUDA(cudaStreamSynchronize(st));
-    inf.spmv_seconds = spmv_ms * 1e-3;
+    inf.spmv_seconds = spmv_ns * 1e-9;
     inf.seconds = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
     if (info) *info = inf;
     ED_REQUIRE(converged, ED_ERR_NOCONV, "Lanczos did not converge within the restart cap");

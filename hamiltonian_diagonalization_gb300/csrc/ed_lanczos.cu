@@ -34,6 +34,7 @@
 #include <vector>
 
 #include "ed_lanczos.h"
+#include "ed_launch.cuh"
 #include "ed_split.h"
 
 namespace edgb {
@@ -133,8 +134,10 @@ __global__ void __launch_bounds__(kThreads) k_local_dot(const double* __restrict
                                                         int64_t n, double* __restrict__ part,
                                                         unsigned int* __restrict__ counter, double* __restrict__ coefcol,
                                                         int j, const double* __restrict__ beta_prev,
-                                                        double* __restrict__ hvnorm2, const int* __restrict__ stop)
+                                                        double* __restrict__ hvnorm2, const int* __restrict__ stop,
+                                                        unsigned long long* __restrict__ ended)
 {
+    if (blockIdx.x == 0) stamp(ended);
     if (*stop) return;
     __shared__ double red[kThreads / 32];
     int64_t r0, r1;
@@ -175,8 +178,10 @@ __global__ void __launch_bounds__(kThreads) k_mdot(const double* __restrict__ V,
                                                    const double* __restrict__ beta_prev, double* __restrict__ part,
                                                    unsigned int* __restrict__ counter, double* __restrict__ c,
                                                    double* __restrict__ coefcol, double* __restrict__ before,
-                                                   const int* __restrict__ run, const int* __restrict__ stop)
+                                                   const int* __restrict__ run, const int* __restrict__ stop,
+                                                   unsigned long long* __restrict__ ended)
 {
+    if (blockIdx.x == 0) stamp(ended);
     if ((run && !*run) || (stop && *stop)) return;
     extern __shared__ double sw[];
     const int64_t r0 = (int64_t)blockIdx.x * R;
@@ -213,6 +218,15 @@ __global__ void __launch_bounds__(kThreads) k_mdot(const double* __restrict__ V,
                     a2 = fma(x[u + 2], sw[r + 32 * (u + 2)], a2);
                     a3 = fma(x[u + 3], sw[r + 32 * (u + 3)], a3);
                 }
+            }
+            for (; R < 512 && r + 96 < len; r += 128) {   // a small sector's slices
+                double x[4];
+#pragma unroll
+                for (int u = 0; u < 4; ++u) x[u] = col[r + 32 * u];
+                a0 = fma(x[0], sw[r], a0);
+                a1 = fma(x[1], sw[r + 32], a1);
+                a2 = fma(x[2], sw[r + 64], a2);
+                a3 = fma(x[3], sw[r + 96], a3);
             }
             for (; r < len; r += 32) a0 = fma(col[r], sw[r], a0);
         } else {
@@ -303,12 +317,15 @@ __global__ void __launch_bounds__(kThreads) k_update(const double* __restrict__ 
 }
 
 __global__ void __launch_bounds__(kThreads) k_scale(double* __restrict__ w, int64_t n,
-                                                    const double* __restrict__ beta, const int* __restrict__ stop)
+                                                    const double* __restrict__ beta, const int* __restrict__ stop,
+                                                    unsigned long long* __restrict__ started)
 {
-    if (stop && *stop) return;
-    const double inv = 1.0 / *beta;
-    for (int64_t r = blockIdx.x * (int64_t)kThreads + threadIdx.x; r < n; r += (int64_t)gridDim.x * kThreads)
-        w[r] *= inv;
+    if (!(stop && *stop)) {
+        const double inv = 1.0 / *beta;
+        for (int64_t r = blockIdx.x * (int64_t)kThreads + threadIdx.x; r < n; r += (int64_t)gridDim.x * kThreads)
+            w[r] *= inv;
+    }
+    stamp(started);
 }
 
 // Seeded uniform(-1,1) vector (splitmix64 of seed and index).
@@ -477,18 +494,17 @@ struct Work {
     RotateScratch rot;               // restart rotation scratch
 
     void mdot(const double* Vb, int J, double* x, int local, const double* alpha, const double* beta_prev,
-              double* coefcol, double* before, const int* run, const int* stop, cudaStream_t st)
+              double* coefcol, double* before, const int* run, const int* stop, cudaStream_t st,
+              unsigned long long* ended = nullptr)
     {
-        k_mdot<<<nbm, kThreads, (size_t)R * 8, st>>>(Vb, n, R, J, x, local, alpha, beta_prev, part.p,
-                                                      counters.p + 1, c.p, coefcol, before, run, stop);
-        ::edgb::count_launch();
+        launch(k_mdot, nbm, kThreads, (size_t)R * 8, st, Vb, n, R, J, x, local, alpha, beta_prev, part.p,
+                                                      counters.p + 1, c.p, coefcol, before, run, stop, ended);
     }
     void update(const double* Vb, int J, double* x, int mode, int force2, const double* before, int* need2,
                 double* b, const double* ref2, int j, const int* run, int* stop, cudaStream_t st)
     {
-        k_update<<<nb, kThreads, (size_t)J * 8, st>>>(Vb, n, J, c.p, x, npart.p, counters.p + 2, mode, force2,
+        launch(k_update, nb, kThreads, (size_t)J * 8, st, Vb, n, J, c.p, x, npart.p, counters.p + 2, mode, force2,
                                                        before, need2, b, ref2, j, run, stop);
-        ::edgb::count_launch();
     }
 };
 
@@ -519,7 +535,7 @@ double orthonormalise_column(Work& w, double* Vbase, int col, cudaStream_t st)
     const double nrm = std::sqrt(host_sum_parts(w.part.p, w.nb, st));
     ED_REQUIRE(nrm > 0.0 && std::isfinite(nrm), ED_ERR_ARG, "start vector is zero or not finite");
     ED_CUDA(cudaMemcpyAsync(w.beta.p + w.m + 1, &nrm, 8, cudaMemcpyHostToDevice, st));
-    k_scale<<<w.nb, kThreads, 0, st>>>(x, w.n, w.beta.p + w.m + 1, nullptr); ::edgb::count_launch();
+    launch(k_scale, w.nb, kThreads, 0, st, x, w.n, w.beta.p + w.m + 1, nullptr, nullptr);
     ED_CUDA(cudaGetLastError());
     ED_CUDA(cudaStreamSynchronize(st));
     return nrm;
@@ -629,15 +645,20 @@ void lanczos_once(const ed_op& op, const ed_lanczos_params& p, const double* v0_
     Work w;
     w.n = n;
     w.m = m;
-    w.nb = (int)std::max<int64_t>(1, std::min<int64_t>(nsm * 4, n / 1024));
+    // rows per block of the row-chunked kernels: few in a small sector, whose
+    // step is a chain of short kernels that are each as long as a thread's rows
+    // (n = 8,512: 128 rows 11.2 ms a solve, 256 11.5, 1024 17.4; n = 45,207:
+    // 256 18.4, 128 19.2, 1024 22.0)
+    const bool small = n < 16384;
+    w.nb = (int)std::max<int64_t>(1, std::min<int64_t>(nsm * 4, n / (small ? 128 : 256)));
     // multi-dot slices: three blocks per SM, a whole wave (a cap of 4096 rows
     // gave 335 blocks at the headline size, 2 or 3 per SM, and a Lanczos phase
     // 2 % longer; 2 or 4 blocks per SM measured 0.3 / 0.6 % longer than 3),
-    // at least 512 and at most 12288 rows (a multiple of 128)
+    // at least 512 (128 in a small sector) and at most 12288 rows (a multiple of 128)
     {
         int64_t nbt = (int64_t)nsm * 3, R = 0;
         for (;;) {
-            R = std::max<int64_t>(512, ((n + nbt - 1) / nbt + 127) / 128 * 128);
+            R = std::max<int64_t>(small ? 128 : 512, ((n + nbt - 1) / nbt + 127) / 128 * 128);
             if (R <= 12288) break;
             nbt += nsm;
         }
@@ -669,12 +690,10 @@ void lanczos_once(const ed_op& op, const ed_lanczos_params& p, const double* v0_
     }
     orthonormalise_column(w, w.V.p, 0, st);
 
-    std::vector<cudaEvent_t> ev(2 * (m + 1), nullptr);
-    for (auto& e : ev) ED_CUDA(cudaEventCreate(&e));
-    struct EvGuard {
-        std::vector<cudaEvent_t>& v;
-        ~EvGuard() { for (auto e : v) if (e) cudaEventDestroy(e); }
-    } evguard{ev};
+    // start and end of each step's product
+    DevBuf<unsigned long long> clock(2 * (size_t)(m + 1));
+    ED_CUDA(cudaMemsetAsync(clock.p, 0, clock.bytes(), st));
+    std::vector<unsigned long long> clock_h(2 * (size_t)(m + 1));
 
     // One restart cycle, steps k..m-1, all on the device: breakdown and the
     // second Gram-Schmidt pass are flags that later kernels read, so the host
@@ -682,41 +701,40 @@ void lanczos_once(const ed_op& op, const ed_lanczos_params& p, const double* v0_
     // replays it as one CUDA graph.
     int* need2 = w.flags.p;
     int* stop = w.flags.p + 1;
-    auto enqueue_cycle = [&](int k, bool capturing) {
-        ED_CUDA(cudaMemsetAsync(w.flags.p, 0, 2 * sizeof(int), st));
-        ED_CUDA(cudaMemsetAsync(w.coef.p + (size_t)k * (m + 1), 0, (size_t)(m - k) * (m + 1) * 8, st));
+    auto enqueue_cycle = [&](int k) {
+        const int64_t coefs = (int64_t)(m - k) * (m + 1);
+        launch(k_cycle_begin, (unsigned)std::min<int64_t>(64, (coefs + 255) / 256), 256, 0, st, w.coef.p + (size_t)k * (m + 1), coefs,
+                   w.flags.p, 2, clock.p + 2 * k);
         for (int j = k; j < m; ++j) {
             double* vj = w.V.p + (int64_t)j * n;
             double* wv = w.V.p + (int64_t)(j + 1) * n;
             double* coefcol = w.coef.p + (size_t)j * (m + 1);
             const bool first = (j == k);
-            if (capturing) ED_CUDA(cudaEventRecordWithFlags(ev[2 * j], st, cudaEventRecordExternal));
-            else ED_CUDA(cudaEventRecord(ev[2 * j], st));
             op_apply(op, vj, wv, st);
-            if (capturing) ED_CUDA(cudaEventRecordWithFlags(ev[2 * j + 1], st, cudaEventRecordExternal));
-            else ED_CUDA(cudaEventRecord(ev[2 * j + 1], st));
+            unsigned long long* ended = clock.p + 2 * j + 1;
             if (!first) {
-                k_local_dot<<<w.nb, kThreads, 0, st>>>(vj, wv, n, w.part.p, w.counters.p, coefcol, j,
-                                                       w.beta.p + (j - 1), w.scal.p + 1, stop); ::edgb::count_launch();
+                launch(k_local_dot, w.nb, kThreads, 0, st, vj, wv, n, w.part.p, w.counters.p, coefcol, j,
+                                                       w.beta.p + (j - 1), w.scal.p + 1, stop, ended);
             }
             const int J = j + 1;
             // pass 1 (with the three-term step on non-first steps), then the
             // DGKS-gated pass 2; breakdown is judged against ||H v_j||
-            w.mdot(w.V.p, J, wv, first ? 0 : 1, coefcol + j, w.beta.p + (j - 1), coefcol, w.scal.p, nullptr, stop, st);
+            w.mdot(w.V.p, J, wv, first ? 0 : 1, coefcol + j, w.beta.p + (j - 1), coefcol, w.scal.p, nullptr, stop, st,
+                   first ? ended : nullptr);
             w.update(w.V.p, J, wv, 1, first ? 1 : 0, w.scal.p, need2, w.beta.p + j,
                      first ? w.scal.p : w.scal.p + 1, j, nullptr, stop, st);
             w.mdot(w.V.p, J, wv, 0, nullptr, nullptr, coefcol, w.scal.p + 2, need2, stop, st);
             w.update(w.V.p, J, wv, 2, 0, nullptr, nullptr, w.beta.p + j, first ? w.scal.p : w.scal.p + 1, j, need2,
                      stop, st);
-            k_scale<<<w.nb, kThreads, 0, st>>>(wv, n, w.beta.p + j, stop); ::edgb::count_launch();
+            launch(k_scale, w.nb, kThreads, 0, st, wv, n, w.beta.p + j, stop, clock.p + 2 * (j + 1));
             ED_CUDA(cudaGetLastError());
         }
     };
     const bool graphs = !op_on_host(op);
     CycleGraphs cache;
     auto run_cycle = [&](int k) {
-        if (!graphs) {
-            enqueue_cycle(k, false);
+        if (!graphs || k == 0) {    // the first cycle runs once: a graph of it would cost more than its launches
+            enqueue_cycle(k);
             return;
         }
         CycleGraphs::Entry* g = cache.find(k, w.V.p);
@@ -724,7 +742,7 @@ void lanczos_once(const ed_op& op, const ed_lanczos_params& p, const double* v0_
             const uint64_t c0 = launch_count();
             ED_CUDA(cudaStreamBeginCapture(st, cudaStreamCaptureModeRelaxed));
             try {
-                enqueue_cycle(k, true);
+                enqueue_cycle(k);
             } catch (...) {
                 cudaGraph_t broken = nullptr;
                 cudaStreamEndCapture(st, &broken);
@@ -751,7 +769,7 @@ void lanczos_once(const ed_op& op, const ed_lanczos_params& p, const double* v0_
     int k = 0, m_eff = m;
     double beta_last = 0.0;
     bool converged = false;
-    double spmv_ms = 0.0;
+    double spmv_ns = 0.0;
     for (;;) {
         run_cycle(k);
         inf.matvecs += m - k;
@@ -759,12 +777,9 @@ void lanczos_once(const ed_op& op, const ed_lanczos_params& p, const double* v0_
         ED_CUDA(cudaMemcpyAsync(&hstop, stop, sizeof(int), cudaMemcpyDeviceToHost, st));
         ED_CUDA(cudaMemcpyAsync(coef_h.data(), w.coef.p, coef_h.size() * 8, cudaMemcpyDeviceToHost, st));
         ED_CUDA(cudaMemcpyAsync(beta_h.data(), w.beta.p, (size_t)(m + 1) * 8, cudaMemcpyDeviceToHost, st));
+        ED_CUDA(cudaMemcpyAsync(clock_h.data(), clock.p, clock.bytes(), cudaMemcpyDeviceToHost, st));
         ED_CUDA(cudaStreamSynchronize(st));
-        for (int j = k; j < m; ++j) {
-            float ms = 0.f;
-            ED_CUDA(cudaEventElapsedTime(&ms, ev[2 * j], ev[2 * j + 1]));
-            spmv_ms += ms;
-        }
+        spmv_ns += stamped_ns(clock_h, k, hstop ? hstop : m);
         m_eff = hstop ? hstop : m;
         if (hstop) ++inf.breakdowns;
         for (int j = k; j < m_eff; ++j)
@@ -824,7 +839,12 @@ void lanczos_once(const ed_op& op, const ed_lanczos_params& p, const double* v0_
             ED_CUDA(cudaGetLastError());
             orthonormalise_column(w, w.V2.p, kk, st);
         }
-        std::swap(w.V, w.V2);
+        // a small sector's basis goes back to where the one graph of the later
+        // cycles expects it; a large one's buffers swap (a graph each)
+        if (n < kCopyBackRows)
+            ED_CUDA(cudaMemcpyAsync(w.V.p, w.V2.p, (size_t)n * (kk + 1) * 8, cudaMemcpyDeviceToDevice, st));
+        else
+            std::swap(w.V, w.V2);
         std::fill(T.begin(), T.end(), 0.0);
         for (int i = 0; i < kk; ++i) {
             T[(size_t)i * m + i] = theta[i];
@@ -862,7 +882,7 @@ void lanczos_once(const ed_op& op, const ed_lanczos_params& p, const double* v0_
     }
     ED_CUDA(cudaStreamSynchronize(st));
     op_check(op, st);
-    inf.spmv_seconds = spmv_ms * 1e-3;
+    inf.spmv_seconds = spmv_ns * 1e-9;
     inf.seconds = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
     if (info) *info = inf;
     ED_REQUIRE(converged, ED_ERR_NOCONV, "Lanczos did not converge within the restart cap");

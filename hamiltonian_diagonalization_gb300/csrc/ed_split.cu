@@ -990,10 +990,9 @@ void launch_pass(const SplitSide& s, const SplitArgs& g, cudaStream_t st)
 {
     if (s.ntasks == 0) return;
     if (s.gammas == kKeepParts)
-        k_split_keep<NATIVE><<<(s.ntasks + kWarps - 1) / kWarps, kThreads, 0, st>>>(g, s.ntasks);
+        launch(k_split_keep<NATIVE>, (s.ntasks + kWarps - 1) / kWarps, kThreads, 0, st, g, s.ntasks);
     else
-        k_split_product<NATIVE><<<s.ntasks, kThreads, (size_t)kWarps * sizeof(Sum) * s.rows + sizeof(int4) * (s.moves + s.gammas - kKeepParts), st>>>(g);
-    count_launch();
+        launch(k_split_product<NATIVE>, s.ntasks, kThreads, (size_t)kWarps * sizeof(Sum) * s.rows + sizeof(int4) * (s.moves + s.gammas - kKeepParts), st, g);
 }
 
 }  // namespace
@@ -1094,8 +1093,7 @@ std::unique_ptr<SplitPlan> split_build(const SplitSource& s, const double* diag,
     // the diagonal's exponent joins the weights'
     const int parts = exp_parts();
     int* part = tmp.take<int>((size_t)parts + 1);
-    k_fix_exp<<<parts, 256, 0, st>>>(diag, n, part);
-    count_launch();
+    launch(k_fix_exp, parts, 256, 0, st, diag, n, part);
     std::vector<int> h(parts);
     ED_CUDA(cudaMemcpyAsync(h.data(), part, (size_t)parts * 4, cudaMemcpyDeviceToHost, st));
     ED_CUDA(cudaStreamSynchronize(st));
@@ -1111,8 +1109,7 @@ std::unique_ptr<SplitPlan> split_build(const SplitSource& s, const double* diag,
     if (!bn.fits() || !bt.fits() || (size_t)n * 56 + bn.bytes() + bt.bytes() > free_b / 2) return nullptr;
     p->diag.alloc((size_t)n);
     ED_CUDA(cudaMemcpyAsync(part, &ea, sizeof(int), cudaMemcpyHostToDevice, st));
-    k_fix_conv<<<sms() * 4, 256, 0, st>>>(diag, n, part, 1, p->diag.p);
-    count_launch();
+    launch(k_fix_conv, sms() * 4, 256, 0, st, diag, n, part, 1, p->diag.p);
     bn.fill(ea);
     bt.fill(ea);
     p->perm.alloc((size_t)n);
@@ -1163,10 +1160,8 @@ const int* split_product(SplitPlan& p, const double* x, double* y, cudaStream_t 
         sc = p.scratch.at({dev, st}).get();
     }
     const int P = exp_parts();
-    k_fix_exp<<<P, 256, 0, st>>>(x, p.n, sc->part.p);
-    count_launch();
-    k_split_conv<<<sms() * 4, 256, 0, st>>>(x, p.n, sc->part.p, P, p.perm.p, sc->x.p, sc->xt.p);
-    count_launch();
+    launch(k_fix_exp, P, 256, 0, st, x, p.n, sc->part.p);
+    launch(k_split_conv, sms() * 4, 256, 0, st, x, p.n, sc->part.p, P, p.perm.p, sc->x.p, sc->xt.p);
     launch_pass<false>(p.trans, args_of(p, p.trans, sc->xt.p, *sc, y, P), st);
     launch_pass<true>(p.native, args_of(p, p.native, sc->x.p, *sc, y, P), st);
     ED_CUDA(cudaGetLastError());

@@ -935,9 +935,14 @@ void sell_launch(const ed_crs& a, const double* x, double* y, cudaStream_t st)
 }  // namespace
 
 // Full-storage matrices of at least kSellMinRows rows and fewer than
-// kSellMaxAvg elements a row on average get the sliced-ELL copy; the others
-// of full storage (the one-level sectors) the fixed-point copy.
-constexpr int64_t kSellMinRows = 4096;
+// kSellMaxAvg elements a row on average get the sliced-ELL copy.  The others
+// from kFixMinRows rows up take the fixed-point row kernel: longer rows (the
+// one-level sectors), and small matrices, where one lane a row leaves most of
+// the GPU idle (rows against sliced ELL on GB300: 8,512 one-level rows of 92
+// elements 16.2 / 24.7 us, 16,276 two-level rows of 22 14.5 / 16.5, 47,044 of
+// 29 19.4 / 18.1).
+constexpr int64_t kSellMinRows = 32768;
+constexpr int64_t kFixMinRows = 4096;
 constexpr double kSellMaxAvg = 96.0;
 
 namespace {
@@ -956,9 +961,8 @@ void fix_build(const ed_crs& a, cudaStream_t st)
     auto fq = std::make_unique<ed_fixq>();
     const int P = fix_parts();
     DevBuf<int> part((size_t)P + 1);
-    k_fix_exp<<<P, 256, 0, st>>>(a.val.p, a.nnz, part.p);
-    count_launch();
-    k_fix_conv<<<1, 256, 0, st>>>(a.val.p, 0, part.p, P, nullptr);   // the bound into part[P]
+    launch(k_fix_exp, P, 256, 0, st, a.val.p, a.nnz, part.p);
+    launch(k_fix_conv, 1, 256, 0, st, a.val.p, 0, part.p, P, nullptr);   // the bound into part[P]
     count_launch();
     ED_CUDA(cudaGetLastError());
     int ea = 1;
@@ -1030,17 +1034,20 @@ bool fix_copy(const ed_crs& a, bool sell, cudaStream_t st)
     ED_CUDA(cudaMemsetAsync(dst.p + cnt, 0, (size_t)kCrsPad * 8, st));
     DevBuf<int> part(2);
     ED_CUDA(cudaMemcpyAsync(part.p, &f.ea, sizeof(int), cudaMemcpyHostToDevice, st));
-    k_fix_conv<<<sms() * 8, 256, 0, st>>>(sell ? a.sell->val.p : a.val.p, cnt, part.p, 1, dst.p);
-    count_launch();
+    launch(k_fix_conv, sms() * 8, 256, 0, st, sell ? a.sell->val.p : a.val.p, cnt, part.p, 1, dst.p);
     ED_CUDA(cudaGetLastError());
     ED_CUDA(cudaStreamSynchronize(st));
     state = 1;
     return true;
 }
 
+bool short_rows(const ed_crs& a) { return (double)a.nnz < kSellMaxAvg * (double)a.n; }
+
+bool sell_shape(const ed_crs& a) { return !a.upper && a.n >= kSellMinRows && short_rows(a); }
+
 bool fix_shape(const ed_crs& a)
 {
-    return !a.upper && a.n > 0 && (double)a.nnz >= kSellMaxAvg * (double)a.n;
+    return !a.upper && a.n > 0 && (!short_rows(a) || (a.n >= kFixMinRows && a.n < kSellMinRows));
 }
 
 // The fixed-point state, the copy of the values in the wanted order and
@@ -1057,10 +1064,7 @@ ed_fixq::Scratch& fix_convert_x(const ed_crs& a, const double* x, cudaStream_t s
 {
     ed_fixq::Scratch& sc = *fix_scratch(a, st);
     const int P = fix_parts();
-    k_fix_exp<<<P, 256, 0, st>>>(x, a.n, sc.part.p);
-    count_launch();
-    k_fix_conv<<<sms() * 4, 256, 0, st>>>(x, a.n, sc.part.p, P, sc.xq.p);
-    count_launch();
+    fix_convert(x, a.n, sc.part.p, P, sms() * 4, sc.xq.p, st);
     return sc;
 }
 
@@ -1089,10 +1093,9 @@ void fix_launch(const ed_crs& a, const double* x, double* y, cudaStream_t st)
     // registers with spills 0.88-1.03; each warp's next row tile prefetched
     // into L2 by cp.async.bulk.prefetch 0.99; the rows staged in shared
     // memory by bulk copies, k_spmv_fix_staged, 1.71)
-    k_spmv_fix<8, 8, 4><<<sms() * 8, 256, 0, st>>>(a.rowptr.p, a.col.p, reinterpret_cast<const int2*>(f.val.p),
+    launch(k_spmv_fix<8, 8, 4>, sms() * 8, 256, 0, st, a.rowptr.p, a.col.p, reinterpret_cast<const int2*>(f.val.p),
                                                    reinterpret_cast<const int2*>(sc.xq.p), sc.part.p + P, f.ea, y,
                                                    a.n);
-    count_launch();
     ED_CUDA(cudaGetLastError());
 }
 
@@ -1101,11 +1104,10 @@ void fix_launch_sell(const ed_crs& a, const double* x, double* y, cudaStream_t s
     const ed_fixq& f = *a.fixq;
     const ed_sell& sl = *a.sell;
     ed_fixq::Scratch& sc = fix_convert_x(a, x, st);
-    k_spmv_sell_fix<8, 4><<<sms() * 8, 256, 0, st>>>(sl.off.p, sl.len.p, sl.row.p, sl.col.p,
+    launch(k_spmv_sell_fix<8, 4>, sms() * 8, 256, 0, st, sl.off.p, sl.len.p, sl.row.p, sl.col.p,
                                                      reinterpret_cast<const int2*>(f.sval.p),
                                                      reinterpret_cast<const int2*>(sc.xq.p), sc.part.p + fix_parts(),
                                                      f.ea, y, sl.nchunks);
-    count_launch();
     ED_CUDA(cudaGetLastError());
 }
 
@@ -1144,12 +1146,8 @@ void spmv_prepare(const ed_crs& a, cudaStream_t st)
     if (k == 0 && split_prepare(a, st)) return;
     if (k == 6 || k == 7 || (k == 0 && fix_shape(a))) fix_ready(a, st);
     if ((k == 4 || k == 5 || k == 8) && a.sell_state == 0) sell_build(a, st);
-    if (k == 0 && a.sell_state == 0) {
-        // one-level sectors (96 and more elements a row) stay with the row lanes
-        if (a.upper || a.n < kSellMinRows || (double)a.nnz >= kSellMaxAvg * (double)a.n) a.sell_state = -1;
-        else sell_build(a, st);
-    }
-    if ((k == 0 || k == 8) && a.sell_state == 1) fix_ready(a, st, true);
+    if (k == 0 && sell_shape(a) && a.sell_state == 0) sell_build(a, st);
+    if ((k == 8 || (k == 0 && sell_shape(a))) && a.sell_state == 1) fix_ready(a, st, true);
 }
 
 void spmv_kernel(const ed_crs& a, int kernel, const double* x, double* y, cudaStream_t st)
@@ -1184,9 +1182,9 @@ void spmv_kernel(const ed_crs& a, int kernel, const double* x, double* y, cudaSt
     const int grid = sms() * 8;
     const int64_t* rp = a.rowptr.p;
     switch (kernel) {
-    case 1: k_spmv_full<8, 4><<<grid, threads, 0, st>>>(rp, a.col.p, a.val.p, x, y, a.n); break;
-    case 2: k_spmv_rows<8, 4, 2><<<grid, threads, 0, st>>>(rp, a.col.p, a.val.p, x, y, a.n); break;
-    case 3: k_spmv_rows<8, 2, 2><<<grid, threads, 0, st>>>(rp, a.col.p, a.val.p, x, y, a.n); break;
+    case 1: launch(k_spmv_full<8, 4>, grid, threads, 0, st, rp, a.col.p, a.val.p, x, y, a.n); break;
+    case 2: launch(k_spmv_rows<8, 4, 2>, grid, threads, 0, st, rp, a.col.p, a.val.p, x, y, a.n); break;
+    case 3: launch(k_spmv_rows<8, 2, 2>, grid, threads, 0, st, rp, a.col.p, a.val.p, x, y, a.n); break;
     default:
         if (a.sell_state == 0 && !stream_capturing(st)) sell_build(a, st);   // any size here
         ED_REQUIRE(a.sell_state == 1, ED_ERR_RANGE, "no sliced-ELL copy (not enough free device memory)");
@@ -1194,8 +1192,6 @@ void spmv_kernel(const ed_crs& a, int kernel, const double* x, double* y, cudaSt
         else sell_launch<8>(a, x, y, st);
         return;
     }
-    count_launch();
-    ED_CUDA(cudaGetLastError());
 }
 
 void spmv_check(const ed_crs& a, cudaStream_t st)
@@ -1234,8 +1230,8 @@ void spmv(const ed_crs& a, const double* x, double* y, cudaStream_t st)
         split_product(*a.split, x, y, st);
         return;
     }
-    if (a.sell_state == 0) spmv_prepare(a, st);   // waits for a solver's explicit call while capturing
-    if (a.sell_state == 1) {
+    if (sell_shape(a) && a.sell_state == 0) spmv_prepare(a, st);   // waits for a solver's explicit call while capturing
+    if (sell_shape(a) && a.sell_state == 1) {
         if (fix_ready(a, st, true)) {
             // the fixed-point sliced ELL (two-level N=8, 2S=21: see
             // k_spmv_sell_fix), else the FP64 kernel below
@@ -1250,6 +1246,10 @@ void spmv(const ed_crs& a, const double* x, double* y, cudaStream_t st)
         sell_launch<16>(a, x, y, st);
         return;
     }
+    if (fix_shape(a) && fix_ready(a, st)) {
+        fix_launch(a, x, y, st);
+        return;
+    }
     const double avg = (double)a.nnz / (double)a.n;
     const int threads = 256;
     const int grid = sms() * 8;
@@ -1260,23 +1260,19 @@ void spmv(const ed_crs& a, const double* x, double* y, cudaStream_t st)
         // loads ahead; N=10 2S=27: 0.1219-0.1226 against 0.1219-0.1232 and
         // 0.14); also the short-row sectors below kSellMinRows rows
         if (avg >= kSellMaxAvg) {
-            if (fix_ready(a, st)) {
-                fix_launch(a, x, y, st);
-                return;
-            }
-            k_spmv_rows<8, 4, 2><<<grid, threads, 0, st>>>(a.rowptr.p, a.col.p, a.val.p, x, y, a.n);
+            launch(k_spmv_rows<8, 4, 2>, grid, threads, 0, st, a.rowptr.p, a.col.p, a.val.p, x, y, a.n);
         } else {
-            k_spmv_rows<8, 2, 2><<<grid, threads, 0, st>>>(a.rowptr.p, a.col.p, a.val.p, x, y, a.n);
+            launch(k_spmv_rows<8, 2, 2>, grid, threads, 0, st, a.rowptr.p, a.col.p, a.val.p, x, y, a.n);
         }
     } else if (!a.upper) {
-        k_spmv_full<2><<<grid, threads, 0, st>>>(a.rowptr.p, a.col.p, a.val.p, x, y, a.n);
+        launch(k_spmv_full<2>, grid, threads, 0, st, a.rowptr.p, a.col.p, a.val.p, x, y, a.n);
     } else {
         ED_CUDA(cudaMemsetAsync(y, 0, (size_t)a.n * sizeof(double), st));
         if (avg >= 48) k_spmv_upper<8><<<grid, threads, 0, st>>>(a.rowptr.p, a.col.p, a.val.p, x, y, a.n);
         else k_spmv_upper<4><<<grid, threads, 0, st>>>(a.rowptr.p, a.col.p, a.val.p, x, y, a.n);
+        count_launch();
+        ED_CUDA(cudaGetLastError());
     }
-    count_launch();
-    ED_CUDA(cudaGetLastError());
 }
 
 std::shared_ptr<SplitPlan> matfree_plan(const ed_basis& b, const ed_terms& t, const double* diag, cudaStream_t st)
