@@ -97,7 +97,9 @@ __global__ void __launch_bounds__(kCThreads) k_cspmv_full(const int64_t* __restr
 // takes 16 mad.wide.s32 into six int64 partial sums of U <= 4 elements,
 // flushed into the lane's two 128-bit sums; the G lanes' sums are added
 // exactly and rounded once to FP64 (rows of at most 1024 elements keep
-// |S| < 2^127).  4 DFMA an element made the FP64 kernel FP64-bound at 2.6 TB/s.
+// |S| < 2^127).  An iteration waits on the x entries of its columns, so the
+// next iteration's columns are fetched with this one's values: one memory
+// access in its chain instead of two.  4 DFMA an element made the FP64 kernel FP64-bound at 2.6 TB/s.
 template <int G, int U, int MINB = 1>
 __global__ void __launch_bounds__(kCThreads, MINB) k_cspmv_fix(const int64_t* __restrict__ rowptr,
                                                          const int32_t* __restrict__ col,
@@ -122,18 +124,18 @@ __global__ void __launch_bounds__(kCThreads, MINB) k_cspmv_fix(const int64_t* __
         const int4* ap = aq + s;
         const int32_t* cp = col + s;
         __int128 sre = 0, sim = 0;
+        int cc[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) cc[u] = sub + u * G < len ? __ldcs(cp + sub + u * G) : 0;
         for (int j0 = sub; j0 < len; j0 += G * U) {
-            int4 av[U];
-            int cc[U];
+            int4 av[U], xv[U];
 #pragma unroll
             for (int u = 0; u < U; ++u) {
-                const bool in = j0 + u * G < len;
-                av[u] = in ? __ldcs(ap + j0 + u * G) : make_int4(0, 0, 0, 0);
-                cc[u] = in ? __ldcs(cp + j0 + u * G) : 0;
+                av[u] = j0 + u * G < len ? __ldcs(ap + j0 + u * G) : make_int4(0, 0, 0, 0);
+                xv[u] = __ldg(xq + cc[u]);
             }
-            int4 xv[U];
 #pragma unroll
-            for (int u = 0; u < U; ++u) xv[u] = __ldg(xq + cc[u]);
+            for (int u = 0; u < U; ++u) cc[u] = j0 + (U + u) * G < len ? __ldcs(cp + j0 + (U + u) * G) : 0;
             long long r2 = 0, r1 = 0, r0 = 0, i2 = 0, i1 = 0, i0 = 0;
 #pragma unroll
             for (int u = 0; u < U; ++u) {
@@ -896,11 +898,13 @@ void cfix_launch(const ed_ccrs& a, const double* x, double* y, cudaStream_t st)
     const int4* A = reinterpret_cast<const int4*>(f.val.p);
     const int4* X = reinterpret_cast<const int4*>(sc.xq.p);
     double2* yy = reinterpret_cast<double2*>(y);
-    // 8 lanes a row, 4 elements ahead, at most 64 registers: four CTAs per SM
-    // (GB300, N=10 on 5x6: 1.363 ms; 92 registers and two CTAs 1.77, 2
-    // ahead 2.69, 16 lanes 2.72, 48 registers with spills 1.62; the FP64
-    // kernel 2.31)
-    if (avg >= 48) launch(k_cspmv_fix<8, 4, 4>, csms() * 8, kCThreads, 0, st, a.rowptr.p, a.col.p, A, X, sc.part.p + P, f.ea, yy, a.n);
+    // 8 lanes a row, 4 elements ahead, at most 80 registers: three CTAs per SM
+    // (GB300, N=10 on 5x6, 1.0M rows of 307: 1.176 ms, 5.2 TB/s; 64 registers
+    // and four CTAs 1.201, two CTAs 1.37, 3 ahead 1.245, 16 lanes 1.26, 4 lanes
+    // 1.169; without the columns' prefetch 1.347; the FP64 kernel 2.31.  N=9 on
+    // 4x6, 0.05M rows: 55.5 us, without it 61.6.  Rows blocked as the real
+    // product's give 1.123 ms for a first product of 5.4 instead of 4.4 ms)
+    if (avg >= 48) launch(k_cspmv_fix<8, 4, 3>, csms() * 8, kCThreads, 0, st, a.rowptr.p, a.col.p, A, X, sc.part.p + P, f.ea, yy, a.n);
     else launch(k_cspmv_fix<4, 4, 4>, csms() * 8, kCThreads, 0, st, a.rowptr.p, a.col.p, A, X, sc.part.p + P, f.ea, yy, a.n);
     ED_CUDA(cudaGetLastError());
 }
