@@ -244,6 +244,12 @@ struct ed_fixq {
     // the sliced-ELL order (nnz_pad + kCrsPad)
     edgb::DevBuf<int64_t> val, sval;
     int val_state = 0, sval_state = 0;
+    // the row-blocked copy (ed_blocked.cuh): offsets of the blocks' steps,
+    // columns and limb pairs; same states
+    edgb::DevBuf<int64_t> boff, bval;
+    edgb::DevBuf<int32_t> bcol;
+    int64_t blocks = 0;
+    int blk_state = 0;
     // the staged kernel's ring: stage capacity (elements) and stage count,
     // 0 when it does not fit; err counts its waits that ran out
     int stage_elems = 0, stages = 0;

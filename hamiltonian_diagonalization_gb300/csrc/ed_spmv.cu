@@ -27,6 +27,7 @@
 #include <map>
 #include <memory>
 
+#include "ed_blocked.cuh"
 #include "ed_fixed.cuh"
 #include "ed_hop.cuh"
 #include "ed_split.h"
@@ -1068,6 +1069,51 @@ ed_fixq::Scratch& fix_convert_x(const ed_crs& a, const double* x, cudaStream_t s
     return sc;
 }
 
+// The row-blocked copy (ed_blocked.cuh) for matrices of at least this many
+// rows, where the matrix streams: k_spmv_fix / k_spmv_blk 29.3 / 28.9 us at
+// 45,207 rows (N=9, 2S=24; for twice the first product's time), 39.0 / 33.9 at
+// 65,809.  Shorter sectors stay in L2, and their products end in the latency
+// of the last rows.
+constexpr int64_t kBlkMinRows = 1 << 16;
+
+// Made once outside a capture; false when it is not there (declined when it
+// would take more than half of the free device memory).
+bool blk_copy(const ed_crs& a, cudaStream_t st)
+{
+    ed_fixq& f = *a.fixq;
+    if (f.blk_state != 0) return f.blk_state == 1;
+    if (stream_capturing(st)) return false;
+    f.blk_state = -1;
+    f.blocks = (a.n + kBlkRows - 1) / kBlkRows;
+    DevBuf<int64_t> off((size_t)f.blocks + 1);
+    int64_t steps = 0;
+    {
+        DevBuf<int64_t> cnt((size_t)f.blocks);
+        launch(k_blk_steps, sms() * 8, 256, 0, st, a.rowptr.p, a.n, f.blocks, cnt.p);
+        exclusive_scan_i64(cnt.p, off.p, f.blocks, st);
+        ED_CUDA(cudaMemcpyAsync(&steps, off.p + f.blocks, 8, cudaMemcpyDeviceToHost, st));
+        ED_CUDA(cudaStreamSynchronize(st));
+    }
+    size_t free_b = 0, total_b = 0;
+    ED_CUDA(cudaMemGetInfo(&free_b, &total_b));
+    if ((size_t)steps * 32 * 12 > free_b / 2) return false;
+    f.bcol.alloc((size_t)steps * 32);
+    f.bval.alloc((size_t)steps * 32);
+    launch(k_blk_fill, sms() * 8, 256, 0, st, a.rowptr.p, a.col.p, a.val.p, a.n, f.blocks, off.p, f.ea, f.bcol.p, f.bval.p);
+    ED_CUDA(cudaStreamSynchronize(st));
+    f.boff = std::move(off);
+    f.blk_state = 1;
+    return true;
+}
+
+bool blk_shape(const ed_crs& a) { return fix_shape(a) && a.n >= kBlkMinRows; }
+
+bool blk_ready(const ed_crs& a, cudaStream_t st)
+{
+    if (a.fix_state == 0 && !stream_capturing(st)) fix_build(a, st);
+    return a.fix_state == 1 && blk_copy(a, st) && fix_scratch(a, st) != nullptr;
+}
+
 void fix_launch_staged(const ed_crs& a, const double* x, double* y, long long stall, cudaStream_t st)
 {
     const ed_fixq& f = *a.fixq;
@@ -1082,13 +1128,22 @@ void fix_launch_staged(const ed_crs& a, const double* x, double* y, long long st
     ED_CUDA(cudaGetLastError());
 }
 
+void blk_launch(const ed_crs& a, const double* x, double* y, cudaStream_t st)
+{
+    const ed_fixq& f = *a.fixq;
+    ed_fixq::Scratch& sc = fix_convert_x(a, x, st);
+    launch(k_spmv_blk<6, 4>, sms() * 8, 256, 0, st, f.boff.p, f.bcol.p, reinterpret_cast<const int2*>(f.bval.p),
+           reinterpret_cast<const int2*>(sc.xq.p), sc.part.p + fix_parts(), f.ea, y, a.n, f.blocks);
+}
+
 void fix_launch(const ed_crs& a, const double* x, double* y, cudaStream_t st)
 {
     const ed_fixq& f = *a.fixq;
     ed_fixq::Scratch& sc = fix_convert_x(a, x, st);
     const int P = fix_parts();
-    // 8 lanes a row, 8 loads ahead, at most 64 registers: four CTAs per SM
-    // (GB300, N=11 2S=30 with the two conversion passes: 0.772 ms; 71
+    // matrices below kBlkMinRows, and those without the memory for the blocked
+    // copy.  8 lanes a row, 8 loads ahead, at most 64 registers: four CTAs per
+    // SM (GB300, N=11 2S=30 with the two conversion passes: 0.772 ms; 71
     // registers and three CTAs 0.877; 4 loads ahead 0.862; 48 or 40
     // registers with spills 0.88-1.03; each warp's next row tile prefetched
     // into L2 by cp.async.bulk.prefetch 0.99; the rows staged in shared
@@ -1115,18 +1170,19 @@ void fix_launch_sell(const ed_crs& a, const double* x, double* y, cudaStream_t s
 
 // Stored matrices of at least this many rows take the split product.  Below,
 // the matrix streams from HBM and L2 faster than the short segments of small
-// sectors can be summed.  Measured on GB300, split against the stored kernel:
-// one level 0.92M rows (N=11, 2S=29) 487 / 474 us, 1.37M (N=11, 2S=30) 709 /
-// 772, 1.44M (N=12, 2S=29) 725 / 812, 3.45M (N=12, 2S=31) 1768 / 2274; two
-// levels 0.90M (N=8, 2S=16) 126 / 108, 1.36M 173 / 177, 2.03M 254 / 281,
-// 5.90M (N=8, 2S=21) 760 / 993.
-constexpr int64_t kSplitMinRows = 1 << 20;
+// sectors can be summed.  Measured on GB300, split against the stored kernels:
+// long rows (one level) 1.37M rows (N=11, 2S=30) 712 / 674 us, 1.44M (N=12,
+// 2S=29) 725 / 709, 2.01M (N=11, 2S=31) 1031 / 1055, 3.45M (N=12, 2S=31) 1763 /
+// 1990; short rows (two levels) 0.90M (N=8, 2S=16) 126 / 108, 1.36M 173 / 177,
+// 2.03M 254 / 281, 5.90M (N=8, 2S=21) 760 / 993.
+constexpr int64_t kSplitMinRows = 3 << 19, kSplitMinRowsShort = 1 << 20;
 
 // The split product's plan and this stream's scratch, made when missing and
 // not capturing; false when the stored product runs instead.
 static bool split_prepare(const ed_crs& a, cudaStream_t st)
 {
-    if (a.n < kSplitMinRows) return false;
+    // the upper triangle has no better stored kernel either
+    if (a.n < (a.upper || short_rows(a) ? kSplitMinRowsShort : kSplitMinRows)) return false;
     if (a.split_state == 0 && !stream_capturing(st)) {
         a.split = split_build_crs(a, st);
         a.split_state = a.split ? 1 : -1;
@@ -1144,6 +1200,7 @@ void spmv_prepare(const ed_crs& a, cudaStream_t st)
     if (a.n == 0 || stream_capturing(st)) return;
     const int k = a.product_kernel;
     if (k == 0 && split_prepare(a, st)) return;
+    if (k == 0 && blk_shape(a) && blk_ready(a, st)) return;
     if (k == 6 || k == 7 || (k == 0 && fix_shape(a))) fix_ready(a, st);
     if ((k == 4 || k == 5 || k == 8) && a.sell_state == 0) sell_build(a, st);
     if (k == 0 && sell_shape(a) && a.sell_state == 0) sell_build(a, st);
@@ -1244,6 +1301,10 @@ void spmv(const ed_crs& a, const double* x, double* y, cudaStream_t st)
         // ahead 0.305 / 1.052 ms (8 ahead 0.326 / 1.110, 24 0.303 / 1.045,
         // 32 0.310 / 1.055) against the best row kernels 0.333 / 1.197
         sell_launch<16>(a, x, y, st);
+        return;
+    }
+    if (blk_shape(a) && blk_ready(a, st)) {
+        blk_launch(a, x, y, st);
         return;
     }
     if (fix_shape(a) && fix_ready(a, st)) {
