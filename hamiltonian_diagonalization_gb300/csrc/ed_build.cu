@@ -9,10 +9,9 @@
 // host folds them, in the reference's visiting order and with its filters,
 // into one value per hop (derive_hop_tables), so the element is
 // sign(state) * W[hop] bit for bit.  The diagonal is summed term by term in
-// the reference order.  Rows are generated one warp per row, sorted by
-// column (in registers, k_fill_reg; in shared memory for rows or sectors too
-// large for 32-bit keys, k_fill) and written coalesced; a count pass sizes
-// the rows first.
+// the reference order.  Rows are generated one warp per row, the real ones in
+// column order (k_fill_rows), the complex ones sorted in registers (k_cfill),
+// and written coalesced; a count pass sizes the rows first.
 #include <algorithm>
 #include <cmath>
 #include <cstdlib>
@@ -20,6 +19,8 @@
 #include <vector>
 
 #include "ed_hop.cuh"
+#include "ed_launch.cuh"
+#include "ed_launch.cuh"
 #include "ed_split.h"
 
 namespace edgb {
@@ -39,22 +40,37 @@ __global__ void k_diag(const uint64_t* __restrict__ words, int64_t n, const doub
         diag[r] = diag_element(hv, words[r]);
 }
 
-// Number of stored entries of each row (upper: col >= row; full: all), and
-// the largest number of admissible hops of a row plus one (the diagonal
-// slot), which sizes the register-sort fill's per-warp task list.  With
-// nozero (no off-diagonal hop weight is zero) a row's count is the popcount
-// of its pairs' target masks.
-__global__ void k_count(const uint64_t* __restrict__ words, int64_t n, const double* __restrict__ diag,
+__device__ __forceinline__ void row_maxes(unsigned tasks, unsigned row, int* maxes)
+{
+    tasks = __reduce_max_sync(0xffffffffu, tasks);
+    row = __reduce_max_sync(0xffffffffu, row);
+    if ((threadIdx.x & 31) == 0) {
+        atomicMax(maxes, (int)tasks);
+        atomicMax(maxes + 1, (int)row);
+    }
+}
+
+// The diagonal, and the number of stored entries of each row (upper: col >=
+// row; full: all); maxes[0]: the largest number of admissible hops of a row
+// plus one (the diagonal slot), which sizes the fill's per-warp task list,
+// maxes[1]: the longest row.  With nozero (no off-diagonal hop weight is zero)
+// a row's count is the popcount of its pairs' target masks.  The diagonal's
+// ordered FP64 sum keeps the FP64 pipe busy while other warps count on the
+// integer pipes (N=10, 2S=27: 111 + 43 us
+// apart, 122 together).
+__global__ void k_count(const uint64_t* __restrict__ words, int64_t n, double* __restrict__ diag,
                         const double* __restrict__ w, int nw, const double* __restrict__ da,
                         const double* __restrict__ db, const int* __restrict__ off, int K, int upper, int nozero,
-                        int64_t* __restrict__ rowlen, int* __restrict__ maxtasks)
+                        int64_t* __restrict__ rowlen, int* __restrict__ maxes)
 {
     extern __shared__ __align__(16) unsigned char smem[];
     const HopView hv = load_hop_smem(smem, w, nw, da, db, off, K);
-    unsigned tmax = 0;
+    unsigned tmax = 0, rmax = 0;
     for (int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; r < n; r += (int64_t)gridDim.x * blockDim.x) {
         const uint64_t in = words[r];
-        int64_t cnt = (fabs(diag[r]) < kSparseZeroTol) ? 0 : 1;
+        const double dv = diag_element(hv, in);
+        diag[r] = dv;
+        unsigned cnt = (fabs(dv) < kSparseZeroTol) ? 0 : 1;
         unsigned tasks = 1;
         for (uint64_t ta = in; ta; ta &= ta - 1) {
             const int a = __ffsll((long long)ta) - 1;
@@ -77,14 +93,14 @@ __global__ void k_count(const uint64_t* __restrict__ words, int64_t n, const dou
             }
         }
         rowlen[r] = cnt;
-        tmax = tasks > tmax ? tasks : tmax;
+        tmax = max(tmax, tasks);
+        rmax = max(rmax, cnt);
     }
-    tmax = __reduce_max_sync(0xffffffffu, tmax);
-    if ((threadIdx.x & 31) == 0) atomicMax(maxtasks, (int)tmax);
+    row_maxes(tmax, rmax, maxes);
 }
 
 // One warp per row: generate (out word, value), sort by word in shared
-// memory, rank, store.  Any row length the shared memory holds, any sector.
+// memory, rank, store (ED_FILL_SORT=smem; rows whose task list does not fit).
 __global__ void k_fill(const uint64_t* __restrict__ words, int64_t n, const double* __restrict__ diag,
                        const double* __restrict__ w, int nw, const double* __restrict__ da,
                        const double* __restrict__ db, const int* __restrict__ off, int K, int N, int upper,
@@ -191,27 +207,260 @@ __global__ void k_fill(const uint64_t* __restrict__ words, int64_t n, const doub
 }
 
 // ---------------------------------------------------------------------------
-// k_fill_reg: the same rows, sorted in registers.  The admissible hops of
-// each occupied pair (hop_targets) are expanded into a task list (a, b, c)
-// in shared memory, so that every task yields an element unless its weight
-// is zero, and the tasks are spread evenly over the lanes.  Each element is
-// ranked as it is generated and stored as a 32-bit key (column << sb | slot),
-// sb = log2(cap), with its value at vals[slot]; the host takes this kernel
-// only when every key fits below 0xFFFFFFFF.  Slots follow the task order
-// (one ballot per 32 tasks) and reuse the task list's storage: a slot never
-// passes the task that fills it.  The keys, padded to 32*E with 0xFFFFFFFF,
-// are sorted by a bitonic network over the element index lane*E + e:
-// exchanges whose partner is nearer than E stay in one lane's registers, the
-// rest take one shuffle.  The sorted keys go back through a swizzled
-// shared-memory image (index i ^ ((i >> 5) & 31), conflict-free both ways)
-// and are written coalesced.
+// k_fill_rows: rows generated in column order, without a sort.  Columns ascend
+// with the words, so a row's order is the order of its words.  The hops of
+// `in` that lower a level's word (d < b) come in the order
+//   b descending, d ascending, a ascending,
+// and those that raise it (d > b) in the order
+//   d ascending, b descending, a descending
+// (compare two results at the highest orbital in which they differ: a larger
+// lost orbital b leaves the smaller word, a larger gained one d the larger;
+// with b and d the same, c = a + b - d moves with a).  For one (b, d) the hops
+// are a mask over a,
+//   in & (empty >> (b - d)) & bits below 2 d - b    (d < b),
+//   in & (empty << (d - b)) & bits below b          (d > b),
+// because c must be empty, and a < b, c < d.  The row of a two-level word
+// (level 0 above level 1) is: level 0 lowering, level 1 lowering, the
+// diagonal, level 1 raising, level 0 raising.
+//
+// A warp takes a row: its task list is made 32 pairs (b, d) of either order at
+// a time (append_hops), the lowering hops from the front and the raising ones
+// from the back of its piece of shared memory; then the list is worked off 32
+// hops at a time (weight, sign, rank), and the elements, compacted by a ballot
+// where a weight is zero, go straight to their places.
+// Integer instructions bound it (79 % of the issue slots).  GB300, against rows
+// generated in any order and sorted in registers: N=10, 2S=27 (245,394 rows of
+// 188) 970 -> 457 us, N=11, 2S=30 with the counts and allocations 10.5 -> 4.4
+// ms.  With 64-bit words 870 us; counting all of a lane's pairs before placing
+// them, two passes over the masks, 508.
+template <class Word>
+__device__ __forceinline__ int bit_count(Word m)
+{
+    return sizeof(Word) == 4 ? __popc((unsigned)m) : __popcll(m);
+}
+
+// One level of a row: its word, the empty orbitals as a mask, and the list of
+// the occupied orbitals (ascending) followed by the empty ones.
+template <class Word>
+struct FillSub {
+    Word in, empty;
+    const unsigned char* orbs;
+    int N, M;
+};
+
+// q-th pair of an outer and an inner index, q = lane, lane + 32, ...
+struct PairWalk {
+    int i, j, di, dj, inner;
+    __device__ __forceinline__ PairWalk(int lane, int n) : inner(n)
+    {
+        // below 2^10, the half keeps the rounded quotient inside its cell
+        const float r = __frcp_rn((float)n);
+        i = (int)(((float)lane + 0.5f) * r);
+        j = lane - i * n;
+        di = (int)(32.5f * r);
+        dj = 32 - di * n;
+    }
+    __device__ __forceinline__ void next()
+    {
+        i += di;
+        j += dj;
+        if (j >= inner) { j -= inner; ++i; }
+    }
+};
+
+// Appends level x's lowering hops at the front of the task list (from
+// `downs`) and level y's raising ones at its back (from `ups`, downwards) as
+// tasks a | b << 6 | d << 12 | tag: the lanes take 32 pairs (b, d) of either
+// order at a time, and one scan of both counts places them.  False when the
+// list is too short.
+template <class Word>
+__device__ __forceinline__ bool append_hops(const FillSub<Word>& x, uint32_t xtag, const FillSub<Word>& y, uint32_t ytag,
+                                            int upper, int lane, uint32_t* tasks, int cap, int& downs, int& ups)
+{
+    const int nx = upper ? 0 : x.N * x.M, ny = y.N * y.M;
+    PairWalk dw(lane, max(1, x.M)), uw(lane, max(1, y.N));
+    for (int q = 0; q < max(nx, ny); q += 32) {
+        Word md = 0, mu = 0;
+        uint32_t td = xtag, tu = ytag;
+        if (q + lane < nx) {
+            const int b = x.orbs[x.N - 1 - dw.i], d = x.orbs[x.N + dw.j];
+            if (d < b && 2 * d > b) md = x.in & (x.empty >> (b - d)) & (((Word)1 << (2 * d - b)) - 1);
+            td |= (uint32_t)(d << 12 | b << 6);
+        }
+        if (q + lane < ny) {
+            const int d = y.orbs[y.N + uw.i], b = y.orbs[y.N - 1 - uw.j];
+            if (d > b) mu = y.in & (y.empty << (d - b)) & (((Word)1 << b) - 1);
+            tu |= (uint32_t)(d << 12 | b << 6);
+        }
+        dw.next();
+        uw.next();
+        const uint32_t c = (uint32_t)(bit_count(md) | bit_count(mu) << 16);
+        uint32_t s = c;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t v = __shfl_up_sync(0xffffffffu, s, o);
+            if (lane >= o) s += v;
+        }
+        const uint32_t all = __shfl_sync(0xffffffffu, s, 31);
+        const int dn = (int)(all & 0xFFFF), un = (int)(all >> 16);
+        if (downs + ups + dn + un >= cap) return false;
+        s -= c;
+        uint32_t* p = tasks + downs + (s & 0xFFFF);
+        for (; md; md &= md - 1)
+            *p++ = td | (uint32_t)(sizeof(Word) == 4 ? __ffs((int)md) - 1 : __ffsll((long long)md) - 1);
+        p = tasks + cap - 1 - ups - (s >> 16);
+        while (mu) {
+            const int a = sizeof(Word) == 4 ? 31 - __clz((int)mu) : 63 - __clzll((long long)mu);
+            *p-- = tu | (uint32_t)a;
+            mu ^= (Word)1 << a;
+        }
+        downs += dn;
+        ups += un;
+    }
+    return true;
+}
+
+// A level's hop table; level 0 is the high part of the word.
+struct FillLevel {
+    const double* w;
+    const int* off;
+    int nw, K;
+};
+
+// In shared memory: the weights, and per pair sum s the pair (offset, count),
+// with which the hop (a, b) -> (c, d) is weight offset + a count + c.
+struct FillTable {
+    const uint64_t* w;
+    const int2* sum;
+};
+
+__host__ __device__ inline size_t fill_table_bytes(const FillLevel& l) { return (((size_t)l.nw * 8 + 15) & ~(size_t)15) + (size_t)l.K * 16; }
+
+__device__ __forceinline__ FillTable load_fill_table(unsigned char* smem, const FillLevel& l)
+{
+    uint64_t* w = reinterpret_cast<uint64_t*>(smem);
+    int2* sum = reinterpret_cast<int2*>(smem + (((size_t)l.nw * 8 + 15) & ~(size_t)15));
+    for (int i = threadIdx.x; i < l.nw; i += blockDim.x) w[i] = (uint64_t)__double_as_longlong(l.w[i]);
+    for (int t = threadIdx.x; t < 2 * l.K; t += blockDim.x) {
+        const int cnt = pair_cnt(t, l.K);
+        sum[t] = make_int2(l.off[t] - pair_lo(t, l.K) * (cnt + 1), cnt);
+    }
+    return FillTable{w, sum};
+}
+
+__host__ __device__ inline size_t fill_list_bytes(int cap) { return ((size_t)cap * 4 + 15) & ~(size_t)15; }
+__host__ __device__ inline size_t fill_warp_bytes(int levels, int cap) { return fill_list_bytes(cap) + 64 * levels; }
+
+// Word: the levels' words, 32 bits up to 32 orbitals a level (two levels:
+// always; 48 bits together).
+template <int LV, class Word>
+__global__ void __launch_bounds__(512) k_fill_rows(
+    const uint64_t* __restrict__ words, int64_t n, const double* __restrict__ diag, FillLevel l0, FillLevel l1,
+    int upper, const int64_t* __restrict__ rowptr, const uint64_t* __restrict__ hi, const uint64_t* __restrict__ lo_tab,
+    int L, int cap, int32_t* __restrict__ col, double* __restrict__ val, int* __restrict__ err)
+{
+    constexpr int kBits = 8 * sizeof(Word);
+    extern __shared__ __align__(16) unsigned char smem[];
+    FillTable tab[LV];
+    tab[0] = load_fill_table(smem, l0);
+    size_t tbytes = fill_table_bytes(l0);
+    if constexpr (LV == 2) {
+        tab[1] = load_fill_table(smem + tbytes, l1);
+        tbytes += fill_table_bytes(l1);
+    }
+    __syncthreads();
+    const int lane = threadIdx.x & 31;
+    unsigned char* wbase = smem + tbytes + (size_t)(threadIdx.x >> 5) * fill_warp_bytes(LV, cap);
+    uint32_t* tasks = reinterpret_cast<uint32_t*>(wbase);
+    unsigned char* orbs = wbase + fill_list_bytes(cap);   // per level: occupied, then empty orbitals
+    const unsigned lt = (1u << lane) - 1u;
+    const int shift = LV == 2 ? l1.K : 0;
+    const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
+    for (int64_t r = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; r < n; r += nwarps) {
+        const uint64_t in = words[r];
+        const int64_t base = rowptr[r];
+        const int want = (int)(rowptr[r + 1] - base);
+        FillSub<Word> sub[LV];
+#pragma unroll
+        for (int v = 0; v < LV; ++v) {
+            const int K = v ? l1.K : l0.K;
+            const Word kmask = K >= kBits ? ~(Word)0 : ((Word)1 << K) - 1;
+            FillSub<Word>& s = sub[v];
+            s.in = v ? (Word)in & kmask : (Word)(in >> shift);
+            s.empty = ~s.in & kmask;
+            s.N = bit_count(s.in);
+            s.M = K - s.N;
+            s.orbs = orbs + 64 * v;
+            for (int o = lane; o < K; o += 32) {
+                const int below = bit_count(s.in & (((Word)1 << o) - 1));
+                orbs[64 * v + (((s.in >> o) & 1) ? below : s.N + o - below)] = (unsigned char)o;
+            }
+        }
+        __syncwarp();
+        // level 0 lowers first and raises last
+        int downs = 0, ups = 0;
+        bool fits = append_hops(sub[0], 0u, sub[LV - 1], (uint32_t)(LV - 1) << 18, upper, lane, tasks, cap, downs, ups);
+        if constexpr (LV == 2)
+            fits = fits && append_hops(sub[1], 1u << 18, sub[0], 0u, upper, lane, tasks, cap, downs, ups);
+        __syncwarp();
+        if (!fits) {   // the count pass sized cap above every row's hops
+            if (lane == 0) atomicOr(err, 4);
+            __syncwarp();
+            continue;
+        }
+        const int all = downs + 1 + ups;
+        int cnt = 0;
+        for (int t0 = 0; t0 < all; t0 += 32) {
+            uint64_t vb = 0, rk = (uint64_t)r;
+            bool ok = false;
+            const int t = t0 + lane;
+            if (t < all) {
+                if (t == downs) {
+                    const double dv = diag[r];
+                    vb = (uint64_t)__double_as_longlong(dv);
+                    ok = !(fabs(dv) < kSparseZeroTol);
+                } else {
+                    const uint32_t task = tasks[t < downs ? t : cap + downs - t];
+                    const bool second = LV == 2 && (task >> 18);
+                    const int a = task & 63, b = (task >> 6) & 63, d = (task >> 12) & 63, c = a + b - d;
+                    const Word s = second ? sub[LV - 1].in : sub[0].in;
+                    const Word A = (Word)1 << a, B = (Word)1 << b, C = (Word)1 << c, D = (Word)1 << d;
+                    const Word o = s ^ A ^ B ^ C ^ D;
+                    const FillTable ft = second ? tab[LV - 1] : tab[0];
+                    const int2 sum = ft.sum[a + b];
+                    vb = ft.w[sum.x + (d > b ? a * sum.y + c : c * sum.y + a)];
+                    ok = !hop_zero(vb);
+                    // hop_parity: the occupied orbitals between a and c and
+                    // between b and d, and one of the four itself
+                    const Word par = s & ((A - 1) ^ (B - 1) ^ (C - 1) ^ (D - 1));
+                    vb ^= (uint64_t)(bit_count(par) & 1) << 63;
+                    rk = rank_in_sector(LV == 1 ? (uint64_t)o : second ? in ^ (uint64_t)(s ^ o) : in ^ ((uint64_t)(s ^ o) << shift),
+                                        hi, lo_tab, L);
+                    if (rk == kMiss) { atomicOr(err, 2); rk = 0; }
+                }
+            }
+            const unsigned m = __ballot_sync(0xffffffffu, ok);
+            const int at = cnt + __popc(m & lt);
+            if (ok && at < want) {
+                col[base + at] = (int32_t)rk;
+                val[base + at] = bits_to_double(vb);
+            }
+            cnt += __popc(m);
+        }
+        if (cnt != want && lane == 0) atomicOr(err, 1);
+        __syncwarp();
+    }
+}
+
+// ---------------------------------------------------------------------------
+// Sort of a row in registers (k_cfill): 32-bit keys (column << sb | slot),
+// padded to 32*E with 0xFFFFFFFF, by a bitonic network over the element index
+// lane*E + e: exchanges whose partner is nearer than E stay in one lane's
+// registers, the rest take one shuffle.  The sorted keys go back through a
+// swizzled shared-memory image (index i ^ ((i >> 5) & 31), conflict-free both
+// ways).
 
 constexpr int kFillMaxE = 32;   // 32 * 32 = 1024 elements per row at most
-
-__host__ __device__ inline size_t fill_reg_warp_bytes(int cap)
-{
-    return ((size_t)cap * 12 + 64 + 15) & ~(size_t)15;
-}
 
 __device__ __forceinline__ int swz(int i) { return i ^ ((i >> 5) & 31); }
 
@@ -270,120 +519,6 @@ __device__ __forceinline__ void sort_row_dispatch(uint32_t* keys, int cnt, int l
     sort_row_keys<E>(keys, cnt, lane);
 }
 
-template <int EM>
-__global__ void __launch_bounds__(256) k_fill_reg(
-    const uint64_t* __restrict__ words, int64_t n, const double* __restrict__ diag, const double* __restrict__ w,
-    int nw, const double* __restrict__ da, const double* __restrict__ db, const int* __restrict__ off, int K, int N,
-    int upper, const int64_t* __restrict__ rowptr, const uint64_t* __restrict__ hi, const uint64_t* __restrict__ lo_tab,
-    int L, int cap, int sb, int32_t* __restrict__ col, double* __restrict__ val, int* __restrict__ err)
-{
-    extern __shared__ __align__(16) unsigned char smem[];
-    const HopView hv = load_hop_smem(smem, w, nw, da, db, off, K);
-    const size_t tbytes = (hop_smem_bytes(K, nw) + 15) & ~(size_t)15;
-    const int warp_in_cta = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int npairs = N * (N - 1) / 2;
-    unsigned char* wbase = smem + tbytes + (size_t)warp_in_cta * fill_reg_warp_bytes(cap);
-    double* vals = reinterpret_cast<double*>(wbase);
-    uint32_t* keys = reinterpret_cast<uint32_t*>(wbase + (size_t)cap * 8);
-    unsigned char* occ = wbase + (size_t)cap * 12;
-    const uint32_t smask = (uint32_t)cap - 1u;
-    const unsigned lt = (1u << lane) - 1u;
-    const int64_t gw = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
-    const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
-    for (int64_t r = gw; r < n; r += nwarps) {
-        const uint64_t in = words[r];
-        const int64_t base = rowptr[r];
-        const int64_t want = rowptr[r + 1] - base;
-        for (int pos0 = 0; pos0 < K; pos0 += 32) {
-            const int pos = pos0 + lane;
-            const bool set = pos < K && ((in >> pos) & 1ull);
-            const unsigned m = __ballot_sync(0xffffffffu, set);
-            if (set) occ[__popc(m & lt) + __popcll(in & ((1ull << pos0) - 1ull))] = (unsigned char)pos;
-        }
-        __syncwarp();
-        // task list: the admissible (a, b, c) of every occupied pair
-        int total = 0;
-        for (int p0 = 0; p0 < npairs; p0 += 32) {
-            const int p = p0 + lane;
-            uint64_t m = 0;
-            int a = 0, b = 0;
-            if (p < npairs) {
-                int j = (int)((1.0f + sqrtf(1.0f + 8.0f * (float)p)) * 0.5f);
-                while (j * (j - 1) / 2 > p) --j;
-                while ((j + 1) * j / 2 <= p) ++j;
-                a = occ[p - j * (j - 1) / 2];
-                b = occ[j];
-                m = hop_targets(in, a, b, K, upper != 0);
-            }
-            const int pc = __popcll(m);
-            int x = pc;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const int y = __shfl_up_sync(0xffffffffu, x, o);
-                if (lane >= o) x += y;
-            }
-            int pos = total + x - pc;
-            for (; m; m &= m - 1, ++pos)
-                if (pos < cap) keys[pos] = (uint32_t)(a | (b << 6) | ((__ffsll((long long)m) - 1) << 12));
-            total += __shfl_sync(0xffffffffu, x, 31);
-        }
-        __syncwarp();
-        if (total >= cap) {   // the count pass sized cap above every row's tasks
-            if (lane == 0) atomicOr(err, 4);
-            __syncwarp();
-            continue;
-        }
-        int cnt = 0;
-        for (int t0 = 0; t0 < total; t0 += 32) {
-            const int t = t0 + lane;
-            const uint32_t task = t < total ? keys[t] : 0u;
-            __syncwarp();
-            uint32_t key = 0;
-            uint64_t vb = 0;
-            bool ok = false;
-            if (t < total) {
-                const int a = task & 63, b = (task >> 6) & 63, c = (task >> 12) & 63, d = a + b - c;
-                const uint64_t out = in ^ (1ull << a) ^ (1ull << b) ^ (1ull << c) ^ (1ull << d);
-                vb = hop_bits(hv, in, out, a, b, c, d);
-                if (!hop_zero(vb)) {
-                    const uint64_t rk = rank_in_sector(out, hi, lo_tab, L);
-                    if (rk == kMiss) atomicOr(err, 2);
-                    key = (uint32_t)rk << sb;
-                    ok = true;
-                }
-            }
-            const unsigned m = __ballot_sync(0xffffffffu, ok);
-            if (ok) {
-                const int slot = cnt + __popc(m & lt);
-                keys[slot] = key | (uint32_t)slot;
-                vals[slot] = bits_to_double(vb);
-            }
-            cnt += __popc(m);
-        }
-        const double dv = diag[r];
-        if (!(fabs(dv) < kSparseZeroTol)) {
-            if (lane == 0 && cnt < cap) {
-                keys[cnt] = ((uint32_t)r << sb) | (uint32_t)cnt;
-                vals[cnt] = dv;
-            }
-            ++cnt;
-        }
-        __syncwarp();
-        if (cnt != want || cnt > cap) {
-            if (lane == 0) atomicOr(err, 1);
-            __syncwarp();
-            continue;
-        }
-        if (cnt > 0) sort_row_dispatch<1, EM>(keys, cnt, lane);
-        for (int t = lane; t < cnt; t += 32) {
-            const uint32_t kk = keys[swz(t)];
-            col[base + t] = (int32_t)(kk >> sb);
-            val[base + t] = vals[kk & smask];
-        }
-        __syncwarp();
-    }
-}
-
 // ---------------------------------------------------------------------------
 // Two Landau levels: TwoLevelSpinlessFermionHamiltonian
 // (two_level_spinless_fermion_hamiltonian.hpp:143-470) as
@@ -413,53 +548,32 @@ __host__ __device__ inline size_t two_level_table_bytes(int K0, int nw0, int K1,
     return ((hop_smem_bytes(K0, nw0) + 15) & ~(size_t)15) + ((hop_smem_bytes(K1, nw1) + 15) & ~(size_t)15);
 }
 
-__global__ void k_diag2(const uint64_t* __restrict__ words, int64_t n, const double* __restrict__ e0,
-                        const double* __restrict__ e1, const double* __restrict__ da0, const double* __restrict__ db0,
-                        int K0, const double* __restrict__ da1, const double* __restrict__ db1, int K1,
-                        double* __restrict__ diag)
-{
-    extern __shared__ __align__(16) unsigned char smem[];
-    double* sda0 = reinterpret_cast<double*>(smem);
-    double* sdb0 = sda0 + K0 * K0;
-    double* sda1 = sdb0 + K0 * K0;
-    double* sdb1 = sda1 + K1 * K1;
-    double* se0 = sdb1 + K1 * K1;
-    double* se1 = se0 + K0;
-    for (int i = threadIdx.x; i < K0 * K0; i += blockDim.x) { sda0[i] = da0[i]; sdb0[i] = db0[i]; }
-    for (int i = threadIdx.x; i < K1 * K1; i += blockDim.x) { sda1[i] = da1[i]; sdb1[i] = db1[i]; }
-    for (int i = threadIdx.x; i < K0; i += blockDim.x) se0[i] = e0[i];
-    for (int i = threadIdx.x; i < K1; i += blockDim.x) se1[i] = e1[i];
-    __syncthreads();
-    const HopView h0{nullptr, sda0, sdb0, nullptr, K0}, h1{nullptr, sda1, sdb1, nullptr, K1};
-    const uint64_t m1 = (1ull << K1) - 1ull;
-    for (int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; r < n; r += (int64_t)gridDim.x * blockDim.x) {
-        const uint64_t w = words[r], first = w >> K1, second = w & m1;
-        double acc = 0.0;
-        for (uint64_t t = first; t; t &= t - 1) acc = acc + se0[__ffsll((long long)t) - 1];
-        for (uint64_t t = second; t; t &= t - 1) acc = acc + se1[__ffsll((long long)t) - 1];
-        acc = diag_element(h0, first, acc);
-        diag[r] = diag_element(h1, second, acc);
-    }
-}
-
-__global__ void k_count2(const uint64_t* __restrict__ words, int64_t n, const double* __restrict__ diag,
+// k_count for two levels.  The diagonal is one running sum: level-0 energies,
+// level-1 energies, then either level's quartic terms.
+__global__ void k_count2(const uint64_t* __restrict__ words, int64_t n, const double* __restrict__ e0,
+                         const double* __restrict__ e1, double* __restrict__ diag,
                          const double* __restrict__ w0, int nw0, const double* __restrict__ da0,
                          const double* __restrict__ db0, const int* __restrict__ off0, int K0, int nozero0,
                          const double* __restrict__ w1, int nw1, const double* __restrict__ da1,
                          const double* __restrict__ db1, const int* __restrict__ off1, int K1, int nozero1, int upper,
-                         int64_t* __restrict__ rowlen, int* __restrict__ maxtasks)
+                         int64_t* __restrict__ rowlen, int* __restrict__ maxes)
 {
     extern __shared__ __align__(16) unsigned char smem[];
     HopView h0, h1;
     load_two_level(smem, w0, nw0, da0, db0, off0, K0, w1, nw1, da1, db1, off1, K1, h0, h1);
     const uint64_t m1 = (1ull << K1) - 1ull;
-    unsigned tmax = 0;
+    unsigned tmax = 0, rmax = 0;
     for (int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; r < n; r += (int64_t)gridDim.x * blockDim.x) {
-        const uint64_t w = words[r];
-        int64_t cnt = (fabs(diag[r]) < kSparseZeroTol) ? 0 : 1;
+        const uint64_t w = words[r], first = w >> K1, second = w & m1;
+        double dv = 0.0;
+        for (uint64_t t = first; t; t &= t - 1) dv = dv + __ldg(e0 + (__ffsll((long long)t) - 1));
+        for (uint64_t t = second; t; t &= t - 1) dv = dv + __ldg(e1 + (__ffsll((long long)t) - 1));
+        dv = diag_element(h1, second, diag_element(h0, first, dv));
+        diag[r] = dv;
+        unsigned cnt = (fabs(dv) < kSparseZeroTol) ? 0 : 1;
         unsigned tasks = 1;
         for (int lvl = 0; lvl < 2; ++lvl) {
-            const uint64_t in = lvl ? (w & m1) : (w >> K1);
+            const uint64_t in = lvl ? second : first;
             const HopView& hv = lvl ? h1 : h0;
             const int K = lvl ? K1 : K0;
             const bool nz = (lvl ? nozero1 : nozero0) != 0;
@@ -484,139 +598,10 @@ __global__ void k_count2(const uint64_t* __restrict__ words, int64_t n, const do
             }
         }
         rowlen[r] = cnt;
-        tmax = tasks > tmax ? tasks : tmax;
+        tmax = max(tmax, tasks);
+        rmax = max(rmax, cnt);
     }
-    tmax = __reduce_max_sync(0xffffffffu, tmax);
-    if ((threadIdx.x & 31) == 0) atomicMax(maxtasks, (int)tmax);
-}
-
-// One warp per row of the two-level Hamiltonian: the admissible hops of every
-// same-level occupied pair as tasks (level << 18 | a | b << 6 | c << 12, level
-// positions), ranked as generated, register-sorted and stored as k_fill_reg does.
-template <int EM>
-__global__ void __launch_bounds__(256) k_fill2(
-    const uint64_t* __restrict__ words, int64_t n, const double* __restrict__ diag, const double* __restrict__ w0,
-    int nw0, const double* __restrict__ da0, const double* __restrict__ db0, const int* __restrict__ off0, int K0,
-    const double* __restrict__ w1, int nw1, const double* __restrict__ da1, const double* __restrict__ db1,
-    const int* __restrict__ off1, int K1, int N, int upper, const int64_t* __restrict__ rowptr,
-    const uint64_t* __restrict__ hi, const uint64_t* __restrict__ lo_tab, int L, int cap, int sb,
-    int32_t* __restrict__ col, double* __restrict__ val, int* __restrict__ err)
-{
-    extern __shared__ __align__(16) unsigned char smem[];
-    HopView h0, h1;
-    load_two_level(smem, w0, nw0, da0, db0, off0, K0, w1, nw1, da1, db1, off1, K1, h0, h1);
-    const size_t tbytes = two_level_table_bytes(K0, nw0, K1, nw1);
-    const int warp_in_cta = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int npairs = N * (N - 1) / 2;
-    const int K = K0 + K1;
-    unsigned char* wbase = smem + tbytes + (size_t)warp_in_cta * fill_reg_warp_bytes(cap);
-    double* vals = reinterpret_cast<double*>(wbase);
-    uint32_t* keys = reinterpret_cast<uint32_t*>(wbase + (size_t)cap * 8);
-    unsigned char* occ = wbase + (size_t)cap * 12;
-    const uint32_t smask = (uint32_t)cap - 1u;
-    const unsigned lt = (1u << lane) - 1u;
-    const uint64_t m1 = (1ull << K1) - 1ull;
-    const int64_t gw = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
-    const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
-    for (int64_t r = gw; r < n; r += nwarps) {
-        const uint64_t in = words[r], first = in >> K1, second = in & m1;
-        const int64_t base = rowptr[r];
-        const int64_t want = rowptr[r + 1] - base;
-        for (int pos0 = 0; pos0 < K; pos0 += 32) {
-            const int pos = pos0 + lane;
-            const bool set = pos < K && ((in >> pos) & 1ull);
-            const unsigned m = __ballot_sync(0xffffffffu, set);
-            if (set) occ[__popc(m & lt) + __popcll(in & ((1ull << pos0) - 1ull))] = (unsigned char)pos;
-        }
-        __syncwarp();
-        int total = 0;
-        for (int p0 = 0; p0 < npairs; p0 += 32) {
-            const int p = p0 + lane;
-            uint64_t m = 0;
-            uint32_t tag = 0;
-            if (p < npairs) {
-                int j = (int)((1.0f + sqrtf(1.0f + 8.0f * (float)p)) * 0.5f);
-                while (j * (j - 1) / 2 > p) --j;
-                while ((j + 1) * j / 2 <= p) ++j;
-                const int a = occ[p - j * (j - 1) / 2], b = occ[j];
-                if (b < K1) {                           // both in level 1 (the low word)
-                    m = hop_targets(second, a, b, K1, upper != 0);
-                    tag = (1u << 18) | (uint32_t)a | ((uint32_t)b << 6);
-                } else if (a >= K1) {                   // both in level 0
-                    m = hop_targets(first, a - K1, b - K1, K0, upper != 0);
-                    tag = (uint32_t)(a - K1) | ((uint32_t)(b - K1) << 6);
-                }
-            }
-            const int pc = __popcll(m);
-            int x = pc;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const int y = __shfl_up_sync(0xffffffffu, x, o);
-                if (lane >= o) x += y;
-            }
-            int pos = total + x - pc;
-            for (; m; m &= m - 1, ++pos)
-                if (pos < cap) keys[pos] = tag | ((uint32_t)(__ffsll((long long)m) - 1) << 12);
-            total += __shfl_sync(0xffffffffu, x, 31);
-        }
-        __syncwarp();
-        if (total >= cap) {
-            if (lane == 0) atomicOr(err, 4);
-            __syncwarp();
-            continue;
-        }
-        int cnt = 0;
-        for (int t0 = 0; t0 < total; t0 += 32) {
-            const int t = t0 + lane;
-            const uint32_t task = t < total ? keys[t] : 0u;
-            __syncwarp();
-            uint32_t key = 0;
-            uint64_t vb = 0;
-            bool ok = false;
-            if (t < total) {
-                const int lvl1 = (task >> 18) & 1;
-                const int a = task & 63, b = (task >> 6) & 63, c = (task >> 12) & 63, d = a + b - c;
-                const uint64_t sub = lvl1 ? second : first;
-                const uint64_t out_sub = sub ^ (1ull << a) ^ (1ull << b) ^ (1ull << c) ^ (1ull << d);
-                vb = hop_bits(lvl1 ? h1 : h0, sub, out_sub, a, b, c, d);
-                if (!hop_zero(vb)) {
-                    const uint64_t out = lvl1 ? ((first << K1) | out_sub) : ((out_sub << K1) | second);
-                    const uint64_t rk = rank_in_sector(out, hi, lo_tab, L);
-                    if (rk == kMiss) atomicOr(err, 2);
-                    key = (uint32_t)rk << sb;
-                    ok = true;
-                }
-            }
-            const unsigned m = __ballot_sync(0xffffffffu, ok);
-            if (ok) {
-                const int slot = cnt + __popc(m & lt);
-                keys[slot] = key | (uint32_t)slot;
-                vals[slot] = bits_to_double(vb);
-            }
-            cnt += __popc(m);
-        }
-        const double dv = diag[r];
-        if (!(fabs(dv) < kSparseZeroTol)) {
-            if (lane == 0 && cnt < cap) {
-                keys[cnt] = ((uint32_t)r << sb) | (uint32_t)cnt;
-                vals[cnt] = dv;
-            }
-            ++cnt;
-        }
-        __syncwarp();
-        if (cnt != want || cnt > cap) {
-            if (lane == 0) atomicOr(err, 1);
-            __syncwarp();
-            continue;
-        }
-        if (cnt > 0) sort_row_dispatch<1, EM>(keys, cnt, lane);
-        for (int t = lane; t < cnt; t += 32) {
-            const uint32_t kk = keys[swz(t)];
-            col[base + t] = (int32_t)(kk >> sb);
-            val[base + t] = vals[kk & smask];
-        }
-        __syncwarp();
-    }
+    row_maxes(tmax, rmax, maxes);
 }
 
 // Level-exchange ladder of the two-level basis: y += T x with T = L0- L1+
@@ -861,6 +846,103 @@ int sm_count()
     return sms;
 }
 
+bool all_hops_nonzero(const ed_terms& t)
+{
+    const int K = t.norb;
+    for (int s = 1; s <= 2 * K - 3; ++s) {
+        const int cnt = pair_cnt(s, K);
+        for (int ia = 0; ia < cnt; ++ia)
+            for (int ic = 0; ic < cnt; ++ic)
+                if (ic != ia && t.hop.w[t.hop.hop_off[s] + ia * cnt + ic] == 0.0) return false;
+    }
+    return true;
+}
+
+FillLevel fill_level(const ed_terms& t) { return FillLevel{t.w_dev.p, t.hop_off_dev.p, (int)t.hop.w.size(), t.norb}; }
+
+// A build's temporaries in one allocation: the diagonal, the rows' lengths,
+// the scan's sums, and {nnz, {most tasks, longest row}, error flag}.
+struct RowCounts {
+    DevBuf<int64_t> buf;
+    int64_t n, *len, *sums, *tail;
+    double* diag;
+    int tasks = 0;
+    RowCounts(int64_t rows, cudaStream_t st) : buf((size_t)(2 * rows + scan_workspace_i64(rows) + 3)), n(rows)
+    {
+        diag = reinterpret_cast<double*>(buf.p);
+        len = buf.p + n;
+        sums = len + n;
+        tail = buf.p + buf.n - 3;
+        ED_CUDA(cudaMemsetAsync(tail, 0, 3 * sizeof(int64_t), st));
+    }
+    int* maxes() { return reinterpret_cast<int*>(tail + 1); }
+    int* err() { return reinterpret_cast<int*>(tail + 2); }
+    // The row pointers from the lengths; a's sizes and arrays.
+    void finish(ed_crs& a, cudaStream_t st)
+    {
+        exclusive_scan_i64(len, a.rowptr.p, n, sums, st);
+        ED_CUDA(cudaMemcpyAsync(tail, a.rowptr.p + n, sizeof(int64_t), cudaMemcpyDeviceToDevice, st));
+        int64_t h[2] = {0, 0};
+        ED_CUDA(cudaMemcpyAsync(h, tail, sizeof(h), cudaMemcpyDeviceToHost, st));
+        ED_CUDA(cudaStreamSynchronize(st));
+        a.nnz = h[0];
+        int m[2];
+        std::memcpy(m, h + 1, sizeof(m));
+        tasks = m[0];
+        a.max_row = m[1];
+        // kCrsPad zeroed elements past the end let the SpMV batches load
+        // without bounds tests (column 0, value 0)
+        a.col.alloc((size_t)a.nnz + kCrsPad);
+        a.val.alloc((size_t)a.nnz + kCrsPad);
+        ED_CUDA(cudaMemsetAsync(a.col.p + a.nnz, 0, kCrsPad * sizeof(int32_t), st));
+        ED_CUDA(cudaMemsetAsync(a.val.p + a.nnz, 0, kCrsPad * sizeof(double), st));
+    }
+    void check(cudaStream_t st, const char* what)
+    {
+        int e = 0;
+        ED_CUDA(cudaMemcpyAsync(&e, err(), sizeof(int), cudaMemcpyDeviceToHost, st));
+        ED_CUDA(cudaStreamSynchronize(st));
+        ED_REQUIRE(e == 0, ED_ERR_INTERNAL, what);
+    }
+};
+
+constexpr size_t kFillSmem = 200 * 1024;
+
+// The rows in column order; false when a row's task list does not fit beside
+// the tables.
+template <int LV, class Word>
+bool fill_rows(const ed_basis& b, const FillLevel& l0, const FillLevel& l1, RowCounts& rows, ed_crs& a, cudaStream_t st)
+{
+    auto kern = k_fill_rows<LV, Word>;
+    const int cap = (rows.tasks + 32) & ~31;   // above every row's hops; below 2^15, so that the packed counts hold
+    const size_t warp_b = fill_warp_bytes(LV, cap), tbytes = fill_table_bytes(l0) + (LV == 2 ? fill_table_bytes(l1) : 0);
+    if (tbytes + warp_b > kFillSmem || cap >= (1 << 15)) return false;
+    // warps per CTA: the most resident warps per SM
+    int wpc = 1, best = 0, blocks = 1;
+    for (int c = 16; c >= 1; c >>= 1) {
+        const size_t smem = tbytes + c * warp_b;
+        if (smem > kFillSmem) continue;
+        ED_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        int ob = 0;
+        ED_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&ob, kern, c * 32, smem));
+        if (ob * c > best) { best = ob * c; wpc = c; blocks = ob; }
+    }
+    const size_t smem = tbytes + wpc * warp_b;
+    ED_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    launch(kern, sm_count() * blocks, wpc * 32, smem, st, b.words.p, a.n, rows.diag, l0, l1, a.upper, a.rowptr.p, b.hi.p,
+           b.lo.p, b.low_bits, cap, a.col.p, a.val.p, rows.err());
+    rows.check(st, "Hamiltonian fill: row count or rank check failed on the device");
+    return true;
+}
+
+template <int LV>
+bool fill_rows(const ed_basis& b, const FillLevel& l0, const FillLevel& l1, RowCounts& rows, ed_crs& a, cudaStream_t st)
+{
+    if constexpr (LV == 1)
+        if (l0.K > 32) return fill_rows<1, uint64_t>(b, l0, l1, rows, a, st);
+    return fill_rows<LV, uint32_t>(b, l0, l1, rows, a, st);
+}
+
 }  // namespace
 
 void ham_diagonal(const ed_basis& b, const ed_terms& t, double* diag, cudaStream_t st)
@@ -893,81 +975,22 @@ void ham_build_crs(const ed_basis& b, const ed_terms& t, int upper, ed_crs& a, c
     const int K = t.norb;
     const int nw = (int)t.hop.w.size();
     const size_t tsm = hop_smem_bytes(K, nw);
-    DevBuf<double> diag(n);
-    ham_diagonal(b, t, diag.p, st);
-    DevBuf<int64_t> rowlen(n);
-    // with no zero off-diagonal weight every admissible hop is stored
-    int nozero = 1;
-    for (int s = 1; s <= 2 * K - 3 && nozero; ++s) {
-        const int cnt = pair_cnt(s, K);
-        for (int ia = 0; ia < cnt && nozero; ++ia)
-            for (int ic = 0; ic < cnt; ++ic)
-                if (ic != ia && t.hop.w[t.hop.hop_off[s] + ia * cnt + ic] == 0.0) { nozero = 0; break; }
-    }
-    DevBuf<int> maxtasks_dev(1);
-    ED_CUDA(cudaMemsetAsync(maxtasks_dev.p, 0, sizeof(int), st));
+    const FillLevel l0 = fill_level(t);
+    RowCounts rows(n, st);
     ED_CUDA(cudaFuncSetAttribute(k_count, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tsm));
-    k_count<<<sm_count() * 4, 256, tsm, st>>>(b.words.p, n, diag.p, t.w_dev.p, nw, t.diag_a_dev.p, t.diag_b_dev.p,
-                                              t.hop_off_dev.p, K, a.upper, nozero, rowlen.p, maxtasks_dev.p);
-    ::edgb::count_launch();
-    ED_CUDA(cudaGetLastError());
-    exclusive_scan_i64(rowlen.p, a.rowptr.p, n, st);
-    ED_CUDA(cudaMemcpyAsync(&a.nnz, a.rowptr.p + n, sizeof(int64_t), cudaMemcpyDeviceToHost, st));
-    int maxtasks = 0;
-    ED_CUDA(cudaMemcpyAsync(&maxtasks, maxtasks_dev.p, sizeof(int), cudaMemcpyDeviceToHost, st));
-    const int64_t maxrow = reduce_max_i64_host(rowlen.p, n, st);
-    ED_CUDA(cudaStreamSynchronize(st));
-    a.max_row = (int)maxrow;
-    // kCrsPad zeroed elements past the end let the SpMV batches load
-    // without bounds tests (column 0, value 0)
-    a.col.alloc((size_t)a.nnz + kCrsPad);
-    a.val.alloc((size_t)a.nnz + kCrsPad);
-    ED_CUDA(cudaMemsetAsync(a.col.p + a.nnz, 0, kCrsPad * sizeof(int32_t), st));
-    ED_CUDA(cudaMemsetAsync(a.val.p + a.nnz, 0, kCrsPad * sizeof(double), st));
-    int cap = 32, sb = 5;
-    while (cap < maxrow) { cap <<= 1; ++sb; }
+    // with no zero off-diagonal weight every admissible hop is stored
+    launch(k_count, sm_count() * 4, 256, tsm, st, b.words.p, n, rows.diag, t.w_dev.p, nw, t.diag_a_dev.p, t.diag_b_dev.p,
+           t.hop_off_dev.p, K, a.upper, all_hops_nonzero(t) ? 1 : 0, rows.len, rows.maxes());
+    rows.finish(a, st);
     const size_t tbytes = (tsm + 15) & ~(size_t)15;
-    const size_t budget = 200 * 1024;
-    DevBuf<int> err(1);
-    ED_CUDA(cudaMemsetAsync(err.p, 0, sizeof(int), st));
-    // register sort when a row's tasks and elements fit 32*kFillMaxE keys of
-    // (column << rsb | slot) below 0xFFFFFFFF; ED_FILL_SORT=smem selects the
-    // shared-memory sort for every sector
-    int rcap = 32, rsb = 5;
-    while (rcap < std::max<int64_t>(maxrow, maxtasks + 1)) { rcap <<= 1; ++rsb; }
-    const size_t reg_warp = fill_reg_warp_bytes(rcap);
+    // ED_FILL_SORT=smem selects the shared-memory sort
     const char* sort_env = std::getenv("ED_FILL_SORT");
-    const bool force_smem = sort_env && std::strcmp(sort_env, "smem") == 0;
-    if (!force_smem && rcap <= 32 * kFillMaxE &&
-        ((((uint64_t)(n - 1)) << rsb) | (uint64_t)(rcap - 1)) < 0xFFFFFFFFull && tbytes + reg_warp <= budget) {
-        const int smax = std::min<int>(8, (int)((budget - tbytes) / reg_warp));
-        auto launch = [&](auto kern) {
-            // warps per CTA: the most resident warps per SM, then the larger CTA
-            int wpc = smax, best = 0, occ_best = 1;
-            for (int c = smax; c >= 1; --c) {
-                const size_t sm_c = tbytes + (size_t)c * reg_warp;
-                ED_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_c));
-                int ob = 0;
-                ED_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&ob, kern, c * 32, sm_c));
-                if (ob * c > best) { best = ob * c; wpc = c; occ_best = ob < 1 ? 1 : ob; }
-            }
-            const size_t smem = tbytes + (size_t)wpc * reg_warp;
-            ED_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-            kern<<<sm_count() * occ_best, wpc * 32, smem, st>>>(
-                b.words.p, n, diag.p, t.w_dev.p, nw, t.diag_a_dev.p, t.diag_b_dev.p, t.hop_off_dev.p, K, b.N,
-                a.upper, a.rowptr.p, b.hi.p, b.lo.p, b.low_bits, rcap, rsb, a.col.p, a.val.p, err.p);
-            ::edgb::count_launch();
-        };
-        if (rcap <= 128) launch(k_fill_reg<4>);
-        else if (rcap <= 512) launch(k_fill_reg<16>);
-        else launch(k_fill_reg<32>);
-        ED_CUDA(cudaGetLastError());
-        int herr = 0;
-        ED_CUDA(cudaMemcpyAsync(&herr, err.p, sizeof(int), cudaMemcpyDeviceToHost, st));
-        ED_CUDA(cudaStreamSynchronize(st));
-        ED_REQUIRE(herr == 0, ED_ERR_INTERNAL, "Hamiltonian fill: row count or rank check failed on the device");
+    if (!(sort_env && std::strcmp(sort_env, "smem") == 0) &&
+        fill_rows<1>(b, l0, l0, rows, a, st))
         return;
-    }
+    int cap = 32;
+    while (cap < a.max_row) cap <<= 1;
+    const size_t budget = kFillSmem;
     const size_t per_warp = (size_t)cap * 16 + 4 + 64;
     ED_REQUIRE(tbytes + per_warp <= budget, ED_ERR_RANGE, "Hamiltonian rows too long for the shared-memory sort");
     int wpc = (int)((budget - tbytes) / per_warp);
@@ -977,30 +1000,11 @@ void ham_build_crs(const ed_basis& b, const ed_terms& t, int upper, ed_crs& a, c
     int occ_blocks = 0;
     ED_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_blocks, k_fill, wpc * 32, smem));
     if (occ_blocks < 1) occ_blocks = 1;
-    k_fill<<<sm_count() * occ_blocks, wpc * 32, smem, st>>>(b.words.p, n, diag.p, t.w_dev.p, nw, t.diag_a_dev.p,
-                                                             t.diag_b_dev.p, t.hop_off_dev.p, K, b.N, a.upper,
-                                                             a.rowptr.p, b.hi.p, b.lo.p, b.low_bits, cap, a.col.p,
-                                                             a.val.p, err.p); ::edgb::count_launch();
-    ED_CUDA(cudaGetLastError());
-    int herr = 0;
-    ED_CUDA(cudaMemcpyAsync(&herr, err.p, sizeof(int), cudaMemcpyDeviceToHost, st));
-    ED_CUDA(cudaStreamSynchronize(st));
-    ED_REQUIRE(herr == 0, ED_ERR_INTERNAL, "Hamiltonian fill: row count or rank check failed on the device");
+    launch(k_fill, sm_count() * occ_blocks, wpc * 32, smem, st, b.words.p, n, rows.diag, t.w_dev.p, nw, t.diag_a_dev.p,
+           t.diag_b_dev.p, t.hop_off_dev.p, K, b.N, a.upper, a.rowptr.p, b.hi.p, b.lo.p, b.low_bits, cap, a.col.p, a.val.p,
+           rows.err());
+    rows.check(st, "Hamiltonian fill: row count or rank check failed on the device");
 }
-
-namespace {
-bool all_hops_nonzero(const ed_terms& t)
-{
-    const int K = t.norb;
-    for (int s = 1; s <= 2 * K - 3; ++s) {
-        const int cnt = pair_cnt(s, K);
-        for (int ia = 0; ia < cnt; ++ia)
-            for (int ic = 0; ic < cnt; ++ic)
-                if (ic != ia && t.hop.w[t.hop.hop_off[s] + ia * cnt + ic] == 0.0) return false;
-    }
-    return true;
-}
-}  // namespace
 
 void ham2_build_crs(const ed_basis& b, const ed_terms& t0, const ed_terms& t1, const double* e0_host,
                     const double* e1_host, int upper, ed_crs& a, cudaStream_t st)
@@ -1031,64 +1035,19 @@ void ham2_build_crs(const ed_basis& b, const ed_terms& t0, const ed_terms& t1, c
     DevBuf<double> de0(K0), de1(K1);
     ED_CUDA(cudaMemcpyAsync(de0.p, e0.data(), K0 * 8, cudaMemcpyHostToDevice, st));
     ED_CUDA(cudaMemcpyAsync(de1.p, e1.data(), K1 * 8, cudaMemcpyHostToDevice, st));
-    DevBuf<double> diag(n);
-    const size_t dsm = ((size_t)2 * K0 * K0 + (size_t)2 * K1 * K1 + K0 + K1) * 8;
-    k_diag2<<<sm_count() * 8, 256, dsm, st>>>(b.words.p, n, de0.p, de1.p, t0.diag_a_dev.p, t0.diag_b_dev.p, K0,
-                                             t1.diag_a_dev.p, t1.diag_b_dev.p, K1, diag.p);
-    ::edgb::count_launch();
-    ED_CUDA(cudaGetLastError());
     const size_t tsm = two_level_table_bytes(K0, nw0, K1, nw1);
-    DevBuf<int64_t> rowlen(n);
-    DevBuf<int> maxtasks_dev(1);
-    ED_CUDA(cudaMemsetAsync(maxtasks_dev.p, 0, sizeof(int), st));
+    RowCounts rows(n, st);
     ED_CUDA(cudaFuncSetAttribute(k_count2, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tsm));
-    k_count2<<<sm_count() * 4, 256, tsm, st>>>(b.words.p, n, diag.p, t0.w_dev.p, nw0, t0.diag_a_dev.p,
-                                               t0.diag_b_dev.p, t0.hop_off_dev.p, K0, all_hops_nonzero(t0) ? 1 : 0,
-                                               t1.w_dev.p, nw1, t1.diag_a_dev.p, t1.diag_b_dev.p, t1.hop_off_dev.p, K1,
-                                               all_hops_nonzero(t1) ? 1 : 0, a.upper, rowlen.p, maxtasks_dev.p);
-    ::edgb::count_launch();
-    ED_CUDA(cudaGetLastError());
-    exclusive_scan_i64(rowlen.p, a.rowptr.p, n, st);
-    ED_CUDA(cudaMemcpyAsync(&a.nnz, a.rowptr.p + n, sizeof(int64_t), cudaMemcpyDeviceToHost, st));
-    int maxtasks = 0;
-    ED_CUDA(cudaMemcpyAsync(&maxtasks, maxtasks_dev.p, sizeof(int), cudaMemcpyDeviceToHost, st));
-    const int64_t maxrow = reduce_max_i64_host(rowlen.p, n, st);
-    ED_CUDA(cudaStreamSynchronize(st));
-    a.max_row = (int)maxrow;
-    a.col.alloc((size_t)a.nnz + kCrsPad);
-    a.val.alloc((size_t)a.nnz + kCrsPad);
-    ED_CUDA(cudaMemsetAsync(a.col.p + a.nnz, 0, kCrsPad * sizeof(int32_t), st));
-    ED_CUDA(cudaMemsetAsync(a.val.p + a.nnz, 0, kCrsPad * sizeof(double), st));
+    launch(k_count2, sm_count() * 4, 256, tsm, st, b.words.p, n, de0.p, de1.p, rows.diag, t0.w_dev.p, nw0, t0.diag_a_dev.p,
+           t0.diag_b_dev.p, t0.hop_off_dev.p, K0, all_hops_nonzero(t0) ? 1 : 0, t1.w_dev.p, nw1, t1.diag_a_dev.p,
+           t1.diag_b_dev.p, t1.hop_off_dev.p, K1, all_hops_nonzero(t1) ? 1 : 0, a.upper, rows.len, rows.maxes());
+    rows.finish(a, st);
     int cap = 32, sb = 5;
-    while (cap < std::max<int64_t>(maxrow, maxtasks + 1)) { cap <<= 1; ++sb; }
-    const size_t tbytes = tsm;
-    const size_t warp_b = fill_reg_warp_bytes(cap);
-    const size_t budget = 200 * 1024;
-    ED_REQUIRE(cap <= 32 * kFillMaxE && ((((uint64_t)(n - 1)) << sb) | (uint64_t)(cap - 1)) < 0xFFFFFFFFull &&
-                   tbytes + warp_b <= budget,
-               ED_ERR_RANGE, "two-level sector too large for the register-sort fill");
-    DevBuf<int> err(1);
-    ED_CUDA(cudaMemsetAsync(err.p, 0, sizeof(int), st));
-    const int wpc = std::min<int>(8, (int)((budget - tbytes) / warp_b));
-    const size_t smem = tbytes + (size_t)wpc * warp_b;
-    auto launch = [&](auto kern) {
-        ED_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        int ob = 0;
-        ED_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&ob, kern, wpc * 32, smem));
-        kern<<<sm_count() * std::max(1, ob), wpc * 32, smem, st>>>(
-            b.words.p, n, diag.p, t0.w_dev.p, nw0, t0.diag_a_dev.p, t0.diag_b_dev.p, t0.hop_off_dev.p, K0, t1.w_dev.p,
-            nw1, t1.diag_a_dev.p, t1.diag_b_dev.p, t1.hop_off_dev.p, K1, b.N, a.upper, a.rowptr.p, b.hi.p, b.lo.p,
-            b.low_bits, cap, sb, a.col.p, a.val.p, err.p);
-        ::edgb::count_launch();
-    };
-    if (cap <= 128) launch(k_fill2<4>);
-    else if (cap <= 512) launch(k_fill2<16>);
-    else launch(k_fill2<32>);
-    ED_CUDA(cudaGetLastError());
-    int herr = 0;
-    ED_CUDA(cudaMemcpyAsync(&herr, err.p, sizeof(int), cudaMemcpyDeviceToHost, st));
-    ED_CUDA(cudaStreamSynchronize(st));
-    ED_REQUIRE(herr == 0, ED_ERR_INTERNAL, "two-level fill: row count or rank check failed on the device");
+    while (cap < std::max(a.max_row, rows.tasks + 1)) { cap <<= 1; ++sb; }
+    // the rows and sectors that this build takes
+    ED_REQUIRE(cap <= 1024 && ((((uint64_t)(n - 1)) << sb) | (uint64_t)(cap - 1)) < 0xFFFFFFFFull &&
+                   fill_rows<2>(b, fill_level(t0), fill_level(t1), rows, a, st),
+               ED_ERR_RANGE, "two-level sector too large for the fill");
 }
 
 void cham_build_crs(const ed_basis& b, const ed_cterms& t, int upper, ed_ccrs& a, cudaStream_t st)

@@ -17,7 +17,7 @@ per second (one FMA per stored element per Hamiltonian, diagonal included).
 With --rotate n,m,k it times the thick-restart rotation of an n x m basis
 into k Ritz vectors (ed_basis_rotate) in FP64 and on the tensor cores.
 With --build it times the whole CRS build (diagonal, count, scan, fill;
-host clock around a synchronised call, best of reps) with the register-sort
+host clock around a synchronised call, best of reps) with the ordered
 fill and with the shared-memory fill (ED_FILL_SORT=smem).  With
 --observables it times the eigenvector observables (density, density-density,
 participation ratio, 100 most probable states) end to end from a host vector.
@@ -52,7 +52,7 @@ def main():
     ap.add_argument("--no-autotune", action="store_true", help="batch: keep the default tile (32 per row, L1)")
     ap.add_argument("--rotate", default="", help="n,m,k: time the restart rotation instead")
     ap.add_argument("--build", action="store_true",
-                    help="time the CRS build instead (register sort, then ED_FILL_SORT=smem)")
+                    help="time the CRS build instead (rows in order, then ED_FILL_SORT=smem)")
     ap.add_argument("--observables", action="store_true",
                     help="time the eigenvector observables on a seeded unit vector of the sector")
     ap.add_argument("--two-level", action="store_true", help="two-Landau-level sector N,norb0,twoLz")
@@ -136,7 +136,7 @@ def build_main(ed, torch, N, norb, tlz, args):
     import time
     T = ed.QuarticTermTables(norb, ed.odd_coulomb_list(norb))
     res = {"sector": [N, norb, tlz], "mode": "build", "layout": "upper" if args.upper else "full"}
-    for name, env in (("register", None), ("smem", "smem")):
+    for name, env in (("ordered", None), ("smem", "smem")):
         if env:
             os.environ["ED_FILL_SORT"] = env
         else:
