@@ -268,6 +268,71 @@ std::vector<int> basis_weights(const ed_basis& b)
 }
 
 namespace {
+// Low words by class: the class of word l is that of l without its lowest bit
+// plus that bit's own, so the tables take one step a word.
+struct LowTables {
+    std::vector<uint64_t> lo;                         // class << 32 | rank within the class
+    std::vector<uint32_t> tables;                     // per class count and start, then the words by class
+    uint32_t *count, *start, *list;
+    int nclass;
+    template <class ClassOf>
+    LowTables(int L, int classes, ClassOf class_of) : lo(1ull << L), tables(2 * (size_t)classes + (1ull << L)), nclass(classes)
+    {
+        count = tables.data();
+        start = count + classes;
+        list = start + classes;
+        const uint64_t nl = 1ull << L;
+        for (uint64_t l = 0; l < nl; ++l) {
+            const uint32_t cls = class_of(l);
+            lo[l] = ((uint64_t)cls << 32) | count[cls]++;
+        }
+        uint32_t acc = 0;
+        for (int c = 0; c < classes; ++c) { start[c] = acc; acc += count[c]; }
+        for (uint64_t l = 0; l < nl; ++l) list[start[lo[l] >> 32] + (uint32_t)lo[l]] = (uint32_t)l;
+    }
+};
+
+// A basis build's temporaries in one allocation: the high halves' counts and
+// offsets, the scan's sums, the class tables, the high bits' weights and the
+// high halves' classes.
+struct BasisTemps {
+    DevBuf<int64_t> buf;
+    int64_t nh, *counts, *offs, *sums;
+    uint32_t *count, *start, *list;
+    int* wh;
+    uint16_t* need;
+    BasisTemps(int H, const LowTables& t, const int* weights, cudaStream_t st)
+        : buf((2ull << H) + 1 + (size_t)scan_workspace_i64(1ll << H) + (t.tables.size() + 64 + 1) / 2 + ((1ull << H) + 3) / 4),
+          nh(1ll << H)
+    {
+        counts = buf.p;
+        offs = counts + nh;
+        sums = offs + nh + 1;
+        count = reinterpret_cast<uint32_t*>(sums + scan_workspace_i64(nh));
+        start = count + t.nclass;
+        list = start + t.nclass;
+        wh = reinterpret_cast<int*>(count + t.tables.size());
+        need = reinterpret_cast<uint16_t*>(wh + 64);
+        ED_CUDA(cudaMemcpyAsync(count, t.tables.data(), t.tables.size() * 4, cudaMemcpyHostToDevice, st));
+        if (weights) ED_CUDA(cudaMemcpyAsync(wh, weights, (size_t)H * sizeof(int), cudaMemcpyHostToDevice, st));
+    }
+    // The sector's dimension from the counts, and its words and high table.
+    void fill(ed_basis& b, cudaStream_t st)
+    {
+        exclusive_scan_i64(counts, offs, nh, sums, st);
+        int64_t dim = 0;
+        ED_CUDA(cudaMemcpyAsync(&dim, offs + nh, sizeof(int64_t), cudaMemcpyDeviceToHost, st));
+        ED_CUDA(cudaStreamSynchronize(st));
+        b.dim = (uint64_t)dim;
+        b.words.alloc(dim > 0 ? (size_t)dim : 1);
+        k_basis_fill<<<grid_for(nh * 32, 256), 256, 0, st>>>(b.high_bits, b.low_bits, offs, counts, need, start, list, b.words.p,
+                                                             b.hi.p);
+        ::edgb::count_launch();
+        ED_CUDA(cudaGetLastError());
+        ED_CUDA(cudaStreamSynchronize(st));
+    }
+};
+
 // Momentum-sector basis (the optical-flux-lattice FermionFockBasis with
 // TestLinearMomentumSector2, linear_momentum_constraints_2D.cpp:38-79).
 void basis_build_momentum(ed_basis& b, cudaStream_t st)
@@ -286,48 +351,24 @@ void basis_build_momentum(ed_basis& b, cudaStream_t st)
     const int nclass = (L + 1) * X * Y;
     ED_REQUIRE(nclass < 0xFFFF, ED_ERR_RANGE, "too many low-word classes");
     const uint64_t nl = 1ull << L;
-    std::vector<uint32_t> ccount(nclass, 0), cstart(nclass, 0), clist(nl), rank_in_class(nl);
-    std::vector<uint64_t> lo(nl);
-    for (uint64_t l = 0; l < nl; ++l) {
-        int sx = 0, sy = 0;
-        for (uint64_t x = l; x; x &= x - 1) {
-            const int p = __builtin_ctzll(x);
-            sx += p / Y;
-            sy += p % Y;
+    std::vector<uint32_t> sums(nl, 0);   // count << 20 | sum kx << 10 | sum ky
+    const LowTables t(L, nclass, [&](uint64_t l) {
+        if (l) {
+            const int p = __builtin_ctzll(l);
+            sums[l] = sums[l & (l - 1)] + (1u << 20 | (uint32_t)(p / Y) << 10 | (uint32_t)(p % Y));
         }
-        const int cls = (__builtin_popcountll(l) * X + sx % X) * Y + sy % Y;
-        rank_in_class[l] = ccount[cls]++;
-        lo[l] = ((uint64_t)cls << 32) | rank_in_class[l];
-    }
-    uint32_t acc = 0;
-    for (int c = 0; c < nclass; ++c) { cstart[c] = acc; acc += ccount[c]; }
-    for (uint64_t l = 0; l < nl; ++l) clist[cstart[lo[l] >> 32] + rank_in_class[l]] = (uint32_t)l;
+        const uint32_t c = sums[l];
+        return ((c >> 20) * X + (c >> 10 & 1023u) % X) * Y + (c & 1023u) % Y;
+    });
     b.lo.alloc(nl);
     b.hi.alloc(1ull << H);
-    DevBuf<uint32_t> d_ccount(nclass), d_cstart(nclass), d_clist(nl);
-    ED_CUDA(cudaMemcpyAsync(b.lo.p, lo.data(), nl * 8, cudaMemcpyHostToDevice, st));
-    ED_CUDA(cudaMemcpyAsync(d_ccount.p, ccount.data(), nclass * 4, cudaMemcpyHostToDevice, st));
-    ED_CUDA(cudaMemcpyAsync(d_cstart.p, cstart.data(), nclass * 4, cudaMemcpyHostToDevice, st));
-    ED_CUDA(cudaMemcpyAsync(d_clist.p, clist.data(), nl * 4, cudaMemcpyHostToDevice, st));
-    const int64_t nh = 1ll << H;
-    DevBuf<int64_t> counts(nh), offs(nh + 1);
-    DevBuf<uint16_t> need(nh);
-    k_basis_count_mom<<<grid_for(nh, 256), 256, 0, st>>>(H, L, N, X, Y, b.kx_tot, b.ky_tot, d_ccount.p, counts.p,
-                                                         need.p);
+    ED_CUDA(cudaMemcpyAsync(b.lo.p, t.lo.data(), nl * 8, cudaMemcpyHostToDevice, st));
+    BasisTemps tmp(H, t, nullptr, st);
+    k_basis_count_mom<<<grid_for(tmp.nh, 256), 256, 0, st>>>(H, L, N, X, Y, b.kx_tot, b.ky_tot, tmp.count, tmp.counts, tmp.need);
     ::edgb::count_launch();
     ED_CUDA(cudaGetLastError());
-    exclusive_scan_i64(counts.p, offs.p, nh, st);
-    int64_t dim = 0;
-    ED_CUDA(cudaMemcpyAsync(&dim, offs.p + nh, sizeof(int64_t), cudaMemcpyDeviceToHost, st));
-    ED_CUDA(cudaStreamSynchronize(st));
-    b.dim = (uint64_t)dim;
-    b.words.alloc(dim > 0 ? (size_t)dim : 1);
-    k_basis_fill<<<grid_for(nh * 32, 256), 256, 0, st>>>(H, L, offs.p, counts.p, need.p, d_cstart.p, d_clist.p,
-                                                         b.words.p, b.hi.p);
-    ::edgb::count_launch();
-    ED_CUDA(cudaGetLastError());
-    ED_CUDA(cudaStreamSynchronize(st));
-    if (dim == 0) b.sector_sum = -1;
+    tmp.fill(b, st);
+    if (b.dim == 0) b.sector_sum = -1;
 }
 }  // namespace
 
@@ -365,46 +406,19 @@ void basis_build(ed_basis& b, cudaStream_t st)
     const int nclass = (L + 1) * (max_sum_low + 1);
     ED_REQUIRE(nclass < 0xFFFF, ED_ERR_RANGE, "too many low-word classes");
     const uint64_t nl = 1ull << L;
-    std::vector<uint32_t> ccount(nclass, 0), cstart(nclass, 0), clist(nl);
-    std::vector<uint64_t> lo(nl);
-    std::vector<uint32_t> rank_in_class(nl);
-    for (uint64_t l = 0; l < nl; ++l) {
-        int pop = __builtin_popcountll(l), sum = 0;
-        for (uint64_t x = l; x; x &= x - 1) sum += w[__builtin_ctzll(x)];
-        const int cls = pop * (max_sum_low + 1) + sum;
-        rank_in_class[l] = ccount[cls]++;
-        lo[l] = ((uint64_t)cls << 32) | rank_in_class[l];
-    }
-    uint32_t acc = 0;
-    for (int c = 0; c < nclass; ++c) { cstart[c] = acc; acc += ccount[c]; }
-    for (uint64_t l = 0; l < nl; ++l) clist[cstart[lo[l] >> 32] + rank_in_class[l]] = (uint32_t)l;
-
+    std::vector<uint32_t> cls(nl, 0);
+    const LowTables low(L, nclass, [&](uint64_t l) {
+        if (l) cls[l] = cls[l & (l - 1)] + (uint32_t)(max_sum_low + 1 + w[__builtin_ctzll(l)]);
+        return cls[l];
+    });
     b.lo.alloc(nl);
     b.hi.alloc(1ull << H);
-    DevBuf<uint32_t> d_ccount(nclass), d_cstart(nclass), d_clist(nl);
-    ED_CUDA(cudaMemcpyAsync(b.lo.p, lo.data(), nl * 8, cudaMemcpyHostToDevice, st));
-    ED_CUDA(cudaMemcpyAsync(d_ccount.p, ccount.data(), nclass * 4, cudaMemcpyHostToDevice, st));
-    ED_CUDA(cudaMemcpyAsync(d_cstart.p, cstart.data(), nclass * 4, cudaMemcpyHostToDevice, st));
-    ED_CUDA(cudaMemcpyAsync(d_clist.p, clist.data(), nl * 4, cudaMemcpyHostToDevice, st));
-
-    const int64_t nh = 1ll << H;
-    DevBuf<int64_t> counts(nh), offs(nh + 1);
-    DevBuf<uint16_t> need(nh);
-    DevBuf<int> d_wh(H);
-    ED_CUDA(cudaMemcpyAsync(d_wh.p, w.data() + L, (size_t)H * sizeof(int), cudaMemcpyHostToDevice, st));
-    k_basis_count<<<grid_for(nh, 256), 256, 0, st>>>(H, L, N, S, max_sum_low, d_ccount.p, d_wh.p, counts.p, need.p);
+    ED_CUDA(cudaMemcpyAsync(b.lo.p, low.lo.data(), nl * 8, cudaMemcpyHostToDevice, st));
+    BasisTemps tmp(H, low, w.data() + L, st);
+    k_basis_count<<<grid_for(tmp.nh, 256), 256, 0, st>>>(H, L, N, S, max_sum_low, tmp.count, tmp.wh, tmp.counts, tmp.need);
     ::edgb::count_launch();
     ED_CUDA(cudaGetLastError());
-    exclusive_scan_i64(counts.p, offs.p, nh, st);
-    int64_t dim = 0;
-    ED_CUDA(cudaMemcpyAsync(&dim, offs.p + nh, sizeof(int64_t), cudaMemcpyDeviceToHost, st));
-    ED_CUDA(cudaStreamSynchronize(st));
-    b.dim = (uint64_t)dim;
-    b.words.alloc(dim > 0 ? (size_t)dim : 1);
-    k_basis_fill<<<grid_for(nh * 32, 256), 256, 0, st>>>(H, L, offs.p, counts.p, need.p, d_cstart.p, d_clist.p,
-                                                         b.words.p, b.hi.p); ::edgb::count_launch();
-    ED_CUDA(cudaGetLastError());
-    ED_CUDA(cudaStreamSynchronize(st));
+    tmp.fill(b, st);
 }
 
 void basis_compact_tables(const ed_basis& b, cudaStream_t st)
