@@ -462,8 +462,10 @@ __device__ __forceinline__ void reduce_per_problem(double v, double* red, int BP
 
 // part[0][blk][p] = v_p . w_p, part[1][blk][p] = w_p . w_p
 __global__ void __launch_bounds__(kBT) k_bdot2(const double* __restrict__ v, const double* __restrict__ w, int64_t n,
-                                               int B, int BP, double* __restrict__ part)
+                                               int B, int BP, double* __restrict__ part,
+                                               unsigned long long* __restrict__ ended)
 {
+    if (blockIdx.x == 0) stamp(ended);
     __shared__ double red[kBT];
     int64_t r0, r1;
     chunk_rows(n, gridDim.x, blockIdx.x, r0, r1);
@@ -480,29 +482,72 @@ __global__ void __launch_bounds__(kBT) k_bdot2(const double* __restrict__ v, con
     reduce_per_problem(c, red, BP, B, part + (int64_t)blockIdx.x * B, sq, 1);
 }
 
+// What follows a sum in a solver's step, done by the thread that has it (t =
+// q B + p, sum in out[t]):
+//   kLocal  (Q = 2: alpha, |H v|^2) column cj gets alpha at row j and
+//           beta_{j-1} at row j-1
+//   kAcc    (Q = J + 1) cj[i][p] += c[i][p] for i < J where the pass ran for p
+//   kNeed   (|w|^2 after the first pass) need[p] = force or |w_after|^2 <
+//           |w_before|^2 / 2 (DGKS); with force, the norm before is |H v|^2
+//   kFinal  (|w|^2) beta_j = |w|, breakdown where it vanishes relative to |H v|
+struct SumThen {
+    enum Kind { kNone, kLocal, kAcc, kNeed, kFinal } kind = kNone;
+    int j = 0, force = 0;
+    double* cj = nullptr;
+    double* beta = nullptr;      // kLocal: beta_{j-1}; kFinal: beta_j
+    const double* before = nullptr;
+    double* ref = nullptr;       // |H v|^2
+    int* need = nullptr;
+    int* brk = nullptr;
+};
+
 // out[q][p] = sum over blocks of part[q][blk][p] for q < Q (t = q*B + p):
-// 32 consecutive t per CTA, its 8 warps split the block range, and the
+// 32 consecutive t per CTA, its 32 warps split the block range, and the
 // partial sums are combined in a fixed order.  With mask given, out[t] is
-// written only where mask[p] != 0.
-__global__ void __launch_bounds__(256) k_bsum(const double* __restrict__ part, int nb, int B, int Q,
-                                              double* __restrict__ out, const int* __restrict__ mask)
+// written only where mask[p] != 0.  Latency bounds it: for 16 problems' 608
+// partials (N=9, 2S=24) 9 us, with the step's scalars; 8 warps with a load at a
+// time took 15 us, a fifth of a step, and the scalars five more launches.
+__global__ void __launch_bounds__(1024) k_bsum(const double* __restrict__ part, int nb, int B, int Q, double* out,
+                                               const int* mask, SumThen then)
 {
-    __shared__ double red[8][33];
+    __shared__ double red[32][33];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int t = blockIdx.x * 32 + lane;
     double s = 0.0;
     if (t < Q * B) {
         const int q = t / B, p = t - q * B;
         const double* src = part + (int64_t)q * nb * B + p;
-        for (int blk = warp; blk < nb; blk += 8) s += src[(int64_t)blk * B];
+#pragma unroll 8
+        for (int blk = warp; blk < nb; blk += 32) s += src[(int64_t)blk * B];
     }
     red[warp][lane] = s;
     __syncthreads();
-    if (warp == 0 && t < Q * B) {
-        double tot = 0.0;
+    if (warp != 0 || t >= Q * B) return;
+    double tot[4] = {0.0, 0.0, 0.0, 0.0};
 #pragma unroll
-        for (int w = 0; w < 8; ++w) tot += red[w][lane];
-        if (!mask || mask[t % B]) out[t] = tot;
+    for (int w = 0; w < 32; ++w) tot[w & 3] += red[w][lane];
+    const int p = t % B;
+    const bool on = !mask || mask[p];
+    const double sum = (tot[0] + tot[1]) + (tot[2] + tot[3]);
+    if (on) out[t] = sum;
+    if (then.kind == SumThen::kLocal) {
+        if (t < B) {
+            then.cj[(size_t)then.j * B + p] = sum;
+            then.cj[(size_t)(then.j - 1) * B + p] = then.beta[p];
+        }
+    } else if (then.kind == SumThen::kAcc) {
+        if (t < then.j * B && (!then.need || then.need[p])) then.cj[t] += sum;
+    } else if (then.kind == SumThen::kNeed) {
+        then.need[p] = (then.force || sum < 0.5 * then.before[p]) ? 1 : 0;
+        if (then.force) then.ref[p] = then.before[p];
+    } else if (then.kind == SumThen::kFinal) {
+        const double b = sqrt(on ? sum : out[t]);
+        if (!(b > 1e-12 * sqrt(fmax(then.ref[p], 0.0)))) {
+            if (then.brk[p] == 0) then.brk[p] = then.j + 1;
+            then.beta[p] = 1.0;          // keeps the (abandoned) vector finite
+        } else {
+            then.beta[p] = b;
+        }
     }
 }
 
@@ -541,8 +586,9 @@ __device__ __forceinline__ void reduce8_per_problem(const double (&acc)[8], int 
 // zeros.
 __global__ void __launch_bounds__(kBT, 4) k_bmdot(const double* __restrict__ V, int64_t n, int B, int BP, int J,
                                                const double* __restrict__ w, double* __restrict__ part,
-                                               const int* __restrict__ need)
+                                               const int* __restrict__ need, unsigned long long* __restrict__ ended)
 {
+    if (blockIdx.x == 0) stamp(ended);
     __shared__ double red[8 * kBT];
     int64_t r0, r1;
     chunk_rows(n, gridDim.x, blockIdx.x, r0, r1);
@@ -618,57 +664,15 @@ __global__ void __launch_bounds__(kBT, 4) k_bupdate(const double* __restrict__ V
     reduce_per_problem(nn, red, BP, B, npart + (int64_t)blockIdx.x * B, 0, 0);
 }
 
-// Local step bookkeeping: column j gets alpha at row j and beta_{j-1} at row j-1.
-__global__ void k_blocal(double* __restrict__ cj, const double* __restrict__ alpha, const double* __restrict__ beta_prev,
-                         int j, int B)
-{
-    for (int p = threadIdx.x; p < B; p += blockDim.x) {
-        cj[(size_t)j * B + p] = alpha[p];
-        cj[(size_t)(j - 1) * B + p] = beta_prev[p];
-    }
-}
-
-// cj[i][p] += c[i][p] for i < J where the pass ran for p
-__global__ void k_bacc(double* __restrict__ cj, const double* __restrict__ c, int J, int B,
-                       const int* __restrict__ need)
-{
-    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < J * B; t += gridDim.x * blockDim.x) {
-        const int p = t % B;
-        if (!need || need[p]) cj[t] += c[t];
-    }
-}
-
-// after pass 1: need2[p] = forced or ||w_after||^2 < eta^2 ||w_before||^2 (DGKS)
-__global__ void k_bneed(const double* __restrict__ after, const double* __restrict__ before, int B, int force,
-                        int* __restrict__ need2)
-{
-    for (int p = threadIdx.x; p < B; p += blockDim.x)
-        need2[p] = (force || after[p] < 0.5 * before[p]) ? 1 : 0;
-}
-
-// beta_j = ||w||; breakdown when it vanishes relative to ||H v_j||
-__global__ void k_bfinal(const double* __restrict__ norm2, const double* __restrict__ ref2, double* __restrict__ beta,
-                         int* __restrict__ brk, int B, int j)
-{
-    for (int p = threadIdx.x; p < B; p += blockDim.x) {
-        const double b = sqrt(norm2[p]);
-        const double ref = sqrt(fmax(ref2[p], 0.0));
-        if (!(b > 1e-12 * ref)) {
-            if (brk[p] == 0) brk[p] = j + 1;
-            beta[p] = 1.0;          // keeps the (abandoned) vector finite
-        } else {
-            beta[p] = b;
-        }
-    }
-}
-
-__global__ void k_bscale(double* __restrict__ w, int64_t n, int B, const double* __restrict__ beta)
+__global__ void k_bscale(double* __restrict__ w, int64_t n, int B, const double* __restrict__ beta,
+                         unsigned long long* __restrict__ started)
 {
     const int64_t total = n * (int64_t)B;
     for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
         const int p = (int)(t % B);
         w[t] = w[t] / beta[p];
     }
+    stamp(started);
 }
 
 // Ritz vectors of selected problems: for q < Bq, s = keep[q] (a column of the
@@ -1052,7 +1056,7 @@ void batch_residuals(const ed_batch& bt, const BlockOperands& o, const double* X
         const double* x = X + (int64_t)i * n * B;
         batch_block_product(bt, o, x, y.p, st);
         k_bresid<<<nb, kBT, 0, st>>>(y.p, x, n, B, BP, dl.p, part.p); count_launch();
-        k_bsum<<<(unsigned)((B + 31) / 32), 256, 0, st>>>(part.p, nb, B, 1, s.p, nullptr); count_launch();
+        launch(k_bsum, (unsigned)((B + 31) / 32), 1024, 0, st, part.p, nb, B, 1, s.p, nullptr, SumThen());
         ED_CUDA(cudaMemcpyAsync(r.data(), s.p, (size_t)B * 8, cudaMemcpyDeviceToHost, st));
         ED_CUDA(cudaStreamSynchronize(st));
         for (int b = 0; b < B; ++b) res[(size_t)b * k + i] = std::sqrt(r[b]);
@@ -1223,13 +1227,13 @@ void batch_solve(const ed_batch& bt, const int* sel, int nsel, const ed_lanczos_
     int64_t vs = vs0;
 
     auto grid_for = [&](int64_t work) { return (int)std::max<int64_t>(1, std::min<int64_t>(sms_b() * 8, (work + 255) / 256)); };
-    auto bsum = [&](const double* src, int Q, double* out, const int* mask) {
-        k_bsum<<<(unsigned)((Q * B + 31) / 32), 256, 0, st>>>(src, nb, B, Q, out, mask); count_launch();
+    auto bsum = [&](const double* src, int Q, double* out, const int* mask, const SumThen& then = SumThen()) {
+        launch(k_bsum, (unsigned)((Q * B + 31) / 32), 1024, 0, st, src, nb, B, Q, out, mask, then);
     };
     if (V0) ED_CUDA(cudaMemcpyAsync(V.p, V0, (size_t)vs * 8, cudaMemcpyDeviceToDevice, st));
     else { k_brandom<<<grid_for(vs), 256, 0, st>>>(V.p, vs, p.seed); count_launch(); }
     {   // normalise every start vector, rejecting zero or non-finite ones
-        k_bdot2<<<nb, kBT, 0, st>>>(V.p, V.p, n, B, BP, part.p); count_launch();
+        launch(k_bdot2, nb, kBT, 0, st, V.p, V.p, n, B, BP, part.p, nullptr);
         bsum(part.p, 1, s2.p, nullptr);
         std::vector<double> nn(B);
         ED_CUDA(cudaMemcpyAsync(nn.data(), s2.p, (size_t)B * 8, cudaMemcpyDeviceToHost, st));
@@ -1239,7 +1243,7 @@ void batch_solve(const ed_batch& bt, const int* sel, int nsel, const ed_lanczos_
             nn[b] = std::sqrt(nn[b]);
         }
         ED_CUDA(cudaMemcpyAsync(s2.p + 2 * B, nn.data(), (size_t)B * 8, cudaMemcpyHostToDevice, st));
-        k_bscale<<<grid_for(vs), 256, 0, st>>>(V.p, n, B, s2.p + 2 * B); count_launch();
+        k_bscale<<<grid_for(vs), 256, 0, st>>>(V.p, n, B, s2.p + 2 * B, nullptr); count_launch();
     }
     ed_batch_info inf;
     std::memset(&inf, 0, sizeof(inf));
@@ -1250,12 +1254,9 @@ void batch_solve(const ed_batch& bt, const int* sel, int nsel, const ed_lanczos_
     std::vector<std::vector<double>> T(B0, std::vector<double>((size_t)m * m, 0.0)), theta(B0), Y(B0);
     std::vector<double> coef_h((size_t)m * (m + 1) * B0), beta_h((size_t)(m + 1) * B0), Yall((size_t)B0 * m * m);
     std::vector<int> brk_h(B0);
-    std::vector<cudaEvent_t> ev(2 * (size_t)(m + 1), nullptr);
-    for (auto& e : ev) ED_CUDA(cudaEventCreate(&e));
-    struct EvG {
-        std::vector<cudaEvent_t>& v;
-        ~EvG() { for (auto e : v) if (e) cudaEventDestroy(e); }
-    } evg{ev};
+    // the steps' products: {latest end of the kernel before, start of the one after}
+    DevBuf<unsigned long long> clock(2 * (size_t)(m + 1));
+    std::vector<unsigned long long> clock_h(2 * (size_t)(m + 1));
     // Ritz coefficients of the active problems, [i][j][column] (column fastest)
     auto pack_Y = [&]() {
         for (int q = 0; q < B; ++q) {
@@ -1284,51 +1285,58 @@ void batch_solve(const ed_batch& bt, const int* sel, int nsel, const ed_lanczos_
         ED_CUDA(cudaStreamSynchronize(st));   // keep/dst are reused right away
     };
 
-    auto enqueue_cycle = [&](int k, bool capturing) {
-        ED_CUDA(cudaMemsetAsync(coef.p, 0, (size_t)m * (m + 1) * B * 8, st));
-        ED_CUDA(cudaMemsetAsync(brk.p, 0, (size_t)B * 4, st));
+    auto enqueue_cycle = [&](int k) {
+        const int64_t coefs = (int64_t)m * (m + 1) * B;
+        ED_CUDA(cudaMemsetAsync(clock.p, 0, clock.bytes(), st));
+        launch(k_cycle_begin, (unsigned)std::min<int64_t>(64, (coefs + 255) / 256), 256, 0, st, coef.p, coefs, brk.p, B,
+               clock.p + 2 * k);
         for (int j = k; j < m; ++j) {
             double* vj = V.p + (int64_t)j * vs;
             double* w = V.p + (int64_t)(j + 1) * vs;
             double* cj = coef.p + (size_t)j * (m + 1) * B;
+            double* ref = s2.p + B;
             const bool first = (j == k);
-            if (capturing) ED_CUDA(cudaEventRecordWithFlags(ev[2 * j], st, cudaEventRecordExternal));
-            else ED_CUDA(cudaEventRecord(ev[2 * j], st));
             if (fixed.ready) fixed_block_product(bt, ops, fixed, tile, vj, w, st);
             else bspmm_variant(bt, ops, tile[0], tile[1], tile[2], tile[3], vj, w, n, nullptr, st);
-            if (capturing) ED_CUDA(cudaEventRecordWithFlags(ev[2 * j + 1], st, cudaEventRecordExternal));
-            else ED_CUDA(cudaEventRecord(ev[2 * j + 1], st));
+            SumThen local, acc, need, fin;
             if (!first) {
-                k_bdot2<<<nb, kBT, 0, st>>>(vj, w, n, B, BP, part.p); count_launch();
-                bsum(part.p, 2, s2.p, nullptr);
-                k_blocal<<<1, 256, 0, st>>>(cj, s2.p, betas.p + (size_t)(j - 1) * B, j, B); count_launch();
-                k_baxpy2<<<grid_for(vs), 256, 0, st>>>(w, vj, V.p + (int64_t)(j - 1) * vs, n, B, s2.p,
-                                                       betas.p + (size_t)(j - 1) * B); count_launch();
+                launch(k_bdot2, nb, kBT, 0, st, vj, w, n, B, BP, part.p, clock.p + 2 * j + 1);
+                local.kind = SumThen::kLocal;
+                local.j = j;
+                local.cj = cj;
+                local.beta = betas.p + (size_t)(j - 1) * B;
+                bsum(part.p, 2, s2.p, nullptr, local);
+                launch(k_baxpy2, grid_for(vs), 256, 0, st, w, vj, V.p + (int64_t)(j - 1) * vs, n, B, s2.p,
+                       betas.p + (size_t)(j - 1) * B);
             }
             const int J = j + 1;
+            acc.kind = SumThen::kAcc;
+            acc.j = J;
+            acc.cj = cj;
+            need.kind = SumThen::kNeed;
+            need.force = first ? 1 : 0;
+            need.before = sc.p + (size_t)J * B;
+            need.ref = ref;
+            need.need = need2.p;
+            fin.kind = SumThen::kFinal;
+            fin.j = j;
+            fin.beta = betas.p + (size_t)j * B;
+            fin.ref = ref;
+            fin.brk = brk.p;
             for (int pass = 0; pass < 2; ++pass) {
-                const int* mask = pass == 0 ? nullptr : need2.p;
-                k_bmdot<<<nb, kBT, 0, st>>>(V.p, n, B, BP, J, w, part.p, mask); count_launch();
-                bsum(part.p, J + 1, sc.p, nullptr);
+                int* mask = pass == 0 ? nullptr : need2.p;
+                launch(k_bmdot, nb, kBT, 0, st, V.p, n, B, BP, J, w, part.p, mask,
+                       first && pass == 0 ? clock.p + 2 * j + 1 : nullptr);
+                acc.need = mask;
+                bsum(part.p, J + 1, sc.p, nullptr, acc);
                 if (upd_stage)
-                    k_bupdate<true><<<nb, kBT, (size_t)J * B * 8, st>>>(V.p, n, B, BP, J, sc.p, w, npart.p, mask);
+                    launch(k_bupdate<true>, nb, kBT, (size_t)J * B * 8, st, V.p, n, B, BP, J, sc.p, w, npart.p, mask);
                 else
-                    k_bupdate<false><<<nb, kBT, 0, st>>>(V.p, n, B, BP, J, sc.p, w, npart.p, mask);
-                count_launch();
-                k_bacc<<<grid_for((int64_t)J * B), 256, 0, st>>>(cj, sc.p, J, B, mask); count_launch();
+                    launch(k_bupdate<false>, nb, kBT, 0, st, V.p, n, B, BP, J, sc.p, w, npart.p, mask);
                 // the norm after the pass, kept from pass 1 for problems that skip pass 2
-                bsum(npart.p, 1, s2.p + 3 * B, mask);
-                if (pass == 0) {
-                    k_bneed<<<1, 256, 0, st>>>(s2.p + 3 * B, sc.p + (size_t)J * B, B, first ? 1 : 0, need2.p);
-                    count_launch();
-                    if (first)   // ||H v_j||^2 is the norm before the first pass
-                        ED_CUDA(cudaMemcpyAsync(s2.p + B, sc.p + (size_t)J * B, (size_t)B * 8, cudaMemcpyDeviceToDevice,
-                                                st));
-                }
+                bsum(npart.p, 1, s2.p + 3 * B, mask, pass == 0 ? need : fin);
             }
-            k_bfinal<<<1, 256, 0, st>>>(s2.p + 3 * B, s2.p + B, betas.p + (size_t)j * B, brk.p, B, j); count_launch();
-            k_bscale<<<grid_for(vs), 256, 0, st>>>(w, n, B, betas.p + (size_t)j * B); count_launch();
-            ED_CUDA(cudaGetLastError());
+            launch(k_bscale, grid_for(vs), 256, 0, st, w, n, B, betas.p + (size_t)j * B, clock.p + 2 * (j + 1));
         }
     };
     CycleGraphs cache;
@@ -1338,7 +1346,7 @@ void batch_solve(const ed_batch& bt, const int* sel, int nsel, const ed_lanczos_
             const uint64_t c0 = launch_count();
             ED_CUDA(cudaStreamBeginCapture(st, cudaStreamCaptureModeRelaxed));
             try {
-                enqueue_cycle(k, true);
+                enqueue_cycle(k);
             } catch (...) {
                 cudaGraph_t broken = nullptr;
                 cudaStreamEndCapture(st, &broken);
@@ -1360,7 +1368,7 @@ void batch_solve(const ed_batch& bt, const int* sel, int nsel, const ed_lanczos_
         count_launches(g->kernels);
     };
 
-    double spmm_ms = 0.0;
+    double spmm_ns = 0.0;
     bool converged = false;
     int finished = 0;
     double retired_res = 0.0;
@@ -1372,12 +1380,9 @@ void batch_solve(const ed_batch& bt, const int* sel, int nsel, const ed_lanczos_
         ED_CUDA(cudaMemcpyAsync(coef_h.data(), coef.p, (size_t)m * (m + 1) * B * 8, cudaMemcpyDeviceToHost, st));
         ED_CUDA(cudaMemcpyAsync(beta_h.data(), betas.p, (size_t)(m + 1) * B * 8, cudaMemcpyDeviceToHost, st));
         ED_CUDA(cudaMemcpyAsync(brk_h.data(), brk.p, (size_t)B * 4, cudaMemcpyDeviceToHost, st));
+        ED_CUDA(cudaMemcpyAsync(clock_h.data(), clock.p, clock.bytes(), cudaMemcpyDeviceToHost, st));
         ED_CUDA(cudaStreamSynchronize(st));
-        for (int j = k; j < m; ++j) {
-            float ms = 0.f;
-            ED_CUDA(cudaEventElapsedTime(&ms, ev[2 * j], ev[2 * j + 1]));
-            spmm_ms += ms;
-        }
+        spmm_ns += stamped_ns(clock_h, k, m);
         std::vector<int> done, live, solved;
         double maxres = 0.0;
         for (int q = 0; q < B; ++q) {
@@ -1526,7 +1531,7 @@ void batch_solve(const ed_batch& bt, const int* sel, int nsel, const ed_lanczos_
         inf.converged = ok_all;
     }
     ED_CUDA(cudaStreamSynchronize(st));
-    inf.spmm_seconds = spmm_ms * 1e-3;
+    inf.spmm_seconds = spmm_ns * 1e-9;
     inf.seconds = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
     if (info) *info = inf;
     ED_REQUIRE(converged, ED_ERR_NOCONV, "batched Lanczos did not converge within the restart cap");
