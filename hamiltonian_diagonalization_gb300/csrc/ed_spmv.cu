@@ -211,7 +211,8 @@ template <int G, int U, int MINB = 1>
 __global__ void __launch_bounds__(256, MINB) k_spmv_fix(const int64_t* __restrict__ rowptr, const int32_t* __restrict__ col,
                                                   const int2* __restrict__ aq, const int2* __restrict__ xq,
                                                   const int* __restrict__ xexp, int ea, double* __restrict__ y,
-                                                  int64_t n)
+                                                  int64_t n, const double* __restrict__ val,
+                                                  const double* __restrict__ x)
 {
     // per element |ah xh| <= 2^56, |ah xl + al xh| < 2^59, 0 <= al xl < 2^60
     static_assert(U >= 1 && U <= 8, "eight elements' products fit the int64 partial sums");
@@ -227,6 +228,14 @@ __global__ void __launch_bounds__(256, MINB) k_spmv_fix(const int64_t* __restric
         const bool valid = r < n;
         const int64_t s = valid ? rowptr[r] : 0;
         const int len = valid ? (int)(rowptr[r + 1] - s) : 0;
+        if (x && !finite) {   // FP64 sums keep what is not finite to the rows that meet it
+            double acc = 0.0;
+            for (int j = sub; j < len; j += G) acc = fma(val[s + j], __ldg(x + col[s + j]), acc);
+#pragma unroll
+            for (int o = G / 2; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o, G);
+            if (valid && sub == 0) y[r] = acc;
+            continue;
+        }
         const int2* ap = aq + s;
         const int32_t* cp = col + s;
         __int128 acc = 0;
@@ -722,13 +731,21 @@ __global__ void __launch_bounds__(256, MINB) k_spmv_sell_fix(const int64_t* __re
     }
 }
 
+__global__ void k_zero_unless_finite(double* __restrict__ y, int64_t n, const int* __restrict__ xexp)
+{
+    if (*xexp < 2047) return;
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) y[i] = 0.0;
+}
+
 // Upper-triangle storage, the reference's layout: gather for the stored
 // part, scatter (atomic) for the transposed part.  y must be zero on entry.
 template <int G>
 __global__ void __launch_bounds__(256) k_spmv_upper(const int64_t* __restrict__ rowptr,
                                                     const int32_t* __restrict__ col, const double* __restrict__ val,
-                                                    const double* __restrict__ x, double* __restrict__ y, int64_t n)
+                                                    const double* __restrict__ x, double* __restrict__ y, int64_t n,
+                                                    const int* __restrict__ xexp)
 {
+    if (xexp && *xexp < 2047) return;   // x is finite: y is there already
     constexpr int RPW = 32 / G;
     const int lane = threadIdx.x & 31, sub = lane & (G - 1), grp = lane / G;
     const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
@@ -1136,7 +1153,8 @@ void blk_launch(const ed_crs& a, const double* x, double* y, cudaStream_t st)
            reinterpret_cast<const int2*>(sc.xq.p), sc.part.p + fix_parts(), f.ea, y, a.n, f.blocks);
 }
 
-void fix_launch(const ed_crs& a, const double* x, double* y, cudaStream_t st)
+// rows: the product in FP64 where x is not finite (else every entry is NaN).
+void fix_launch(const ed_crs& a, const double* x, double* y, cudaStream_t st, bool rows = false)
 {
     const ed_fixq& f = *a.fixq;
     ed_fixq::Scratch& sc = fix_convert_x(a, x, st);
@@ -1150,7 +1168,7 @@ void fix_launch(const ed_crs& a, const double* x, double* y, cudaStream_t st)
     // memory by bulk copies, k_spmv_fix_staged, 1.71)
     launch(k_spmv_fix<8, 8, 4>, sms() * 8, 256, 0, st, a.rowptr.p, a.col.p, reinterpret_cast<const int2*>(f.val.p),
                                                    reinterpret_cast<const int2*>(sc.xq.p), sc.part.p + P, f.ea, y,
-                                                   a.n);
+                                                   a.n, a.val.p, rows ? x : nullptr);
     ED_CUDA(cudaGetLastError());
 }
 
@@ -1166,6 +1184,16 @@ void fix_launch_sell(const ed_crs& a, const double* x, double* y, cudaStream_t s
     ED_CUDA(cudaGetLastError());
 }
 
+}  // namespace
+
+namespace {
+void upper_launch(const ed_crs& a, const double* x, double* y, const int* xexp, cudaStream_t st)
+{
+    if ((double)a.nnz >= 48.0 * (double)a.n)
+        launch(k_spmv_upper<8>, sms() * 8, 256, 0, st, a.rowptr.p, a.col.p, a.val.p, x, y, a.n, xexp);
+    else
+        launch(k_spmv_upper<4>, sms() * 8, 256, 0, st, a.rowptr.p, a.col.p, a.val.p, x, y, a.n, xexp);
+}
 }  // namespace
 
 // Stored matrices of at least this many rows take the split product.  Below,
@@ -1284,7 +1312,11 @@ void spmv(const ed_crs& a, const double* x, double* y, cudaStream_t st)
         return;
     }
     if (split_prepare(a, st)) {
-        split_product(*a.split, x, y, st);
+        const int* xexp = split_product(*a.split, x, y, st);
+        if (a.upper) {
+            launch(k_zero_unless_finite, sms() * 4, 256, 0, st, y, a.n, xexp);
+            upper_launch(a, x, y, xexp, st);
+        }
         return;
     }
     if (sell_shape(a) && a.sell_state == 0) spmv_prepare(a, st);   // waits for a solver's explicit call while capturing
@@ -1308,7 +1340,7 @@ void spmv(const ed_crs& a, const double* x, double* y, cudaStream_t st)
         return;
     }
     if (fix_shape(a) && fix_ready(a, st)) {
-        fix_launch(a, x, y, st);
+        fix_launch(a, x, y, st, short_rows(a));
         return;
     }
     const double avg = (double)a.nnz / (double)a.n;
@@ -1329,10 +1361,7 @@ void spmv(const ed_crs& a, const double* x, double* y, cudaStream_t st)
         launch(k_spmv_full<2>, grid, threads, 0, st, a.rowptr.p, a.col.p, a.val.p, x, y, a.n);
     } else {
         ED_CUDA(cudaMemsetAsync(y, 0, (size_t)a.n * sizeof(double), st));
-        if (avg >= 48) k_spmv_upper<8><<<grid, threads, 0, st>>>(a.rowptr.p, a.col.p, a.val.p, x, y, a.n);
-        else k_spmv_upper<4><<<grid, threads, 0, st>>>(a.rowptr.p, a.col.p, a.val.p, x, y, a.n);
-        count_launch();
-        ED_CUDA(cudaGetLastError());
+        upper_launch(a, x, y, nullptr, st);
     }
 }
 

@@ -121,3 +121,24 @@ def test_split_products_on_two_streams_and_in_a_solve(cuda):
     v0 = np.random.default_rng(9).uniform(-1, 1, n)
     assert free.LanczosDiagonalize(3, tol=1e-10, v0=v0) and stored.LanczosDiagonalize(3, tol=1e-10, v0=v0)
     assert np.array_equal(free.m_eigenvalues, stored.m_eigenvalues)
+
+
+# what took FP64 sums before they were fixed point still keeps a NaN to the
+# rows that meet it: the upper triangle of a large sector, short rows of a small one
+@pytest.mark.parametrize("make,case,kw", [(two_level, (8, 18, 2), dict(store_upper=True)), (two_level, (6, 13, 0), {})])
+def test_products_keep_a_nan_to_its_rows(cuda, make, case, kw):
+    torch = cuda
+    H = make(*case, **kw)
+    rowptr, col, _ = H.m_crsSparseMatrix.to_host()
+    n = len(rowptr) - 1
+    x = torch.from_numpy(np.random.default_rng(5).uniform(-1, 1, n)).cuda()
+    clean = product(torch, H, x).cpu().numpy()
+    x[n // 2] = float("nan")
+    y = product(torch, H, x).cpu().numpy()
+    rows = np.repeat(np.arange(n), np.diff(rowptr))
+    hit = np.zeros(n, bool)
+    hit[rows[col == n // 2]] = True
+    if kw:
+        hit[col[rows == n // 2]] = True
+    assert np.array_equal(np.isnan(y), hit)
+    assert np.max(np.abs(y[~hit] - clean[~hit])) <= 1e-13 * np.abs(clean).max()
