@@ -1187,12 +1187,18 @@ void fix_launch_sell(const ed_crs& a, const double* x, double* y, cudaStream_t s
 }  // namespace
 
 namespace {
+// Four times the resident blocks: the stored rows get shorter towards the end
+// of the matrix, and later blocks fill the places that short ones leave
+// (GB300, 8 / 32 / 64 blocks per SM: N=10, 2S=27 135.4 / 123.6 / 123.4 us, N=9,
+// 2S=24 28.7 / 26.7 / 26.7, two levels N=8, 2S=16 147.9 / 134.3 / 130.8, N=6,
+// 2S=12 10.3 / 10.3 / 12.3).  The atomic additions bound it: two or four
+// elements ahead, 4 or 16 lanes a row are slower.
 void upper_launch(const ed_crs& a, const double* x, double* y, const int* xexp, cudaStream_t st)
 {
     if ((double)a.nnz >= 48.0 * (double)a.n)
-        launch(k_spmv_upper<8>, sms() * 8, 256, 0, st, a.rowptr.p, a.col.p, a.val.p, x, y, a.n, xexp);
+        launch(k_spmv_upper<8>, sms() * 32, 256, 0, st, a.rowptr.p, a.col.p, a.val.p, x, y, a.n, xexp);
     else
-        launch(k_spmv_upper<4>, sms() * 8, 256, 0, st, a.rowptr.p, a.col.p, a.val.p, x, y, a.n, xexp);
+        launch(k_spmv_upper<4>, sms() * 32, 256, 0, st, a.rowptr.p, a.col.p, a.val.p, x, y, a.n, xexp);
 }
 }  // namespace
 
