@@ -331,10 +331,12 @@ __global__ void __launch_bounds__(kCThreads) k_cmdot(const double2* __restrict__
                                                      unsigned int* __restrict__ counter, double2* __restrict__ c,
                                                      double* __restrict__ coefcol, double* __restrict__ before,
                                                      const int* __restrict__ run, const int* __restrict__ stop,
-                                                     unsigned long long* __restrict__ ended)
+                                                     unsigned long long* __restrict__ ended,
+                                                     unsigned long long* __restrict__ absmax)
 {
     if (blockIdx.x == 0) stamp(ended);
     if ((run && !*run) || (stop && *stop)) return;
+    if (absmax && blockIdx.x == 0 && threadIdx.x == 0) *absmax = 0ull;   // k_cupd's
     extern __shared__ double2 csw[];
     const int64_t r0 = (int64_t)blockIdx.x * R;
     const int len = (int)min((int64_t)R, n - r0);
@@ -431,16 +433,20 @@ __global__ void __launch_bounds__(kCThreads) k_cupd(const double2* __restrict__ 
                                                     int mode, int force2, const double* __restrict__ before,
                                                     int* __restrict__ need2, double* __restrict__ beta,
                                                     const double* __restrict__ ref2, int j,
-                                                    const int* __restrict__ run, int* __restrict__ stop)
+                                                    const int* __restrict__ run, int* __restrict__ stop,
+                                                    unsigned long long* __restrict__ absmax)
 {
     if ((run && !*run) || (stop && *stop)) return;
     extern __shared__ double2 cc[];
     __shared__ double red[kCThreads / 32];
+    __shared__ unsigned long long top;
+    if (threadIdx.x == 0) top = 0ull;
     for (int i = threadIdx.x; i < J; i += kCThreads) cc[i] = c[i];
     __syncthreads();
     int64_t r0, r1;
     cchunk(n, gridDim.x, blockIdx.x, r0, r1);
     double nn = 0.0;
+    unsigned long long mx = 0ull;
     for (int64_t r = r0 + threadIdx.x; r < r1; r += kCThreads) {
         double2 a = w[r], b = make_double2(0.0, 0.0);
         int i = 0;
@@ -473,9 +479,14 @@ __global__ void __launch_bounds__(kCThreads) k_cupd(const double2* __restrict__ 
         w[r] = a;
         nn = fma(a.x, a.x, nn);
         nn = fma(a.y, a.y, nn);
+        mx = max(mx, max(abs_bits(a.x), abs_bits(a.y)));
     }
+    if (absmax) block_absmax(mx, &top);
     nn = cblock_sum(nn, red);
-    if (threadIdx.x == 0) npart[blockIdx.x] = nn;
+    if (threadIdx.x == 0) {
+        npart[blockIdx.x] = nn;
+        if (absmax) atomicMax(absmax, top);
+    }
     if (mode == 0 || !clast_block(counter)) return;
     const double s = csum_parts(npart, gridDim.x, 1, red);
     if (threadIdx.x == 0) {
@@ -493,18 +504,23 @@ __global__ void __launch_bounds__(kCThreads) k_cupd(const double2* __restrict__ 
     }
 }
 
-// w /= *beta unless the cycle stopped.
+// w /= *beta unless the cycle stopped; with q also the product's fixed-point
+// copy (as the real solver's k_scale).
 __global__ void __launch_bounds__(kCThreads) k_cscale_dev(double2* __restrict__ w, int64_t n,
                                                           const double* __restrict__ beta, const int* __restrict__ stop,
-                                                          unsigned long long* __restrict__ started)
+                                                          unsigned long long* __restrict__ started,
+                                                          const unsigned long long* __restrict__ absmax, FixTarget t)
 {
     if (!*stop) {
         const double inv = 1.0 / *beta;
+        const int E = t.q ? fix_exp(__longlong_as_double((long long)*absmax) * inv) : 0;
+        if (t.q && blockIdx.x == 0 && threadIdx.x == 0) *t.bound = E;
         for (int64_t r = blockIdx.x * (int64_t)kCThreads + threadIdx.x; r < n; r += (int64_t)gridDim.x * kCThreads) {
             double2 a = w[r];
             a.x *= inv;
             a.y *= inv;
             w[r] = a;
+            if (t.q) reinterpret_cast<longlong2*>(t.q)[r] = make_longlong2(fix_pair(a.x, E), fix_pair(a.y, E));
         }
     }
     stamp(started);
@@ -583,6 +599,7 @@ struct CWork {
     int m = 0;
     int nb = 1;            // blocks of the row-chunked kernels
     int R = 512, nbm = 1;  // multi-dot: rows per block, blocks
+    DevBuf<unsigned long long> absmax;   // of w, where the scaling also converts it (else empty)
     DevBuf<double> part, npart, coef, beta, c, scal;
     DevBuf<int> flags;
     DevBuf<unsigned int> counters;
@@ -593,14 +610,14 @@ struct CWork {
     {
         launch(k_cmdot, nbm, kCThreads, (size_t)R * 16, st, V, n, R, J, w, local, alpha, beta_prev, part.p,
                                                         counters.p + 1, reinterpret_cast<double2*>(c.p), coefcol,
-                                                        before, run, stop, ended);
+                                                        before, run, stop, ended, absmax.p);
     }
     void update(const double2* V, int J, double2* w, int mode, int force2, const double* before, int* need2,
                 double* b, const double* ref2, int j, const int* run, int* stop, cudaStream_t st)
     {
         launch(k_cupd, nb, kCThreads, (size_t)J * 16, st, V, n, J, reinterpret_cast<const double2*>(c.p), w, npart.p,
                                                       counters.p + 2, mode, force2, before, need2, b, ref2, j, run,
-                                                      stop);
+                                                      stop, absmax.p);
     }
 };
 
@@ -888,12 +905,13 @@ bool cfix_ready(const ed_ccrs& a, cudaStream_t st)
     return a.fix_state == 1 && cfix_scratch(a, st) != nullptr;
 }
 
+// x null: its fixed-point copy is there already
 void cfix_launch(const ed_ccrs& a, const double* x, double* y, cudaStream_t st)
 {
     const ed_fixq& f = *a.fixq;
     ed_fixq::Scratch& sc = *cfix_scratch(a, st);
     const int P = cfix_parts();
-    fix_convert(x, 2 * a.n, sc.part.p, P, csms() * 4, sc.xq.p, st);
+    if (x) fix_convert(x, 2 * a.n, sc.part.p, P, csms() * 4, sc.xq.p, st);
     const double avg = (double)a.nnz / (double)a.n;
     const int4* A = reinterpret_cast<const int4*>(f.val.p);
     const int4* X = reinterpret_cast<const int4*>(sc.xq.p);
@@ -947,6 +965,18 @@ void cspmv(const ed_ccrs& a, const double* x, double* y, cudaStream_t st)
     }
     cspmv_fp64(a, x, y, st);
 }
+
+FixTarget cspmv_target(const ed_ccrs& a, cudaStream_t st)
+{
+    FixTarget t;
+    if (a.n == 0 || a.upper || !cfix_ready(a, st)) return t;
+    ed_fixq::Scratch& sc = *cfix_scratch(a, st);
+    t.q = sc.xq.p;
+    t.bound = sc.part.p + cfix_parts();
+    return t;
+}
+
+void cspmv_converted(const ed_ccrs& a, double* y, cudaStream_t st) { cfix_launch(a, nullptr, y, st); }
 
 void cspmv_kernel(const ed_ccrs& a, int kernel, const double* x, double* y, cudaStream_t st)
 {
@@ -1054,6 +1084,8 @@ void clanczos_solve(const ed_ccrs& a, const ed_lanczos_params& p, const double* 
     // the cycle is replayed as one CUDA graph.
     int* need2 = cw.flags.p;
     int* stop = cw.flags.p + 1;
+    const FixTarget target = cspmv_target(a, st);
+    if (target.q) cw.absmax.alloc(1);
     auto enqueue_cycle = [&](double2* V, int k) {
         const int64_t coefs = (int64_t)(m - k) * (m + 1);
         launch(k_cycle_begin, (unsigned)std::min<int64_t>(64, (coefs + 255) / 256), 256, 0, st, cw.coef.p + (size_t)k * (m + 1), coefs,
@@ -1063,7 +1095,8 @@ void clanczos_solve(const ed_ccrs& a, const ed_lanczos_params& p, const double* 
             double2* w = V + (int64_t)(j + 1) * n;
             double* coefcol = cw.coef.p + (size_t)j * (m + 1);
             const bool first = (j == k);
-            cspmv(a, reinterpret_cast<const double*>(vj), reinterpret_cast<double*>(w), st);
+            if (!first && target.q) cspmv_converted(a, reinterpret_cast<double*>(w), st);
+            else cspmv(a, reinterpret_cast<const double*>(vj), reinterpret_cast<double*>(w), st);
             unsigned long long* ended = clock.p + 2 * j + 1;
             if (!first) {
                 launch(k_clocal, cw.nb, kCThreads, 0, st, vj, w, n, cw.part.p, cw.counters.p, coefcol, j,
@@ -1076,7 +1109,8 @@ void clanczos_solve(const ed_ccrs& a, const ed_lanczos_params& p, const double* 
             cw.update(V, J, w, 1, first ? 1 : 0, cw.scal.p, need2, cw.beta.p + j, ref2, j, nullptr, stop, st);
             cw.mdot(V, J, w, 0, nullptr, nullptr, coefcol, cw.scal.p + 2, need2, stop, st);
             cw.update(V, J, w, 2, 0, nullptr, nullptr, cw.beta.p + j, ref2, j, need2, stop, st);
-            launch(k_cscale_dev, cw.nb, kCThreads, 0, st, w, n, cw.beta.p + j, stop, clock.p + 2 * (j + 1));
+            launch(k_cscale_dev, cw.nb, kCThreads, 0, st, w, n, cw.beta.p + j, stop, clock.p + 2 * (j + 1), cw.absmax.p,
+                   j + 1 < m ? target : FixTarget());
             ED_CUDA(cudaGetLastError());
         }
     };

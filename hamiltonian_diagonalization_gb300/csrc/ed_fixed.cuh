@@ -109,6 +109,20 @@ __device__ __forceinline__ double round_i128(__int128 S, int sc)
     return round_u128((unsigned long long)(M >> 64), (unsigned long long)M, neg, sc);
 }
 
+// The largest |v| of a block's threads (as the bits without the sign, which
+// order as the values) into *at; m is a shared word, zero at the start.
+__device__ __forceinline__ unsigned long long abs_bits(double v)
+{
+    return (unsigned long long)__double_as_longlong(v) & 0x7FFFFFFFFFFFFFFFull;
+}
+
+__device__ __forceinline__ void block_absmax(unsigned long long v, unsigned long long* m)
+{
+    const unsigned hi = (unsigned)(v >> 32), top = __reduce_max_sync(0xffffffffu, hi);
+    const unsigned lo = __reduce_max_sync(0xffffffffu, hi == top ? (unsigned)v : 0u);
+    if ((threadIdx.x & 31) == 0) atomicMax(m, (unsigned long long)top << 32 | lo);
+}
+
 // Per-block maxima of fix_exp over v[0, n) into part[blockIdx.x].
 __global__ void __launch_bounds__(256) k_fix_exp(const double* __restrict__ v, int64_t n, int* __restrict__ part)
 {

@@ -333,6 +333,19 @@ void two_level_ladder(const ed_basis& b, const double* x, double* y, int dir, cu
 void cterms_derive(ed_cterms& t);
 void cham_build_crs(const ed_basis& b, const ed_cterms& t, int upper, ed_ccrs& a, cudaStream_t st);
 void cspmv(const ed_ccrs& a, const double* x, double* y, cudaStream_t st);
+
+// Where the product of this matrix on this stream reads x in fixed point, for
+// a solver whose last kernel before the product writes it there: q = x's limb
+// pairs, *bound = the exponent bound.  q is null where the product reads x
+// itself.  *_converted runs the product that reads them.
+struct FixTarget {
+    int64_t* q = nullptr;
+    int* bound = nullptr;
+};
+FixTarget cspmv_target(const ed_ccrs& a, cudaStream_t st);
+void cspmv_converted(const ed_ccrs& a, double* y, cudaStream_t st);
+FixTarget spmv_target(const ed_crs& a, cudaStream_t st);
+void spmv_converted(const ed_crs& a, const double* x, double* y, cudaStream_t st);
 // kernel 0: as cspmv; 1: the FP64 row kernel; 2: the fixed-point integer kernel (full storage)
 void cspmv_kernel(const ed_ccrs& a, int kernel, const double* x, double* y, cudaStream_t st);
 // the complex product's fixed-point copy, made before a solver captures its cycles

@@ -21,7 +21,8 @@
 // Kernels per step: the product, k_local_dot (alpha, ||H v_j||), k_mdot with
 // the three-term step folded into its staging, k_update, the gated second
 // k_mdot/k_update pair (an early return when the DGKS test passed) and
-// k_scale.  Each reduction is finished by the last block of its own launch.
+// k_scale, which also writes the next product's fixed-point copy of the vector.
+// Each reduction is finished by the last block of its own launch.
 // Every decision (second pass, breakdown) is a device flag, so a whole cycle
 // is enqueued without host round trips and replayed as a CUDA graph.
 // After m steps the m x m projected matrix is diagonalised on the host, the
@@ -34,7 +35,7 @@
 #include <vector>
 
 #include "ed_lanczos.h"
-#include "ed_launch.cuh"
+#include "ed_fixed.cuh"
 #include "ed_split.h"
 
 namespace edgb {
@@ -179,10 +180,12 @@ __global__ void __launch_bounds__(kThreads) k_mdot(const double* __restrict__ V,
                                                    unsigned int* __restrict__ counter, double* __restrict__ c,
                                                    double* __restrict__ coefcol, double* __restrict__ before,
                                                    const int* __restrict__ run, const int* __restrict__ stop,
-                                                   unsigned long long* __restrict__ ended)
+                                                   unsigned long long* __restrict__ ended,
+                                                   unsigned long long* __restrict__ absmax)
 {
     if (blockIdx.x == 0) stamp(ended);
     if ((run && !*run) || (stop && *stop)) return;
+    if (absmax && blockIdx.x == 0 && threadIdx.x == 0) *absmax = 0ull;   // k_update's
     extern __shared__ double sw[];
     const int64_t r0 = (int64_t)blockIdx.x * R;
     const int len = (int)min((int64_t)R, n - r0);
@@ -261,23 +264,28 @@ __global__ void __launch_bounds__(kThreads) k_mdot(const double* __restrict__ V,
 //   mode 2 (second pass): beta and the breakdown test;
 //   mode 0: nothing (the counter is not touched).
 // beta = ||w||; breakdown (stop = j + 1) when beta <= 1e-12 sqrt(*ref2), the
-// new direction having vanished relative to ||H v_j||.
+// new direction having vanished relative to ||H v_j||.  *absmax (when given)
+// takes the largest |w_r|, for k_scale's fixed-point copy.
 __global__ void __launch_bounds__(kThreads) k_update(const double* __restrict__ V, int64_t n, int J,
                                                      const double* __restrict__ c, double* __restrict__ w,
                                                      double* __restrict__ npart, unsigned int* __restrict__ counter,
                                                      int mode, int force2, const double* __restrict__ before,
                                                      int* __restrict__ need2, double* __restrict__ beta,
                                                      const double* __restrict__ ref2, int j,
-                                                     const int* __restrict__ run, int* __restrict__ stop)
+                                                     const int* __restrict__ run, int* __restrict__ stop,
+                                                     unsigned long long* __restrict__ absmax)
 {
     if ((run && !*run) || (stop && *stop)) return;
     extern __shared__ double sc[];
     __shared__ double red[kThreads / 32];
+    __shared__ unsigned long long top;
+    if (threadIdx.x == 0) top = 0ull;
     for (int i = threadIdx.x; i < J; i += kThreads) sc[i] = -c[i];
     __syncthreads();
     int64_t r0, r1;
     chunk(n, gridDim.x, blockIdx.x, r0, r1);
     double nn = 0.0;
+    unsigned long long mx = 0ull;
     for (int64_t r = r0 + threadIdx.x; r < r1; r += kThreads) {
         // eight column loads in flight, two FMA chains (even / odd columns)
         double acc = w[r], acc2 = 0.0;
@@ -296,9 +304,14 @@ __global__ void __launch_bounds__(kThreads) k_update(const double* __restrict__ 
         acc += acc2;
         w[r] = acc;
         nn = fma(acc, acc, nn);
+        mx = max(mx, abs_bits(acc));
     }
+    if (absmax) block_absmax(mx, &top);
     nn = block_sum(nn, red);
-    if (threadIdx.x == 0) npart[blockIdx.x] = nn;
+    if (threadIdx.x == 0) {
+        npart[blockIdx.x] = nn;
+        if (absmax) atomicMax(absmax, top);
+    }
     if (mode == 0 || !last_block(counter)) return;
     const double s = sum_parts(npart, gridDim.x, red);
     if (threadIdx.x == 0) {
@@ -316,14 +329,26 @@ __global__ void __launch_bounds__(kThreads) k_update(const double* __restrict__ 
     }
 }
 
+// w /= *beta (unless the cycle stopped); with q also the product's fixed-point
+// copy of the result: rounding keeps the order, so the largest entry is the
+// rounded quotient of the largest |w_r|, which k_update left in *absmax.  (A
+// product's own conversion passes over the vector once for the bound and once
+// for the copy: 5.4 us of a step's 56 at n = 8,512, 8.7 of 140 at 54,484
+// complex rows.)
 __global__ void __launch_bounds__(kThreads) k_scale(double* __restrict__ w, int64_t n,
                                                     const double* __restrict__ beta, const int* __restrict__ stop,
-                                                    unsigned long long* __restrict__ started)
+                                                    unsigned long long* __restrict__ started,
+                                                    const unsigned long long* __restrict__ absmax, FixTarget t)
 {
     if (!(stop && *stop)) {
         const double inv = 1.0 / *beta;
-        for (int64_t r = blockIdx.x * (int64_t)kThreads + threadIdx.x; r < n; r += (int64_t)gridDim.x * kThreads)
-            w[r] *= inv;
+        const int E = t.q ? fix_exp(__longlong_as_double((long long)*absmax) * inv) : 0;
+        if (t.q && blockIdx.x == 0 && threadIdx.x == 0) *t.bound = E;
+        for (int64_t r = blockIdx.x * (int64_t)kThreads + threadIdx.x; r < n; r += (int64_t)gridDim.x * kThreads) {
+            const double x = w[r] * inv;
+            w[r] = x;
+            if (t.q) t.q[r] = fix_pair(x, E);
+        }
     }
     stamp(started);
 }
@@ -487,6 +512,7 @@ struct Work {
     DevBuf<double> beta;             // m+2
     DevBuf<double> c;                // m+2
     DevBuf<double> junk;             // m+2, coefficient sink for host-side orthonormalisation
+    DevBuf<unsigned long long> absmax;   // of w, where the scaling also converts it (else empty)
     DevBuf<double> scal;             // [0] ||w||^2 before pass 1, [1] ||H v_j||^2, [2] before pass 2
     DevBuf<int> flags;               // [0] second pass wanted, [1] breakdown step + 1
     DevBuf<unsigned int> counters;   // last-block counters: [0] local dot, [1] multi-dot, [2] update
@@ -498,13 +524,13 @@ struct Work {
               unsigned long long* ended = nullptr)
     {
         launch(k_mdot, nbm, kThreads, (size_t)R * 8, st, Vb, n, R, J, x, local, alpha, beta_prev, part.p,
-                                                      counters.p + 1, c.p, coefcol, before, run, stop, ended);
+                                                      counters.p + 1, c.p, coefcol, before, run, stop, ended, absmax.p);
     }
     void update(const double* Vb, int J, double* x, int mode, int force2, const double* before, int* need2,
                 double* b, const double* ref2, int j, const int* run, int* stop, cudaStream_t st)
     {
         launch(k_update, nb, kThreads, (size_t)J * 8, st, Vb, n, J, c.p, x, npart.p, counters.p + 2, mode, force2,
-                                                       before, need2, b, ref2, j, run, stop);
+                                                       before, need2, b, ref2, j, run, stop, absmax.p);
     }
 };
 
@@ -535,7 +561,7 @@ double orthonormalise_column(Work& w, double* Vbase, int col, cudaStream_t st)
     const double nrm = std::sqrt(host_sum_parts(w.part.p, w.nb, st));
     ED_REQUIRE(nrm > 0.0 && std::isfinite(nrm), ED_ERR_ARG, "start vector is zero or not finite");
     ED_CUDA(cudaMemcpyAsync(w.beta.p + w.m + 1, &nrm, 8, cudaMemcpyHostToDevice, st));
-    launch(k_scale, w.nb, kThreads, 0, st, x, w.n, w.beta.p + w.m + 1, nullptr, nullptr);
+    launch(k_scale, w.nb, kThreads, 0, st, x, w.n, w.beta.p + w.m + 1, nullptr, nullptr, nullptr, FixTarget());
     ED_CUDA(cudaGetLastError());
     ED_CUDA(cudaStreamSynchronize(st));
     return nrm;
@@ -701,6 +727,8 @@ void lanczos_once(const ed_op& op, const ed_lanczos_params& p, const double* v0_
     // replays it as one CUDA graph.
     int* need2 = w.flags.p;
     int* stop = w.flags.p + 1;
+    const FixTarget target = op.kind == ed_op::CRS ? spmv_target(*op.crs, st) : FixTarget();
+    if (target.q) w.absmax.alloc(1);
     auto enqueue_cycle = [&](int k) {
         const int64_t coefs = (int64_t)(m - k) * (m + 1);
         launch(k_cycle_begin, (unsigned)std::min<int64_t>(64, (coefs + 255) / 256), 256, 0, st, w.coef.p + (size_t)k * (m + 1), coefs,
@@ -710,7 +738,8 @@ void lanczos_once(const ed_op& op, const ed_lanczos_params& p, const double* v0_
             double* wv = w.V.p + (int64_t)(j + 1) * n;
             double* coefcol = w.coef.p + (size_t)j * (m + 1);
             const bool first = (j == k);
-            op_apply(op, vj, wv, st);
+            if (!first && target.q) spmv_converted(*op.crs, vj, wv, st);
+            else op_apply(op, vj, wv, st);
             unsigned long long* ended = clock.p + 2 * j + 1;
             if (!first) {
                 launch(k_local_dot, w.nb, kThreads, 0, st, vj, wv, n, w.part.p, w.counters.p, coefcol, j,
@@ -726,7 +755,8 @@ void lanczos_once(const ed_op& op, const ed_lanczos_params& p, const double* v0_
             w.mdot(w.V.p, J, wv, 0, nullptr, nullptr, coefcol, w.scal.p + 2, need2, stop, st);
             w.update(w.V.p, J, wv, 2, 0, nullptr, nullptr, w.beta.p + j, first ? w.scal.p : w.scal.p + 1, j, need2,
                      stop, st);
-            launch(k_scale, w.nb, kThreads, 0, st, wv, n, w.beta.p + j, stop, clock.p + 2 * (j + 1));
+            launch(k_scale, w.nb, kThreads, 0, st, wv, n, w.beta.p + j, stop, clock.p + 2 * (j + 1), w.absmax.p,
+                   j + 1 < m ? target : FixTarget());
             ED_CUDA(cudaGetLastError());
         }
     };

@@ -1077,12 +1077,13 @@ bool fix_ready(const ed_crs& a, cudaStream_t st, bool sell = false)
     return a.fix_state == 1 && fix_copy(a, sell, st) && fix_scratch(a, st) != nullptr;
 }
 
-// x's fixed-point copy into the stream's scratch; returns the scratch.
-ed_fixq::Scratch& fix_convert_x(const ed_crs& a, const double* x, cudaStream_t st)
+// x's fixed-point copy into the stream's scratch (or it is there already);
+// returns the scratch.
+ed_fixq::Scratch& fix_convert_x(const ed_crs& a, const double* x, cudaStream_t st, bool converted = false)
 {
     ed_fixq::Scratch& sc = *fix_scratch(a, st);
     const int P = fix_parts();
-    fix_convert(x, a.n, sc.part.p, P, sms() * 4, sc.xq.p, st);
+    if (!converted) fix_convert(x, a.n, sc.part.p, P, sms() * 4, sc.xq.p, st);
     return sc;
 }
 
@@ -1145,19 +1146,19 @@ void fix_launch_staged(const ed_crs& a, const double* x, double* y, long long st
     ED_CUDA(cudaGetLastError());
 }
 
-void blk_launch(const ed_crs& a, const double* x, double* y, cudaStream_t st)
+void blk_launch(const ed_crs& a, const double* x, double* y, cudaStream_t st, bool converted)
 {
     const ed_fixq& f = *a.fixq;
-    ed_fixq::Scratch& sc = fix_convert_x(a, x, st);
+    ed_fixq::Scratch& sc = fix_convert_x(a, x, st, converted);
     launch(k_spmv_blk<6, 4>, sms() * 8, 256, 0, st, f.boff.p, f.bcol.p, reinterpret_cast<const int2*>(f.bval.p),
            reinterpret_cast<const int2*>(sc.xq.p), sc.part.p + fix_parts(), f.ea, y, a.n, f.blocks);
 }
 
 // rows: the product in FP64 where x is not finite (else every entry is NaN).
-void fix_launch(const ed_crs& a, const double* x, double* y, cudaStream_t st, bool rows = false)
+void fix_launch(const ed_crs& a, const double* x, double* y, cudaStream_t st, bool rows = false, bool converted = false)
 {
     const ed_fixq& f = *a.fixq;
-    ed_fixq::Scratch& sc = fix_convert_x(a, x, st);
+    ed_fixq::Scratch& sc = fix_convert_x(a, x, st, converted);
     const int P = fix_parts();
     // matrices below kBlkMinRows, and those without the memory for the blocked
     // copy.  8 lanes a row, 8 loads ahead, at most 64 registers: four CTAs per
@@ -1172,11 +1173,11 @@ void fix_launch(const ed_crs& a, const double* x, double* y, cudaStream_t st, bo
     ED_CUDA(cudaGetLastError());
 }
 
-void fix_launch_sell(const ed_crs& a, const double* x, double* y, cudaStream_t st)
+void fix_launch_sell(const ed_crs& a, const double* x, double* y, cudaStream_t st, bool converted = false)
 {
     const ed_fixq& f = *a.fixq;
     const ed_sell& sl = *a.sell;
-    ed_fixq::Scratch& sc = fix_convert_x(a, x, st);
+    ed_fixq::Scratch& sc = fix_convert_x(a, x, st, converted);
     launch(k_spmv_sell_fix<8, 4>, sms() * 8, 256, 0, st, sl.off.p, sl.len.p, sl.row.p, sl.col.p,
                                                      reinterpret_cast<const int2*>(f.sval.p),
                                                      reinterpret_cast<const int2*>(sc.xq.p), sc.part.p + fix_parts(),
@@ -1310,6 +1311,39 @@ int spmv_staged_wait_test(const ed_crs& a, const double* x, double* y, long long
     return e;
 }
 
+// The fixed-point kernel that a matrix below the split product's sizes takes,
+// with what it needs made when missing and not capturing.
+enum class FixRoute { kNone, kSell, kBlocked, kRows };
+
+static FixRoute fix_route(const ed_crs& a, cudaStream_t st)
+{
+    if (sell_shape(a) && a.sell_state == 0) spmv_prepare(a, st);   // waits for a solver's explicit call while capturing
+    if (sell_shape(a) && a.sell_state == 1) return fix_ready(a, st, true) ? FixRoute::kSell : FixRoute::kNone;
+    if (blk_shape(a) && blk_ready(a, st)) return FixRoute::kBlocked;
+    if (fix_shape(a) && fix_ready(a, st)) return FixRoute::kRows;
+    return FixRoute::kNone;
+}
+
+FixTarget spmv_target(const ed_crs& a, cudaStream_t st)
+{
+    FixTarget t;
+    if (a.n == 0 || a.product_kernel > 0 || split_prepare(a, st) || fix_route(a, st) == FixRoute::kNone) return t;
+    ed_fixq::Scratch& sc = *fix_scratch(a, st);
+    t.q = sc.xq.p;
+    t.bound = sc.part.p + fix_parts();
+    return t;
+}
+
+void spmv_converted(const ed_crs& a, const double* x, double* y, cudaStream_t st)
+{
+    switch (fix_route(a, st)) {
+    case FixRoute::kSell: fix_launch_sell(a, x, y, st, true); return;
+    case FixRoute::kBlocked: blk_launch(a, x, y, st, true); return;
+    case FixRoute::kRows: fix_launch(a, x, y, st, short_rows(a), true); return;
+    case FixRoute::kNone: throw Error(ED_ERR_INTERNAL, "a converted product without a fixed-point kernel");
+    }
+}
+
 void spmv(const ed_crs& a, const double* x, double* y, cudaStream_t st)
 {
     if (a.n == 0) return;
@@ -1325,28 +1359,19 @@ void spmv(const ed_crs& a, const double* x, double* y, cudaStream_t st)
         }
         return;
     }
-    if (sell_shape(a) && a.sell_state == 0) spmv_prepare(a, st);   // waits for a solver's explicit call while capturing
+    switch (fix_route(a, st)) {
+    case FixRoute::kSell: fix_launch_sell(a, x, y, st); return;
+    case FixRoute::kBlocked: blk_launch(a, x, y, st, false); return;
+    case FixRoute::kRows: fix_launch(a, x, y, st, short_rows(a)); return;
+    case FixRoute::kNone: break;
+    }
     if (sell_shape(a) && a.sell_state == 1) {
-        if (fix_ready(a, st, true)) {
-            // the fixed-point sliced ELL (two-level N=8, 2S=21: see
-            // k_spmv_sell_fix), else the FP64 kernel below
-            fix_launch_sell(a, x, y, st);
-            return;
-        }
         // rows of fewer than 96 elements (two-level sectors, small one-level
         // ones), measured on GB300 at two-level N=8, 2S=18 (2.03M rows of 59
         // on average) / 2S=21 (5.90M rows of 73): sliced ELL with 16 loads
         // ahead 0.305 / 1.052 ms (8 ahead 0.326 / 1.110, 24 0.303 / 1.045,
         // 32 0.310 / 1.055) against the best row kernels 0.333 / 1.197
         sell_launch<16>(a, x, y, st);
-        return;
-    }
-    if (blk_shape(a) && blk_ready(a, st)) {
-        blk_launch(a, x, y, st);
-        return;
-    }
-    if (fix_shape(a) && fix_ready(a, st)) {
-        fix_launch(a, x, y, st, short_rows(a));
         return;
     }
     const double avg = (double)a.nnz / (double)a.n;
