@@ -11,8 +11,8 @@ reorthogonalisation -> verified residuals.
          left in HBM), seconds per solve, CUDA events on the launching stream
   e2e    the one-call public API ed_solve_sector from host buffers: start
          vector in, eigenvalues and eigenvectors out, copies inside the timing
-  roofline  the stored-CRS SpMV (the fixed-point integer kernel with its two
-         passes over x), algorithmic bytes per product
+  roofline  the stored-CRS SpMV (the fixed-point integer kernel on the
+         row-blocked copy of the matrix), algorithmic bytes of the CRS per product
          nnz*(8+4) + (n+1)*8 + 2*n*8 over its average in-solve duration
   max_rel_eig_vs_fixture  the eigenvalues against the committed ARPACK run
          of the same Hamiltonian (tests/golden/arpack_n11_2s30_lz0.json)
@@ -470,7 +470,7 @@ def main():
                       "nnz_full": nnz},
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                          "traffic": (traffic or {}).get("bytes_per_launch"),
-                         "kernel": "k_spmv_fix<8,8> (+ k_fix_exp, k_fix_conv on x)", "bytes_per_launch": bytes_per,
+                         "kernel": "k_spmv_blk<6,4>", "bytes_per_launch": bytes_per,
                          "avg_launch_ms": spmv_s * 1000.0, "standalone_launch_ms": r["spmv_ms_alone"],
                          "peak_source": f"{peak_kind} (MEASURED_PEAKS.json hbm_gbs)" if peak_kind == "measured"
                          else "fallback 6.8 TB/s"},

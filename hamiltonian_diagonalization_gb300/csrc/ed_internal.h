@@ -360,9 +360,9 @@ void terms_upload(ed_terms& t);
 void ham_diagonal(const ed_basis& b, const ed_terms& t, double* diag, cudaStream_t st);
 void ham_build_crs(const ed_basis& b, const ed_terms& t, int upper, ed_crs& a, cudaStream_t st);
 void spmv(const ed_crs& a, const double* x, double* y, cudaStream_t st);
-// Make the product's sliced-ELL copy of a full-storage CRS now (a no-op when
-// made, declined, or the stream is capturing); solvers call it before they
-// capture their cycles.
+// Make what the default product needs (split plan, row-blocked or sliced-ELL
+// copy) now (a no-op when made, declined, or the stream is capturing); solvers
+// call it before they capture their cycles.
 void spmv_prepare(const ed_crs& a, cudaStream_t st);
 // Gives back what products on st keep for that stream, before it is destroyed.
 void spmv_release(const ed_crs& a, cudaStream_t st);

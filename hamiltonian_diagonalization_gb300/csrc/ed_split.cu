@@ -18,7 +18,7 @@
 // warp, and the gathers of x run along a segment.  (The stored-matrix kernels
 // are bound by L1 gather wavefronts: a warp's 32 gathers of a CRS row hit
 // 12 different lines on average and take 13 of its 19 wavefronts per 32
-// elements, 87 % of the L1's rate; profiles in the repository's notes.)
+// elements, 87 % of the L1's rate.)
 //
 // Two passes cover all hops: the native pass (P = high part, rows in the
 // basis order) takes the hops that leave S alone, change one of its orbitals
@@ -589,6 +589,13 @@ __device__ __forceinline__ void move_lists(const SplitArgs& g, int a0, int a1, i
 // lists of the other gammas are taken by the block's warps from a queue; each
 // warp keeps its own exact sums of the segment's rows in shared memory, and
 // 32 consecutive entries hold 32 different rows, so it adds without atomics.
+//
+// Instruction issue and shared-memory latency bound it, so the blocks are
+// small (64 threads, 18 per SM) to keep many segments in flight.  GB300, both
+// passes with the conversion of x, against the element-generating kernel: N=11,
+// 2S=30 2.76 -> 0.73 ms, N=12, 2S=33 18.3 -> 4.13 ms; against the stored kernels
+// see the dispatch in ed_spmv.cu.  Move lists by (orbital, orbital) instead of
+// by distance took 1.53 ms at N=11.
 template <bool NATIVE>
 __global__ void __launch_bounds__(kThreads, 18) k_split_product(SplitArgs g)
 {
@@ -689,7 +696,9 @@ __device__ __forceinline__ void keep_task(const SplitArgs& g, int p, int size, i
 
 // Hops that leave S alone only (two levels): a warp takes one primary word
 // and 32 * kIdRows rows of its segment, or, where segments are short, up to
-// 32 / width words with `width` lanes each.
+// 32 / width words with `width` lanes each.  The gathers of x from L2 bound it:
+// GB300, N=8, 2S=18 254 us against 281 of the sliced ELL copy, N=8, 2S=21 760
+// against 993; segments staged in shared memory were slower.
 template <bool NATIVE>
 __global__ void __launch_bounds__(kThreads, 20) k_split_keep(SplitArgs g, int ntasks)
 {

@@ -9,14 +9,16 @@
 // FP64 product is FP64-bound before it is HBM-bound.  The default products of
 // full storage therefore run on the integer pipes in exact fixed-point
 // arithmetic (ed_fixed.cuh: values and x in 58-bit fixed point, exact 128-bit
-// row sums, one rounding to FP64), in one of two layouts:
-//  - rows of 96 and more elements (the one-level sectors): k_spmv_fix, 8
-//    lanes a row, each lane's exact sum over its share of the row, the lanes'
-//    sums added exactly;
+// row sums, one rounding to FP64), in one of these layouts:
+//  - small sectors: k_spmv_fix on the CRS, 8 lanes a row, each lane's exact
+//    sum over its share of the row, the lanes' sums added exactly;
+//  - rows of 96 and more elements (the one-level sectors): k_spmv_blk over
+//    blocks of eight rows (ed_blocked.cuh);
 //  - shorter rows (two-level sectors): k_spmv_sell_fix over a sliced-ELL copy
 //    (rows sorted by length within windows, chunks of 32 rows transposed), one
-//    lane a row, no reduction, and the lanes of a chunk finish together.
-// Both give the same bits.  The FP64 kernels (k_spmv_full, k_spmv_rows,
+//    lane a row, no reduction, and the lanes of a chunk finish together;
+//  - the largest sectors: no elements at all, the split product (ed_split.cu).
+// All give the same bits.  The FP64 kernels (k_spmv_full, k_spmv_rows,
 // k_spmv_sell) remain as selectable alternatives, spending FP64 instructions
 // only where they must: one FMA per element, as few additions as the
 // reduction allows, none for lanes with no element.  Column and value streams

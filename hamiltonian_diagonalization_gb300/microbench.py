@@ -47,7 +47,7 @@ def main():
     ap.add_argument("--reps", type=int, default=20)
     ap.add_argument("--warmup", type=int, default=3)
     ap.add_argument("--upper", action="store_true", help="store the upper triangle (the reference's layout)")
-    ap.add_argument("--matfree", action="store_true", help="regenerate elements on the fly")
+    ap.add_argument("--matfree", action="store_true", help="without a stored matrix")
     ap.add_argument("--batch", type=int, default=0, help="time the block product of this many Hamiltonians")
     ap.add_argument("--no-autotune", action="store_true", help="batch: keep the default tile (32 per row, L1)")
     ap.add_argument("--rotate", default="", help="n,m,k: time the restart rotation instead")

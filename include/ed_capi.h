@@ -168,13 +168,20 @@ ed_status ed_ham_diagonal(const ed_basis* b, const ed_terms* t, double* diag_dev
 /* y = H x from a stored CRS (either storage).  Device vectors of n doubles.
  * Replaces MatrixVectorFunction::Simple (hamiltonians/matrix_vector_routines.hpp:94-104)
  * -> SymmetricMatrixVectorMultiply (utilities/mathematics/sparse_linear_algebra.hpp:78-168).
- * Full storage uses the fixed-point integer kernels (kernel 6 below for 96
- * and more elements a row on average, the one-level sectors; kernel 8 on
- * the sliced-ELL copy for shorter rows from 4096 rows up, the two-level
- * sectors): the first product makes a fixed-point copy of the values (8
- * bytes an element) and, per stream, an n-element scratch for x; products of
- * one matrix on one stream must not overlap (they share that stream's
- * scratch). */
+ * Full storage uses fixed-point integer arithmetic (kernel 6 below) in the
+ * layout that suits the size:
+ *   - 96 and more elements a row on average (the one-level sectors): kernel 6,
+ *     from 65,536 rows a row-blocked copy of the matrix (12.5 bytes an
+ *     element; the same bits), from 1,572,864 rows the split product;
+ *   - shorter rows (the two-level sectors): kernel 6 from 4,096 rows, kernel 8
+ *     on the sliced-ELL copy from 32,768, the split product from 1,048,576.
+ * The split product sums over the moves of two parts of the Fock word instead
+ * of over the elements (the same bits); it needs a matrix built by this
+ * library, in either storage.  Where the memory for a copy or plan is
+ * missing, the next simpler kernel runs.  Other matrices take FP64 kernels.
+ * The first product makes the copies and, per stream, an n-element scratch
+ * for x; products of one matrix on one stream must not overlap (they share
+ * that stream's scratch). */
 ed_status ed_spmv(const ed_crs* a, const double* x_dev, double* y_dev, ed_stream stream);
 
 /* The same product with a chosen kernel of the full storage, for measuring
@@ -267,7 +274,7 @@ typedef struct {
     int64_t matvecs;
     double max_residual;    /* max over returned pairs of the residual (true one if verify) */
     double seconds;         /* wall time of the solve                                  */
-    double spmv_seconds;    /* device time inside the H*v products                     */
+    double spmv_seconds;    /* device time inside the H*v products (the device's clock) */
     int breakdowns;
 } ed_solve_info;
 
@@ -389,7 +396,7 @@ typedef struct {
     int64_t block_products;   /* each applies every Hamiltonian of the batch once   */
     double max_residual;
     double seconds;
-    double spmm_seconds;      /* device time inside the block products               */
+    double spmm_seconds;      /* device time inside the block products (its clock)   */
     int breakdowns;
     int tile_hamiltonians;    /* autotuned Hamiltonians per row tile of the block product */
     int tile_unroll;          /* autotuned loads in flight per lane                  */
