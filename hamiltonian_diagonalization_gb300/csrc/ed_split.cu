@@ -34,6 +34,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <numeric>
 
 #include "ed_fixed.cuh"
 #include "ed_hop.cuh"
@@ -59,7 +60,7 @@ static_assert(kSegRows == 1 << kRowBits, "row field");
 
 enum GammaType { kKeep = 0, kEmpty = 1, kFill = 2 };   // and the moves, in lists of their own
 constexpr int kKeepParts = 8;        // kKeep's alpha entries are listed in so many parts, one after another
-constexpr int kMaxSideBits = 24;     // tables over one part's words
+constexpr int kMaxSideBits = 24;     // tables over one part's words (PartArgs::w)
 
 int sms()
 {
@@ -152,6 +153,46 @@ __device__ __forceinline__ bool gamma_acts(const GenArgs& g, uint32_t S, int gm,
     const uint32_t mask = g.slo < g.plo ? ~((2u << o) - 1u) : (1u << o) - 1u;
     odd = __popc(S & out & mask) & 1;
     return true;
+}
+
+// Words of one part: how many choices of p of the orbitals below b have the
+// weight sum s, count[(b (N + 1) + p) span + s].
+struct PartArgs {
+    int bits, N, span;
+    int w[24];
+    const int *count, *cls, *start;   // cls: per popcount span + sum, -1 where the sector has none
+};
+
+// Every word of a class to its place: classes one after another, ascending
+// within a class.  The rank in its class is the sum over its orbitals b of the
+// words that agree above b and leave b empty.  base (when wanted): the
+// segment's first row in the transposed order, cbase[c] + rank size[c].  (The
+// host enumerating the words by popcount and uploading them took 1.6 ms of a
+// first product's 4.0 at two levels N=8, 2S=18, with 4e5 words in either part.)
+__global__ void k_split_words(PartArgs a, uint32_t* __restrict__ word, int* __restrict__ cls, int* __restrict__ base,
+                              const int* __restrict__ cbase, const int* __restrict__ size)
+{
+    const uint32_t end = 1u << a.bits;
+    for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < end; v += gridDim.x * blockDim.x) {
+        const int pop = __popc(v);
+        if (pop > a.N) continue;
+        int sum = 0;
+        for (uint32_t m = v; m; m &= m - 1) sum += a.w[__ffs((int)m) - 1];
+        const int c = a.cls[pop * a.span + sum];
+        if (c < 0) continue;
+        int rank = 0, p = pop;
+        for (uint32_t m = v; m;) {
+            const int b = 31 - __clz((int)m);
+            rank += a.count[(b * (a.N + 1) + p) * a.span + sum];
+            --p;
+            sum -= a.w[b];
+            m ^= 1u << b;
+        }
+        const int at = a.start[c] + rank;
+        word[at] = v;
+        cls[at] = c;
+        if (base) base[at] = cbase[c] + rank * size[c];
+    }
 }
 
 // table[word] = segment length of the primary word, for the scan of bases
@@ -719,40 +760,30 @@ __global__ void __launch_bounds__(kThreads, 20) k_split_keep(SplitArgs g, int nt
 
 // ------------------------------------------------------------------ the plan
 
-// The words of one part with at most N bits set, grouped by class.
+// The words of one part that the sector's classes hold, by class, ascending
+// within each (on the device), and the classes' places and sizes.
 struct PartWords {
-    std::vector<uint32_t> word;      // by class, ascending
-    std::vector<int> cls;            // class of each
-    std::vector<int> start, size;    // per class
+    int count = 0;
+    uint32_t* word = nullptr;
+    int *cls = nullptr, *base = nullptr;
+    std::vector<int> start, size;
 };
 
-// words of each key = popcount * span + weight sum, up to N bits set
-void count_part(const std::vector<int>& w, int N, int span, std::vector<int>& count)
+// count[(b (N + 1) + p) span + s]: choices of p of the first b orbitals with
+// weight sum s, b = 0 .. bits
+std::vector<int> part_counts(const std::vector<int>& w, int N, int span)
 {
-    count[0] = 1;
-    for (int wk : w)
-        for (int pop = N; pop >= 1; --pop)
-            for (int sum = span - 1; sum >= wk; --sum) count[pop * span + sum] += count[(pop - 1) * span + sum - wk];
-}
-
-// f(key, word) for every word of min_pop .. N bits set, ascending within each
-// key = popcount * span + weight sum
-template <class F>
-void for_part(const std::vector<int>& w, int N, int min_pop, int span, F&& f)
-{
-    const int B = (int)w.size(), lo_bits = std::min(B, 12);
-    std::vector<int> lo(1u << lo_bits), hi(1u << (B - lo_bits));
-    for (size_t i = 1; i < lo.size(); ++i) lo[i] = lo[i & (i - 1)] + w[__builtin_ctzll(i)];
-    for (size_t i = 1; i < hi.size(); ++i) hi[i] = hi[i & (i - 1)] + w[lo_bits + __builtin_ctzll(i)];
-    for (int pop = std::max(0, min_pop); pop <= std::min(N, B); ++pop) {
-        uint64_t v = (1ull << pop) - 1, end = 1ull << B;
-        while (v < end) {
-            f(pop * span + lo[v & ((1u << lo_bits) - 1)] + hi[v >> lo_bits], (uint32_t)v);
-            if (v == 0) break;
-            const uint64_t r = v + (v & (0 - v));   // next word of the same popcount
-            v = r | ((v ^ r) >> (2 + __builtin_ctzll(v)));
-        }
+    const size_t layer = (size_t)(N + 1) * span;
+    std::vector<int> t(layer * (w.size() + 1), 0);
+    t[0] = 1;
+    for (size_t b = 0; b < w.size(); ++b) {
+        const int *from = t.data() + layer * b, wb = w[b];
+        int* to = t.data() + layer * (b + 1);
+        std::copy(from, from + layer, to);
+        for (int p = 1; p <= N; ++p)
+            for (int sum = wb; sum < span; ++sum) to[(size_t)p * span + sum] += from[(size_t)(p - 1) * span + sum - wb];
     }
+    return t;
 }
 
 template <class T>
@@ -839,11 +870,11 @@ struct SideBuild {
         count_launch();
     }
 
-    // given_base: the segments' bases (transposed pass), else the scan over
-    // the primary words in ascending order (native)
-    bool count(const std::vector<int>* given_base)
+    // given_base: the segments' bases are P's (transposed pass), else the scan
+    // over the primary words in ascending order (native)
+    bool count(bool given_base)
     {
-        np = (int)P.word.size();
+        np = P.count;
         nc = (int)P.start.size();
         out.gammas = g.gammas = G = (int)gamma.size();
         int longest = 0;
@@ -852,16 +883,18 @@ struct SideBuild {
         if (lists && longest > (int)kRankMask) return false;
         out.nseg = (longest + kSegRows - 1) / kSegRows;
         out.rows = (std::min(longest, kSegRows) + 31) / 32 * 32;
-        pword = tmp.put(P.word, st);
+        pword = P.word;
         g.gamma = tmp.put(gamma, st);
-        upload(out.pcls, P.cls, st);
+        out.pcls.alloc(np);
+        ED_CUDA(cudaMemcpyAsync(out.pcls.p, P.cls, (size_t)np * 4, cudaMemcpyDeviceToDevice, st));
         upload(out.ssize, S.size, st);
         const int64_t nw = 1ll << g.pbits;
         by_word = tmp.take<int>((size_t)nw);
         ED_CUDA(cudaMemsetAsync(by_word, 0xFF, (size_t)nw * 4, st));
         int64_t* scan = nullptr;
         if (given_base) {
-            upload(out.pbase, *given_base, st);
+            out.pbase.alloc(np);
+            ED_CUDA(cudaMemcpyAsync(out.pbase.p, P.base, (size_t)np * 4, cudaMemcpyDeviceToDevice, st));
         } else {
             int64_t* len = tmp.take<int64_t>((size_t)nw);
             scan = tmp.take<int64_t>((size_t)nw + 1);
@@ -878,11 +911,10 @@ struct SideBuild {
             k_split_alpha<<<grid_of(na, 128), 128, 0, st>>>(g, pword, np, by_word, cnt, nullptr, 0, nullptr);
         });
         if (lists) {
-            sword = tmp.put(S.word, st);
+            sword = S.word;
             sstart = tmp.put(S.start, st);
             rank = tmp.take<int>((size_t)1 << g.sbits);
-            k_split_ranks<<<grid_of((int64_t)S.word.size(), 256), 256, 0, st>>>(sword, tmp.put(S.cls, st), sstart, (int)S.word.size(),
-                                                                               rank);
+            k_split_ranks<<<grid_of(S.count, 256), 256, 0, st>>>(sword, S.cls, sstart, S.count, rank);
             count_launch();
             counted(list, (int64_t)nc * G * out.nseg, [&](int64_t* cnt) {
                 k_split_lists<<<sms() * 8, 256, 0, st>>>(g, sword, sstart, out.ssize.p, rank, nc, out.nseg, cnt, nullptr, nullptr);
@@ -1030,48 +1062,33 @@ std::unique_ptr<SplitPlan> split_build(const SplitSource& s, const double* diag,
             wmax = std::max(wmax, std::fabs(w));
         }
     // words of both parts by (popcount, weight sum), then the classes the sector joins
-    int span = 1;
-    for (int w : wl) span += w;
-    for (int w : wh) span += w;
-    const int nkeys = (s.N + 1) * span;
-    std::vector<int> lcount(nkeys, 0), hcount(nkeys, 0), lclass(nkeys, -1), hclass(nkeys, -1);
-    count_part(wl, s.N, span, lcount);
-    count_part(wh, s.N, span, hcount);
+    const int lspan = 1 + std::accumulate(wl.begin(), wl.end(), 0), hspan = 1 + std::accumulate(wh.begin(), wh.end(), 0);
+    const std::vector<int> ltab = part_counts(wl, s.N, lspan), htab = part_counts(wh, s.N, hspan);
+    const int *lcount = ltab.data() + (size_t)B0 * (s.N + 1) * lspan, *hcount = htab.data() + (size_t)B1 * (s.N + 1) * hspan;
+    std::vector<int> lclass((size_t)(s.N + 1) * lspan, -1), hclass((size_t)(s.N + 1) * hspan, -1);
     PartWords L, H;
     int64_t rows = 0;
-    for (int k = 0; k < nkeys; ++k) {
-        const int pop = k / span, sum = k % span;
+    for (int k = 0; k < (int)lclass.size(); ++k) {
+        const int pop = k / lspan, sum = k % lspan;
         const int64_t sh = s.sector_sum - sum;
-        if (!lcount[k] || sh < 0 || sh >= span) continue;
-        const int kh = (s.N - pop) * span + (int)sh;
+        if (!lcount[k] || sh < 0 || sh >= hspan) continue;
+        const int kh = (s.N - pop) * hspan + (int)sh;
         if (!hcount[kh]) continue;
         lclass[k] = hclass[kh] = (int)L.start.size();
-        L.start.push_back((int)L.word.size());
-        H.start.push_back((int)H.word.size());
+        L.start.push_back(L.count);
+        H.start.push_back(H.count);
         L.size.push_back(lcount[k]);
         H.size.push_back(hcount[kh]);
-        L.word.resize(L.word.size() + lcount[k]);
-        H.word.resize(H.word.size() + hcount[kh]);
+        L.count += lcount[k];
+        H.count += hcount[kh];
         rows += (int64_t)lcount[k] * hcount[kh];
     }
     if (rows != n) return nullptr;
-    for (auto* part : {&L, &H}) {
-        auto& cls = part == &L ? lclass : hclass;
-        std::vector<int> at = part->start;
-        part->cls.resize(part->word.size());
-        for_part(part == &L ? wl : wh, s.N, s.N - (part == &L ? B1 : B0), span, [&](int key, uint32_t word) {
-            const int c = cls[key];
-            if (c < 0) return;
-            part->cls[at[c]] = c;
-            part->word[at[c]++] = word;
-        });
-    }
     const int nc = (int)L.start.size();
-    std::vector<int> cbase(nc), tbase(L.word.size());
+    std::vector<int> cbase(nc);
     int64_t run = 0;
     for (int c = 0; c < nc; ++c) {
         cbase[c] = (int)run;
-        for (int i = 0; i < L.size[c]; ++i) tbase[L.start[c] + i] = (int)(run + (int64_t)i * H.size[c]);
         run += (int64_t)L.size[c] * H.size[c];
     }
 
@@ -1096,9 +1113,21 @@ std::unique_ptr<SplitPlan> split_build(const SplitSource& s, const double* diag,
         gn = GenArgs{0, B1, 0, B0, 0, nullptr, s.norb0, w0, off0};
         gt = GenArgs{0, B0, 0, B1, 0, nullptr, s.norb1, w1, off1};
     }
+    auto words = [&](PartWords& part, const std::vector<int>& w, int span, const std::vector<int>& tab, const std::vector<int>& cls,
+                     bool base) {
+        PartArgs a{(int)w.size(), s.N, span, {}, tmp.put(tab, st), tmp.put(cls, st), tmp.put(part.start, st)};
+        std::copy(w.begin(), w.end(), a.w);
+        part.word = tmp.take<uint32_t>(part.count);
+        part.cls = tmp.take<int>(part.count);
+        if (base) part.base = tmp.take<int>(part.count);
+        launch(k_split_words, grid_of(1ll << a.bits, 256), 256, 0, st, a, part.word, part.cls, part.base,
+               base ? tmp.put(cbase, st) : nullptr, base ? tmp.put(H.size, st) : nullptr);
+    };
+    words(L, wl, lspan, ltab, lclass, true);
+    words(H, wh, hspan, htab, hclass, false);
     SideBuild bn{p->native, H, L, gn, gamman, s.levels == 1, tmp, st};
     SideBuild bt{p->trans, L, H, gt, gammat, false, tmp, st};
-    if (!bn.count(nullptr) || !bt.count(&tbase)) return nullptr;
+    if (!bn.count(false) || !bt.count(true)) return nullptr;
     // the diagonal's exponent joins the weights'
     const int parts = exp_parts();
     int* part = tmp.take<int>((size_t)parts + 1);
@@ -1123,7 +1152,7 @@ std::unique_ptr<SplitPlan> split_build(const SplitSource& s, const double* diag,
     bt.fill(ea);
     p->perm.alloc((size_t)n);
     k_split_perm<<<sms() * 8, 256, 0, st>>>(p->native.pbase.p, p->native.pcls.p, tmp.put(H.start, st), tmp.put(H.size, st),
-                                            p->native.ssize.p, tmp.put(cbase, st), (int)H.word.size(), p->perm.p);
+                                            p->native.ssize.p, tmp.put(cbase, st), H.count, p->perm.p);
     count_launch();
     ED_CUDA(cudaGetLastError());
     ED_CUDA(cudaStreamSynchronize(st));   // the temporaries and the host vectors go
