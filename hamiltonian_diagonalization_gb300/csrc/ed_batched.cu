@@ -499,6 +499,11 @@ struct SumThen {
     double* ref = nullptr;       // |H v|^2
     int* need = nullptr;
     int* brk = nullptr;
+    // where the scaling also writes the product's fixed-point copy: per problem
+    // the largest |w_p| (k_bupdate's, cleared by kAcc) and the copy's exponent
+    // bounds, the largest of them after the last (kFinal)
+    unsigned long long* absmax = nullptr;
+    int* ex = nullptr;
 };
 
 // out[q][p] = sum over blocks of part[q][blk][p] for q < Q (t = q*B + p):
@@ -536,7 +541,10 @@ __global__ void __launch_bounds__(1024) k_bsum(const double* __restrict__ part, 
             then.cj[(size_t)(then.j - 1) * B + p] = then.beta[p];
         }
     } else if (then.kind == SumThen::kAcc) {
-        if (t < then.j * B && (!then.need || then.need[p])) then.cj[t] += sum;
+        const bool ran = !then.need || then.need[p];
+        if (t < then.j * B && ran) then.cj[t] += sum;
+        if (then.absmax && t < B && ran) then.absmax[p] = 0ull;
+        if (then.absmax && t == 0 && !then.need) then.ex[B] = 0;
     } else if (then.kind == SumThen::kNeed) {
         then.need[p] = (then.force || sum < 0.5 * then.before[p]) ? 1 : 0;
         if (then.force) then.ref[p] = then.before[p];
@@ -547,6 +555,11 @@ __global__ void __launch_bounds__(1024) k_bsum(const double* __restrict__ part, 
             then.beta[p] = 1.0;          // keeps the (abandoned) vector finite
         } else {
             then.beta[p] = b;
+        }
+        if (then.absmax) {   // rounding keeps the order: the largest entry of w_p / beta
+            const int E = fix_exp(__longlong_as_double((long long)then.absmax[p]) / then.beta[p]);
+            then.ex[p] = E;
+            atomicMax(then.ex + B, E);
         }
     }
 }
@@ -626,7 +639,8 @@ __global__ void __launch_bounds__(kBT, 4) k_bmdot(const double* __restrict__ V, 
 template <bool SC>
 __global__ void __launch_bounds__(kBT, 4) k_bupdate(const double* __restrict__ V, int64_t n, int B, int BP, int J,
                                                  const double* __restrict__ c, double* __restrict__ w,
-                                                 double* __restrict__ npart, const int* __restrict__ need)
+                                                 double* __restrict__ npart, const int* __restrict__ need,
+                                                 unsigned long long* __restrict__ absmax)
 {
     __shared__ double red[kBT];
     extern __shared__ double sc[];   // SC: -c[i][p], J * B values staged once per block
@@ -640,6 +654,7 @@ __global__ void __launch_bounds__(kBT, 4) k_bupdate(const double* __restrict__ V
     auto coef = [&](int i) { return SC ? sc[i * B + p] : -__ldg(c + i * B + p); };
     const int64_t vs = n * (int64_t)B;
     double nn = 0.0;
+    unsigned long long mx = 0ull;
     if (p < B && (!need || need[p])) {
 #pragma unroll 2
         for (int64_t r = r0 + rl; r < r1; r += nrl) {
@@ -659,18 +674,31 @@ __global__ void __launch_bounds__(kBT, 4) k_bupdate(const double* __restrict__ V
             acc += acc2;
             w[r * B + p] = acc;
             nn = fma(acc, acc, nn);
+            mx = max(mx, abs_bits(acc));
         }
     }
     reduce_per_problem(nn, red, BP, B, npart + (int64_t)blockIdx.x * B, 0, 0);
+    if (!absmax) return;
+    red[threadIdx.x] = __longlong_as_double((long long)mx);
+    __syncthreads();
+    if (threadIdx.x < B) {
+        for (int q = threadIdx.x + BP; q < kBT; q += BP) mx = max(mx, abs_bits(red[q]));
+        if (mx) atomicMax(absmax + threadIdx.x, mx);
+    }
 }
 
+// w_p /= beta_p, with q also the block product's fixed-point copy at the bounds
+// ex (its own two passes over the block and the clearing before them took 12
+// us of a step's 330 for 16 problems at N=9, 2S=24).
 __global__ void k_bscale(double* __restrict__ w, int64_t n, int B, const double* __restrict__ beta,
-                         unsigned long long* __restrict__ started)
+                         unsigned long long* __restrict__ started, const int* __restrict__ ex, int64_t* __restrict__ q)
 {
     const int64_t total = n * (int64_t)B;
     for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
         const int p = (int)(t % B);
-        w[t] = w[t] / beta[p];
+        const double x = w[t] / beta[p];
+        w[t] = x;
+        if (q) q[t] = fix_pair(x, ex[p]);
     }
     stamp(started);
 }
@@ -989,13 +1017,15 @@ bool fix_operands(const ed_batch& bt, const BlockOperands& o, BlockFixed& f, cud
 // Y = H X through the fixed-point operands f of o; where X is not finite the
 // FP64 kernel of tile t follows and its answer stands.
 void fixed_block_product(const ed_batch& bt, const BlockOperands& o, const BlockFixed& f, const std::array<int, 4>& t,
-                         const double* X, double* Y, cudaStream_t st)
+                         const double* X, double* Y, cudaStream_t st, bool converted)
 {
     const int B = o.B, T = column_threads(B);
     const int64_t total = bt.n * B;
-    ED_CUDA(cudaMemsetAsync(f.ex.p, 0, (size_t)(B + 1) * 4, st));
-    k_bfix_exp<<<column_grid(total, B), T, B * 4, st>>>(X, total, B, f.ex.p); count_launch();
-    k_bfix_conv<<<column_grid(total, B), T, 0, st>>>(X, total, B, f.ex.p, 0, f.x.p); count_launch();
+    if (!converted) {
+        ED_CUDA(cudaMemsetAsync(f.ex.p, 0, (size_t)(B + 1) * 4, st));
+        k_bfix_exp<<<column_grid(total, B), T, B * 4, st>>>(X, total, B, f.ex.p); count_launch();
+        k_bfix_conv<<<column_grid(total, B), T, 0, st>>>(X, total, B, f.ex.p, 0, f.x.p); count_launch();
+    }
     if (B > 16) launch_bspmm_fix<32>(bt, f, B, Y, st);
     else if (B > 8) launch_bspmm_fix<16>(bt, f, B, Y, st);
     else if (B > 4) launch_bspmm_fix<8>(bt, f, B, Y, st);
@@ -1031,7 +1061,7 @@ BlockFixed* batch_fixed(const ed_batch& bt, const BlockOperands& o, cudaStream_t
 void batch_block_product(const ed_batch& bt, const BlockOperands& o, const double* X, double* Y, cudaStream_t st)
 {
     const std::array<int, 4> t = batch_tile(bt, o, st);
-    if (BlockFixed* f = batch_fixed(bt, o, st)) fixed_block_product(bt, o, *f, t, X, Y, st);
+    if (BlockFixed* f = batch_fixed(bt, o, st)) fixed_block_product(bt, o, *f, t, X, Y, st, false);
     else bspmm_variant(bt, o, t[0], t[1], t[2], t[3], X, Y, bt.n, nullptr, st);
 }
 
@@ -1202,6 +1232,7 @@ void batch_solve(const ed_batch& bt, const int* sel, int nsel, const ed_lanczos_
     DevBuf<double> part((size_t)(m + 2) * nb * B0), npart((size_t)nb * B0);
     DevBuf<double> sc((size_t)(m + 2) * B0);
     DevBuf<double> s2((size_t)6 * B0);   // [0] alpha [1] |Hv|^2 [2] scratch [3] |w|^2 after a pass
+    DevBuf<unsigned long long> absmax(B0);
     DevBuf<int> need2(B0), brk(B0), iota(B0), keep(B0), dst(B0);
     DevBuf<double> coef((size_t)m * (m + 1) * B0);
     DevBuf<double> betas((size_t)(m + 1) * B0);
@@ -1243,7 +1274,7 @@ void batch_solve(const ed_batch& bt, const int* sel, int nsel, const ed_lanczos_
             nn[b] = std::sqrt(nn[b]);
         }
         ED_CUDA(cudaMemcpyAsync(s2.p + 2 * B, nn.data(), (size_t)B * 8, cudaMemcpyHostToDevice, st));
-        k_bscale<<<grid_for(vs), 256, 0, st>>>(V.p, n, B, s2.p + 2 * B, nullptr); count_launch();
+        k_bscale<<<grid_for(vs), 256, 0, st>>>(V.p, n, B, s2.p + 2 * B, nullptr, nullptr, nullptr); count_launch();
     }
     ed_batch_info inf;
     std::memset(&inf, 0, sizeof(inf));
@@ -1296,7 +1327,7 @@ void batch_solve(const ed_batch& bt, const int* sel, int nsel, const ed_lanczos_
             double* cj = coef.p + (size_t)j * (m + 1) * B;
             double* ref = s2.p + B;
             const bool first = (j == k);
-            if (fixed.ready) fixed_block_product(bt, ops, fixed, tile, vj, w, st);
+            if (fixed.ready) fixed_block_product(bt, ops, fixed, tile, vj, w, st, !first);
             else bspmm_variant(bt, ops, tile[0], tile[1], tile[2], tile[3], vj, w, n, nullptr, st);
             SumThen local, acc, need, fin;
             if (!first) {
@@ -1323,6 +1354,9 @@ void batch_solve(const ed_batch& bt, const int* sel, int nsel, const ed_lanczos_
             fin.beta = betas.p + (size_t)j * B;
             fin.ref = ref;
             fin.brk = brk.p;
+            unsigned long long* amax = fixed.ready ? absmax.p : nullptr;
+            acc.absmax = fin.absmax = amax;
+            acc.ex = fin.ex = fixed.ex.p;
             for (int pass = 0; pass < 2; ++pass) {
                 int* mask = pass == 0 ? nullptr : need2.p;
                 launch(k_bmdot, nb, kBT, 0, st, V.p, n, B, BP, J, w, part.p, mask,
@@ -1330,13 +1364,14 @@ void batch_solve(const ed_batch& bt, const int* sel, int nsel, const ed_lanczos_
                 acc.need = mask;
                 bsum(part.p, J + 1, sc.p, nullptr, acc);
                 if (upd_stage)
-                    launch(k_bupdate<true>, nb, kBT, (size_t)J * B * 8, st, V.p, n, B, BP, J, sc.p, w, npart.p, mask);
+                    launch(k_bupdate<true>, nb, kBT, (size_t)J * B * 8, st, V.p, n, B, BP, J, sc.p, w, npart.p, mask, amax);
                 else
-                    launch(k_bupdate<false>, nb, kBT, 0, st, V.p, n, B, BP, J, sc.p, w, npart.p, mask);
+                    launch(k_bupdate<false>, nb, kBT, 0, st, V.p, n, B, BP, J, sc.p, w, npart.p, mask, amax);
                 // the norm after the pass, kept from pass 1 for problems that skip pass 2
                 bsum(npart.p, 1, s2.p + 3 * B, mask, pass == 0 ? need : fin);
             }
-            launch(k_bscale, grid_for(vs), 256, 0, st, w, n, B, betas.p + (size_t)j * B, clock.p + 2 * (j + 1));
+            launch(k_bscale, grid_for(vs), 256, 0, st, w, n, B, betas.p + (size_t)j * B, clock.p + 2 * (j + 1), fixed.ex.p,
+                   amax && j + 1 < m ? fixed.x.p : nullptr);
         }
     };
     CycleGraphs cache;
