@@ -1169,11 +1169,16 @@ std::unique_ptr<SplitPlan> split_build_crs(const ed_crs& a, cudaStream_t st)
     return split_build(*a.source, d.p, a.n, a.upper ? 0 : a.max_row, st);
 }
 
-bool split_ready(SplitPlan& p, cudaStream_t st)
+static SplitPlan::StreamKey stream_key(cudaStream_t st)
 {
     int dev = 0;
     ED_CUDA(cudaGetDevice(&dev));
-    const std::pair<int, cudaStream_t> key(dev, st);
+    return {dev, st, st == cudaStreamPerThread ? std::this_thread::get_id() : std::thread::id()};
+}
+
+bool split_ready(SplitPlan& p, cudaStream_t st)
+{
+    const SplitPlan::StreamKey key = stream_key(st);
     std::lock_guard<std::mutex> lk(p.mu);
     if (p.scratch.count(key)) return true;
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
@@ -1190,12 +1195,10 @@ bool split_ready(SplitPlan& p, cudaStream_t st)
 
 const int* split_product(SplitPlan& p, const double* x, double* y, cudaStream_t st)
 {
-    int dev = 0;
-    ED_CUDA(cudaGetDevice(&dev));
     SplitPlan::Scratch* sc;
     {
         std::lock_guard<std::mutex> lk(p.mu);
-        sc = p.scratch.at({dev, st}).get();
+        sc = p.scratch.at(stream_key(st)).get();
     }
     const int P = exp_parts();
     launch(k_fix_exp, P, 256, 0, st, x, p.n, sc->part.p);
@@ -1211,7 +1214,7 @@ void split_release(SplitPlan& p, cudaStream_t st)
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess) return;
     std::lock_guard<std::mutex> lk(p.mu);
-    p.scratch.erase({dev, st});
+    p.scratch.erase({dev, st, std::thread::id()});   // a solver's own stream
 }
 
 }  // namespace edgb

@@ -1,6 +1,9 @@
 // Products of the sphere Hamiltonians by splitting the Fock word (ed_split.cu).
 #pragma once
 
+#include <thread>
+#include <tuple>
+
 #include "ed_internal.h"
 
 namespace edgb {
@@ -48,8 +51,16 @@ struct SplitPlan {
         DevBuf<int> part;           // per-block exponent maxima and the bound
         DevBuf<ulonglong2> acct;    // the transposed pass's exact sums
     };
+    // a stream: the device, the handle and, for the per-thread default stream
+    // (one handle, as many streams as threads), the thread
+    using StreamKey = std::tuple<int, cudaStream_t, std::thread::id>;
     std::mutex mu;
-    std::map<std::pair<int, cudaStream_t>, std::unique_ptr<Scratch>> scratch;   // by (device, stream)
+    std::map<StreamKey, std::unique_ptr<Scratch>> scratch;
+    // Held over all launches of a product, the kernel gated on x's bound
+    // included: several operators share a plan through their terms, and two
+    // threads may enqueue their products on one stream, whose scratch holds
+    // one x at a time.
+    std::mutex order;
 };
 
 struct SplitArgs {
@@ -84,7 +95,7 @@ std::unique_ptr<SplitPlan> split_build(const SplitSource& s, const double* diag,
 std::unique_ptr<SplitPlan> split_build_crs(const ed_crs& a, cudaStream_t st);
 // The stream's scratch, made outside a capture; false when it is missing.
 bool split_ready(SplitPlan& p, cudaStream_t st);
-// y = H x on a stream that split_ready accepted; returns the device word with
+// y = H x on a stream that split_ready accepted, p.order held; returns the device word with
 // x's exponent bound (2047: a non-finite entry, y is all NaN).
 const int* split_product(SplitPlan& p, const double* x, double* y, cudaStream_t st);
 // Gives back the stream's scratch (before a solver's stream is destroyed).

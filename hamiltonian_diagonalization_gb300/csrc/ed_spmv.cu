@@ -1354,6 +1354,7 @@ void spmv(const ed_crs& a, const double* x, double* y, cudaStream_t st)
         return;
     }
     if (split_prepare(a, st)) {
+        std::lock_guard<std::mutex> order(a.split->order);
         const int* xexp = split_product(*a.split, x, y, st);
         if (a.upper) {
             launch(k_zero_unless_finite, sms() * 4, 256, 0, st, y, a.n, xexp);
@@ -1430,7 +1431,11 @@ void hv_matfree(const ed_basis& b, const ed_terms& t, SplitPlan* plan, const dou
     ED_REQUIRE(b.levels == 1 && b.dimX == 0, ED_ERR_ARG, "the matrix-free product takes a one-level Lz basis");
     if (b.dim == 0) return;
     const int* xexp = nullptr;
-    if (plan && split_ready(*plan, st)) xexp = split_product(*plan, x, y, st);
+    std::unique_lock<std::mutex> order;
+    if (plan && split_ready(*plan, st)) {
+        order = std::unique_lock<std::mutex>(plan->order);
+        xexp = split_product(*plan, x, y, st);
+    }
     if (plan) diag = plan->values.p;
     const int K = t.norb;
     const int nw = (int)t.hop.w.size();

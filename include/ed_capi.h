@@ -226,7 +226,10 @@ ed_status ed_fp64_fma_rate(int iters, int blocks_per_sm, double* fma_per_second)
 
 /* y = H x with the matrix elements regenerated on the fly from the basis and
  * the term tables (no stored matrix).  Stands in for the reference's
- * unfinished MatrixVectorFunction::Recalculate (matrix_vector_routines.hpp:112-143). */
+ * unfinished MatrixVectorFunction::Recalculate (matrix_vector_routines.hpp:112-143).
+ * The first product of a sector makes its plan (ed_split.cu), kept with the
+ * term tables, and, per stream, a scratch for x; operators and calls on the
+ * same term tables share both, from several threads and streams. */
 ed_status ed_hv_matfree(const ed_basis* b, const ed_terms* t, const double* x_dev, double* y_dev,
                         ed_stream stream);
 
