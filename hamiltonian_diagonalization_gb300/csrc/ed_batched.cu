@@ -1037,20 +1037,21 @@ void fixed_block_product(const ed_batch& bt, const BlockOperands& o, const Block
 namespace {
 
 // The whole batch's fixed-point operands with this stream's scratch for X,
-// made when missing and not capturing; null for a part of the batch or where
-// they do not apply.
+// made when missing; null for a part of the batch, where they do not apply and
+// in a capture: a graph may be replayed on any stream beside other products,
+// so it must not hold a stream's scratch.
 BlockFixed* batch_fixed(const ed_batch& bt, const BlockOperands& o, cudaStream_t st)
 {
     if (o.w != bt.w.p) return nullptr;
     int dev = 0;
     ED_CUDA(cudaGetDevice(&dev));
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    ED_CUDA(cudaStreamIsCapturing(st, &cs));
+    if (cs != cudaStreamCaptureStatusNone) return nullptr;
     const std::pair<int, cudaStream_t> key(dev, st);
     std::lock_guard<std::mutex> lk(bt.fix_mu);
     auto it = bt.fixed.find(key);
     if (it != bt.fixed.end()) return it->second->ready ? it->second.get() : nullptr;
-    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-    ED_CUDA(cudaStreamIsCapturing(st, &cs));
-    if (cs != cudaStreamCaptureStatusNone) return nullptr;
     auto f = std::make_unique<BlockFixed>();
     fix_operands(bt, o, *f, st);
     return (bt.fixed[key] = std::move(f))->ready ? bt.fixed[key].get() : nullptr;

@@ -359,7 +359,8 @@ void ham2_build_crs(const ed_basis& b, const ed_terms& t0, const ed_terms& t1, c
 void terms_upload(ed_terms& t);
 void ham_diagonal(const ed_basis& b, const ed_terms& t, double* diag, cudaStream_t st);
 void ham_build_crs(const ed_basis& b, const ed_terms& t, int upper, ed_crs& a, cudaStream_t st);
-void spmv(const ed_crs& a, const double* x, double* y, cudaStream_t st);
+// solver: called by a solver on its own stream.
+void spmv(const ed_crs& a, const double* x, double* y, cudaStream_t st, bool solver = false);
 // Make what the default product needs (split plan, row-blocked or sliced-ELL
 // copy) now (a no-op when made, declined, or the stream is capturing); solvers
 // call it before they capture their cycles.

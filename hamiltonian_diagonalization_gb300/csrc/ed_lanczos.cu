@@ -465,7 +465,7 @@ void op_apply(const ed_op& op, const double* x, double* y, cudaStream_t st)
 {
     switch (op.kind) {
     case ed_op::CRS:
-        spmv(*op.crs, x, y, st);
+        spmv(*op.crs, x, y, st, true);
         break;
     case ed_op::MATFREE:
         if (!op.plan) op.plan = matfree_plan(*op.basis, *op.terms, op.diag.p, st);

@@ -1061,6 +1061,11 @@ bool fix_copy(const ed_crs& a, bool sell, cudaStream_t st)
     return true;
 }
 
+// Whether a product must keep nothing: one that a caller captures (a graph may
+// be replayed on any stream beside other products, so it must not hold a
+// stream's scratch).  A solver's cycles replay on its own stream.
+bool stateless(cudaStream_t st, bool solver) { return !solver && stream_capturing(st); }
+
 bool short_rows(const ed_crs& a) { return (double)a.nnz < kSellMaxAvg * (double)a.n; }
 
 bool sell_shape(const ed_crs& a) { return !a.upper && a.n >= kSellMinRows && short_rows(a); }
@@ -1317,8 +1322,10 @@ int spmv_staged_wait_test(const ed_crs& a, const double* x, double* y, long long
 // with what it needs made when missing and not capturing.
 enum class FixRoute { kNone, kSell, kBlocked, kRows };
 
-static FixRoute fix_route(const ed_crs& a, cudaStream_t st)
+static FixRoute fix_route(const ed_crs& a, cudaStream_t st, bool solver)
 {
+    // short rows of a small sector: their FP64 kernel needs no scratch
+    if (fix_shape(a) && short_rows(a) && stateless(st, solver)) return FixRoute::kNone;
     if (sell_shape(a) && a.sell_state == 0) spmv_prepare(a, st);   // waits for a solver's explicit call while capturing
     if (sell_shape(a) && a.sell_state == 1) return fix_ready(a, st, true) ? FixRoute::kSell : FixRoute::kNone;
     if (blk_shape(a) && blk_ready(a, st)) return FixRoute::kBlocked;
@@ -1329,7 +1336,7 @@ static FixRoute fix_route(const ed_crs& a, cudaStream_t st)
 FixTarget spmv_target(const ed_crs& a, cudaStream_t st)
 {
     FixTarget t;
-    if (a.n == 0 || a.product_kernel > 0 || split_prepare(a, st) || fix_route(a, st) == FixRoute::kNone) return t;
+    if (a.n == 0 || a.product_kernel > 0 || split_prepare(a, st) || fix_route(a, st, true) == FixRoute::kNone) return t;
     ed_fixq::Scratch& sc = *fix_scratch(a, st);
     t.q = sc.xq.p;
     t.bound = sc.part.p + fix_parts();
@@ -1338,7 +1345,7 @@ FixTarget spmv_target(const ed_crs& a, cudaStream_t st)
 
 void spmv_converted(const ed_crs& a, const double* x, double* y, cudaStream_t st)
 {
-    switch (fix_route(a, st)) {
+    switch (fix_route(a, st, true)) {
     case FixRoute::kSell: fix_launch_sell(a, x, y, st, true); return;
     case FixRoute::kBlocked: blk_launch(a, x, y, st, true); return;
     case FixRoute::kRows: fix_launch(a, x, y, st, short_rows(a), true); return;
@@ -1346,14 +1353,14 @@ void spmv_converted(const ed_crs& a, const double* x, double* y, cudaStream_t st
     }
 }
 
-void spmv(const ed_crs& a, const double* x, double* y, cudaStream_t st)
+void spmv(const ed_crs& a, const double* x, double* y, cudaStream_t st, bool solver)
 {
     if (a.n == 0) return;
     if (a.product_kernel > 0) {
         spmv_kernel(a, a.product_kernel, x, y, st);
         return;
     }
-    if (split_prepare(a, st)) {
+    if (!(a.upper && stateless(st, solver)) && split_prepare(a, st)) {
         std::lock_guard<std::mutex> order(a.split->order);
         const int* xexp = split_product(*a.split, x, y, st);
         if (a.upper) {
@@ -1362,7 +1369,7 @@ void spmv(const ed_crs& a, const double* x, double* y, cudaStream_t st)
         }
         return;
     }
-    switch (fix_route(a, st)) {
+    switch (fix_route(a, st, solver)) {
     case FixRoute::kSell: fix_launch_sell(a, x, y, st); return;
     case FixRoute::kBlocked: blk_launch(a, x, y, st, false); return;
     case FixRoute::kRows: fix_launch(a, x, y, st, short_rows(a)); return;
