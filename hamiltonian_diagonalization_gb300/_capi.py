@@ -67,6 +67,7 @@ _SIGS = {
     "ed_status_string": (ctypes.c_char_p, [c_int]),
     "ed_last_error": (ctypes.c_char_p, []),
     "ed_device_count": (c_int, []),
+    "ed_memory_limit": (None, [c_i64]),
     "ed_coulomb_pseudopotentials": (c_int, [c_int, P(c_double)]),
     "ed_quartic_tables": (c_int, [c_int, P(c_double), c_int, P(ctypes.c_uint16), P(c_double)]),
     "ed_clebsch_gordan": (c_double, [c_int] * 6),

@@ -1,6 +1,7 @@
 // C ABI of libedgb300: argument checks, handle management, error capture.
 // No C++ exception crosses this boundary; every entry returns ed_status and
 // leaves a message for ed_last_error() on failure.
+#include <algorithm>
 #include <atomic>
 #include <cstring>
 #include <new>
@@ -46,6 +47,37 @@ void count_launch() { g_launches.fetch_add(1, std::memory_order_relaxed); }
 void count_launches(int64_t d) { g_launches.fetch_add((uint64_t)d, std::memory_order_relaxed); }
 uint64_t launch_count() { return g_launches.load(std::memory_order_relaxed); }
 
+namespace {
+thread_local int64_t g_memory_left = -1;   // negative: no limit
+}
+
+void* device_alloc(size_t bytes)
+{
+    void* p = nullptr;
+    const bool over = g_memory_left >= 0 && bytes > (size_t)g_memory_left;
+    const cudaError_t e = over ? cudaErrorMemoryAllocation : cudaMalloc(&p, bytes);
+    if (e == cudaErrorMemoryAllocation) {
+        cudaGetLastError();   // the caller may go on with less
+        throw Error(ED_ERR_OOM, "no device memory for " + std::to_string(bytes) + " bytes");
+    }
+    ED_CUDA(e);
+    if (g_memory_left >= 0) g_memory_left -= (int64_t)bytes;
+    return p;
+}
+
+void device_release(void* p, size_t bytes)
+{
+    cudaFree(p);
+    if (g_memory_left >= 0) g_memory_left += (int64_t)bytes;
+}
+
+size_t device_memory_free()
+{
+    size_t free_b = 0, total_b = 0;
+    ED_CUDA(cudaMemGetInfo(&free_b, &total_b));
+    return g_memory_left >= 0 ? std::min(free_b, (size_t)g_memory_left) : free_b;
+}
+
 void terms_upload(ed_terms& t)
 {
     t.w_dev.alloc(t.hop.w.size());
@@ -87,6 +119,8 @@ const char* ed_status_string(ed_status s)
 }
 
 const char* ed_last_error(void) { return g_last_error.c_str(); }
+
+void ed_memory_limit(int64_t bytes) { g_memory_left = bytes; }
 
 int ed_device_count(void)
 {

@@ -855,8 +855,7 @@ bool capturing(cudaStream_t st)
 // half of the free device memory, for long rows or a non-finite value).
 void cfix_build(const ed_ccrs& a, cudaStream_t st)
 {
-    size_t free_b = 0, total_b = 0;
-    ED_CUDA(cudaMemGetInfo(&free_b, &total_b));
+    const size_t free_b = device_memory_free();
     const size_t need = (size_t)(a.nnz + kCrsPad) * 16 + (size_t)a.n * 16;
     if (a.upper || need > free_b / 2 || a.max_row > kCFixMaxRow) {
         a.fix_state = -1;

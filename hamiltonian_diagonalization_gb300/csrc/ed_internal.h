@@ -81,6 +81,12 @@ ed_status guard(F&& f)
     }
 }
 
+// Device memory within the calling thread's limit (ed_memory_limit): the
+// allocation, its release and what is free.
+void* device_alloc(size_t bytes);
+void device_release(void* p, size_t bytes);
+size_t device_memory_free();
+
 // Owning device buffer.
 template <class T>
 struct DevBuf {
@@ -98,11 +104,11 @@ struct DevBuf {
     ~DevBuf() { release(); }
     void alloc(size_t count) {
         release();
-        if (count) ED_CUDA(cudaMalloc(reinterpret_cast<void**>(&p), count * sizeof(T)));
+        if (count) p = static_cast<T*>(device_alloc(count * sizeof(T)));
         n = count;
     }
     void release() {
-        if (p) cudaFree(p);
+        if (p) device_release(p, n * sizeof(T));
         p = nullptr;
         n = 0;
     }
@@ -112,6 +118,19 @@ struct DevBuf {
         if (count > n) alloc(count);
     }
 };
+
+// f(), or false where device memory ran out for it: what it had allocated is
+// given back, once the device is done with it (cudaFree waits).
+template <class F>
+bool if_memory(F&& f)
+{
+    try {
+        return f();
+    } catch (const Error& e) {
+        if (e.code != ED_ERR_OOM) throw;
+        return false;
+    }
+}
 
 // ------------------------------------------------------------ host tables
 

@@ -447,6 +447,14 @@ void op_prepare(const ed_op& op, cudaStream_t st)
     }
 }
 
+// Whether the operator's product runs without any memory of its own too, only
+// slower: no stored matrix, or its upper triangle.
+static bool op_optional(const ed_op& op)
+{
+    if (op.kind == ed_op::DEFLATED && op.inner) return op_optional(*op.inner);
+    return op.kind == ed_op::MATFREE || (op.kind == ed_op::CRS && op.crs->upper);
+}
+
 void op_release(const ed_op& op, cudaStream_t st)
 {
     if (op.kind == ed_op::CRS) spmv_release(*op.crs, st);
@@ -633,7 +641,9 @@ void lanczos_once(const ed_op& op, const ed_lanczos_params& p, const double* v0_
     SolveStream ss(caller_stream);
     cudaStream_t st = ss.s;
     const int nsm = sm_count();
-    op_prepare(op, st);
+    // what these products keep is theirs to leave out: it comes after the basis vectors
+    const bool late = op_optional(op);
+    if (!late) op_prepare(op, st);
     struct Release {     // before the stream goes
         const ed_op& op;
         cudaStream_t st;
@@ -715,6 +725,7 @@ void lanczos_once(const ed_op& op, const ed_lanczos_params& p, const double* v0_
         ED_CUDA(cudaGetLastError());
     }
     orthonormalise_column(w, w.V.p, 0, st);
+    if (late) op_prepare(op, st);
 
     // start and end of each step's product
     DevBuf<unsigned long long> clock(2 * (size_t)(m + 1));

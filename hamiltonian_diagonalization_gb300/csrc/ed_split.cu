@@ -1038,7 +1038,7 @@ void launch_pass(const SplitSide& s, const SplitArgs& g, cudaStream_t st)
 
 }  // namespace
 
-std::unique_ptr<SplitPlan> split_build(const SplitSource& s, const double* diag, int64_t n, int max_row, cudaStream_t st)
+static std::unique_ptr<SplitPlan> plan_of(const SplitSource& s, const double* diag, int64_t n, int max_row, cudaStream_t st)
 {
     // the low part S-side bits first: one level splits its orbitals in two
     // (the low part one longer for odd counts), two levels by level
@@ -1142,8 +1142,7 @@ std::unique_ptr<SplitPlan> split_build(const SplitSource& s, const double* diag,
     // pairs, is well above the single weights)
     if ((double)max_row * (std::ldexp(wmax, 1050 - ea) + 1.0) >= std::ldexp(1.0, 34)) return nullptr;
     p->ea = ea;
-    size_t free_b = 0, total_b = 0;
-    ED_CUDA(cudaMemGetInfo(&free_b, &total_b));
+    const size_t free_b = device_memory_free();
     if (!bn.fits() || !bt.fits() || (size_t)n * 56 + bn.bytes() + bt.bytes() > free_b / 2) return nullptr;
     p->diag.alloc((size_t)n);
     ED_CUDA(cudaMemcpyAsync(part, &ea, sizeof(int), cudaMemcpyHostToDevice, st));
@@ -1159,14 +1158,29 @@ std::unique_ptr<SplitPlan> split_build(const SplitSource& s, const double* diag,
     return p;
 }
 
+std::unique_ptr<SplitPlan> split_build(const SplitSource& s, const double* diag, int64_t n, int max_row, cudaStream_t st)
+{
+    std::unique_ptr<SplitPlan> p;
+    const bool made = if_memory([&] {
+        p = plan_of(s, diag, n, max_row, st);
+        return p != nullptr;
+    });
+    return made ? std::move(p) : nullptr;
+}
+
 std::unique_ptr<SplitPlan> split_build_crs(const ed_crs& a, cudaStream_t st)
 {
     if (!a.source || a.n < 1) return nullptr;
-    DevBuf<double> d((size_t)a.n);
-    k_split_crs_diag<<<grid_of(a.n, 256), 256, 0, st>>>(a.rowptr.p, a.col.p, a.val.p, a.n, d.p);
-    count_launch();
-    ED_CUDA(cudaGetLastError());
-    return split_build(*a.source, d.p, a.n, a.upper ? 0 : a.max_row, st);
+    std::unique_ptr<SplitPlan> p;
+    const bool made = if_memory([&] {
+        DevBuf<double> d((size_t)a.n);
+        k_split_crs_diag<<<grid_of(a.n, 256), 256, 0, st>>>(a.rowptr.p, a.col.p, a.val.p, a.n, d.p);
+        count_launch();
+        ED_CUDA(cudaGetLastError());
+        p = plan_of(*a.source, d.p, a.n, a.upper ? 0 : a.max_row, st);
+        return p != nullptr;
+    });
+    return made ? std::move(p) : nullptr;
 }
 
 static SplitPlan::StreamKey stream_key(cudaStream_t st)
@@ -1184,13 +1198,16 @@ bool split_ready(SplitPlan& p, cudaStream_t st)
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     ED_CUDA(cudaStreamIsCapturing(st, &cs));
     if (cs != cudaStreamCaptureStatusNone) return false;
-    auto sc = std::make_unique<SplitPlan::Scratch>();
-    sc->x.alloc((size_t)p.n);
-    sc->xt.alloc((size_t)p.n);
-    sc->acct.alloc((size_t)p.n);
-    sc->part.alloc((size_t)exp_parts() + 1);
-    p.scratch.emplace(key, std::move(sc));
-    return true;
+    if ((size_t)p.n * 32 > device_memory_free() / 2) return false;
+    return if_memory([&] {
+        auto sc = std::make_unique<SplitPlan::Scratch>();
+        sc->x.alloc((size_t)p.n);
+        sc->xt.alloc((size_t)p.n);
+        sc->acct.alloc((size_t)p.n);
+        sc->part.alloc((size_t)exp_parts() + 1);
+        p.scratch.emplace(key, std::move(sc));
+        return true;
+    });
 }
 
 const int* split_product(SplitPlan& p, const double* x, double* y, cudaStream_t st)

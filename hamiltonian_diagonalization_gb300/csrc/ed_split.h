@@ -93,7 +93,8 @@ struct SplitArgs {
 std::unique_ptr<SplitPlan> split_build(const SplitSource& s, const double* diag, int64_t n, int max_row, cudaStream_t st);
 // The plan of a stored matrix: its own diagonal, its source's weights.
 std::unique_ptr<SplitPlan> split_build_crs(const ed_crs& a, cudaStream_t st);
-// The stream's scratch, made outside a capture; false when it is missing.
+// The stream's scratch, made outside a capture where it takes at most half of
+// the free device memory; false when it is missing.
 bool split_ready(SplitPlan& p, cudaStream_t st);
 // y = H x on a stream that split_ready accepted, p.order held; returns the device word with
 // x's exponent bound (2047: a non-finite entry, y is all NaN).

@@ -895,7 +895,7 @@ int sms()
 
 namespace {
 
-void sell_build(const ed_crs& a, cudaStream_t st)
+void sell_make(const ed_crs& a, cudaStream_t st)
 {
     const int64_t n = a.n;
     const int64_t nwin = (n + kSellWindow - 1) / kSellWindow;
@@ -916,8 +916,7 @@ void sell_build(const ed_crs& a, cudaStream_t st)
     }
     // the copy must leave room: decline when it would take more than half
     // of the free device memory
-    size_t free_b = 0, total_b = 0;
-    ED_CUDA(cudaMemGetInfo(&free_b, &total_b));
+    const size_t free_b = device_memory_free();
     const size_t need = (size_t)sl->nnz_pad * 12 + (size_t)kCrsPad * 12;
     if (need > free_b / 2) {
         a.sell_state = -1;
@@ -933,6 +932,16 @@ void sell_build(const ed_crs& a, cudaStream_t st)
     ED_CUDA(cudaGetLastError());
     a.sell = std::move(sl);
     a.sell_state = 1;
+}
+
+// The copy, or its state -1 where the memory ran out for it.
+void sell_build(const ed_crs& a, cudaStream_t st)
+{
+    if (!if_memory([&] {
+            sell_make(a, st);
+            return true;
+        }))
+        a.sell_state = -1;
 }
 
 bool stream_capturing(cudaStream_t st)
@@ -1043,8 +1052,7 @@ bool fix_copy(const ed_crs& a, bool sell, cudaStream_t st)
     if (sell && a.sell_state != 1) return false;
     if (stream_capturing(st)) return false;
     const int64_t cnt = sell ? a.sell->nnz_pad : a.nnz;
-    size_t free_b = 0, total_b = 0;
-    ED_CUDA(cudaMemGetInfo(&free_b, &total_b));
+    const size_t free_b = device_memory_free();
     if ((size_t)(cnt + kCrsPad) * 8 > free_b / 2) {
         state = -1;
         return false;
@@ -1080,8 +1088,10 @@ bool fix_shape(const ed_crs& a)
 // of them is not there.
 bool fix_ready(const ed_crs& a, cudaStream_t st, bool sell = false)
 {
-    if (a.fix_state == 0 && !stream_capturing(st)) fix_build(a, st);
-    return a.fix_state == 1 && fix_copy(a, sell, st) && fix_scratch(a, st) != nullptr;
+    return if_memory([&] {
+        if (a.fix_state == 0 && !stream_capturing(st)) fix_build(a, st);
+        return a.fix_state == 1 && fix_copy(a, sell, st) && fix_scratch(a, st) != nullptr;
+    });
 }
 
 // x's fixed-point copy into the stream's scratch (or it is there already);
@@ -1119,8 +1129,7 @@ bool blk_copy(const ed_crs& a, cudaStream_t st)
         ED_CUDA(cudaMemcpyAsync(&steps, off.p + f.blocks, 8, cudaMemcpyDeviceToHost, st));
         ED_CUDA(cudaStreamSynchronize(st));
     }
-    size_t free_b = 0, total_b = 0;
-    ED_CUDA(cudaMemGetInfo(&free_b, &total_b));
+    const size_t free_b = device_memory_free();
     if ((size_t)steps * 32 * 12 > free_b / 2) return false;
     f.bcol.alloc((size_t)steps * 32);
     f.bval.alloc((size_t)steps * 32);
@@ -1135,8 +1144,10 @@ bool blk_shape(const ed_crs& a) { return fix_shape(a) && a.n >= kBlkMinRows; }
 
 bool blk_ready(const ed_crs& a, cudaStream_t st)
 {
-    if (a.fix_state == 0 && !stream_capturing(st)) fix_build(a, st);
-    return a.fix_state == 1 && blk_copy(a, st) && fix_scratch(a, st) != nullptr;
+    return if_memory([&] {
+        if (a.fix_state == 0 && !stream_capturing(st)) fix_build(a, st);
+        return a.fix_state == 1 && blk_copy(a, st) && fix_scratch(a, st) != nullptr;
+    });
 }
 
 void fix_launch_staged(const ed_crs& a, const double* x, double* y, long long stall, cudaStream_t st)
@@ -1421,12 +1432,14 @@ std::shared_ptr<SplitPlan> matfree_plan(const ed_basis& b, const ed_terms& t, co
         ham_diagonal(b, t, own.p, st);
     }
     std::shared_ptr<SplitPlan> p = split_build(split_source(b, t), diag ? diag : own.p, (int64_t)b.dim, 0, st);
-    if (p) {
-        // the row kernel's diagonal, for an x that is not finite
-        p->values.alloc((size_t)b.dim);
-        ED_CUDA(cudaMemcpyAsync(p->values.p, diag ? diag : own.p, (size_t)b.dim * 8, cudaMemcpyDeviceToDevice, st));
-        ED_CUDA(cudaStreamSynchronize(st));
-    }
+    if (p && !if_memory([&] {
+            // the row kernel's diagonal, for an x that is not finite
+            p->values.alloc((size_t)b.dim);
+            ED_CUDA(cudaMemcpyAsync(p->values.p, diag ? diag : own.p, (size_t)b.dim * 8, cudaMemcpyDeviceToDevice, st));
+            ED_CUDA(cudaStreamSynchronize(st));
+            return true;
+        }))
+        p.reset();
     if (t.plans.size() == kMaxPlans) t.plans.erase(t.plans.begin());
     t.plans.push_back({key, p});
     return p;

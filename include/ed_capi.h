@@ -65,6 +65,10 @@ const char* ed_last_error(void);
 /* Kernels launched by this library since it was loaded (a counter kept on
  * the host at every launch site). */
 uint64_t ed_kernel_launches(void);
+/* For tests of what happens where device memory is short: from now on the
+ * calling thread's allocations in this library fail beyond bytes more (what it
+ * frees counts back); negative: no limit, the default. */
+void ed_memory_limit(int64_t bytes);
 /* Number of visible CUDA devices (0 without a GPU); never fails. */
 int ed_device_count(void);
 
