@@ -10,12 +10,16 @@
 namespace edgb {
 // A block product's operands in the integer product's fixed point: weights
 // [2 nhop][B] (each hop and its negative), diagonals [n][B], the exponent bound
-// of each Hamiltonian; and the scratch for X [n][B] with its bounds (the last
-// entry the largest of all).
+// of each Hamiltonian.
 struct BlockFixed {
     bool ready = false;
-    DevBuf<int64_t> w, diag, x;
-    DevBuf<int> ea, ex;
+    DevBuf<int64_t> w, diag;
+    DevBuf<int> ea;
+};
+// The scratch for X [n][B] with its bounds (the last entry the largest of all).
+struct BlockScratch {
+    DevBuf<int64_t> x;
+    DevBuf<int> ex;
 };
 }  // namespace edgb
 
@@ -40,9 +44,12 @@ struct ed_batch {
     int tb = 32, unroll = 4, nt = 256, l1 = 1;
     int tuned = 0;                // 1 after batch_autotune: subsets get their own tuned tiles
     int max_row = 0;              // most off-diagonal entries of a row
-    // the fixed-point operands of ed_batch_spmm, per (device, stream)
+    // the fixed-point operands of ed_batch_spmm (state 0 not yet tried, 1 made,
+    // -1 declined), and the scratch of each (device, stream)
     mutable std::mutex fix_mu;
-    mutable std::map<std::pair<int, cudaStream_t>, std::unique_ptr<edgb::BlockFixed>> fixed;
+    mutable edgb::BlockFixed fixed;
+    mutable int fixed_state = 0;
+    mutable std::map<std::pair<int, cudaStream_t>, std::unique_ptr<edgb::BlockScratch>> fixed_x;
 };
 
 namespace edgb {
@@ -74,9 +81,11 @@ std::array<int, 4> batch_tile(const ed_batch& bt, const BlockOperands& o, cudaSt
 void batch_block_product(const ed_batch& bt, const BlockOperands& o, const double* X, double* Y, cudaStream_t st);
 
 // res[b * k + i] = || H_b x_{i,b} - lam[b * k + i] x_{i,b} || for the o.B
-// problems of o, X [k][n][o.B] on the device, lam and res on the host.
+// problems of o, X [k][n][o.B] on the device, lam and res on the host.  fixed
+// and scratch: o's fixed-point operands with room for X, or null for the whole
+// batch's.
 void batch_residuals(const ed_batch& bt, const BlockOperands& o, const double* X, const double* lam, int k,
-                     double* res, cudaStream_t st);
+                     double* res, cudaStream_t st, const BlockFixed* fixed = nullptr, BlockScratch* scratch = nullptr);
 
 // Lockstep thick-restart Lanczos for the problems sel[0..nsel) of the batch
 // (all of them when sel is null); V0 [n][nsel], evals [nsel][nev], evecs

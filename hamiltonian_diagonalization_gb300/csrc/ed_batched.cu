@@ -962,18 +962,23 @@ int column_grid(int64_t total, int B)
 }
 
 template <int TB>
-void launch_bspmm_fix(const ed_batch& bt, const BlockFixed& f, int B, double* Y, cudaStream_t st)
+void launch_bspmm_fix(const ed_batch& bt, const BlockFixed& f, const BlockScratch& v, int B, double* Y, cudaStream_t st)
 {
     const int64_t rows_per_block = 256 / TB;
     dim3 grid((unsigned)std::max<int64_t>(1, std::min<int64_t>(sms_b() * 16, (bt.n + rows_per_block - 1) / rows_per_block)),
               (unsigned)((B + TB - 1) / TB));
     k_bspmm_fix<TB><<<grid, 256, 0, st>>>(bt.rowptr.p, bt.col.p, bt.code.p, reinterpret_cast<const int2*>(f.w.p),
                                           reinterpret_cast<const int2*>(f.diag.p), f.ea.p,
-                                          reinterpret_cast<const int2*>(f.x.p), f.ex.p, Y, bt.n, B);
+                                          reinterpret_cast<const int2*>(v.x.p), v.ex.p, Y, bt.n, B);
     count_launch();
 }
 
-}  // namespace
+// The scratch of B columns.
+void fix_room(const ed_batch& bt, int B, BlockScratch& v)
+{
+    v.x.alloc_at_least((size_t)bt.n * B);
+    v.ex.alloc_at_least(B + 1);
+}
 
 // The operands' fixed-point form; false where the exact sums do not apply
 // (a weight or diagonal entry that is not finite, a row of more than 2048
@@ -986,10 +991,8 @@ bool fix_operands(const ed_batch& bt, const BlockOperands& o, BlockFixed& f, cud
     if (bt.max_row > kFixMaxRow || bt.n * B >= (1ll << 32)) return false;
     const int64_t nw = (int64_t)bt.nhop * B, nd = bt.n * B;
     f.ea.alloc_at_least(B + 1);
-    f.ex.alloc_at_least(B + 1);
     f.w.alloc_at_least((size_t)(2 * nw));
     f.diag.alloc_at_least((size_t)nd);
-    f.x.alloc_at_least((size_t)nd);
     DevBuf<int> ew(B + 1);
     ED_CUDA(cudaMemsetAsync(f.ea.p, 0, (size_t)(B + 1) * 4, st));
     ED_CUDA(cudaMemsetAsync(ew.p, 0, (size_t)(B + 1) * 4, st));
@@ -1016,53 +1019,61 @@ bool fix_operands(const ed_batch& bt, const BlockOperands& o, BlockFixed& f, cud
 
 // Y = H X through the fixed-point operands f of o; where X is not finite the
 // FP64 kernel of tile t follows and its answer stands.
-void fixed_block_product(const ed_batch& bt, const BlockOperands& o, const BlockFixed& f, const std::array<int, 4>& t,
-                         const double* X, double* Y, cudaStream_t st, bool converted)
+void fixed_block_product(const ed_batch& bt, const BlockOperands& o, const BlockFixed& f, BlockScratch& v,
+                         const std::array<int, 4>& t, const double* X, double* Y, cudaStream_t st, bool converted)
 {
     const int B = o.B, T = column_threads(B);
     const int64_t total = bt.n * B;
     if (!converted) {
-        ED_CUDA(cudaMemsetAsync(f.ex.p, 0, (size_t)(B + 1) * 4, st));
-        k_bfix_exp<<<column_grid(total, B), T, B * 4, st>>>(X, total, B, f.ex.p); count_launch();
-        k_bfix_conv<<<column_grid(total, B), T, 0, st>>>(X, total, B, f.ex.p, 0, f.x.p); count_launch();
+        ED_CUDA(cudaMemsetAsync(v.ex.p, 0, (size_t)(B + 1) * 4, st));
+        k_bfix_exp<<<column_grid(total, B), T, B * 4, st>>>(X, total, B, v.ex.p); count_launch();
+        k_bfix_conv<<<column_grid(total, B), T, 0, st>>>(X, total, B, v.ex.p, 0, v.x.p); count_launch();
     }
-    if (B > 16) launch_bspmm_fix<32>(bt, f, B, Y, st);
-    else if (B > 8) launch_bspmm_fix<16>(bt, f, B, Y, st);
-    else if (B > 4) launch_bspmm_fix<8>(bt, f, B, Y, st);
-    else launch_bspmm_fix<4>(bt, f, B, Y, st);
+    if (B > 16) launch_bspmm_fix<32>(bt, f, v, B, Y, st);
+    else if (B > 8) launch_bspmm_fix<16>(bt, f, v, B, Y, st);
+    else if (B > 4) launch_bspmm_fix<8>(bt, f, v, B, Y, st);
+    else launch_bspmm_fix<4>(bt, f, v, B, Y, st);
     ED_CUDA(cudaGetLastError());
-    bspmm_variant(bt, o, t[0], t[1], t[2], t[3], X, Y, bt.n, f.ex.p + B, st);
+    bspmm_variant(bt, o, t[0], t[1], t[2], t[3], X, Y, bt.n, v.ex.p + B, st);
 }
 
-namespace {
-
-// The whole batch's fixed-point operands with this stream's scratch for X,
-// made when missing; null for a part of the batch, where they do not apply and
-// in a capture: a graph may be replayed on any stream beside other products,
-// so it must not hold a stream's scratch.
-BlockFixed* batch_fixed(const ed_batch& bt, const BlockOperands& o, cudaStream_t st)
+// The whole batch's fixed-point operands, made when missing; false for a part
+// of the batch and where they were declined.
+bool whole_fixed(const ed_batch& bt, const BlockOperands& o, cudaStream_t st)
 {
-    if (o.w != bt.w.p) return nullptr;
+    if (o.w != bt.w.p) return false;
+    std::lock_guard<std::mutex> lk(bt.fix_mu);
+    if (bt.fixed_state == 0) bt.fixed_state = fix_operands(bt, o, bt.fixed, st) ? 1 : -1;
+    return bt.fixed_state == 1;
+}
+
+// This stream's scratch for the whole batch, made when missing.
+BlockScratch* whole_scratch(const ed_batch& bt, cudaStream_t st)
+{
     int dev = 0;
     ED_CUDA(cudaGetDevice(&dev));
-    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-    ED_CUDA(cudaStreamIsCapturing(st, &cs));
-    if (cs != cudaStreamCaptureStatusNone) return nullptr;
-    const std::pair<int, cudaStream_t> key(dev, st);
     std::lock_guard<std::mutex> lk(bt.fix_mu);
-    auto it = bt.fixed.find(key);
-    if (it != bt.fixed.end()) return it->second->ready ? it->second.get() : nullptr;
-    auto f = std::make_unique<BlockFixed>();
-    fix_operands(bt, o, *f, st);
-    return (bt.fixed[key] = std::move(f))->ready ? bt.fixed[key].get() : nullptr;
+    std::unique_ptr<BlockScratch>& v = bt.fixed_x[{dev, st}];
+    if (!v) {
+        auto made = std::make_unique<BlockScratch>();
+        fix_room(bt, bt.B, *made);
+        v = std::move(made);
+    }
+    return v.get();
 }
 
 }  // namespace
 
+// In a capture without fixed point: a graph may be replayed on any stream
+// beside other products, so it must not hold a stream's scratch.
 void batch_block_product(const ed_batch& bt, const BlockOperands& o, const double* X, double* Y, cudaStream_t st)
 {
     const std::array<int, 4> t = batch_tile(bt, o, st);
-    if (BlockFixed* f = batch_fixed(bt, o, st)) fixed_block_product(bt, o, *f, t, X, Y, st, false);
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    ED_CUDA(cudaStreamIsCapturing(st, &cs));
+    BlockScratch* v = nullptr;
+    if (cs == cudaStreamCaptureStatusNone && whole_fixed(bt, o, st)) v = whole_scratch(bt, st);
+    if (v) fixed_block_product(bt, o, bt.fixed, *v, t, X, Y, st, false);
     else bspmm_variant(bt, o, t[0], t[1], t[2], t[3], X, Y, bt.n, nullptr, st);
 }
 
@@ -1072,7 +1083,7 @@ void batch_spmm(const ed_batch& bt, const double* X, double* Y, cudaStream_t st)
 }
 
 void batch_residuals(const ed_batch& bt, const BlockOperands& o, const double* X, const double* lam, int k,
-                     double* res, cudaStream_t st)
+                     double* res, cudaStream_t st, const BlockFixed* fixed, BlockScratch* scratch)
 {
     const int B = o.B;
     int BP = 1;
@@ -1081,11 +1092,19 @@ void batch_residuals(const ed_batch& bt, const BlockOperands& o, const double* X
     const int nb = (int)std::max<int64_t>(1, std::min<int64_t>(sms_b() * 4, n / 128));
     DevBuf<double> y((size_t)n * B), part((size_t)nb * B), s(B), dl(B);
     std::vector<double> l(B), r(B);
+    const std::array<int, 4> t = batch_tile(bt, o, st);
+    BlockScratch own;      // for this call: its stream may not live longer
+    if (!fixed && whole_fixed(bt, o, st)) fixed = &bt.fixed;
+    if (fixed && !scratch) {
+        fix_room(bt, B, own);
+        scratch = &own;
+    }
     for (int i = 0; i < k; ++i) {
         for (int b = 0; b < B; ++b) l[b] = lam[(size_t)b * k + i];
         ED_CUDA(cudaMemcpyAsync(dl.p, l.data(), (size_t)B * 8, cudaMemcpyHostToDevice, st));
         const double* x = X + (int64_t)i * n * B;
-        batch_block_product(bt, o, x, y.p, st);
+        if (fixed && fixed->ready && scratch) fixed_block_product(bt, o, *fixed, *scratch, t, x, y.p, st, false);
+        else bspmm_variant(bt, o, t[0], t[1], t[2], t[3], x, y.p, n, nullptr, st);
         k_bresid<<<nb, kBT, 0, st>>>(y.p, x, n, B, BP, dl.p, part.p); count_launch();
         launch(k_bsum, (unsigned)((B + 31) / 32), 1024, 0, st, part.p, nb, B, 1, s.p, nullptr, SumThen());
         ED_CUDA(cudaMemcpyAsync(r.data(), s.p, (size_t)B * 8, cudaMemcpyDeviceToHost, st));
@@ -1254,8 +1273,6 @@ void batch_solve(const ed_batch& bt, const int* sel, int nsel, const ed_lanczos_
     const BlockOperands ops0 = sel ? gather_operands(bt, sel, nsel, wsel, dsel, st) : full_operands(bt);
     BlockOperands ops = ops0;
     std::array<int, 4> tile = batch_tile(bt, ops, st);
-    BlockFixed fixed;
-    fix_operands(bt, ops, fixed, st);
     int64_t vs = vs0;
 
     auto grid_for = [&](int64_t work) { return (int)std::max<int64_t>(1, std::min<int64_t>(sms_b() * 8, (work + 255) / 256)); };
@@ -1305,6 +1322,9 @@ void batch_solve(const ed_batch& bt, const int* sel, int nsel, const ed_lanczos_
         xtmp.alloc((size_t)vs0 * nev);
         X = xtmp.p;
     }
+    BlockFixed fixed;
+    BlockScratch fixed_x;
+    if (fix_operands(bt, ops, fixed, st)) fix_room(bt, B0, fixed_x);
     auto write_ritz = [&](const std::vector<int>& cols) {   // cols: active columns whose pairs are final
         if (!X || cols.empty()) return;
         std::vector<int> d(cols.size());
@@ -1328,7 +1348,7 @@ void batch_solve(const ed_batch& bt, const int* sel, int nsel, const ed_lanczos_
             double* cj = coef.p + (size_t)j * (m + 1) * B;
             double* ref = s2.p + B;
             const bool first = (j == k);
-            if (fixed.ready) fixed_block_product(bt, ops, fixed, tile, vj, w, st, !first);
+            if (fixed.ready) fixed_block_product(bt, ops, fixed, fixed_x, tile, vj, w, st, !first);
             else bspmm_variant(bt, ops, tile[0], tile[1], tile[2], tile[3], vj, w, n, nullptr, st);
             SumThen local, acc, need, fin;
             if (!first) {
@@ -1357,7 +1377,7 @@ void batch_solve(const ed_batch& bt, const int* sel, int nsel, const ed_lanczos_
             fin.brk = brk.p;
             unsigned long long* amax = fixed.ready ? absmax.p : nullptr;
             acc.absmax = fin.absmax = amax;
-            acc.ex = fin.ex = fixed.ex.p;
+            acc.ex = fin.ex = fixed_x.ex.p;
             for (int pass = 0; pass < 2; ++pass) {
                 int* mask = pass == 0 ? nullptr : need2.p;
                 launch(k_bmdot, nb, kBT, 0, st, V.p, n, B, BP, J, w, part.p, mask,
@@ -1371,8 +1391,8 @@ void batch_solve(const ed_batch& bt, const int* sel, int nsel, const ed_lanczos_
                 // the norm after the pass, kept from pass 1 for problems that skip pass 2
                 bsum(npart.p, 1, s2.p + 3 * B, mask, pass == 0 ? need : fin);
             }
-            launch(k_bscale, grid_for(vs), 256, 0, st, w, n, B, betas.p + (size_t)j * B, clock.p + 2 * (j + 1), fixed.ex.p,
-                   amax && j + 1 < m ? fixed.x.p : nullptr);
+            launch(k_bscale, grid_for(vs), 256, 0, st, w, n, B, betas.p + (size_t)j * B, clock.p + 2 * (j + 1), fixed_x.ex.p,
+                   amax && j + 1 < m ? fixed_x.x.p : nullptr);
         }
     };
     CycleGraphs cache;
@@ -1512,7 +1532,7 @@ void batch_solve(const ed_batch& bt, const int* sel, int nsel, const ed_lanczos_
             ED_CUDA(cudaGetLastError());
             ops = {wc[nxt].p, dc[nxt].p, Bn};
             tile = batch_tile(bt, ops, st);
-            fix_operands(bt, ops, fixed, st);
+            if (fixed.ready) fix_operands(bt, ops, fixed, st);   // into the same buffers
             std::vector<int> no(Bn);
             for (int q = 0; q < Bn; ++q) no[q] = orig[live[q]];
             orig = no;
@@ -1549,7 +1569,8 @@ void batch_solve(const ed_batch& bt, const int* sel, int nsel, const ed_lanczos_
     if (p.verify && X) {
         // true residuals of every problem, through its own operator
         std::vector<double> res((size_t)B0 * nev);
-        batch_residuals(bt, ops0, X, evals, nev, res.data(), st);
+        if (fixed.ready && ops.w != ops0.w) fix_operands(bt, ops0, fixed, st);   // compacted meanwhile
+        batch_residuals(bt, ops0, X, evals, nev, res.data(), st, &fixed, &fixed_x);
         inf.block_products += nev;
         inf.problem_products += (int64_t)nev * B0;
         double worst = 0.0;

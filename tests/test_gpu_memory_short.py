@@ -109,3 +109,49 @@ def test_a_solve_that_fills_the_device(cuda, kw):
     with memory(basis + (3 + nev) * n * 8 + (8 << 20)):
         assert K.LanczosDiagonalize(nev, tol=1e-10, v0=v0)
     assert np.max(np.abs(K.m_eigenvalues - want)) <= 1e-11 * np.abs(want).max()
+
+
+def sweep(N, norb, count):
+    basis = ed.FermionFockBasis()
+    basis.GenerateFockSpace(N, norb, 0)
+    vs = []
+    for v1 in np.linspace(0.5, 3.0, count):
+        v = ed.odd_coulomb_list(norb)
+        v[1] = v1
+        vs.append(v)
+    return ed.HamiltonianBatch(basis, vs, autotune=False)
+
+
+def block(torch, bt, seed):
+    X = torch.from_numpy(np.random.default_rng(seed).uniform(-1, 1, (bt.n, bt.nham))).cuda()
+    torch.cuda.synchronize()
+    return X
+
+
+def held(torch):
+    torch.cuda.synchronize()
+    return -torch.cuda.mem_get_info()[0]
+
+
+def test_solves_and_streams_leave_one_set_of_operands(cuda):
+    torch = cuda
+    N, norb, count = 9, 25, 16
+    X = block(torch, sweep(N, norb, count), 8)
+    Y = torch.empty_like(X)
+    warm = sweep(N, norb, count)      # modules and the like
+    warm.solve(2, V0=X)
+    warm.spmm(X, Y)
+    bt = sweep(N, norb, count)
+    one, slack = bt.n * count * 8, 2 << 20      # a block of vectors; the allocator's granularity
+    before = held(torch)
+    for _ in range(3):
+        bt.solve(2, V0=X)
+    assert held(torch) - before <= slack
+    bt.spmm(X, Y)
+    torch.cuda.synchronize()
+    first = held(torch)
+    streams = [torch.cuda.Stream() for _ in range(3)]
+    for s in streams:
+        bt.spmm(X, Y, stream=s.cuda_stream)
+        torch.cuda.synchronize()
+    assert held(torch) - first <= len(streams) * (one + slack)
