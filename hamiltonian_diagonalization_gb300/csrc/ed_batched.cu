@@ -973,27 +973,41 @@ void launch_bspmm_fix(const ed_batch& bt, const BlockFixed& f, const BlockScratc
     count_launch();
 }
 
-// The scratch of B columns.
-void fix_room(const ed_batch& bt, int B, BlockScratch& v)
+// The scratch of B columns, or false where it would leave less than as much
+// free and the reserve (bytes that the caller will need).
+bool fix_room(const ed_batch& bt, int B, BlockScratch& v, size_t reserve)
 {
-    v.x.alloc_at_least((size_t)bt.n * B);
-    v.ex.alloc_at_least(B + 1);
+    const size_t count = (size_t)bt.n * B;
+    if (count > v.x.n && 16 * count + reserve > device_memory_free()) return false;
+    return if_memory([&] {
+        v.x.alloc_at_least(count);
+        v.ex.alloc_at_least(B + 1);
+        return true;
+    });
 }
 
 // The operands' fixed-point form; false where the exact sums do not apply
 // (a weight or diagonal entry that is not finite, a row of more than 2048
 // elements, weights so near the diagonal's size that a row's high limb
-// products could pass 2^62).  Waits for the stream.
-bool fix_operands(const ed_batch& bt, const BlockOperands& o, BlockFixed& f, cudaStream_t st)
+// products could pass 2^62) or where it would leave less than as much free and
+// the reserve.  Waits for the stream.
+bool fix_operands(const ed_batch& bt, const BlockOperands& o, BlockFixed& f, size_t reserve, cudaStream_t st)
 {
     f.ready = false;
     const int B = o.B;
     if (bt.max_row > kFixMaxRow || bt.n * B >= (1ll << 32)) return false;
     const int64_t nw = (int64_t)bt.nhop * B, nd = bt.n * B;
-    f.ea.alloc_at_least(B + 1);
-    f.w.alloc_at_least((size_t)(2 * nw));
-    f.diag.alloc_at_least((size_t)nd);
-    DevBuf<int> ew(B + 1);
+    const size_t need = ((size_t)(2 * nw) > f.w.n ? 16 * (size_t)nw : 0) + ((size_t)nd > f.diag.n ? 8 * (size_t)nd : 0);
+    if (need && 2 * need + reserve > device_memory_free()) return false;
+    DevBuf<int> ew;
+    if (!if_memory([&] {
+            f.ea.alloc_at_least(B + 1);
+            ew.alloc(B + 1);
+            f.w.alloc_at_least((size_t)(2 * nw));
+            f.diag.alloc_at_least((size_t)nd);
+            return true;
+        }))
+        return false;
     ED_CUDA(cudaMemsetAsync(f.ea.p, 0, (size_t)(B + 1) * 4, st));
     ED_CUDA(cudaMemsetAsync(ew.p, 0, (size_t)(B + 1) * 4, st));
     const int T = column_threads(B);
@@ -1043,11 +1057,12 @@ bool whole_fixed(const ed_batch& bt, const BlockOperands& o, cudaStream_t st)
 {
     if (o.w != bt.w.p) return false;
     std::lock_guard<std::mutex> lk(bt.fix_mu);
-    if (bt.fixed_state == 0) bt.fixed_state = fix_operands(bt, o, bt.fixed, st) ? 1 : -1;
+    if (bt.fixed_state == 0) bt.fixed_state = fix_operands(bt, o, bt.fixed, 8 * (size_t)bt.n * bt.B, st) ? 1 : -1;
     return bt.fixed_state == 1;
 }
 
-// This stream's scratch for the whole batch, made when missing.
+// This stream's scratch for the whole batch, made when missing; null where the
+// memory is short.
 BlockScratch* whole_scratch(const ed_batch& bt, cudaStream_t st)
 {
     int dev = 0;
@@ -1056,7 +1071,7 @@ BlockScratch* whole_scratch(const ed_batch& bt, cudaStream_t st)
     std::unique_ptr<BlockScratch>& v = bt.fixed_x[{dev, st}];
     if (!v) {
         auto made = std::make_unique<BlockScratch>();
-        fix_room(bt, bt.B, *made);
+        if (!fix_room(bt, bt.B, *made, 0)) return nullptr;
         v = std::move(made);
     }
     return v.get();
@@ -1095,10 +1110,7 @@ void batch_residuals(const ed_batch& bt, const BlockOperands& o, const double* X
     const std::array<int, 4> t = batch_tile(bt, o, st);
     BlockScratch own;      // for this call: its stream may not live longer
     if (!fixed && whole_fixed(bt, o, st)) fixed = &bt.fixed;
-    if (fixed && !scratch) {
-        fix_room(bt, B, own);
-        scratch = &own;
-    }
+    if (fixed && !scratch && fix_room(bt, B, own, 0)) scratch = &own;
     for (int i = 0; i < k; ++i) {
         for (int b = 0; b < B; ++b) l[b] = lam[(size_t)b * k + i];
         ED_CUDA(cudaMemcpyAsync(dl.p, l.data(), (size_t)B * 8, cudaMemcpyHostToDevice, st));
@@ -1322,9 +1334,14 @@ void batch_solve(const ed_batch& bt, const int* sel, int nsel, const ed_lanczos_
         xtmp.alloc((size_t)vs0 * nev);
         X = xtmp.p;
     }
+    // the fixed-point operands, where the memory has room for them beside what
+    // the solve may still need: two sets of compacted operands, a residual's
+    // product and a tile's tuning
+    const size_t later = 16 * (size_t)bt.nhop * B0 + 5 * 8 * (size_t)vs0;
     BlockFixed fixed;
     BlockScratch fixed_x;
-    if (fix_operands(bt, ops, fixed, st)) fix_room(bt, B0, fixed_x);
+    if (fix_room(bt, B0, fixed_x, later)) fix_operands(bt, ops, fixed, later, st);
+    if (!fixed.ready) fixed_x = BlockScratch();
     auto write_ritz = [&](const std::vector<int>& cols) {   // cols: active columns whose pairs are final
         if (!X || cols.empty()) return;
         std::vector<int> d(cols.size());
@@ -1532,7 +1549,7 @@ void batch_solve(const ed_batch& bt, const int* sel, int nsel, const ed_lanczos_
             ED_CUDA(cudaGetLastError());
             ops = {wc[nxt].p, dc[nxt].p, Bn};
             tile = batch_tile(bt, ops, st);
-            if (fixed.ready) fix_operands(bt, ops, fixed, st);   // into the same buffers
+            if (fixed.ready) fix_operands(bt, ops, fixed, 0, st);   // into the same buffers
             std::vector<int> no(Bn);
             for (int q = 0; q < Bn; ++q) no[q] = orig[live[q]];
             orig = no;
@@ -1569,7 +1586,7 @@ void batch_solve(const ed_batch& bt, const int* sel, int nsel, const ed_lanczos_
     if (p.verify && X) {
         // true residuals of every problem, through its own operator
         std::vector<double> res((size_t)B0 * nev);
-        if (fixed.ready && ops.w != ops0.w) fix_operands(bt, ops0, fixed, st);   // compacted meanwhile
+        if (fixed.ready && ops.w != ops0.w) fix_operands(bt, ops0, fixed, 0, st);   // compacted meanwhile
         batch_residuals(bt, ops0, X, evals, nev, res.data(), st, &fixed, &fixed_x);
         inf.block_products += nev;
         inf.problem_products += (int64_t)nev * B0;

@@ -128,6 +128,38 @@ def block(torch, bt, seed):
     return X
 
 
+def test_block_product_without_room(cuda):
+    torch = cuda
+    X = block(torch, sweep(7, 19, 6), 6)
+    Y, want = torch.empty_like(X), torch.empty_like(X)
+    bt = sweep(7, 19, 6)
+    with memory(1 << 12):
+        bt.spmm(X, Y)
+    sweep(7, 19, 6).spmm(X, want)
+    torch.cuda.synchronize()
+    assert close(torch, Y, want)
+    first = sweep(7, 19, 6)
+    first.spmm(X, Y)
+    with memory(1 << 12):       # the operands are there, another stream's scratch is not
+        first.spmm(X, Y, stream=torch.cuda.Stream().cuda_stream)
+    torch.cuda.synchronize()
+    assert close(torch, Y, want)
+
+
+# the solve's own vectors, a second set of operands, and a residual's product: all that the FP64 products need
+def test_a_batched_solve_that_fills_the_device(cuda):
+    torch = cuda
+    N, norb, count, nev = 9, 25, 16, 2
+    bt = sweep(N, norb, count)
+    X = block(torch, bt, 7)
+    want, _, _ = bt.solve(nev, V0=X)
+    m, vs = 2 * nev + 21, bt.n * count
+    short = sweep(N, norb, count)
+    with memory((2 * (m + 1) + nev + 3) * vs * 8 + (4 << 20)):
+        got, _, info = short.solve(nev, V0=X)
+    assert info["converged"] == count and np.max(np.abs(got - want)) <= 1e-11 * np.abs(want).max()
+
+
 def held(torch):
     torch.cuda.synchronize()
     return -torch.cuda.mem_get_info()[0]
