@@ -343,20 +343,25 @@ __global__ void __launch_bounds__(256) k_bfix_exp(const double* __restrict__ v, 
 }
 
 // q = v in fixed point by column; with both, rows 2h and 2h + 1 of q are row h
-// of v and its negative.
-__global__ void __launch_bounds__(256) k_bfix_conv(const double* __restrict__ v, int64_t total, int B,
-                                                   const int* __restrict__ exps, int both, int64_t* __restrict__ q)
+// of v and its negative.  exps[B] becomes kFixLost where an entry is lost.
+__global__ void __launch_bounds__(256) k_bfix_conv(const double* __restrict__ v, int64_t total, int B, int* exps, int both,
+                                                   int64_t* __restrict__ q)
 {
     const int E = exps[threadIdx.x % B];
+    bool lost = false;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
+        const double x = v[i];
+        const int64_t a = fix_pair(x, E);
+        lost |= fix_lost(x, a);
         if (both) {
             const int64_t h = i / B, b = i - h * B;
-            q[2 * h * B + b] = fix_pair(v[i], E);
-            q[(2 * h + 1) * B + b] = fix_pair(-v[i], E);
+            q[2 * h * B + b] = a;
+            q[(2 * h + 1) * B + b] = fix_pair(-x, E);
         } else {
-            q[i] = fix_pair(v[i], E);
+            q[i] = a;
         }
     }
+    if (lost) atomicMax(exps + B, kFixLost);
 }
 
 // The eight elements at k (a multiple of 8) of a row whose elements are
@@ -688,18 +693,24 @@ __global__ void __launch_bounds__(kBT, 4) k_bupdate(const double* __restrict__ V
 }
 
 // w_p /= beta_p, with q also the block product's fixed-point copy at the bounds
-// ex (its own two passes over the block and the clearing before them took 12
+// ex, ex[B] raised to kFixLost where an entry is lost (its own two passes over the block and the clearing before them took 12
 // us of a step's 330 for 16 problems at N=9, 2S=24).
 __global__ void k_bscale(double* __restrict__ w, int64_t n, int B, const double* __restrict__ beta,
-                         unsigned long long* __restrict__ started, const int* __restrict__ ex, int64_t* __restrict__ q)
+                         unsigned long long* __restrict__ started, int* ex, int64_t* __restrict__ q)
 {
     const int64_t total = n * (int64_t)B;
+    bool lost = false;
     for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
         const int p = (int)(t % B);
         const double x = w[t] / beta[p];
         w[t] = x;
-        if (q) q[t] = fix_pair(x, ex[p]);
+        if (q) {
+            const int64_t a = fix_pair(x, ex[p]);
+            lost |= fix_lost(x, a);
+            q[t] = a;
+        }
     }
+    if (lost) atomicMax(ex + B, kFixLost);
     stamp(started);
 }
 
@@ -989,7 +1000,7 @@ bool fix_room(const ed_batch& bt, int B, BlockScratch& v, size_t reserve)
 // The operands' fixed-point form; false where the exact sums do not apply
 // (a weight or diagonal entry that is not finite, a row of more than 2048
 // elements, weights so near the diagonal's size that a row's high limb
-// products could pass 2^62) or where it would leave less than as much free and
+// products could pass 2^62, a weight or diagonal entry lost) or where it would leave less than as much free and
 // the reserve.  Waits for the stream.
 bool fix_operands(const ed_batch& bt, const BlockOperands& o, BlockFixed& f, size_t reserve, cudaStream_t st)
 {
@@ -1026,13 +1037,14 @@ bool fix_operands(const ed_batch& bt, const BlockOperands& o, BlockFixed& f, siz
     k_bfix_conv<<<column_grid(nw, B), T, 0, st>>>(o.w, nw, B, f.ea.p, 1, f.w.p); count_launch();
     k_bfix_conv<<<column_grid(nd, B), T, 0, st>>>(o.diag, nd, B, f.ea.p, 0, f.diag.p); count_launch();
     ED_CUDA(cudaGetLastError());
+    ED_CUDA(cudaMemcpyAsync(ea.data(), f.ea.p + B, 4, cudaMemcpyDeviceToHost, st));
     ED_CUDA(cudaStreamSynchronize(st));   // ew goes
-    f.ready = true;
-    return true;
+    f.ready = ea[0] < kFixLost;
+    return f.ready;
 }
 
-// Y = H X through the fixed-point operands f of o; where X is not finite the
-// FP64 kernel of tile t follows and its answer stands.
+// Y = H X through the fixed-point operands f of o; where an entry of X is not
+// finite, or lost, the FP64 kernel of tile t follows and its answer stands.
 void fixed_block_product(const ed_batch& bt, const BlockOperands& o, const BlockFixed& f, BlockScratch& v,
                          const std::array<int, 4>& t, const double* X, double* Y, cudaStream_t st, bool converted)
 {

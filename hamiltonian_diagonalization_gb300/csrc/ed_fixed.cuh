@@ -123,9 +123,19 @@ __device__ __forceinline__ void block_absmax(unsigned long long v, unsigned long
     if ((threadIdx.x & 31) == 0) atomicMax(m, (unsigned long long)top << 32 | lo);
 }
 
-// Per-block maxima of fix_exp over v[0, n) into part[blockIdx.x].
+// Whether v, converted to q, is lost: not zero, but zero in fixed point
+// (below 2^(E - 1081): its exponent field is below E - 58).  A product whose
+// FP64 kernel stands behind it takes that one for a vector with such an entry:
+// its conversion raises the vector's bound to 2047, as an entry that is not
+// finite does.
+__device__ __forceinline__ bool fix_lost(double v, int64_t q) { return q == 0 && abs_bits(v) != 0; }
+constexpr int kFixLost = 2047;
+
+// Per-block maxima of fix_exp over v[0, n) into part[blockIdx.x]; the word
+// after them, which the conversion raises to the bound, is zeroed.
 __global__ void __launch_bounds__(256) k_fix_exp(const double* __restrict__ v, int64_t n, int* __restrict__ part)
 {
+    if (blockIdx.x == 0 && threadIdx.x == 0) part[gridDim.x] = 0;
     __shared__ int sm[8];
     int m = 1;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
@@ -140,10 +150,10 @@ __global__ void __launch_bounds__(256) k_fix_exp(const double* __restrict__ v, i
     }
 }
 
-// q[i] = fix_pair(v[i], E) with E the maximum of part[0, nparts); block 0
-// also stores E in part[nparts] for the product.
+// q[i] = fix_pair(v[i], E) with E the maximum of part[0, nparts); part[nparts]
+// is raised to E for the product, with mark to kFixLost where an entry is lost.
 __global__ void __launch_bounds__(256) k_fix_conv(const double* __restrict__ v, int64_t n, int* __restrict__ part,
-                                                  int nparts, int64_t* __restrict__ q)
+                                                  int nparts, int64_t* __restrict__ q, bool mark)
 {
     __shared__ int sE;
     if (threadIdx.x < 32) {
@@ -152,13 +162,19 @@ __global__ void __launch_bounds__(256) k_fix_conv(const double* __restrict__ v, 
         m = __reduce_max_sync(0xffffffffu, m);
         if (threadIdx.x == 0) {
             sE = m;
-            if (blockIdx.x == 0) part[nparts] = m;
+            if (blockIdx.x == 0) atomicMax(part + nparts, m);
         }
     }
     __syncthreads();
     const int E = sE;
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-        q[i] = fix_pair(v[i], E);
+    bool lost = false;
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+        const double x = v[i];
+        const int64_t a = fix_pair(x, E);
+        lost |= fix_lost(x, a);
+        q[i] = a;
+    }
+    if (mark && lost) atomicMax(part + nparts, kFixLost);
 }
 
 // Both at once for a short vector (one launch less in a solver's step): every
@@ -166,33 +182,46 @@ __global__ void __launch_bounds__(256) k_fix_conv(const double* __restrict__ v, 
 constexpr int64_t kFixOnePass = 16384;   // n = 8,512: 7.7 us a product's step less; at 45,207 the two passes are shorter
 
 __global__ void __launch_bounds__(256) k_fix_one(const double* __restrict__ v, int64_t n, int* __restrict__ bound,
-                                                 int64_t* __restrict__ q)
+                                                 int64_t* __restrict__ q, bool mark)
 {
-    __shared__ int sm[8];
-    int m = 1;
+    __shared__ int sm[8], sl[8];
+    int m = 1, low = kFixLost;
 #pragma unroll 8
-    for (int64_t i = threadIdx.x; i < n; i += 256) m = max(m, fix_exp(v[i]));
+    for (int64_t i = threadIdx.x; i < n; i += 256) {
+        const double x = v[i];
+        const int e = fix_exp(x);
+        m = max(m, e);
+        if (abs_bits(x) != 0) low = min(low, e);
+    }
     m = __reduce_max_sync(0xffffffffu, m);
-    if ((threadIdx.x & 31) == 0) sm[threadIdx.x >> 5] = m;
+    low = __reduce_min_sync(0xffffffffu, low);
+    if ((threadIdx.x & 31) == 0) {
+        sm[threadIdx.x >> 5] = m;
+        sl[threadIdx.x >> 5] = low;
+    }
     __syncthreads();
     int E = sm[0];
 #pragma unroll
-    for (int w = 1; w < 8; ++w) E = max(E, sm[w]);
-    if (blockIdx.x == 0 && threadIdx.x == 0) *bound = E;
+    for (int w = 1; w < 8; ++w) {
+        E = max(E, sm[w]);
+        low = min(low, sl[w]);
+    }
+    if (blockIdx.x == 0 && threadIdx.x == 0) *bound = mark && low < E - 58 ? kFixLost : E;
     const int64_t i = blockIdx.x * (int64_t)256 + threadIdx.x;
     if (i < n) q[i] = fix_pair(v[i], E);
 }
 
 // q = v in fixed point, its exponent bound in part[parts]; blocks: the grid of
-// the conversion of a long vector.
-inline void fix_convert(const double* v, int64_t n, int* part, int parts, int blocks, int64_t* q, cudaStream_t st)
+// the conversion of a long vector; mark: kFixLost where an entry is lost.
+inline void fix_convert(const double* v, int64_t n, int* part, int parts, int blocks, int64_t* q, cudaStream_t st,
+                        bool mark = false)
 {
     if (n <= kFixOnePass) {
-        launch(k_fix_one, (unsigned)((n + 255) / 256), 256, 0, st, v, n, part + parts, q);
+        launch(k_fix_one, (unsigned)((n + 255) / 256), 256, 0, st, v, n, part + parts, q, mark);
         return;
     }
     launch(k_fix_exp, parts, 256, 0, st, v, n, part);
-    launch(k_fix_conv, blocks, 256, 0, st, v, n, part, parts, q);
+    launch(k_fix_conv, blocks, 256, 0, st, v, n, part, parts, q, mark);
 }
 
 // p2, p1, p0 += the three limb products of a b (weights 2^60, 2^30, 1).

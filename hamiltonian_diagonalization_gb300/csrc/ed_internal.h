@@ -263,6 +263,7 @@ struct ed_fixq {
     // the sliced-ELL order (nnz_pad + kCrsPad)
     edgb::DevBuf<int64_t> val, sval;
     int val_state = 0, sval_state = 0;
+    bool lost = false;   // a value of the copy became zero
     // the row-blocked copy (ed_blocked.cuh): offsets of the blocks' steps,
     // columns and limb pairs; same states
     edgb::DevBuf<int64_t> boff, bval;
@@ -356,10 +357,12 @@ void cspmv(const ed_ccrs& a, const double* x, double* y, cudaStream_t st);
 // Where the product of this matrix on this stream reads x in fixed point, for
 // a solver whose last kernel before the product writes it there: q = x's limb
 // pairs, *bound = the exponent bound.  q is null where the product reads x
-// itself.  *_converted runs the product that reads them.
+// itself.  *_converted runs the product that reads them.  mark: the bound is
+// kFixLost where an entry is lost.
 struct FixTarget {
     int64_t* q = nullptr;
     int* bound = nullptr;
+    bool mark = false;
 };
 FixTarget cspmv_target(const ed_ccrs& a, cudaStream_t st);
 void cspmv_converted(const ed_ccrs& a, double* y, cudaStream_t st);

@@ -181,11 +181,14 @@ __global__ void __launch_bounds__(kThreads) k_mdot(const double* __restrict__ V,
                                                    double* __restrict__ coefcol, double* __restrict__ before,
                                                    const int* __restrict__ run, const int* __restrict__ stop,
                                                    unsigned long long* __restrict__ ended,
-                                                   unsigned long long* __restrict__ absmax)
+                                                   unsigned long long* __restrict__ absmax, FixTarget t)
 {
     if (blockIdx.x == 0) stamp(ended);
     if ((run && !*run) || (stop && *stop)) return;
-    if (absmax && blockIdx.x == 0 && threadIdx.x == 0) *absmax = 0ull;   // k_update's
+    if (absmax && blockIdx.x == 0 && threadIdx.x == 0) {
+        *absmax = 0ull;               // k_update's
+        if (t.mark) *t.bound = 0;     // k_scale's
+    }
     extern __shared__ double sw[];
     const int64_t r0 = (int64_t)blockIdx.x * R;
     const int len = (int)min((int64_t)R, n - r0);
@@ -343,12 +346,21 @@ __global__ void __launch_bounds__(kThreads) k_scale(double* __restrict__ w, int6
     if (!(stop && *stop)) {
         const double inv = 1.0 / *beta;
         const int E = t.q ? fix_exp(__longlong_as_double((long long)*absmax) * inv) : 0;
-        if (t.q && blockIdx.x == 0 && threadIdx.x == 0) *t.bound = E;
+        if (t.q && blockIdx.x == 0 && threadIdx.x == 0) {
+            if (t.mark) atomicMax(t.bound, E);
+            else *t.bound = E;
+        }
+        bool lost = false;
         for (int64_t r = blockIdx.x * (int64_t)kThreads + threadIdx.x; r < n; r += (int64_t)gridDim.x * kThreads) {
             const double x = w[r] * inv;
             w[r] = x;
-            if (t.q) t.q[r] = fix_pair(x, E);
+            if (t.q) {
+                const int64_t a = fix_pair(x, E);
+                lost |= fix_lost(x, a);
+                t.q[r] = a;
+            }
         }
+        if (t.mark && lost) atomicMax(t.bound, kFixLost);
     }
     stamp(started);
 }
@@ -521,6 +533,7 @@ struct Work {
     DevBuf<double> c;                // m+2
     DevBuf<double> junk;             // m+2, coefficient sink for host-side orthonormalisation
     DevBuf<unsigned long long> absmax;   // of w, where the scaling also converts it (else empty)
+    FixTarget target;                    // where it writes the copy
     DevBuf<double> scal;             // [0] ||w||^2 before pass 1, [1] ||H v_j||^2, [2] before pass 2
     DevBuf<int> flags;               // [0] second pass wanted, [1] breakdown step + 1
     DevBuf<unsigned int> counters;   // last-block counters: [0] local dot, [1] multi-dot, [2] update
@@ -532,7 +545,7 @@ struct Work {
               unsigned long long* ended = nullptr)
     {
         launch(k_mdot, nbm, kThreads, (size_t)R * 8, st, Vb, n, R, J, x, local, alpha, beta_prev, part.p,
-                                                      counters.p + 1, c.p, coefcol, before, run, stop, ended, absmax.p);
+                                                      counters.p + 1, c.p, coefcol, before, run, stop, ended, absmax.p, target);
     }
     void update(const double* Vb, int J, double* x, int mode, int force2, const double* before, int* need2,
                 double* b, const double* ref2, int j, const int* run, int* stop, cudaStream_t st)
@@ -740,6 +753,7 @@ void lanczos_once(const ed_op& op, const ed_lanczos_params& p, const double* v0_
     int* stop = w.flags.p + 1;
     const FixTarget target = op.kind == ed_op::CRS ? spmv_target(*op.crs, st) : FixTarget();
     if (target.q) w.absmax.alloc(1);
+    w.target = target;
     auto enqueue_cycle = [&](int k) {
         const int64_t coefs = (int64_t)(m - k) * (m + 1);
         launch(k_cycle_begin, (unsigned)std::min<int64_t>(64, (coefs + 255) / 256), 256, 0, st, w.coef.p + (size_t)k * (m + 1), coefs,

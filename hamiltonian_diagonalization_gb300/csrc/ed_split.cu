@@ -434,7 +434,7 @@ __global__ void k_split_crs_diag(const int64_t* __restrict__ rowptr, const int32
 // in the native order and in the transposed one.
 __global__ void __launch_bounds__(256) k_split_conv(const double* __restrict__ v, int64_t n, int* __restrict__ part,
                                                     int nparts, const int* __restrict__ perm, int64_t* __restrict__ q,
-                                                    int64_t* __restrict__ qt)
+                                                    int64_t* __restrict__ qt, bool mark)
 {
     __shared__ int sE;
     if (threadIdx.x < 32) {
@@ -443,16 +443,20 @@ __global__ void __launch_bounds__(256) k_split_conv(const double* __restrict__ v
         m = __reduce_max_sync(0xffffffffu, m);
         if (threadIdx.x == 0) {
             sE = m;
-            if (blockIdx.x == 0) part[nparts] = m;
+            if (blockIdx.x == 0) atomicMax(part + nparts, m);
         }
     }
     __syncthreads();
     const int E = sE;
+    bool lost = false;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t a = fix_pair(v[i], E);
+        const double x = v[i];
+        const int64_t a = fix_pair(x, E);
+        lost |= fix_lost(x, a);
         q[i] = a;
         qt[perm[i]] = a;
     }
+    if (mark && lost) atomicMax(part + nparts, kFixLost);
 }
 
 using Sum = FixSum;
@@ -1142,11 +1146,17 @@ static std::unique_ptr<SplitPlan> plan_of(const SplitSource& s, const double* di
     // pairs, is well above the single weights)
     if ((double)max_row * (std::ldexp(wmax, 1050 - ea) + 1.0) >= std::ldexp(1.0, 34)) return nullptr;
     p->ea = ea;
+    // no weight may be lost either (nor, below, an entry of the diagonal)
+    for (const HopTables* h : {&s.hop0, &s.hop1})
+        for (double w : h->w)
+            if (w != 0.0 && std::ldexp(std::fabs(w), 1080 - ea) < 0.5) return nullptr;
     const size_t free_b = device_memory_free();
     if (!bn.fits() || !bt.fits() || (size_t)n * 56 + bn.bytes() + bt.bytes() > free_b / 2) return nullptr;
     p->diag.alloc((size_t)n);
-    ED_CUDA(cudaMemcpyAsync(part, &ea, sizeof(int), cudaMemcpyHostToDevice, st));
-    launch(k_fix_conv, sms() * 4, 256, 0, st, diag, n, part, 1, p->diag.p);
+    int bound[2] = {ea, 0};
+    ED_CUDA(cudaMemcpyAsync(part, bound, sizeof(bound), cudaMemcpyHostToDevice, st));
+    launch(k_fix_conv, sms() * 4, 256, 0, st, diag, n, part, 1, p->diag.p, true);
+    ED_CUDA(cudaMemcpyAsync(bound, part, sizeof(bound), cudaMemcpyDeviceToHost, st));
     bn.fill(ea);
     bt.fill(ea);
     p->perm.alloc((size_t)n);
@@ -1155,7 +1165,7 @@ static std::unique_ptr<SplitPlan> plan_of(const SplitSource& s, const double* di
     count_launch();
     ED_CUDA(cudaGetLastError());
     ED_CUDA(cudaStreamSynchronize(st));   // the temporaries and the host vectors go
-    return p;
+    return bound[1] == kFixLost ? nullptr : std::move(p);
 }
 
 std::unique_ptr<SplitPlan> split_build(const SplitSource& s, const double* diag, int64_t n, int max_row, cudaStream_t st)
@@ -1210,7 +1220,7 @@ bool split_ready(SplitPlan& p, cudaStream_t st)
     });
 }
 
-const int* split_product(SplitPlan& p, const double* x, double* y, cudaStream_t st)
+const int* split_product(SplitPlan& p, const double* x, double* y, bool mark, cudaStream_t st)
 {
     SplitPlan::Scratch* sc;
     {
@@ -1219,7 +1229,7 @@ const int* split_product(SplitPlan& p, const double* x, double* y, cudaStream_t 
     }
     const int P = exp_parts();
     launch(k_fix_exp, P, 256, 0, st, x, p.n, sc->part.p);
-    launch(k_split_conv, sms() * 4, 256, 0, st, x, p.n, sc->part.p, P, p.perm.p, sc->x.p, sc->xt.p);
+    launch(k_split_conv, sms() * 4, 256, 0, st, x, p.n, sc->part.p, P, p.perm.p, sc->x.p, sc->xt.p, mark);
     launch_pass<false>(p.trans, args_of(p, p.trans, sc->xt.p, *sc, y, P), st);
     launch_pass<true>(p.native, args_of(p, p.native, sc->x.p, *sc, y, P), st);
     ED_CUDA(cudaGetLastError());

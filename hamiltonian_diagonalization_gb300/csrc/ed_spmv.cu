@@ -230,7 +230,7 @@ __global__ void __launch_bounds__(256, MINB) k_spmv_fix(const int64_t* __restric
         const bool valid = r < n;
         const int64_t s = valid ? rowptr[r] : 0;
         const int len = valid ? (int)(rowptr[r + 1] - s) : 0;
-        if (x && !finite) {   // FP64 sums keep what is not finite to the rows that meet it
+        if (x && !finite) {   // FP64 sums: what is not finite stays with the rows that meet it, and nothing is lost
             double acc = 0.0;
             for (int j = sub; j < len; j += G) acc = fma(val[s + j], __ldg(x + col[s + j]), acc);
 #pragma unroll
@@ -991,7 +991,7 @@ void fix_build(const ed_crs& a, cudaStream_t st)
     const int P = fix_parts();
     DevBuf<int> part((size_t)P + 1);
     launch(k_fix_exp, P, 256, 0, st, a.val.p, a.nnz, part.p);
-    launch(k_fix_conv, 1, 256, 0, st, a.val.p, 0, part.p, P, nullptr);   // the bound into part[P]
+    launch(k_fix_conv, 1, 256, 0, st, a.val.p, 0, part.p, P, nullptr, false);   // the bound into part[P]
     count_launch();
     ED_CUDA(cudaGetLastError());
     int ea = 1;
@@ -1040,6 +1040,12 @@ ed_fixq::Scratch* fix_scratch(const ed_crs& a, cudaStream_t st)
     return f.scratch.emplace(key, std::move(sc)).first->second.get();
 }
 
+bool short_rows(const ed_crs& a) { return (double)a.nnz < kSellMaxAvg * (double)a.n; }
+
+// Short rows of a small sector, whose FP64 kernel stands behind the fixed-point
+// one: for a value or an entry of x that would be lost, as for what is not finite.
+bool small_short(const ed_crs& a) { return !a.upper && short_rows(a) && a.n >= kFixMinRows && a.n < kSellMinRows; }
+
 // The values' limb pairs in the CRS order (sell false) or the sliced-ELL
 // order (sell true, after sell_build), made once outside a capture; false
 // when the copy is not there (declined when it would take more than half of
@@ -1061,10 +1067,12 @@ bool fix_copy(const ed_crs& a, bool sell, cudaStream_t st)
     dst.alloc((size_t)(cnt + kCrsPad));
     ED_CUDA(cudaMemsetAsync(dst.p + cnt, 0, (size_t)kCrsPad * 8, st));
     DevBuf<int> part(2);
-    ED_CUDA(cudaMemcpyAsync(part.p, &f.ea, sizeof(int), cudaMemcpyHostToDevice, st));
-    launch(k_fix_conv, sms() * 8, 256, 0, st, sell ? a.sell->val.p : a.val.p, cnt, part.p, 1, dst.p);
-    ED_CUDA(cudaGetLastError());
+    int bound[2] = {f.ea, 0};
+    ED_CUDA(cudaMemcpyAsync(part.p, bound, sizeof(bound), cudaMemcpyHostToDevice, st));
+    launch(k_fix_conv, sms() * 8, 256, 0, st, sell ? a.sell->val.p : a.val.p, cnt, part.p, 1, dst.p, true);
+    ED_CUDA(cudaMemcpyAsync(bound, part.p, sizeof(bound), cudaMemcpyDeviceToHost, st));
     ED_CUDA(cudaStreamSynchronize(st));
+    f.lost = bound[1] == kFixLost;
     state = 1;
     return true;
 }
@@ -1074,13 +1082,11 @@ bool fix_copy(const ed_crs& a, bool sell, cudaStream_t st)
 // stream's scratch).  A solver's cycles replay on its own stream.
 bool stateless(cudaStream_t st, bool solver) { return !solver && stream_capturing(st); }
 
-bool short_rows(const ed_crs& a) { return (double)a.nnz < kSellMaxAvg * (double)a.n; }
-
 bool sell_shape(const ed_crs& a) { return !a.upper && a.n >= kSellMinRows && short_rows(a); }
 
 bool fix_shape(const ed_crs& a)
 {
-    return !a.upper && a.n > 0 && (!short_rows(a) || (a.n >= kFixMinRows && a.n < kSellMinRows));
+    return !a.upper && a.n > 0 && (!short_rows(a) || small_short(a));
 }
 
 // The fixed-point state, the copy of the values in the wanted order and
@@ -1096,11 +1102,11 @@ bool fix_ready(const ed_crs& a, cudaStream_t st, bool sell = false)
 
 // x's fixed-point copy into the stream's scratch (or it is there already);
 // returns the scratch.
-ed_fixq::Scratch& fix_convert_x(const ed_crs& a, const double* x, cudaStream_t st, bool converted = false)
+ed_fixq::Scratch& fix_convert_x(const ed_crs& a, const double* x, cudaStream_t st, bool converted = false, bool mark = false)
 {
     ed_fixq::Scratch& sc = *fix_scratch(a, st);
     const int P = fix_parts();
-    if (!converted) fix_convert(x, a.n, sc.part.p, P, sms() * 4, sc.xq.p, st);
+    if (!converted) fix_convert(x, a.n, sc.part.p, P, sms() * 4, sc.xq.p, st, mark);
     return sc;
 }
 
@@ -1172,11 +1178,12 @@ void blk_launch(const ed_crs& a, const double* x, double* y, cudaStream_t st, bo
            reinterpret_cast<const int2*>(sc.xq.p), sc.part.p + fix_parts(), f.ea, y, a.n, f.blocks);
 }
 
-// rows: the product in FP64 where x is not finite (else every entry is NaN).
+// rows: the product in FP64 where an entry of x is not finite or lost (else
+// what is not finite makes every entry NaN, and what is lost counts as zero).
 void fix_launch(const ed_crs& a, const double* x, double* y, cudaStream_t st, bool rows = false, bool converted = false)
 {
     const ed_fixq& f = *a.fixq;
-    ed_fixq::Scratch& sc = fix_convert_x(a, x, st, converted);
+    ed_fixq::Scratch& sc = fix_convert_x(a, x, st, converted, rows);
     const int P = fix_parts();
     // matrices below kBlkMinRows, and those without the memory for the blocked
     // copy.  8 lanes a row, 8 loads ahead, at most 64 registers: four CTAs per
@@ -1336,11 +1343,11 @@ enum class FixRoute { kNone, kSell, kBlocked, kRows };
 static FixRoute fix_route(const ed_crs& a, cudaStream_t st, bool solver)
 {
     // short rows of a small sector: their FP64 kernel needs no scratch
-    if (fix_shape(a) && short_rows(a) && stateless(st, solver)) return FixRoute::kNone;
+    if (small_short(a) && stateless(st, solver)) return FixRoute::kNone;
     if (sell_shape(a) && a.sell_state == 0) spmv_prepare(a, st);   // waits for a solver's explicit call while capturing
     if (sell_shape(a) && a.sell_state == 1) return fix_ready(a, st, true) ? FixRoute::kSell : FixRoute::kNone;
     if (blk_shape(a) && blk_ready(a, st)) return FixRoute::kBlocked;
-    if (fix_shape(a) && fix_ready(a, st)) return FixRoute::kRows;
+    if (fix_shape(a) && fix_ready(a, st) && !(small_short(a) && a.fixq->lost)) return FixRoute::kRows;
     return FixRoute::kNone;
 }
 
@@ -1351,6 +1358,7 @@ FixTarget spmv_target(const ed_crs& a, cudaStream_t st)
     ed_fixq::Scratch& sc = *fix_scratch(a, st);
     t.q = sc.xq.p;
     t.bound = sc.part.p + fix_parts();
+    t.mark = small_short(a);
     return t;
 }
 
@@ -1359,7 +1367,7 @@ void spmv_converted(const ed_crs& a, const double* x, double* y, cudaStream_t st
     switch (fix_route(a, st, true)) {
     case FixRoute::kSell: fix_launch_sell(a, x, y, st, true); return;
     case FixRoute::kBlocked: blk_launch(a, x, y, st, true); return;
-    case FixRoute::kRows: fix_launch(a, x, y, st, short_rows(a), true); return;
+    case FixRoute::kRows: fix_launch(a, x, y, st, small_short(a), true); return;
     case FixRoute::kNone: throw Error(ED_ERR_INTERNAL, "a converted product without a fixed-point kernel");
     }
 }
@@ -1373,7 +1381,7 @@ void spmv(const ed_crs& a, const double* x, double* y, cudaStream_t st, bool sol
     }
     if (!(a.upper && stateless(st, solver)) && split_prepare(a, st)) {
         std::lock_guard<std::mutex> order(a.split->order);
-        const int* xexp = split_product(*a.split, x, y, st);
+        const int* xexp = split_product(*a.split, x, y, a.upper, st);
         if (a.upper) {
             launch(k_zero_unless_finite, sms() * 4, 256, 0, st, y, a.n, xexp);
             upper_launch(a, x, y, xexp, st);
@@ -1383,7 +1391,7 @@ void spmv(const ed_crs& a, const double* x, double* y, cudaStream_t st, bool sol
     switch (fix_route(a, st, solver)) {
     case FixRoute::kSell: fix_launch_sell(a, x, y, st); return;
     case FixRoute::kBlocked: blk_launch(a, x, y, st, false); return;
-    case FixRoute::kRows: fix_launch(a, x, y, st, short_rows(a)); return;
+    case FixRoute::kRows: fix_launch(a, x, y, st, small_short(a)); return;
     case FixRoute::kNone: break;
     }
     if (sell_shape(a) && a.sell_state == 1) {
@@ -1454,7 +1462,7 @@ void hv_matfree(const ed_basis& b, const ed_terms& t, SplitPlan* plan, const dou
     std::unique_lock<std::mutex> order;
     if (plan && split_ready(*plan, st)) {
         order = std::unique_lock<std::mutex>(plan->order);
-        xexp = split_product(*plan, x, y, st);
+        xexp = split_product(*plan, x, y, true, st);
     }
     if (plan) diag = plan->values.p;
     const int K = t.norb;
