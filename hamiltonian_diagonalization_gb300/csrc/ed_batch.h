@@ -44,6 +44,7 @@ struct ed_batch {
     int tb = 32, unroll = 4, nt = 256, l1 = 1;
     int tuned = 0;                // 1 after batch_autotune: subsets get their own tuned tiles
     int max_row = 0;              // most off-diagonal entries of a row
+    bool fp64 = false;            // block products in FP64
     // the fixed-point operands of ed_batch_spmm (state 0 not yet tried, 1 made,
     // -1 declined), and the scratch of each (device, stream)
     mutable std::mutex fix_mu;

@@ -1067,7 +1067,7 @@ void fixed_block_product(const ed_batch& bt, const BlockOperands& o, const Block
 // of the batch and where they were declined.
 bool whole_fixed(const ed_batch& bt, const BlockOperands& o, cudaStream_t st)
 {
-    if (o.w != bt.w.p) return false;
+    if (bt.fp64 || o.w != bt.w.p) return false;
     std::lock_guard<std::mutex> lk(bt.fix_mu);
     if (bt.fixed_state == 0) bt.fixed_state = fix_operands(bt, o, bt.fixed, 8 * (size_t)bt.n * bt.B, st) ? 1 : -1;
     return bt.fixed_state == 1;
@@ -1352,7 +1352,7 @@ void batch_solve(const ed_batch& bt, const int* sel, int nsel, const ed_lanczos_
     const size_t later = 16 * (size_t)bt.nhop * B0 + 5 * 8 * (size_t)vs0;
     BlockFixed fixed;
     BlockScratch fixed_x;
-    if (fix_room(bt, B0, fixed_x, later)) fix_operands(bt, ops, fixed, later, st);
+    if (!bt.fp64 && fix_room(bt, B0, fixed_x, later)) fix_operands(bt, ops, fixed, later, st);
     if (!fixed.ready) fixed_x = BlockScratch();
     auto write_ritz = [&](const std::vector<int>& cols) {   // cols: active columns whose pairs are final
         if (!X || cols.empty()) return;
@@ -1650,6 +1650,14 @@ ed_status ed_batch_create(const ed_basis* b, int nham, const uint16_t* ktable, c
 ed_status ed_batch_free(ed_batch* bt)
 {
     return guard([&] { delete bt; });
+}
+
+ed_status ed_batch_set_fp64(ed_batch* bt, int on)
+{
+    return guard([&] {
+        ED_REQUIRE(bt, ED_ERR_ARG, "NULL batch");
+        bt->fp64 = on != 0;
+    });
 }
 
 ed_status ed_batch_dims(const ed_batch* bt, int64_t* n, int64_t* nnz, int* nham)

@@ -302,6 +302,16 @@ ed_status ed_terms_set(int norb, const uint16_t* ktable, const double* vtable, e
     });
 }
 
+ed_status ed_terms_set_fp64(ed_terms* t, int on)
+{
+    return guarded([&] {
+        ED_NONNULL(t);
+        std::lock_guard<std::mutex> lk(t->plans_mu);
+        t->fp64 = on != 0;
+        t->plans.clear();
+    });
+}
+
 ed_status ed_terms_free(ed_terms* t)
 {
     return guarded([&] { delete t; });
@@ -441,6 +451,14 @@ ed_status ed_crs_set_product_kernel(ed_crs* a, int kernel)
         ED_REQUIRE(kernel >= 0 && kernel <= 8, ED_ERR_ARG, "kernel: 0 (chosen by shape) or 1-8 (ed_spmv_kernel)");
         ED_REQUIRE(kernel == 0 || !a->upper, ED_ERR_ARG, "kernels 1-8 take full storage");
         a->product_kernel = kernel;
+    });
+}
+
+ed_status ed_crs_set_fp64(ed_crs* a, int on)
+{
+    return guarded([&] {
+        ED_NONNULL(a);
+        a->fp64 = on != 0;
     });
 }
 

@@ -228,6 +228,7 @@ struct ed_terms {
     edgb::DevBuf<double> diag_b_dev;  // hop.diag_b
     // plans of the matrix-free product by sector (N, twice Lz), the latest
     // few; null where the row kernel runs instead
+    bool fp64 = false;                // no plans: the row kernel's FP64 sums
     mutable std::mutex plans_mu;
     mutable std::vector<std::pair<std::pair<int, int>, std::shared_ptr<edgb::SplitPlan>>> plans;
 };
@@ -304,6 +305,7 @@ struct ed_crs {
     mutable std::shared_ptr<edgb::SplitPlan> split;
     mutable int split_state = 0;
     int product_kernel = 0;   // 0: chosen by shape; else an ed_spmv_kernel id for every product
+    bool fp64 = false;        // of the kernels by shape only the FP64 ones
 };
 
 // Complex momentum-conserving terms (the optical-flux-lattice QuarticTermTables

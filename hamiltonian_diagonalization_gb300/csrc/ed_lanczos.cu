@@ -488,7 +488,7 @@ void op_apply(const ed_op& op, const double* x, double* y, cudaStream_t st)
         spmv(*op.crs, x, y, st, true);
         break;
     case ed_op::MATFREE:
-        if (!op.plan) op.plan = matfree_plan(*op.basis, *op.terms, op.diag.p, st);
+        if (!op.plan || op.terms->fp64) op.plan = matfree_plan(*op.basis, *op.terms, op.diag.p, st);
         hv_matfree(*op.basis, *op.terms, op.plan.get(), op.diag.p, x, y, st);
         break;
     case ed_op::HOST: {

@@ -1242,7 +1242,7 @@ constexpr int64_t kSplitMinRows = 3 << 19, kSplitMinRowsShort = 1 << 20;
 static bool split_prepare(const ed_crs& a, cudaStream_t st)
 {
     // the upper triangle has no better stored kernel either
-    if (a.n < (a.upper || short_rows(a) ? kSplitMinRowsShort : kSplitMinRows)) return false;
+    if (a.fp64 || a.n < (a.upper || short_rows(a) ? kSplitMinRowsShort : kSplitMinRows)) return false;
     if (a.split_state == 0 && !stream_capturing(st)) {
         a.split = split_build_crs(a, st);
         a.split_state = a.split ? 1 : -1;
@@ -1260,11 +1260,11 @@ void spmv_prepare(const ed_crs& a, cudaStream_t st)
     if (a.n == 0 || stream_capturing(st)) return;
     const int k = a.product_kernel;
     if (k == 0 && split_prepare(a, st)) return;
-    if (k == 0 && blk_shape(a) && blk_ready(a, st)) return;
-    if (k == 6 || k == 7 || (k == 0 && fix_shape(a))) fix_ready(a, st);
+    if (k == 0 && !a.fp64 && blk_shape(a) && blk_ready(a, st)) return;
+    if (k == 6 || k == 7 || (k == 0 && !a.fp64 && fix_shape(a))) fix_ready(a, st);
     if ((k == 4 || k == 5 || k == 8) && a.sell_state == 0) sell_build(a, st);
     if (k == 0 && sell_shape(a) && a.sell_state == 0) sell_build(a, st);
-    if ((k == 8 || (k == 0 && sell_shape(a))) && a.sell_state == 1) fix_ready(a, st, true);
+    if ((k == 8 || (k == 0 && !a.fp64 && sell_shape(a))) && a.sell_state == 1) fix_ready(a, st, true);
 }
 
 void spmv_kernel(const ed_crs& a, int kernel, const double* x, double* y, cudaStream_t st)
@@ -1345,6 +1345,7 @@ static FixRoute fix_route(const ed_crs& a, cudaStream_t st, bool solver)
     // short rows of a small sector: their FP64 kernel needs no scratch
     if (small_short(a) && stateless(st, solver)) return FixRoute::kNone;
     if (sell_shape(a) && a.sell_state == 0) spmv_prepare(a, st);   // waits for a solver's explicit call while capturing
+    if (a.fp64) return FixRoute::kNone;
     if (sell_shape(a) && a.sell_state == 1) return fix_ready(a, st, true) ? FixRoute::kSell : FixRoute::kNone;
     if (blk_shape(a) && blk_ready(a, st)) return FixRoute::kBlocked;
     if (fix_shape(a) && fix_ready(a, st) && !(small_short(a) && a.fixq->lost)) return FixRoute::kRows;
@@ -1431,6 +1432,7 @@ std::shared_ptr<SplitPlan> matfree_plan(const ed_basis& b, const ed_terms& t, co
     if (b.levels != 1 || b.dimX != 0 || b.dim == 0 || t.norb != b.norb) return nullptr;
     const std::pair<int, int> key(b.N, b.two_lz);
     std::lock_guard<std::mutex> lk(t.plans_mu);
+    if (t.fp64) return nullptr;
     for (auto& e : t.plans)
         if (e.first == key) return e.second;
     if (stream_capturing(st)) return nullptr;

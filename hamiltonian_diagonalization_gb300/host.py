@@ -96,6 +96,10 @@ class QuarticTermTables:
         self.m_vTable = np.ascontiguousarray(vtable, dtype=np.float64)
         self._h = None
 
+    def set_fp64(self, on: bool = True):
+        """Matrix-free products with these tables in FP64, or (False) the default (ed_terms_set_fp64)."""
+        check(lib().ed_terms_set_fp64(self.handle(), int(on)))
+
     # term_tables.cpp:109-124
     def GetMaxKCount(self) -> int:
         return 1
@@ -296,6 +300,11 @@ class CrsSparseMatrix:
         """Kernel of every later product, eigensolvers included
         (ed_crs_set_product_kernel; 0 restores the choice by shape)."""
         check(lib().ed_crs_set_product_kernel(self._h, int(kernel)))
+
+    def set_fp64(self, on: bool = True):
+        """FP64 kernels alone for every later product, eigensolvers included,
+        or (False) the default (ed_crs_set_fp64)."""
+        check(lib().ed_crs_set_fp64(self._h, int(on)))
 
     def multiply(self, x, y, kernel: int = 0, stream=None):
         """y = A x on device vectors with a chosen product kernel (ed_spmv_kernel:
@@ -1297,6 +1306,10 @@ class HamiltonianBatch:
         n, nnz, nh = ctypes.c_int64(), ctypes.c_int64(), ctypes.c_int()
         check(lib().ed_batch_dims(h, ctypes.byref(n), ctypes.byref(nnz), ctypes.byref(nh)))
         self.n, self.nnz = int(n.value), int(nnz.value)
+
+    def set_fp64(self, on: bool = True):
+        """Block products and solves in FP64, or (False) the default (ed_batch_set_fp64)."""
+        check(lib().ed_batch_set_fp64(self._h, int(on)))
 
     def spmm(self, X, Y, stream=None):
         """Y[:, b] = H_b X[:, b] on device [n][nham] arrays (torch CUDA tensors)."""

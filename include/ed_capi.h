@@ -214,6 +214,24 @@ ed_status ed_spmv_kernel(const ed_crs* a, int kernel, const double* x_dev, doubl
  * later product of a, including those inside the eigensolvers. */
 ed_status ed_crs_set_product_kernel(ed_crs* a, int kernel);
 
+/* The default products' arithmetic.  Fixed point (kernels 6-8, the split
+ * product, the integer block product): values and x rounded to 58 bits under
+ * their largest entries, the sums exact, one rounding to FP64.  Row r of y is
+ * off by at most
+ *   2^-58 (max|x| sum_j |H_rj| + max|H| sum_j |x_j|) + 2^-53 |y_r|,
+ * j over the row's columns: about a tenth of an FP64 sum's error for the
+ * vector as a whole, more than it in rows that are far smaller than the
+ * vector.  A vector with an entry that would round to zero, or that is not
+ * finite, takes the FP64 kernel in the matrix-free product, the block product,
+ * the upper triangle and the short rows of sectors below 32,768 states.
+ * With on != 0 the handle's later products, those inside the eigensolvers
+ * included, use the FP64 kernels alone (a chosen product kernel stands); 0
+ * restores the default.  ed_crs_set_fp64: stored matrices of either storage;
+ * ed_terms_set_fp64: the matrix-free products of these tables (their plans
+ * are given back); ed_batch_set_fp64: block products and batched solves. */
+ed_status ed_crs_set_fp64(ed_crs* a, int on);
+ed_status ed_terms_set_fp64(ed_terms* t, int on);
+
 /* A test of the staged kernel's (ed_spmv_kernel 7) bounded waits on the
  * legacy stream: the kernel runs with its first stage never filled and every
  * wait limited to wait_cycles SM clock cycles, so that the waits run out; it
@@ -421,6 +439,8 @@ typedef struct {
 ed_status ed_batch_create(const ed_basis* b, int nham, const uint16_t* ktable, const double* vtables, int autotune,
                           ed_batch** out);
 ed_status ed_batch_free(ed_batch* bt);
+/* As ed_crs_set_fp64. */
+ed_status ed_batch_set_fp64(ed_batch* bt, int on);
 ed_status ed_batch_dims(const ed_batch* bt, int64_t* n, int64_t* nnz_offdiag, int* nham);
 /* Y[:, b] = H_b X[:, b] for every Hamiltonian b (device [n][nham] arrays). */
 ed_status ed_batch_spmm(const ed_batch* bt, const double* X_dev, double* Y_dev, ed_stream stream);

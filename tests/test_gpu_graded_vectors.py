@@ -110,3 +110,76 @@ def test_a_solve_from_a_graded_vector(cuda):
     want = H.m_eigenvalues
     assert H.LanczosDiagonalize(3, tol=1e-10, v0=graded(n, 6, 1e-22))
     assert np.max(np.abs(H.m_eigenvalues - want)) <= 1e-10 * np.abs(want).max()
+
+
+def assert_default_bound(torch, A, lengths, x, y):
+    """The bound that ed_capi.h states for the fixed-point products, beside the comparison's own FP64 sums."""
+    a, ones = torch.sparse_csr_tensor(A.crow_indices(), A.col_indices(), A.values().abs(), A.shape), torch.ones_like(x)
+    pattern = torch.sparse_csr_tensor(A.crow_indices(), A.col_indices(), torch.ones_like(A.values()), A.shape)
+    scale = a @ x.abs()
+    bound = 2.0 ** -58 * (x.abs().max() * (a @ ones) + A.values().abs().max() * (pattern @ x.abs())) + 2.0 ** -53 * y.abs()
+    assert bool(((y - A @ x).abs() <= bound + (lengths + 2) * 2.0 ** -52 * scale).all())
+
+
+def levelled(n, seed, level):
+    """Entries of the level to within a factor of two, one of 1: none is lost, all keep few bits."""
+    r = np.random.default_rng(seed)
+    x = level * r.uniform(0.5, 1.0, n) * r.choice([-1.0, 1.0], n)
+    x[n // 2] = 1.0
+    return x
+
+
+# entries that fixed point keeps to a few bits: the handles' FP64 choice keeps all of them
+@pytest.mark.parametrize("make,case,kw", [(one_level, (8, 22, 0), dict(matrix_free=True)), (one_level, (9, 26, 1), {}),
+                                          (two_level, (6, 13, 0), {}), (two_level, (7, 15, 0), {}),
+                                          (two_level, (8, 18, 2), {}), (two_level, (8, 18, 2), dict(store_upper=True))])
+def test_products_in_fp64_by_choice(cuda, make, case, kw):
+    torch = cuda
+    full = make(*case)
+    A, lengths = csr(torch, full)
+    x = torch.from_numpy(levelled(len(lengths), 7, 1e-15)).cuda()
+    H = make(*case, **kw) if kw else full
+    handle = H.m_terms if H.m_crsSparseMatrix is None else H.m_crsSparseMatrix
+    default = product(torch, H, x)
+    assert_default_bound(torch, A, lengths, x, default)
+    handle.set_fp64()
+    assert_rows(torch, A, lengths, x, product(torch, H, x))
+    handle.set_fp64(False)
+    assert torch.equal(product(torch, H, x).view(torch.int64), default.view(torch.int64))
+
+
+def test_solves_in_fp64_by_choice(cuda):
+    for kw in ({}, dict(matrix_free=True)):
+        H = one_level(8, 22, 0, **kw)
+        v0 = np.random.default_rng(8).uniform(-1, 1, H.GetDimension())
+        assert H.LanczosDiagonalize(3, tol=1e-10, v0=v0)
+        want = H.m_eigenvalues
+        (H.m_terms if kw else H.m_crsSparseMatrix).set_fp64()
+        assert H.LanczosDiagonalize(3, tol=1e-10, v0=v0)
+        assert np.max(np.abs(H.m_eigenvalues - want)) <= 1e-11 * np.abs(want).max()
+
+
+def test_block_product_in_fp64_by_choice(cuda):
+    torch = cuda
+    N, norb = 8, 20
+    basis = ed.FermionFockBasis()
+    basis.GenerateFockSpace(N, norb, 0)
+    v = ed.odd_coulomb_list(norb)
+    bt = ed.HamiltonianBatch(basis, [v, v, v], autotune=False)
+    H = ed.SpinlessFermionHamiltonian()
+    H.Initialize(N, norb, twoLz=0)
+    H.Add_CdCdCC_Terms(ed.QuarticTermTables(norb, v))
+    A, lengths = csr(torch, H)
+    X = torch.from_numpy(np.stack([levelled(bt.n, i, 1e-15) for i in range(3)], 1)).cuda()
+    Y = torch.empty_like(X)
+    bt.spmm(X, Y)
+    torch.cuda.synchronize()
+    assert_default_bound(torch, A, lengths, X[:, 1].contiguous(), Y[:, 1].contiguous())
+    bt.set_fp64()
+    bt.spmm(X, Y)
+    torch.cuda.synchronize()
+    assert_rows(torch, A, lengths, X[:, 1].contiguous(), Y[:, 1].contiguous())
+    want, _, _ = bt.solve(2, V0=X)
+    bt.set_fp64(False)
+    got, _, _ = bt.solve(2, V0=X)
+    assert np.max(np.abs(got - want)) <= 1e-11 * np.abs(want).max()
