@@ -992,7 +992,6 @@ void fix_build(const ed_crs& a, cudaStream_t st)
     DevBuf<int> part((size_t)P + 1);
     launch(k_fix_exp, P, 256, 0, st, a.val.p, a.nnz, part.p);
     launch(k_fix_conv, 1, 256, 0, st, a.val.p, 0, part.p, P, nullptr, false);   // the bound into part[P]
-    count_launch();
     ED_CUDA(cudaGetLastError());
     int ea = 1;
     ED_CUDA(cudaMemcpyAsync(&ea, part.p + P, sizeof(int), cudaMemcpyDeviceToHost, st));
