@@ -20,7 +20,6 @@
 
 #include "ed_hop.cuh"
 #include "ed_launch.cuh"
-#include "ed_launch.cuh"
 #include "ed_split.h"
 
 namespace edgb {

@@ -609,15 +609,15 @@ struct CWork {
               unsigned long long* ended = nullptr)
     {
         launch(k_cmdot, nbm, kCThreads, (size_t)R * 16, st, V, n, R, J, w, local, alpha, beta_prev, part.p,
-                                                        counters.p + 1, reinterpret_cast<double2*>(c.p), coefcol,
-                                                        before, run, stop, ended, absmax.p);
+               counters.p + 1, reinterpret_cast<double2*>(c.p), coefcol,
+               before, run, stop, ended, absmax.p);
     }
     void update(const double2* V, int J, double2* w, int mode, int force2, const double* before, int* need2,
                 double* b, const double* ref2, int j, const int* run, int* stop, cudaStream_t st)
     {
         launch(k_cupd, nb, kCThreads, (size_t)J * 16, st, V, n, J, reinterpret_cast<const double2*>(c.p), w, npart.p,
-                                                      counters.p + 2, mode, force2, before, need2, b, ref2, j, run,
-                                                      stop, absmax.p);
+               counters.p + 2, mode, force2, before, need2, b, ref2, j, run,
+               stop, absmax.p);
     }
 };
 
@@ -1088,7 +1088,7 @@ void clanczos_solve(const ed_ccrs& a, const ed_lanczos_params& p, const double* 
     auto enqueue_cycle = [&](double2* V, int k) {
         const int64_t coefs = (int64_t)(m - k) * (m + 1);
         launch(k_cycle_begin, (unsigned)std::min<int64_t>(64, (coefs + 255) / 256), 256, 0, st, cw.coef.p + (size_t)k * (m + 1), coefs,
-                   cw.flags.p, 2, clock.p + 2 * k);
+               cw.flags.p, 2, clock.p + 2 * k);
         for (int j = k; j < m; ++j) {
             double2* vj = V + (int64_t)j * n;
             double2* w = V + (int64_t)(j + 1) * n;
@@ -1099,7 +1099,7 @@ void clanczos_solve(const ed_ccrs& a, const ed_lanczos_params& p, const double* 
             unsigned long long* ended = clock.p + 2 * j + 1;
             if (!first) {
                 launch(k_clocal, cw.nb, kCThreads, 0, st, vj, w, n, cw.part.p, cw.counters.p, coefcol, j,
-                                                      cw.beta.p + (j - 1), cw.scal.p + 1, stop, ended);
+                       cw.beta.p + (j - 1), cw.scal.p + 1, stop, ended);
             }
             const int J = j + 1;
             const double* ref2 = first ? cw.scal.p : cw.scal.p + 1;

@@ -109,13 +109,13 @@ __device__ __forceinline__ double round_i128(__int128 S, int sc)
     return round_u128((unsigned long long)(M >> 64), (unsigned long long)M, neg, sc);
 }
 
-// The largest |v| of a block's threads (as the bits without the sign, which
-// order as the values) into *at; m is a shared word, zero at the start.
+// |v| as its bits without the sign, which order as the values.
 __device__ __forceinline__ unsigned long long abs_bits(double v)
 {
     return (unsigned long long)__double_as_longlong(v) & 0x7FFFFFFFFFFFFFFFull;
 }
 
+// The largest v of a block's threads into the shared word m, zero at the start.
 __device__ __forceinline__ void block_absmax(unsigned long long v, unsigned long long* m)
 {
     const unsigned hi = (unsigned)(v >> 32), top = __reduce_max_sync(0xffffffffu, hi);

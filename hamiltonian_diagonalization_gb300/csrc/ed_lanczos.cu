@@ -545,13 +545,13 @@ struct Work {
               unsigned long long* ended = nullptr)
     {
         launch(k_mdot, nbm, kThreads, (size_t)R * 8, st, Vb, n, R, J, x, local, alpha, beta_prev, part.p,
-                                                      counters.p + 1, c.p, coefcol, before, run, stop, ended, absmax.p, target);
+               counters.p + 1, c.p, coefcol, before, run, stop, ended, absmax.p, target);
     }
     void update(const double* Vb, int J, double* x, int mode, int force2, const double* before, int* need2,
                 double* b, const double* ref2, int j, const int* run, int* stop, cudaStream_t st)
     {
         launch(k_update, nb, kThreads, (size_t)J * 8, st, Vb, n, J, c.p, x, npart.p, counters.p + 2, mode, force2,
-                                                       before, need2, b, ref2, j, run, stop, absmax.p);
+               before, need2, b, ref2, j, run, stop, absmax.p);
     }
 };
 
@@ -757,7 +757,7 @@ void lanczos_once(const ed_op& op, const ed_lanczos_params& p, const double* v0_
     auto enqueue_cycle = [&](int k) {
         const int64_t coefs = (int64_t)(m - k) * (m + 1);
         launch(k_cycle_begin, (unsigned)std::min<int64_t>(64, (coefs + 255) / 256), 256, 0, st, w.coef.p + (size_t)k * (m + 1), coefs,
-                   w.flags.p, 2, clock.p + 2 * k);
+               w.flags.p, 2, clock.p + 2 * k);
         for (int j = k; j < m; ++j) {
             double* vj = w.V.p + (int64_t)j * n;
             double* wv = w.V.p + (int64_t)(j + 1) * n;
@@ -768,7 +768,7 @@ void lanczos_once(const ed_op& op, const ed_lanczos_params& p, const double* v0_
             unsigned long long* ended = clock.p + 2 * j + 1;
             if (!first) {
                 launch(k_local_dot, w.nb, kThreads, 0, st, vj, wv, n, w.part.p, w.counters.p, coefcol, j,
-                                                       w.beta.p + (j - 1), w.scal.p + 1, stop, ended);
+                       w.beta.p + (j - 1), w.scal.p + 1, stop, ended);
             }
             const int J = j + 1;
             // pass 1 (with the three-term step on non-first steps), then the

@@ -837,8 +837,8 @@ struct Arena {
 };
 
 // One pass: primary words P (by class), secondary words S of the same classes.
-// count() enqueues the list lengths' counts and scans, fill(), after the
-// stream has been waited for, allocates and enqueues the lists.
+// count() sizes the lists (each total's copy to the host waits for its scan),
+// fill() allocates them and enqueues their kernels.
 struct SideBuild {
     SplitSide& out;
     const PartWords &P, &S;
@@ -1098,7 +1098,6 @@ static std::unique_ptr<SplitPlan> plan_of(const SplitSource& s, const double* di
 
     auto p = std::make_unique<SplitPlan>();
     p->n = n;
-    p->lists = s.levels == 1;
     Arena tmp;
     GenArgs gn{}, gt{};
     std::vector<int> gamman, gammat;

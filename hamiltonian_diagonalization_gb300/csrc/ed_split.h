@@ -41,7 +41,6 @@ struct SplitSide {
 struct SplitPlan {
     int64_t n = 0;
     int ea = 1;                     // exponent bound of the weights and the diagonal
-    bool lists = false;             // gammas other than "nothing" (one level)
     SplitSide native, trans;
     DevBuf<int> perm;               // native row -> transposed row
     DevBuf<int64_t> diag;           // the diagonal's limb pairs

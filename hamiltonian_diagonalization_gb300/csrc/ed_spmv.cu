@@ -1192,8 +1192,8 @@ void fix_launch(const ed_crs& a, const double* x, double* y, cudaStream_t st, bo
     // into L2 by cp.async.bulk.prefetch 0.99; the rows staged in shared
     // memory by bulk copies, k_spmv_fix_staged, 1.71)
     launch(k_spmv_fix<8, 8, 4>, sms() * 8, 256, 0, st, a.rowptr.p, a.col.p, reinterpret_cast<const int2*>(f.val.p),
-                                                   reinterpret_cast<const int2*>(sc.xq.p), sc.part.p + P, f.ea, y,
-                                                   a.n, a.val.p, rows ? x : nullptr);
+           reinterpret_cast<const int2*>(sc.xq.p), sc.part.p + P, f.ea, y,
+           a.n, a.val.p, rows ? x : nullptr);
     ED_CUDA(cudaGetLastError());
 }
 
@@ -1203,9 +1203,9 @@ void fix_launch_sell(const ed_crs& a, const double* x, double* y, cudaStream_t s
     const ed_sell& sl = *a.sell;
     ed_fixq::Scratch& sc = fix_convert_x(a, x, st, converted);
     launch(k_spmv_sell_fix<8, 4>, sms() * 8, 256, 0, st, sl.off.p, sl.len.p, sl.row.p, sl.col.p,
-                                                     reinterpret_cast<const int2*>(f.sval.p),
-                                                     reinterpret_cast<const int2*>(sc.xq.p), sc.part.p + fix_parts(),
-                                                     f.ea, y, sl.nchunks);
+           reinterpret_cast<const int2*>(f.sval.p),
+           reinterpret_cast<const int2*>(sc.xq.p), sc.part.p + fix_parts(),
+           f.ea, y, sl.nchunks);
     ED_CUDA(cudaGetLastError());
 }
 
