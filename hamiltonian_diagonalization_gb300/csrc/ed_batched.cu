@@ -343,8 +343,10 @@ __global__ void __launch_bounds__(256) k_bfix_exp(const double* __restrict__ v, 
 }
 
 // q = v in fixed point by column; with both, rows 2h and 2h + 1 of q are row h
-// of v and its negative.  exps[B] becomes kFixLost where an entry is lost.
-__global__ void __launch_bounds__(256) k_bfix_conv(const double* __restrict__ v, int64_t total, int B, int* exps, int both,
+// of v and its negative.  *bound (after the exps) is raised to kFixLost where
+// an entry is lost.
+__global__ void __launch_bounds__(256) k_bfix_conv(const double* __restrict__ v, int64_t total, int B,
+                                                   const int* __restrict__ exps, int* __restrict__ bound, int both,
                                                    int64_t* __restrict__ q)
 {
     const int E = exps[threadIdx.x % B];
@@ -361,7 +363,7 @@ __global__ void __launch_bounds__(256) k_bfix_conv(const double* __restrict__ v,
             q[i] = a;
         }
     }
-    if (lost) atomicMax(exps + B, kFixLost);
+    if (lost) atomicMax(bound, kFixLost);
 }
 
 // The eight elements at k (a multiple of 8) of a row whose elements are
@@ -419,7 +421,7 @@ __global__ void __launch_bounds__(256, 4) k_bspmm_fix(const int64_t* __restrict_
     const int b = blockIdx.y * TB + (lane % TB);
     const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
     const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
-    if (b >= B) return;
+    if (b >= B || ex[B] >= 2047) return;   // the FP64 kernel answers
     const int e_x = ex[b];
     for (int64_t r = warp * RPW + lane / TB; r < n; r += nwarps * RPW) {
         const int64_t s = rowptr[r], e = rowptr[r + 1];
@@ -435,7 +437,7 @@ __global__ void __launch_bounds__(256, 4) k_bspmm_fix(const int64_t* __restrict_
         long long q2 = 0, q1 = 0, q0 = 0;
         fix_mac(d, x, q2, q1, q0);
         const __int128 S = ((__int128)p2 << 60) + (__int128)(unsigned long long)p0 + fix_combine(q2, q1, q0);
-        Y[r * B + b] = e_x < 2047 ? round_i128(S, ea[b] + e_x - 2160) : __longlong_as_double(0x7FF8000000000000ll);
+        Y[r * B + b] = round_i128(S, ea[b] + e_x - 2160);
     }
 }
 
@@ -693,10 +695,11 @@ __global__ void __launch_bounds__(kBT, 4) k_bupdate(const double* __restrict__ V
 }
 
 // w_p /= beta_p, with q also the block product's fixed-point copy at the bounds
-// ex, ex[B] raised to kFixLost where an entry is lost (its own two passes over the block and the clearing before them took 12
+// ex, *bound raised to kFixLost where an entry is lost (its own two passes over the block and the clearing before them took 12
 // us of a step's 330 for 16 problems at N=9, 2S=24).
 __global__ void k_bscale(double* __restrict__ w, int64_t n, int B, const double* __restrict__ beta,
-                         unsigned long long* __restrict__ started, int* ex, int64_t* __restrict__ q)
+                         unsigned long long* __restrict__ started, const int* __restrict__ ex, int* __restrict__ bound,
+                         int64_t* __restrict__ q)
 {
     const int64_t total = n * (int64_t)B;
     bool lost = false;
@@ -710,7 +713,7 @@ __global__ void k_bscale(double* __restrict__ w, int64_t n, int B, const double*
             q[t] = a;
         }
     }
-    if (lost) atomicMax(ex + B, kFixLost);
+    if (lost) atomicMax(bound, kFixLost);
     stamp(started);
 }
 
@@ -1034,8 +1037,8 @@ bool fix_operands(const ed_batch& bt, const BlockOperands& o, BlockFixed& f, siz
         const double high = std::ldexp(1.0, 28 + eh[b] - ea[b]) + 1.0;
         if (ea[b] >= 2047 || (double)bt.max_row * high >= std::ldexp(1.0, 34)) return false;
     }
-    k_bfix_conv<<<column_grid(nw, B), T, 0, st>>>(o.w, nw, B, f.ea.p, 1, f.w.p); count_launch();
-    k_bfix_conv<<<column_grid(nd, B), T, 0, st>>>(o.diag, nd, B, f.ea.p, 0, f.diag.p); count_launch();
+    k_bfix_conv<<<column_grid(nw, B), T, 0, st>>>(o.w, nw, B, f.ea.p, f.ea.p + B, 1, f.w.p); count_launch();
+    k_bfix_conv<<<column_grid(nd, B), T, 0, st>>>(o.diag, nd, B, f.ea.p, f.ea.p + B, 0, f.diag.p); count_launch();
     ED_CUDA(cudaGetLastError());
     ED_CUDA(cudaMemcpyAsync(ea.data(), f.ea.p + B, 4, cudaMemcpyDeviceToHost, st));
     ED_CUDA(cudaStreamSynchronize(st));   // ew goes
@@ -1053,7 +1056,7 @@ void fixed_block_product(const ed_batch& bt, const BlockOperands& o, const Block
     if (!converted) {
         ED_CUDA(cudaMemsetAsync(v.ex.p, 0, (size_t)(B + 1) * 4, st));
         k_bfix_exp<<<column_grid(total, B), T, B * 4, st>>>(X, total, B, v.ex.p); count_launch();
-        k_bfix_conv<<<column_grid(total, B), T, 0, st>>>(X, total, B, v.ex.p, 0, v.x.p); count_launch();
+        k_bfix_conv<<<column_grid(total, B), T, 0, st>>>(X, total, B, v.ex.p, v.ex.p + B, 0, v.x.p); count_launch();
     }
     if (B > 16) launch_bspmm_fix<32>(bt, f, v, B, Y, st);
     else if (B > 8) launch_bspmm_fix<16>(bt, f, v, B, Y, st);
@@ -1316,7 +1319,7 @@ void batch_solve(const ed_batch& bt, const int* sel, int nsel, const ed_lanczos_
             nn[b] = std::sqrt(nn[b]);
         }
         ED_CUDA(cudaMemcpyAsync(s2.p + 2 * B, nn.data(), (size_t)B * 8, cudaMemcpyHostToDevice, st));
-        k_bscale<<<grid_for(vs), 256, 0, st>>>(V.p, n, B, s2.p + 2 * B, nullptr, nullptr, nullptr); count_launch();
+        k_bscale<<<grid_for(vs), 256, 0, st>>>(V.p, n, B, s2.p + 2 * B, nullptr, nullptr, nullptr, nullptr); count_launch();
     }
     ed_batch_info inf;
     std::memset(&inf, 0, sizeof(inf));
@@ -1420,7 +1423,7 @@ void batch_solve(const ed_batch& bt, const int* sel, int nsel, const ed_lanczos_
                 // the norm after the pass, kept from pass 1 for problems that skip pass 2
                 bsum(npart.p, 1, s2.p + 3 * B, mask, pass == 0 ? need : fin);
             }
-            launch(k_bscale, grid_for(vs), 256, 0, st, w, n, B, betas.p + (size_t)j * B, clock.p + 2 * (j + 1), fixed_x.ex.p,
+            launch(k_bscale, grid_for(vs), 256, 0, st, w, n, B, betas.p + (size_t)j * B, clock.p + 2 * (j + 1), fixed_x.ex.p, fixed_x.ex.p + B,
                    amax && j + 1 < m ? fixed_x.x.p : nullptr);
         }
     };

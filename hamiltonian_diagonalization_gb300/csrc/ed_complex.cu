@@ -866,7 +866,7 @@ void cfix_build(const ed_ccrs& a, cudaStream_t st)
     DevBuf<int> part((size_t)P + 1);
     fq->val.alloc(2 * (size_t)(a.nnz + kCrsPad));
     ED_CUDA(cudaMemsetAsync(fq->val.p + 2 * a.nnz, 0, (size_t)kCrsPad * 16, st));
-    launch(k_fix_exp, P, 256, 0, st, a.val.p, 2 * a.nnz, part.p);
+    launch(k_fix_exp, P, 256, 0, st, a.val.p, 2 * a.nnz, part.p, 1);
     launch(k_fix_conv, csms() * 8, 256, 0, st, a.val.p, 2 * a.nnz, part.p, P, fq->val.p, false);
     ED_CUDA(cudaGetLastError());
     int ea = 1;

@@ -128,14 +128,18 @@ __device__ __forceinline__ void block_absmax(unsigned long long v, unsigned long
 // FP64 kernel stands behind it takes that one for a vector with such an entry:
 // its conversion raises the vector's bound to 2047, as an entry that is not
 // finite does.
-__device__ __forceinline__ bool fix_lost(double v, int64_t q) { return q == 0 && abs_bits(v) != 0; }
+__device__ __forceinline__ bool fix_lost(double v, int64_t q)
+{
+    return q == 0 && (((unsigned)__double2hiint(v) << 1) | (unsigned)__double2loint(v)) != 0u;
+}
 constexpr int kFixLost = 2047;
 
 // Per-block maxima of fix_exp over v[0, n) into part[blockIdx.x]; the word
-// after them, which the conversion raises to the bound, is zeroed.
-__global__ void __launch_bounds__(256) k_fix_exp(const double* __restrict__ v, int64_t n, int* __restrict__ part)
+// after them, which the conversion raises to the bound, is cleared (clear
+// words, with k_fix_one's flags).
+__global__ void __launch_bounds__(256) k_fix_exp(const double* __restrict__ v, int64_t n, int* __restrict__ part, int clear)
 {
-    if (blockIdx.x == 0 && threadIdx.x == 0) part[gridDim.x] = 0;
+    if (blockIdx.x == 0 && threadIdx.x < clear) part[gridDim.x + threadIdx.x] = 0;
     __shared__ int sm[8];
     int m = 1;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
@@ -178,50 +182,77 @@ __global__ void __launch_bounds__(256) k_fix_conv(const double* __restrict__ v, 
 }
 
 // Both at once for a short vector (one launch less in a solver's step): every
-// block finds the bound of all of v, then converts its own 256 entries.
+// block finds the bound of all of v, then converts its own kFixOneThreads
+// entries.  The latency of the loads bounds it, so each thread has seventeen
+// in flight.  With mark, each warp tells of a lost entry in a byte of its own
+// of the kFixFlags bytes after the bound (no byte is both cleared and raised in
+// a launch, and no block waits for its warps).
 constexpr int64_t kFixOnePass = 16384;   // n = 8,512: 7.7 us a product's step less; at 45,207 the two passes are shorter
+constexpr int kFixOneThreads = 512, kFixOneLoads = 17;
+constexpr int kFixFlags = 512, kFixWords = 1 + 4 + kFixFlags / 4;   // the bound, alignment, the flags
+static_assert(kFixFlags * 32 >= kFixOnePass, "a flag a warp");
 
-__global__ void __launch_bounds__(256) k_fix_one(const double* __restrict__ v, int64_t n, int* __restrict__ bound,
-                                                 int64_t* __restrict__ q, bool mark)
+__device__ __forceinline__ unsigned char* fix_flags(int* bound)
 {
-    __shared__ int sm[8], sl[8];
-    int m = 1, low = kFixLost;
-#pragma unroll 8
-    for (int64_t i = threadIdx.x; i < n; i += 256) {
-        const double x = v[i];
-        const int e = fix_exp(x);
-        m = max(m, e);
-        if (abs_bits(x) != 0) low = min(low, e);
+    return reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(bound + 1) + 15) & ~(uintptr_t)15);
+}
+
+__global__ void __launch_bounds__(kFixOneThreads) k_fix_one(const double* __restrict__ v, int64_t n, int* __restrict__ bound,
+                                                            int64_t* __restrict__ q, bool mark)
+{
+    constexpr int T = kFixOneThreads, U = kFixOneLoads;
+    __shared__ unsigned sm[T / 32];
+    unsigned m = 0u;                 // the largest high word
+    for (int i = threadIdx.x; i < n; i += U * T) {
+        unsigned hi[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) hi[u] = i + u * T < n ? (unsigned)(abs_bits(__ldg(v + i + u * T)) >> 32) : 0u;
+#pragma unroll
+        for (int u = 0; u < U; ++u) m = max(m, hi[u]);
     }
     m = __reduce_max_sync(0xffffffffu, m);
-    low = __reduce_min_sync(0xffffffffu, low);
-    if ((threadIdx.x & 31) == 0) {
-        sm[threadIdx.x >> 5] = m;
-        sl[threadIdx.x >> 5] = low;
-    }
+    if ((threadIdx.x & 31) == 0) sm[threadIdx.x >> 5] = m;
     __syncthreads();
-    int E = sm[0];
 #pragma unroll
-    for (int w = 1; w < 8; ++w) {
-        E = max(E, sm[w]);
-        low = min(low, sl[w]);
+    for (int w = 0; w < T / 32; ++w) m = max(m, sm[w]);
+    const int E = max((int)(m >> 20), 1);
+    if (blockIdx.x == 0 && threadIdx.x == 0) *bound = E;
+    const int i = blockIdx.x * T + threadIdx.x;
+    bool lost = false;
+    if (i < n) {
+        const double x = v[i];
+        const int64_t a = fix_pair(x, E);
+        lost = fix_lost(x, a);
+        q[i] = a;
     }
-    if (blockIdx.x == 0 && threadIdx.x == 0) *bound = mark && low < E - 58 ? kFixLost : E;
-    const int64_t i = blockIdx.x * (int64_t)256 + threadIdx.x;
-    if (i < n) q[i] = fix_pair(v[i], E);
+    if (!mark) return;
+    unsigned char* flags = fix_flags(bound);
+    const int any = __any_sync(0xffffffffu, lost);
+    if ((threadIdx.x & 31) == 0) flags[i / 32] = (unsigned char)any;
+    if (blockIdx.x == 0 && threadIdx.x >= gridDim.x * (T / 32) && threadIdx.x < kFixFlags) flags[threadIdx.x] = 0;
 }
 
 // q = v in fixed point, its exponent bound in part[parts]; blocks: the grid of
-// the conversion of a long vector; mark: kFixLost where an entry is lost.
+// the conversion of a long vector; mark: kFixLost where an entry is lost, or
+// a flag after it (fix_finite).
 inline void fix_convert(const double* v, int64_t n, int* part, int parts, int blocks, int64_t* q, cudaStream_t st,
                         bool mark = false)
 {
     if (n <= kFixOnePass) {
-        launch(k_fix_one, (unsigned)((n + 255) / 256), 256, 0, st, v, n, part + parts, q, mark);
+        launch(k_fix_one, (unsigned)((n + kFixOneThreads - 1) / kFixOneThreads), kFixOneThreads, 0, st, v, n, part + parts, q, mark);
         return;
     }
-    launch(k_fix_exp, parts, 256, 0, st, v, n, part);
+    launch(k_fix_exp, parts, 256, 0, st, v, n, part, mark ? kFixWords : 1);
     launch(k_fix_conv, blocks, 256, 0, st, v, n, part, parts, q, mark);
+}
+
+// Whether the product may go by the marked copy whose bound is at xexp: the
+// vector is finite and no entry lost.  The whole warp calls it.
+__device__ __forceinline__ bool fix_finite(const int* __restrict__ xexp)
+{
+    static_assert(kFixFlags == 32 * 16, "sixteen flags a lane");
+    const uint4 f = __ldg(reinterpret_cast<const uint4*>(fix_flags(const_cast<int*>(xexp))) + (threadIdx.x & 31));
+    return __ldg(xexp) < 2047 && !__any_sync(0xffffffffu, (f.x | f.y | f.z | f.w) != 0u);
 }
 
 // p2, p1, p0 += the three limb products of a b (weights 2^60, 2^30, 1).

@@ -185,10 +185,8 @@ __global__ void __launch_bounds__(kThreads) k_mdot(const double* __restrict__ V,
 {
     if (blockIdx.x == 0) stamp(ended);
     if ((run && !*run) || (stop && *stop)) return;
-    if (absmax && blockIdx.x == 0 && threadIdx.x == 0) {
-        *absmax = 0ull;               // k_update's
-        if (t.mark) *t.bound = 0;     // k_scale's
-    }
+    if (absmax && blockIdx.x == 0 && threadIdx.x == 0) *absmax = 0ull;                       // k_update's
+    if (t.mark && blockIdx.x == 0 && threadIdx.x < kFixWords) t.bound[threadIdx.x] = 0;   // k_scale's
     extern __shared__ double sw[];
     const int64_t r0 = (int64_t)blockIdx.x * R;
     const int len = (int)min((int64_t)R, n - r0);

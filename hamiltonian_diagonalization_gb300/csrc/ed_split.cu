@@ -648,6 +648,7 @@ __global__ void __launch_bounds__(kThreads, 18) k_split_product(SplitArgs g)
     __shared__ int queue, count;
     Sum* acc = reinterpret_cast<Sum*>(smem);                     // [warp][rows]
     int4* lists = reinterpret_cast<int4*>(acc + kWarps * g.rows);   // alpha and entry ranges of each list
+    if (g.gated && __ldg(g.xexp) >= 2047) return;
     const int2 task = g.task[blockIdx.x];
     const int p = task.x, seg = task.y;
     const int c = g.pcls[p];
@@ -749,7 +750,7 @@ __global__ void __launch_bounds__(kThreads, 20) k_split_keep(SplitArgs g, int nt
 {
     __shared__ int4 stages[kWarps][32];
     const int t = (int)((blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5);
-    if (t >= ntasks) return;
+    if (t >= ntasks || (g.gated && __ldg(g.xexp) >= 2047)) return;
     const int2 task = g.task[t];
     const int lane = threadIdx.x & 31;
     const int width = task.y & 63, cnt = (task.y >> 6) & 63, seg = task.y >> 12;
@@ -999,7 +1000,8 @@ struct SideBuild {
     }
 };
 
-SplitArgs args_of(const SplitPlan& p, const SplitSide& s, const int64_t* x, const SplitPlan::Scratch& sc, double* y, int parts)
+SplitArgs args_of(const SplitPlan& p, const SplitSide& s, const int64_t* x, const SplitPlan::Scratch& sc, double* y, int parts,
+                  bool gated)
 {
     SplitArgs g;
     g.task = s.task.p;
@@ -1027,6 +1029,7 @@ SplitArgs args_of(const SplitPlan& p, const SplitSide& s, const int64_t* x, cons
     g.diag = reinterpret_cast<const int2*>(p.diag.p);
     g.y = y;
     g.ea = p.ea;
+    g.gated = gated;
     return g;
 }
 
@@ -1134,7 +1137,7 @@ static std::unique_ptr<SplitPlan> plan_of(const SplitSource& s, const double* di
     // the diagonal's exponent joins the weights'
     const int parts = exp_parts();
     int* part = tmp.take<int>((size_t)parts + 1);
-    launch(k_fix_exp, parts, 256, 0, st, diag, n, part);
+    launch(k_fix_exp, parts, 256, 0, st, diag, n, part, 1);
     std::vector<int> h(parts);
     ED_CUDA(cudaMemcpyAsync(h.data(), part, (size_t)parts * 4, cudaMemcpyDeviceToHost, st));
     ED_CUDA(cudaStreamSynchronize(st));
@@ -1227,10 +1230,10 @@ const int* split_product(SplitPlan& p, const double* x, double* y, bool mark, cu
         sc = p.scratch.at(stream_key(st)).get();
     }
     const int P = exp_parts();
-    launch(k_fix_exp, P, 256, 0, st, x, p.n, sc->part.p);
+    launch(k_fix_exp, P, 256, 0, st, x, p.n, sc->part.p, 1);
     launch(k_split_conv, sms() * 4, 256, 0, st, x, p.n, sc->part.p, P, p.perm.p, sc->x.p, sc->xt.p, mark);
-    launch_pass<false>(p.trans, args_of(p, p.trans, sc->xt.p, *sc, y, P), st);
-    launch_pass<true>(p.native, args_of(p, p.native, sc->x.p, *sc, y, P), st);
+    launch_pass<false>(p.trans, args_of(p, p.trans, sc->xt.p, *sc, y, P, mark), st);
+    launch_pass<true>(p.native, args_of(p, p.native, sc->x.p, *sc, y, P, mark), st);
     ED_CUDA(cudaGetLastError());
     return sc->part.p + P;
 }

@@ -84,6 +84,7 @@ struct SplitArgs {
     const int2* diag;
     double* y;
     int ea;
+    bool gated;     // another kernel answers for a bound of 2047
 };
 
 // The plan of a Hamiltonian with the given diagonal (device, n entries), or
@@ -96,8 +97,8 @@ std::unique_ptr<SplitPlan> split_build_crs(const ed_crs& a, cudaStream_t st);
 // the free device memory; false when it is missing.
 bool split_ready(SplitPlan& p, cudaStream_t st);
 // y = H x on a stream that split_ready accepted, p.order held; returns the device word with
-// x's exponent bound (2047: a non-finite entry or, with mark, one that is lost
-// in fixed point; y is all NaN).
+// x's exponent bound (2047: a non-finite entry, y is all NaN; with mark also
+// where an entry is lost in fixed point, and y is left to the caller's kernel).
 const int* split_product(SplitPlan& p, const double* x, double* y, bool mark, cudaStream_t st);
 // Gives back the stream's scratch (before a solver's stream is destroyed).
 void split_release(SplitPlan& p, cudaStream_t st);

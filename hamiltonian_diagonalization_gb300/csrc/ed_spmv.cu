@@ -223,7 +223,7 @@ __global__ void __launch_bounds__(256, MINB) k_spmv_fix(const int64_t* __restric
     const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
     const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
     const int ex = __ldg(xexp);
-    const bool finite = ex < 2047;
+    const bool finite = x ? fix_finite(xexp) : ex < 2047;
     const int sc = ea + ex - 2160;
     for (int64_t rb = warp * RPW; rb < n; rb += nwarps * RPW) {   // warp-uniform loop
         const int64_t r = rb + grp;
@@ -990,7 +990,7 @@ void fix_build(const ed_crs& a, cudaStream_t st)
     auto fq = std::make_unique<ed_fixq>();
     const int P = fix_parts();
     DevBuf<int> part((size_t)P + 1);
-    launch(k_fix_exp, P, 256, 0, st, a.val.p, a.nnz, part.p);
+    launch(k_fix_exp, P, 256, 0, st, a.val.p, a.nnz, part.p, 1);
     launch(k_fix_conv, 1, 256, 0, st, a.val.p, 0, part.p, P, nullptr, false);   // the bound into part[P]
     ED_CUDA(cudaGetLastError());
     int ea = 1;
@@ -1035,7 +1035,7 @@ ed_fixq::Scratch* fix_scratch(const ed_crs& a, cudaStream_t st)
     if (stream_capturing(st)) return nullptr;
     auto sc = std::make_unique<ed_fixq::Scratch>();
     sc->xq.alloc((size_t)a.n);
-    sc->part.alloc((size_t)fix_parts() + 1);
+    sc->part.alloc((size_t)fix_parts() + kFixWords);
     return f.scratch.emplace(key, std::move(sc)).first->second.get();
 }
 
