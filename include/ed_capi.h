@@ -181,11 +181,13 @@ ed_status ed_ham_diagonal(const ed_basis* b, const ed_terms* t, double* diag_dev
  *     on the sliced-ELL copy from 32,768, the split product from 1,048,576.
  * The split product sums over the moves of two parts of the Fock word instead
  * of over the elements (the same bits); it needs a matrix built by this
- * library, in either storage.  Where the memory for a copy or plan is
- * missing, the next simpler kernel runs.  Other matrices take FP64 kernels.
+ * library, in either storage.  Where the memory for a copy, plan or scratch
+ * is missing, the next simpler kernel runs.  Other matrices take FP64 kernels.
  * The first product makes the copies and, per stream, an n-element scratch
  * for x; products of one matrix on one stream must not overlap (they share
- * that stream's scratch). */
+ * that stream's scratch), nor graphs captured from them on one stream. Inside a
+ * caller's capture the upper triangle and kernel 6 on short rows give way to
+ * the FP64 kernels, which need no scratch. */
 ed_status ed_spmv(const ed_crs* a, const double* x_dev, double* y_dev, ed_stream stream);
 
 /* The same product with a chosen kernel of the full storage, for measuring
@@ -423,7 +425,8 @@ typedef struct {
     double seconds;
     double spmm_seconds;      /* device time inside the block products (its clock)   */
     int breakdowns;
-    int tile_hamiltonians;    /* autotuned Hamiltonians per row tile of the block product */
+    int tile_hamiltonians;    /* autotuned Hamiltonians per row tile of the FP64 block product,
+                                 which runs where the integer one does not (ed_batch_spmm) */
     int tile_unroll;          /* autotuned loads in flight per lane                  */
     int tile_l1;              /* 1: hop values read through L1, 0: staged in shared memory */
     int tile_threads;         /* threads per CTA of the block product                */
@@ -442,7 +445,12 @@ ed_status ed_batch_free(ed_batch* bt);
 /* As ed_crs_set_fp64. */
 ed_status ed_batch_set_fp64(ed_batch* bt, int on);
 ed_status ed_batch_dims(const ed_batch* bt, int64_t* n, int64_t* nnz_offdiag, int* nham);
-/* Y[:, b] = H_b X[:, b] for every Hamiltonian b (device [n][nham] arrays). */
+/* Y[:, b] = H_b X[:, b] for every Hamiltonian b (device [n][nham] arrays), in
+ * exact fixed point (ed_crs_set_fp64): the first product makes the batch's
+ * fixed-point operands (8 bytes a row and Hamiltonian) and each stream a
+ * scratch for X as large; products on one stream must not overlap.  The FP64
+ * kernel runs where their memory is missing, inside a caller's capture, by
+ * choice, and for an X with an entry that is not finite or would be lost. */
 ed_status ed_batch_spmm(const ed_batch* bt, const double* X_dev, double* Y_dev, ed_stream stream);
 /* Lowest p->nev eigenpairs of every Hamiltonian, all in lockstep (the
  * thick-restart Lanczos of ed_lanczos, batched).  V0_dev: [n][nham] start
